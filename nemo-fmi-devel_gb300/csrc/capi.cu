@@ -104,10 +104,10 @@ struct nemo_ctx {
   float* spg_ff = nullptr;  // mixed form: compensated sub-step sums, 10 x nmem x n2
   unsigned int* bar_mem = nullptr;  // count, gen
   int* err_flag = nullptr;
-  // EOS-80 tables (eos80.h): raw FP64 [3][4][7][7]; FP32 re-expanded about s0 =
+  // EOS-80 tables (eos80.h): FP64 as they stand; FP32 re-expanded about s0 =
   // sqrt((35 + 20) / 40), and the density at (35 psu, 0 degC, 0 m)
-  double* e80_raw = nullptr;
-  float* e80_tay = nullptr;
+  nemo::E80Tab<double> e80_raw{};
+  nemo::E80Tab<float> e80_tay{};
   double e80_s0 = 0.0, e80_rho0 = 0.0;
   // stp_ctl (block partials, per-member results, the blow-up flag) and dia_hsb
   double* ctl_part = nullptr;
@@ -1358,7 +1358,8 @@ EosArgs<T> eos_args(const nemo_ctx* c, int what) {
   a.gdept = (const T*)c->f[NEMO_F_GDEPT_N]; a.gdepw = (const T*)c->f[NEMO_F_GDEPW_N];
   a.what = what;
   a.eos80 = nm.ln_eos80;
-  a.e80_raw = c->e80_raw; a.e80_tay = c->e80_tay;
+  if constexpr (sizeof(T) == 8) a.e80 = c->e80_raw;
+  else a.e80 = c->e80_tay;
   a.e80_s0 = (float)c->e80_s0; a.e80_rho0 = (float)c->e80_rho0; a.e80_anom = (float)(c->e80_rho0 - nm.rau0);
   return a;
 }
@@ -1762,40 +1763,43 @@ int run_hotpath(nemo_ctx* c, int kt, bool staged, bool model = false) {
 // ================================================================== C ABI
 extern "C" {
 
-// The EOS-80 tables on the device. FP32 evaluates each polynomial re-expanded in
-// s' = zs - s0 about the reference salinity's s0 = sqrt((35 + 20) / 40), with the
-// density's constant term (its value at 35 psu, 0 degC, 0 m) kept apart: in the
-// monomial basis about zs = 0 the terms reach ~900 kg/m3 and cancel to the density,
-// so FP32 would lose the density anomaly (~1e-4 kg/m3 against neighbour differences
-// of 1e-3..1e-1); about s0 the terms are of the size of the anomaly itself. The
-// re-expansion is exact in FP64 (binomial sums) and then rounded to FP32.
-int upload_eos80(nemo_ctx* c) {
+// The EOS-80 tables the kernels take as arguments. FP32 evaluates each polynomial
+// re-expanded in s' = zs - s0 about the reference salinity's s0 = sqrt((35 + 20) / 40),
+// with the density's constant term (its value at 35 psu, 0 degC, 0 m) kept apart: in
+// the monomial basis about zs = 0 the terms reach ~900 kg/m3 and cancel to the
+// density, so FP32 would lose the density anomaly (~1e-4 kg/m3 against neighbour
+// differences of 1e-3..1e-1); about s0 the terms are of the size of the anomaly
+// itself. The re-expansion is exact in FP64 (binomial sums) and then rounded to FP32.
+void form_eos80(nemo_ctx* c) {
   static const double raw[3][4][7][7] = NEMO_EOS80_TABLE;
   const double s0 = std::sqrt((35.0 + NEMO_EOS80_RDELTAS) * NEMO_EOS80_R1_S0);
-  std::vector<float> tay(3 * 4 * 49, 0.0f);
   double binom[7][7] = {};
   for (int n = 0; n < 7; ++n) {
     binom[n][0] = 1.0;
     for (int r = 1; r <= n; ++r) binom[n][r] = binom[n - 1][r - 1] + (r <= n - 1 ? binom[n - 1][r] : 0.0);
   }
-  for (int t = 0; t < 3; ++t)
-    for (int k = 0; k < 4; ++k)
-      for (int j = 0; j < 7; ++j)
-        for (int ip = 0; ip < 7; ++ip) {
+  double* const rt[3] = {c->e80_raw.eos, c->e80_raw.alp, c->e80_raw.bet};
+  unsigned long long* const tt[3] = {c->e80_tay.eos, c->e80_tay.alp, c->e80_tay.bet};
+  for (int t = 0; t < 3; ++t) {
+    int at = 0;
+    for (int k = 0; k < 4; ++k) {
+      const int D = t == 0 ? nemo::E80_DEN[k] : nemo::E80_EXP[k];
+      for (int ip = 0; ip <= D; ++ip)
+        for (int j = 0; j <= D - ip; ++j, ++at) {
           double v = 0.0;
           for (int i = ip; i < 7; ++i) v += raw[t][k][i][j] * binom[i][ip] * std::pow(s0, i - ip);
-          tay[((t * 4 + k) * 7 + ip) * 7 + j] = (float)v;
+          rt[t][at] = raw[t][k][ip][j];
+          const float f = t == 0 && at == 0 ? 0.0f : (float)v;  // the density's constant term apart
+          const float two[2] = {f, f};
+          memcpy(&tt[t][at], two, sizeof(two));
         }
+    }
+  }
   // the density at (s' = 0, zt = 0, zh = 0): the constant term of the surface table
   double rho0 = 0.0;
   for (int i = 0; i < 7; ++i) rho0 += raw[0][0][i][0] * std::pow(s0, i);
   c->e80_s0 = s0;
   c->e80_rho0 = rho0;
-  if (cudaMalloc(&c->e80_raw, sizeof(raw)) != cudaSuccess) return NEMO_ERR_NOMEM;
-  if (cudaMalloc(&c->e80_tay, tay.size() * sizeof(float)) != cudaSuccess) return NEMO_ERR_NOMEM;
-  cudaMemcpy(c->e80_raw, raw, sizeof(raw), cudaMemcpyHostToDevice);
-  cudaMemcpy(c->e80_tay, tay.data(), tay.size() * sizeof(float), cudaMemcpyHostToDevice);
-  return NEMO_OK;
 }
 
 // The sub-step kernel and its grid: one block per 32 x 8 tile, at most all
@@ -1916,7 +1920,7 @@ int nemo_gpu_create(const nemo_dom_desc* dm, const nemo_namelist* nam, int nmemb
   cudaMemset(c->err_flag, 0, sizeof(int));
   select_p2(c);
   if (nam->ln_eos80 && nam->ln_seos) return bad(NEMO_ERR_ARG);  // eos_init: exactly one equation of state
-  if (nam->ln_eos80 && upload_eos80(c)) return bad(NEMO_ERR_NOMEM);
+  if (nam->ln_eos80) form_eos80(c);
   // stp_ctl: one column a thread (at most 2048 blocks of DG_THREADS, then a grid stride)
   c->ctl_nblk = (int)std::min<long>(2048, (c->n2 + DG_THREADS - 1) / DG_THREADS);
   c->hsb_nblk = 2 * c->nsm;
@@ -1963,7 +1967,6 @@ int nemo_gpu_destroy(nemo_ctx* c) {
   cudaFree(c->d_wgt1); cudaFree(c->d_wgt2); cudaFree(c->d_wgtf);
   cudaFree(c->bar_mem); cudaFree(c->err_flag);
   cudaFree(c->ctl_part); cudaFree(c->ctl_out); cudaFree(c->ctl_idx); cudaFree(c->ctl_flag);
-  cudaFree(c->e80_raw); cudaFree(c->e80_tay);
   cudaFree(c->hsb_mem); cudaFree(c->hsb_part); cudaFree(c->hsb_state); cudaFree(c->hsb_out);
   cudaFree(c->gs_part); cudaFree(c->gs_out);
   for (auto e : c->tev)

@@ -12,6 +12,17 @@ template <class T>
 dim3 s_col(const Dom<T>& d) { return dim3((d.jpi + SX - 1) / SX, (d.jpj + SY - 1) / SY, d.nmem); }
 template <class T>
 dim3 s_pt(const Dom<T>& d) { return dim3((d.jpi + SX - 1) / SX, (d.jpj + SY - 1) / SY, d.nmem * d.jpk); }
+// Levels a thread of a level-march kernel walks: the longest of 4, 2, 1 times `step`
+// that still gives every SM its resident warps twice over (64 warps of 32 points),
+// so that a long march amortises its column's metrics on a large grid and a small one
+// still fills the chip.
+template <class T>
+int level_chunk(const Dom<T>& d, int block, int step) {
+  const long planes = (d.n2 + block - 1) / block * d.nmem;
+  for (int f = 4; f > 1; f /= 2)
+    if (planes * ((d.jpk + f * step - 1) / (f * step)) * block >= 152L * 64 * 32) return f * step;
+  return step;
+}
 }  // namespace
 
 template <class T>
@@ -117,7 +128,12 @@ cudaError_t launch_tra_qsr(const Dom<T>& d, const QsrArgs<T>& a, cudaStream_t s)
 
 template <class T>
 cudaError_t launch_eos(const Dom<T>& d, const EosArgs<T>& a, cudaStream_t s) {
-  k_eos<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
+  const int kch = level_chunk(d, EOS_BLOCK, EOS_U);
+  const dim3 g((unsigned)((d.n2 + EOS_BLOCK - 1) / EOS_BLOCK), (d.jpk - 1 + kch - 1) / kch, d.nmem);
+  if (a.what == 3) k_bn2<T><<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
+  else if (a.what == 0) (a.eos80 ? k_eos<T, 0, true> : k_eos<T, 0, false>)<<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
+  else if (a.what == 1) (a.eos80 ? k_eos<T, 1, true> : k_eos<T, 1, false>)<<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
+  else (a.eos80 ? k_eos<T, 2, true> : k_eos<T, 2, false>)<<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
   ktick(a.what == 3 ? NEMO_K_BN2 : NEMO_K_EOS, s);
   return cudaGetLastError();
 }

@@ -628,95 +628,165 @@ __global__ void k_tra_qsr(Dom<T> d, QsrArgs<T> a) {
   a.fraq[(long)m * d.n2 + ij] = qsr != T(0) ? h1 / (a.r1_rau0_rcp * qsr) : T(1);
 }
 
-// ------------------------------------------- the simplified equation of state
-// eos_insitu (eosbn2.F90:276-292), eos_insitu_pot (:440-462), rab_3d (:645-661)
-// with np_seos, and bn2 (:889-933), one point per thread, each expression in the
-// reference's association.
+// --------------------------------------------------------- equations of state
+// eos_insitu, eos_insitu_pot, rab_3d and bn2, EOS-80 or the simplified one (np_seos),
+// each FP64 expression in the reference's association.
 // ---- EOS-80. FP64: one power k of the depth of a table in the reference's
 // association (eosbn2.F90:242-265): acc = C(0,D); for j = D-1 .. 0,
 // acc = (acc*zt + H_j*zs) + C(0,j), H_j = (..(C(n,j)*zs + C(n-1,j))*zs .. + C(1,j)),
-// n = D - j. C points at [i][j] (7 x 7) of that k.
+// n = D - j.
 template <int D>
-__device__ __forceinline__ double e80_zn(const double* __restrict__ C, double zt, double zs) {
-  double acc = __ldg(C + D);
+__device__ __forceinline__ double e80_zn(const double* C, double zt, double zs) {
+  double acc = C[e80_at(D, 0, D)];
 #pragma unroll
   for (int j = D - 1; j >= 0; --j) {
     const int n = D - j;
-    double h = __ldg(C + n * 7 + j);
+    double h = C[e80_at(D, n, j)];
 #pragma unroll
-    for (int i = n - 1; i >= 1; --i) h = h * zs + __ldg(C + i * 7 + j);
-    acc = (acc * zt + h * zs) + __ldg(C + j);
+    for (int i = n - 1; i >= 1; --i) h = h * zs + C[e80_at(D, i, j)];
+    acc = (acc * zt + h * zs) + C[e80_at(D, 0, j)];
   }
   return acc;
 }
-// table t (0 EOS: degrees 6 4 2 1 in zt; 1 ALP, 2 BET: 5 3 1 0), all depth powers
+// all depth powers of a table; zn0: the surface part
 template <int D0, int D1, int D2, int D3>
-__device__ __forceinline__ double e80_poly(const double* __restrict__ tab, double zt, double zs, double zh,
-                                           double& zn0) {
-  const double z3 = e80_zn<D3>(tab + 3 * 49, zt, zs), z2 = e80_zn<D2>(tab + 2 * 49, zt, zs);
-  const double z1 = e80_zn<D1>(tab + 49, zt, zs);
-  zn0 = e80_zn<D0>(tab, zt, zs);
+__device__ __forceinline__ double e80_poly(const double* C, double zt, double zs, double zh, double& zn0) {
+  constexpr int o1 = e80_len(D0), o2 = o1 + e80_len(D1), o3 = o2 + e80_len(D2);
+  const double z3 = e80_zn<D3>(C + o3, zt, zs), z2 = e80_zn<D2>(C + o2, zt, zs);
+  const double z1 = e80_zn<D1>(C + o1, zt, zs);
+  zn0 = e80_zn<D0>(C, zt, zs);
   return ((z3 * zh + z2) * zh + z1) * zh + zn0;
 }
-// FP32: the re-expanded table (in s' = zs - s0), Horner in s', zt, zh; skip00 leaves
-// out the constant term of the surface part (the density's, added apart)
-template <int D>
-__device__ __forceinline__ float e80_q32(const float* __restrict__ C, float zt, float sp, bool skip00) {
-  float acc = 0.f;
+// FP32: Horner in s' = zs - s0, zt and zh with fused multiply-adds, two points to an
+// instruction (fma.rn.f32x2), NP pairs of points a coefficient: the polynomials are
+// issue-bound (70 multiply-adds a point in rab_3d, one coefficient load each).
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(F2 r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+template <int D, int NP>
+__device__ __forceinline__ void e80_zn(const F2* C, const F2 (&zt)[NP], const F2 (&sp)[NP], F2 (&acc)[NP]) {
 #pragma unroll
-  for (int j = D; j >= 0; --j) {
-    float h = 0.f;
+  for (int n = 0; n < NP; ++n) acc[n] = C[e80_at(D, 0, D)];
 #pragma unroll
-    for (int i = D - j; i >= 0; --i) h = h * sp + ((skip00 && i == 0 && j == 0) ? 0.f : __ldg(C + i * 7 + j));
-    acc = acc * zt + h;
+  for (int j = D - 1; j >= 0; --j) {
+    F2 h[NP];
+#pragma unroll
+    for (int n = 0; n < NP; ++n) h[n] = C[e80_at(D, D - j, j)];
+#pragma unroll
+    for (int i = D - j - 1; i >= 0; --i) {
+      const F2 c = C[e80_at(D, i, j)];
+#pragma unroll
+      for (int n = 0; n < NP; ++n) h[n] = f2_fma(h[n], sp[n], c);
+    }
+#pragma unroll
+    for (int n = 0; n < NP; ++n) acc[n] = f2_fma(acc[n], zt[n], h[n]);
   }
-  return acc;
 }
-template <int D0, int D1, int D2, int D3>
-__device__ __forceinline__ float e80_poly32(const float* __restrict__ tab, float zt, float sp, float zh,
-                                            bool skip00, float& zn0) {
-  const float z3 = e80_q32<D3>(tab + 3 * 49, zt, sp, false), z2 = e80_q32<D2>(tab + 2 * 49, zt, sp, false);
-  const float z1 = e80_q32<D1>(tab + 49, zt, sp, false);
-  zn0 = e80_q32<D0>(tab, zt, sp, skip00);
-  return ((z3 * zh + z2) * zh + z1) * zh + zn0;
+template <int D0, int D1, int D2, int D3, int NP>
+__device__ __forceinline__ void e80_poly(const F2* C, const F2 (&zt)[NP], const F2 (&sp)[NP], const F2 (&zh)[NP],
+                                         F2 (&zn)[NP], F2 (&zn0)[NP]) {
+  constexpr int o1 = e80_len(D0), o2 = o1 + e80_len(D1), o3 = o2 + e80_len(D2);
+  F2 z[NP];
+  e80_zn<D3>(C + o3, zt, sp, zn);
+  e80_zn<D2>(C + o2, zt, sp, z);
+#pragma unroll
+  for (int n = 0; n < NP; ++n) zn[n] = f2_fma(zn[n], zh[n], z[n]);
+  e80_zn<D1>(C + o1, zt, sp, z);
+#pragma unroll
+  for (int n = 0; n < NP; ++n) zn[n] = f2_fma(zn[n], zh[n], z[n]);
+  e80_zn<D0>(C, zt, sp, zn0);
+#pragma unroll
+  for (int n = 0; n < NP; ++n) zn[n] = f2_fma(zn[n], zh[n], zn0[n]);
 }
 
-// eos_insitu, eos_insitu_pot and rab_3d with EOS-80 (eosbn2.F90:236-270, :400-436,
-// :588-642) at point q (temperature qt, salinity qs)
-template <class T>
-__device__ __forceinline__ void eos80_point(const EosArgs<T>& a, long q, long qt, long qs, T ztm) {
-  constexpr double r1_Z0 = 1.e-4, r1_T0 = 1.0 / 40.0, r1_S0 = 1.0 / 40.0, rdeltaS = 20.0;
-  const T dep = a.what == 2 ? a.gdept[q] : a.pdep[q];
-  if constexpr (sizeof(T) == 8) {
-    const double zh = dep * r1_Z0, zt = a.pts[qt] * r1_T0;
-    const double zs = sqrt(fabs(a.pts[qs] + rdeltaS) * r1_S0);
-    double zn0;
-    if (a.what == 2) {
-      double zn = e80_poly<5, 3, 1, 0>(a.e80_raw + 196, zt, zs, zh, zn0);
-      a.pab[qt] = zn * a.r1_rau0 * ztm;
-      zn = e80_poly<5, 3, 1, 0>(a.e80_raw + 392, zt, zs, zh, zn0);
-      a.pab[qs] = zn / zs * a.r1_rau0 * ztm;
-    } else {
-      const double zn = e80_poly<6, 4, 2, 1>(a.e80_raw, zt, zs, zh, zn0);
-      if (a.what == 1) a.prhop[q] = zn0 * ztm;
-      a.prd[q] = (zn * a.r1_rau0 - 1.0) * ztm;
+// The unmasked density anomaly and surface (potential) density (eos_insitu,
+// eos_insitu_pot; eosbn2.F90:236-292, :400-462), or the expansion coefficients
+// (rab_3d; :588-661), of U points: x = anomaly or alpha, y = rhop or beta.
+template <bool RAB, bool E80, int U, class T>
+__device__ __forceinline__ void eos_points(const EosArgs<T>& a, const T (&t)[U], const T (&s)[U], const T (&dep)[U],
+                                           T (&x)[U], T (&y)[U]) {
+  constexpr T r1_Z0 = T(1.e-4), r1_T0 = T(1.0 / 40.0), r1_S0 = T(1.0 / 40.0), rdeltaS = T(20.0);
+  if constexpr (!E80) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const T zt = t[u] - T(10), zs = s[u] - T(35), zh = dep[u];
+      if constexpr (RAB) {
+        T zn = a.a0 * (T(1) + a.lambda1 * zt + a.mu1 * zh) + a.nu * zs;
+        x[u] = zn * a.r1_rau0;
+        zn = a.b0 * (T(1) - a.lambda2 * zs - a.mu2 * zh) - a.nu * zt;
+        y[u] = zn * a.r1_rau0;
+      } else {
+        T zn = -a.a0 * (T(1) + T(0.5) * a.lambda1 * zt) * zt + a.b0 * (T(1) - T(0.5) * a.lambda2 * zs) * zs -
+               a.nu * zt * zs;
+        y[u] = a.rau0 + zn;
+        zn = zn - (a.a0 * a.mu1 * zt + a.b0 * a.mu2 * zs) * zh;
+        x[u] = zn * a.r1_rau0;
+      }
+    }
+  } else if constexpr (sizeof(T) == 8) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const T zh = dep[u] * r1_Z0, zt = t[u] * r1_T0, zs = sqrt(fabs(s[u] + rdeltaS) * r1_S0);
+      T zn0;
+      if constexpr (RAB) {
+        x[u] = e80_poly<5, 3, 1, 0>(a.e80.alp, zt, zs, zh, zn0) * a.r1_rau0;
+        y[u] = e80_poly<5, 3, 1, 0>(a.e80.bet, zt, zs, zh, zn0) / zs * a.r1_rau0;
+      } else {
+        x[u] = e80_poly<6, 4, 2, 1>(a.e80.eos, zt, zs, zh, zn0) * a.r1_rau0 - T(1);
+        y[u] = zn0;
+      }
     }
   } else {
-    const float zh = dep * (float)r1_Z0, zt = a.pts[qt] * (float)r1_T0;
-    const float x = fabsf(a.pts[qs] + (float)rdeltaS) * (float)r1_S0;
-    const float zs = sqrtf(x);
-    const float sp = (x - a.e80_s0 * a.e80_s0) / (zs + a.e80_s0);  // zs - s0 without cancellation
-    float zn0;
-    if (a.what == 2) {
-      float zn = e80_poly32<5, 3, 1, 0>(a.e80_tay + 196, zt, sp, zh, false, zn0);
-      a.pab[qt] = zn * a.r1_rau0 * ztm;
-      zn = e80_poly32<5, 3, 1, 0>(a.e80_tay + 392, zt, sp, zh, false, zn0);
-      a.pab[qs] = zn / zs * a.r1_rau0 * ztm;
-    } else {
-      // the anomaly of the density about its value at (35 psu, 0 degC, 0 m) first
-      const float zn = e80_poly32<6, 4, 2, 1>(a.e80_tay, zt, sp, zh, true, zn0);
-      if (a.what == 1) a.prhop[q] = (zn0 + a.e80_rho0) * ztm;
-      a.prd[q] = ((zn + a.e80_anom) * a.r1_rau0) * ztm;
+    constexpr int NP = (U + 1) / 2;
+    float zs[2 * NP];
+    F2 zt[NP], sp[NP], zh[NP], zn[NP], zn0[NP];
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+      float w[2], h[2], v[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int u = 2 * n + e < U ? 2 * n + e : U - 1;
+        h[e] = dep[u] * r1_Z0;
+        w[e] = t[u] * r1_T0;
+        const float s2 = fabsf(s[u] + rdeltaS) * r1_S0;
+        zs[2 * n + e] = sqrtf(s2);
+        v[e] = (s2 - a.e80_s0 * a.e80_s0) / (zs[2 * n + e] + a.e80_s0);  // zs - s0 without cancellation
+      }
+      zt[n] = f2_pack(w[0], w[1]);
+      zh[n] = f2_pack(h[0], h[1]);
+      sp[n] = f2_pack(v[0], v[1]);
+    }
+    float p[2 * NP], q[2 * NP];
+    if constexpr (RAB) {
+      e80_poly<5, 3, 1, 0>(a.e80.alp, zt, sp, zh, zn, zn0);
+#pragma unroll
+      for (int n = 0; n < NP; ++n) f2_unpack(zn[n], p[2 * n], p[2 * n + 1]);
+      e80_poly<5, 3, 1, 0>(a.e80.bet, zt, sp, zh, zn, zn0);
+#pragma unroll
+      for (int n = 0; n < NP; ++n) f2_unpack(zn[n], q[2 * n], q[2 * n + 1]);
+    } else {  // the anomaly about the value at (35 psu, 0 degC, 0 m) first
+      e80_poly<6, 4, 2, 1>(a.e80.eos, zt, sp, zh, zn, zn0);
+#pragma unroll
+      for (int n = 0; n < NP; ++n) {
+        f2_unpack(zn[n], p[2 * n], p[2 * n + 1]);
+        f2_unpack(zn0[n], q[2 * n], q[2 * n + 1]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      x[u] = RAB ? p[u] * a.r1_rau0 : (p[u] + a.e80_anom) * a.r1_rau0;
+      y[u] = RAB ? q[u] / zs[u] * a.r1_rau0 : q[u] + a.e80_rho0;
     }
   }
 }
@@ -724,19 +794,10 @@ __device__ __forceinline__ void eos80_point(const EosArgs<T>& a, long q, long qt
 template <class T>
 __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
   if (a.eos80) {
-    constexpr double r1_Z0 = 1.e-4, r1_T0 = 1.0 / 40.0, r1_S0 = 1.0 / 40.0, rdeltaS = 20.0;
-    if constexpr (sizeof(T) == 8) {
-      const double zh = dep * r1_Z0, zt = t * r1_T0, zs = sqrt(fabs(sal + rdeltaS) * r1_S0);
-      double zn0;
-      return e80_poly<6, 4, 2, 1>(a.e80_raw, zt, zs, zh, zn0) * a.r1_rau0 - 1.0;
-    } else {
-      const float zh = dep * (float)r1_Z0, zt = t * (float)r1_T0;
-      const float x = fabsf(sal + (float)rdeltaS) * (float)r1_S0;
-      const float zs = sqrtf(x);
-      const float sp = (x - a.e80_s0 * a.e80_s0) / (zs + a.e80_s0);
-      float zn0;
-      return (e80_poly32<6, 4, 2, 1>(a.e80_tay, zt, sp, zh, true, zn0) + a.e80_anom) * a.r1_rau0;
-    }
+    const T t1[1] = {t}, s1[1] = {sal}, h1[1] = {dep};
+    T rd[1], rhop[1];
+    eos_points<false, true>(a, t1, s1, h1, rd, rhop);
+    return rd[0];
   }
   const T zt = t - T(10), zs = sal - T(35);
   const T zn = -a.a0 * (T(1) + T(0.5) * a.lambda1 * zt + a.mu1 * dep) * zt +
@@ -744,47 +805,96 @@ __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
   return zn * a.r1_rau0;
 }
 
+// eos_insitu (WHAT 0), eos_insitu_pot (1) and rab_3d (2) on levels 1..jpk-1: a thread
+// owns one (i,j) of the flat 2-D plane (no stencil, so no ragged tiles) and a chunk of
+// levels, EOS_U of them loaded before the first polynomial. The polynomials' operands
+// come from the constant bank; the kernels are bound by memory in FP32 (rab_3d moves
+// 5 fields, eos_insitu 4) and by the FP64 pipe in FP64. As one point a thread, with
+// the coefficients loaded from global memory, the six calls of a step's density (two
+// rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32.
+constexpr int EOS_U = 4, EOS_BLOCK = 256;
+template <class T, int WHAT, bool E80>
+__global__ void __launch_bounds__(EOS_BLOCK) k_eos(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
+  const long p = (long)blockIdx.x * EOS_BLOCK + threadIdx.x;
+  if (p >= d.n2) return;
+  const int m = blockIdx.z, k0 = blockIdx.y * kch + 1, k1 = min(k0 + kch - 1, d.jpk - 1);
+  const long c3 = (long)m * d.n3 + p, c4 = 2 * (long)m * d.n3 + p;
+  const ColInfo ci = d.ci[p];
+  const T* __restrict__ ts = a.pts + c4;
+  const T* __restrict__ dep = (WHAT == 2 ? a.gdept : a.pdep) + c3;
+  for (int k = k0; k <= k1; k += EOS_U) {
+    T t[EOS_U], s[EOS_U], h[EOS_U];
+#pragma unroll
+    for (int u = 0; u < EOS_U; ++u) {
+      const int ku = k + u <= k1 ? k + u : k1;
+      const long o = (long)(ku - 1) * d.n2;
+      t[u] = __ldg(ts + o);
+      s[u] = __ldg(ts + d.n3 + o);
+      h[u] = __ldg(dep + o);
+    }
+    T x[EOS_U], y[EOS_U];
+    if constexpr (WHAT == 0 && !E80) {
+#pragma unroll
+      for (int u = 0; u < EOS_U; ++u) x[u] = eos_rd_2d(a, t[u], s[u], h[u]);
+    } else {
+      eos_points<WHAT == 2, E80>(a, t, s, h, x, y);
+    }
+#pragma unroll
+    for (int u = 0; u < EOS_U; ++u) {
+      if (k + u > k1) break;
+      const long o = (long)(k + u - 1) * d.n2;
+      const T tm = tmsk<T>(ci, k + u);
+      if constexpr (WHAT == 2) {
+        a.pab[c4 + o] = x[u] * tm;
+        a.pab[c4 + d.n3 + o] = y[u] * tm;
+      } else {
+        if constexpr (WHAT == 1) a.prhop[c3 + o] = y[u] * tm;
+        a.prd[c3 + o] = x[u] * tm;
+      }
+    }
+  }
+}
+
+// bn2 (eosbn2.F90:889-933) on levels 2..jpk-1: a thread marches down a chunk of one
+// flat (i,j)'s levels and carries T, S, the expansion coefficients and the depth of
+// the level above, so that each of the 7 fields is read once.
 template <class T>
-__global__ void k_eos(Dom<T> d, EosArgs<T> a) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || c.k > d.jpk - 1) return;
-  const long q = (long)c.m * d.n3 + c.q;          // one 3-D field
-  const long qt = 2 * (long)c.m * d.n3 + c.q;     // temperature of (jpi,jpj,jpk,2)
-  const long qs = qt + d.n3;
-  const ColInfo ci = d.ci[c.ij];
-  if (a.eos80 && a.what != 3) {
-    eos80_point(a, q, qt, qs, tmsk<T>(ci, c.k));
-    return;
-  }
-  if (a.what == 3) {
-    if (c.k < 2) return;
-    const T zrw = (a.gdepw[q] - a.gdept[q]) / (a.gdept[q - d.n2] - a.gdept[q]);
-    const T zaw = a.pab_in[qt] * (T(1) - zrw) + a.pab_in[qt - d.n2] * zrw;
-    const T zbw = a.pab_in[qs] * (T(1) - zrw) + a.pab_in[qs - d.n2] * zrw;
-    a.pn2[q] = a.grav * (zaw * (a.pts[qt - d.n2] - a.pts[qt]) - zbw * (a.pts[qs - d.n2] - a.pts[qs])) /
-               d.e3w_n(c.ij, c.k, c.m) * wmsk<T>(ci, c.k);
-    return;
-  }
-  const T zt = a.pts[qt] - T(10), zs = a.pts[qs] - T(35), ztm = tmsk<T>(ci, c.k);
-  if (a.what == 2) {
-    const T zh = a.gdept[q];
-    T zn = a.a0 * (T(1) + a.lambda1 * zt + a.mu1 * zh) + a.nu * zs;
-    a.pab[qt] = zn * a.r1_rau0 * ztm;
-    zn = a.b0 * (T(1) - a.lambda2 * zs - a.mu2 * zh) - a.nu * zt;
-    a.pab[qs] = zn * a.r1_rau0 * ztm;
-    return;
-  }
-  const T zh = a.pdep[q];
-  if (a.what == 0) {
-    const T zn = -a.a0 * (T(1) + T(0.5) * a.lambda1 * zt + a.mu1 * zh) * zt +
-                 a.b0 * (T(1) - T(0.5) * a.lambda2 * zs - a.mu2 * zh) * zs - a.nu * zt * zs;
-    a.prd[q] = zn * a.r1_rau0 * ztm;
-  } else {
-    T zn = -a.a0 * (T(1) + T(0.5) * a.lambda1 * zt) * zt + a.b0 * (T(1) - T(0.5) * a.lambda2 * zs) * zs -
-           a.nu * zt * zs;
-    a.prhop[q] = (a.rau0 + zn) * ztm;
-    zn = zn - (a.a0 * a.mu1 * zt + a.b0 * a.mu2 * zs) * zh;
-    a.prd[q] = zn * a.r1_rau0 * ztm;
+__global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
+  const long p = (long)blockIdx.x * EOS_BLOCK + threadIdx.x;
+  if (p >= d.n2) return;
+  const int m = blockIdx.z, k0 = blockIdx.y * kch + 2, k1 = min(k0 + kch - 1, d.jpk - 1);
+  if (k0 > k1) return;
+  const long c3 = (long)m * d.n3 + p, c4 = 2 * (long)m * d.n3 + p, n3 = d.n3;
+  const ColInfo ci = d.ci[p];
+  const T* __restrict__ ts = a.pts + c4;
+  const T* __restrict__ ab = a.pab_in + c4;
+  const T* __restrict__ gt = a.gdept + c3;
+  const T* __restrict__ gw = a.gdepw + c3;
+  long o = (long)(k0 - 2) * d.n2;
+  T tu = __ldg(ts + o), su = __ldg(ts + n3 + o), au = __ldg(ab + o), bu = __ldg(ab + n3 + o), hu = __ldg(gt + o);
+  for (int k = k0; k <= k1; k += EOS_U) {
+    T t[EOS_U], s[EOS_U], x[EOS_U], y[EOS_U], h[EOS_U], w[EOS_U];
+#pragma unroll
+    for (int u = 0; u < EOS_U; ++u) {
+      const int ku = k + u <= k1 ? k + u : k1;
+      o = (long)(ku - 1) * d.n2;
+      t[u] = __ldg(ts + o);
+      s[u] = __ldg(ts + n3 + o);
+      x[u] = __ldg(ab + o);
+      y[u] = __ldg(ab + n3 + o);
+      h[u] = __ldg(gt + o);
+      w[u] = __ldg(gw + o);
+    }
+#pragma unroll
+    for (int u = 0; u < EOS_U; ++u) {
+      if (k + u > k1) break;
+      const T zrw = (w[u] - h[u]) / (hu - h[u]);
+      const T zaw = x[u] * (T(1) - zrw) + au * zrw;
+      const T zbw = y[u] * (T(1) - zrw) + bu * zrw;
+      a.pn2[c3 + (long)(k + u - 1) * d.n2] =
+          a.grav * (zaw * (tu - t[u]) - zbw * (su - s[u])) / d.e3w_n(p, k + u, m) * wmsk<T>(ci, k + u);
+      tu = t[u]; su = s[u]; au = x[u]; bu = y[u]; hu = h[u];
+    }
   }
 }
 

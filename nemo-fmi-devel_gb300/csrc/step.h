@@ -50,6 +50,24 @@ struct QsrArgs {
   int nksr, mode;
 };
 
+// EOS-80 coefficients of a kernel's arguments: the nonzero ones of each table packed
+// as [k][i][j], i + j <= D(k), so that a compiled-in index is a constant-bank operand
+// of the multiply-add that uses it and costs no load.
+__host__ __device__ constexpr int e80_at(int D, int i, int j) { return i * (D + 1) - i * (i - 1) / 2 + j; }
+__host__ __device__ constexpr int e80_len(int D) { return (D + 1) * (D + 2) / 2; }
+constexpr int E80_DEN[4] = {6, 4, 2, 1};  // degrees in zt (and zs) of the density's powers of zh
+constexpr int E80_EXP[4] = {5, 3, 1, 0};  // and of the expansion coefficients'
+constexpr int E80_NDEN = e80_len(6) + e80_len(4) + e80_len(2) + e80_len(1);
+constexpr int E80_NEXP = e80_len(5) + e80_len(3) + e80_len(1) + e80_len(0);
+// FP32 holds each coefficient twice, the operand of a packed multiply-add of two points.
+template <class T> struct E80Coef { typedef T type; };
+template <> struct E80Coef<float> { typedef unsigned long long type; };
+template <class T>
+struct E80Tab {
+  typedef typename E80Coef<T>::type C;
+  C eos[E80_NDEN], alp[E80_NEXP], bet[E80_NEXP];
+};
+
 // The simplified equation of state (np_seos), rab_3d and bn2; member strides are
 // those of the bound fields (2 x n3 for pts and pab, n3 for the others).
 template <class T>
@@ -58,13 +76,12 @@ struct EosArgs {
   T *prd, *prhop, *pab, *pn2;
   T a0, b0, lambda1, lambda2, mu1, mu2, nu, rau0, r1_rau0, grav;
   int what;  // 0 eos_insitu, 1 eos_insitu_pot, 2 rab_3d, 3 bn2
-  // EOS-80 (ln_eos80): FP64 evaluates the reference's table in its association
-  // (e80_raw: [table][k][i][j], eos80.h); FP32 the same polynomials re-expanded about
-  // the salinity 35 (e80_tay, same layout, in s' = zs - e80_s0), the density's
-  // constant term kept apart (e80_rho0, and e80_anom = e80_rho0 - rau0)
+  // EOS-80 (ln_eos80): FP64 evaluates the reference's table (eos80.h) in its
+  // association; FP32 the same polynomials re-expanded about the salinity 35 (in
+  // s' = zs - e80_s0), the density's constant term kept apart and zero in the table
+  // (e80_rho0, and e80_anom = e80_rho0 - rau0)
   int eos80;
-  const double* e80_raw;
-  const float* e80_tay;
+  E80Tab<T> e80;
   float e80_s0, e80_rho0, e80_anom;
 };
 
