@@ -19,6 +19,7 @@ struct LdfAdj {
   RO<double> lam;           // pta_ad
   double *tb_ad, *tbb_ad;   // tbb_ad: kpass 2 of the bilaplacian iso operator only
   double* G;                // work: zsign lam r1_e1e2t / e3t_n on the interior cells
+  double *su, *sv, *t3, *t4;  // work: the products of the face and w-point coefficients
   double *dit, *djt, *dk;   // work: adjoints of the gradients (jpi,jpj,jpk,kjpt)
 };
 

@@ -20,7 +20,12 @@ dim3 acol_grid(const Dom<T>& d) {
 }  // namespace
 
 cudaError_t launch_fct_adj(const Dom<double>& d, const FctAdj& a, cudaStream_t s) {
-  k_fct_adj<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a);
+  if (a.kh == 2) {
+    const dim3 g((d.jpi + 29) / 30, (d.jpj + FADJ_Y - 3) / (FADJ_Y - 2), d.nmem * ((d.jpk - 1 + FADJ_K - 1) / FADJ_K));
+    k_fct_adj2<<<g, dim3(32, FADJ_Y), 0, s>>>(d, a);
+  } else {
+    k_fct_adj<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a);
+  }
   ktick(NEMO_K_FCT_ADJ, s);
   if (a.kv == 4) {
     k_fct_adj_v4<<<acol_grid(d), dim3(AX, AY), 0, s>>>(d, a);
@@ -37,6 +42,7 @@ cudaError_t launch_lap_adj(const Dom<double>& d, const LdfArgs<double>& a, const
 
 cudaError_t launch_iso_adj(const Dom<double>& d, const LdfArgs<double>& a, const LdfAdj& b, cudaStream_t s) {
   k_iso_adj_g<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a, b);
+  k_iso_adj_prod<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a, b);
   k_iso_adj_grad<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a, b);
   k_iso_adj_tb<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a, b);
   ktick(NEMO_K_ISO_ADJ, s);

@@ -81,7 +81,7 @@ struct nemo_ctx {
   void* fct_w[6] = {};
   void* fct_ztw = nullptr;
   void* iso_w[3] = {};         // iso-neutral fluxes zftu, zftv, ztfw
-  void* adj_w[4] = {};         // iso-neutral adjoint: G and the gradient adjoints
+  void* adj_w[8] = {};         // iso-neutral adjoint: G, the gradient adjoints, the coefficient products
   double* spgadj_w = nullptr;  // dyn_spg_ts adjoint: 18 (jpi,jpj) arrays per member
   double* wzvadj_w = nullptr;  // wzv adjoint: one (jpi,jpj,jpk) array per member
   int adj_kjpt = 0;
@@ -2769,6 +2769,7 @@ int nemo_gpu_tra_ldf_iso_adj(nemo_ctx* c, int kt, int kit000, const char* cdtype
   LdfAdj b{};
   b.lam = (const double*)pta_ad; b.tb_ad = (double*)ptb_ad; b.tbb_ad = (double*)ptbb_ad;
   b.G = (double*)c->adj_w[0]; b.dit = (double*)c->adj_w[1]; b.djt = (double*)c->adj_w[2]; b.dk = (double*)c->adj_w[3];
+  b.su = (double*)c->adj_w[4]; b.sv = (double*)c->adj_w[5]; b.t3 = (double*)c->adj_w[6]; b.t4 = (double*)c->adj_w[7];
   cudaError_t e = launch_iso_adj(dom_now<double>(c), a, b, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "tra_ldf_iso_adj launch");
   return NEMO_OK;

@@ -37,6 +37,19 @@ struct Pt3 {
 template <class T>
 __device__ __forceinline__ Pt3 pt3(const Dom<T>& d) { return Pt3{d.jpi, d.jpj, d.jpk, d.n2}; }
 
+// x / e3t_n(k) and x / e3w_n(k): through the reciprocal profile (divq, the correctly
+// rounded quotient) where the now scale factor is the rest-state profile
+__device__ __forceinline__ double over_e3t(const Dom<double>& d, double x, long ij, int k, int m) {
+  const double e = d.e3t_n(ij, k, m);
+  return d.r1_e3t && d.e3t_n.s == 0 ? divq(x, e, d.r1_e3t[k - 1]) : x / e;
+}
+__device__ __forceinline__ double over_e3w(const Dom<double>& d, double x, long ij, int k, int m) {
+  const double e = d.e3w_n(ij, k, m);
+  return d.r1_e3w && d.e3w_n.s == 0 ? divq(x, e, d.r1_e3w[k - 1]) : x / e;
+}
+// x != 0 on the integer pipe (NaN counts as nonzero)
+__device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
 // ------------------------------------------------------------------ tra_adv_fct
 // Adjoint of tra_adv_fct (traadv_fct.F90:54-327) at one point; with kn_fct_h = 4 the
 // 4th-order centred horizontal fluxes (:191-227), with kn_fct_v = 4 the compact
@@ -74,7 +87,7 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
     auto g = [&](int ii, int jj, int kk) -> double {
       if (!P.cell(ii, jj, kk)) return 0.0;
       const long o = P.ij(ii, jj);
-      return lam[P.q(ii, jj, kk)] * d.r1_e1e2t[o] / d.e3t_n(o, kk, c.m);
+      return over_e3t(d, lam[P.q(ii, jj, kk)] * d.r1_e1e2t[o], o, kk, c.m);
     };
     const double gc = g(i, j, k), ge = g(i + 1, j, k), gw = g(i - 1, j, k), gn = g(i, j + 1, k),
                  gs = g(i, j - 1, k), gu = g(i, j, k - 1), gd = g(i, j, k + 1);
@@ -141,6 +154,120 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
     if (k == 1 && a.linssh) tbv += wn[q] * fzt;  // surface flux w tb (:146-156)
     a.tb_ad[mo + q] += tbv;
     a.tn_ad[mo + q] += tnv;
+  }
+}
+
+// tra_adv_fct's adjoint with kn_fct_h = 2: a block marches down a chunk of levels over
+// a tile of 32 x FADJ_Y points, one column a thread; each weight g and each face adjoint
+// is formed once a tile, by the point that owns it, and passed to its neighbour by a
+// shuffle (i) or through shared memory (j). The outer ring of the tile only feeds its
+// inside (30 x (FADJ_Y - 2) points are written). Bound by the FP64 pipe: a point of
+// k_fct_adj divides seven times a tracer and forms all six faces (1053 us at
+// 302x202x31, T and S). Values as k_fct_adj's: an upstream flux's adjoint f reaches the
+// point upstream of its face as u f and the other as 0 (0.5 (u + |u|) is u or 0).
+constexpr int FADJ_Y = 16, FADJ_K = 8;
+__global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj a) {
+  constexpr int NT = 2;
+  __shared__ double sg[NT][FADJ_Y][32], sp[NT][FADJ_Y][32], sr[NT][FADJ_Y][32];
+  const int lane = threadIdx.x, row = threadIdx.y, jpi = d.jpi, jpk = d.jpk;
+  const int i = blockIdx.x * 30 + lane, j = blockIdx.y * (FADJ_Y - 2) + row;  // 1-based, 0: outside
+  const int nch = (jpk - 1 + FADJ_K - 1) / FADJ_K, m = blockIdx.z / nch;
+  const int k0 = (int)(blockIdx.z - m * nch) * FADJ_K + 1, k1 = min(k0 + FADJ_K - 1, jpk - 1);
+  const Pt3 P = pt3(d);
+  const bool in = i >= 1 && i <= jpi && j >= 1 && j <= d.jpj;
+  const bool own = in && lane >= 1 && lane <= 30 && row >= 1 && row <= FADJ_Y - 2;
+  const bool ic = in && P.icol(i, j), face = in && i <= jpi - 1 && j <= d.jpj - 1;
+  // the halo's weights are needed inside; its faces west and south of the tile's inside
+  const long ij = in ? P.ij(i, j) : 0, n2 = d.n2, n3 = d.n3, mv = (long)m * n3;
+  const bool last = lane == 31 || row == FADJ_Y - 1;  // no east / north neighbour in the tile
+  const bool fx = face && !last;
+  const ColInfo ci = d.ci[ij];
+  ColInfo ce{}, cn{};
+  if (fx) {
+    ce = d.ci[ij + 1];
+    cn = d.ci[ij + jpi];
+  }
+  const double r1 = d.r1_e1e2t[ij];
+  const RO<double> un = a.pun + mv, vn = a.pvn + mv, wn = a.pwn + mv;
+  for (int n0 = 0; n0 < a.kjpt; n0 += NT) {
+    const int nt = a.kjpt - n0 < NT ? a.kjpt - n0 : NT;
+    auto g = [&](int n, int k) -> double {  // lam r1_e1e2t / e3t_n of the own column
+      return ic && k <= jpk - 1 ? over_e3t(d, a.lam[((long)m * a.kjpt + n) * n3 + ij + (long)(k - 1) * n2] * r1, ij, k, m)
+                                : 0.0;
+    };
+    // carried: g(k); the parts of the top face of level k that its column gets below it
+    double gc[NT] = {}, pz[NT] = {}, rz[NT] = {};
+    // the vertical face between levels k-1 and k (weights gu, gk): its centred part on tn
+    // and its upstream part, with w > 0 for the level below (k), w < 0 for that above
+    auto zface = [&](int n, int k, double gu, double gk, double& p, double& r) {
+      p = 0.0;
+      r = 0.0;
+      if (!in || k < 2 || k > jpk - 1) return;
+      const long q = ij + (long)(k - 1) * n2;
+      const double w = wn[q], wm = wmsk<double>(ci, k);
+      double az = 0.0;
+      if (ic) {
+        az = msel(a.tape[(((long)m * a.kjpt + n) * 3 + 2) * n3 + q] * (gu - gk), wm);
+        if (a.kv == 2) p = w * 0.5 * az;
+      }
+      const double fz = -az + (msel(gu, tmsk<double>(ci, k - 1)) - msel(gk, tmsk<double>(ci, k)));
+      r = msel(w * fz, wm);
+    };
+    for (int nn = 0; nn < nt; ++nn) {
+      gc[nn] = g(n0 + nn, k0);
+      if (k0 > 1) zface(n0 + nn, k0, g(n0 + nn, k0 - 1), gc[nn], pz[nn], rz[nn]);
+    }
+    for (int k = k0; k <= k1; ++k) {
+      const long q = ij + (long)(k - 1) * n2;
+#pragma unroll
+      for (int nn = 0; nn < NT; ++nn) sg[nn][row][lane] = gc[nn];
+      __syncthreads();
+      const double u = fx ? un[q] : 0.0, v = fx ? vn[q] : 0.0;
+      const double tm = tmsk<double>(ci, k);
+      double px[NT], rx[NT], py[NT], ry[NT];
+#pragma unroll
+      for (int nn = 0; nn < NT; ++nn) {
+        const double ge = __shfl_down_sync(0xffffffffu, gc[nn], 1);
+        px[nn] = rx[nn] = py[nn] = ry[nn] = 0.0;
+        if (fx && nn < nt) {
+          const RO<double> tx = a.tape + ((long)m * a.kjpt + n0 + nn) * 3 * n3;
+          const double gn = sg[nn][row + 1][lane], hc = msel(gc[nn], tm);
+          const double ax = tx[q] * (ge - gc[nn]), ay = tx[n3 + q] * (gn - gc[nn]);
+          px[nn] = 0.5 * u * ax;
+          py[nn] = 0.5 * v * ay;
+          rx[nn] = u * (-ax + (msel(ge, tmsk<double>(ce, k)) - hc));
+          ry[nn] = v * (-ay + (msel(gn, tmsk<double>(cn, k)) - hc));
+        }
+        sp[nn][row][lane] = py[nn];
+        sr[nn][row][lane] = sgn_pos(v) ? 0.0 : ry[nn];  // for the northern point
+      }
+      __syncthreads();
+      const double wt = own && k >= 2 ? wn[q] : 0.0;
+      const double wb = own && k + 1 <= jpk - 1 ? wn[q + n2] : 0.0;
+#pragma unroll
+      for (int nn = 0; nn < NT; ++nn) {
+        const double pw = __shfl_up_sync(0xffffffffu, px[nn], 1);
+        const double rw = __shfl_up_sync(0xffffffffu, sgn_pos(u) ? 0.0 : rx[nn], 1);
+        if (nn >= nt) continue;
+        const int n = n0 + nn;
+        const double gd = g(n, k + 1);
+        double pb, rb;
+        zface(n, k + 1, gc[nn], gd, pb, rb);
+        if (own) {
+          const double tnv = px[nn] + pw + py[nn] + sp[nn][row - 1][lane] + pz[nn] + pb;
+          double tbv = (sgn_pos(u) ? rx[nn] : 0.0) + rw + (sgn_pos(v) ? ry[nn] : 0.0) + sr[nn][row - 1][lane];
+          tbv += sgn_pos(wt) ? rz[nn] : 0.0;
+          tbv += sgn_pos(wb) ? 0.0 : rb;
+          if (k == 1 && a.linssh) tbv += wn[q] * -msel(gc[nn], tm);  // surface flux w tb (:146-156)
+          const long o = ((long)m * a.kjpt + n) * n3 + q;
+          a.tb_ad[o] += tbv;
+          a.tn_ad[o] += tnv;
+        }
+        gc[nn] = gd;
+        pz[nn] = pb;
+        rz[nn] = rb;
+      }
+    }
   }
 }
 
@@ -264,6 +391,13 @@ __global__ void __launch_bounds__(128) k_lap_adj(Dom<double> d, LdfArgs<double> 
 }
 
 // ------------------------------------------------------------------ tra_ldf_iso
+// The adjoint runs at the FP64 rate (1/58 of FP32: one FP64 operation per tracer cell
+// costs as much time as 13 bytes of HBM traffic), so each coefficient and each product
+// is formed once, by the point that owns its face, and kept in work arrays; as one
+// gather kernel, in which every point formed the coefficients of its six w-points and
+// eight faces for each tracer, the gradient stage alone took 2254 us at 302x202x31
+// (T and S).
+//
 // Stage 0: G = zsign lam r1_e1e2t / e3t_n on the interior cells, 0 elsewhere (the
 // adjoint weight of a divergence, :278-284 and :359-366).
 __global__ void __launch_bounds__(128) k_iso_adj_g(Dom<double> d, LdfArgs<double> a, LdfAdj b) {
@@ -272,141 +406,120 @@ __global__ void __launch_bounds__(128) k_iso_adj_g(Dom<double> d, LdfArgs<double
   const Pt3 P = pt3(d);
   for (int n = 0; n < a.kjpt; ++n) {
     const long o = ((long)c.m * a.kjpt + n) * d.n3 + c.q;
-    b.G[o] = P.cell(c.i, c.j, c.k) ? a.zsign * b.lam[o] * d.r1_e1e2t[c.ij] / d.e3t_n(c.ij, c.k, c.m) : 0.0;
+    b.G[o] = P.cell(c.i, c.j, c.k) ? over_e3t(d, a.zsign * b.lam[o] * d.r1_e1e2t[c.ij], c.ij, c.k, c.m) : 0.0;
   }
 }
 
-// Coefficients of the iso-neutral fluxes at one face or w-point, as the forward
-// kernel forms them (traldf_iso.F90:255-276 horizontal, :297-357 vertical).
-struct IsoAdjCoef {
-  const Dom<double>& d;
-  const LdfArgs<double>& a;
-  Pt3 P;
-  int m;
-  long m3;
-  // zcof1 * umask of the u face (ii,jj,kk); zabe1 * umask
-  __device__ __forceinline__ double cof1(int ii, int jj, int kk) const {
-    const long o = P.ij(ii, jj);
-    const ColInfo cc = d.ci[o], ce = d.ci[o + 1];
-    const double pah = ahu(d, a, cc, o, kk, m);
-    const double zm = rcount(wmsk<double>(ce, kk) + wmsk<double>(cc, kk + 1) + wmsk<double>(ce, kk + 1) +
-                             wmsk<double>(cc, kk));
-    return -pah * d.e2u[o] * a.uslp[m3 + o + (long)(kk - 1) * P.n2] * zm * umsk<double>(cc, kk);
-  }
-  __device__ __forceinline__ double cof2(int ii, int jj, int kk) const {
-    const long o = P.ij(ii, jj);
-    const ColInfo cc = d.ci[o], cn = d.ci[o + P.jpi];
-    const double pah = ahv(d, a, cc, o, kk, m);
-    const double zm = rcount(wmsk<double>(cn, kk) + wmsk<double>(cc, kk + 1) + wmsk<double>(cn, kk + 1) +
-                             wmsk<double>(cc, kk));
-    return -pah * d.e1v[o] * a.vslp[m3 + o + (long)(kk - 1) * P.n2] * zm * vmsk<double>(cc, kk);
-  }
-  __device__ __forceinline__ double abe1(int ii, int jj, int kk) const {
-    const long o = P.ij(ii, jj);
-    const ColInfo cc = d.ci[o];
-    return ahu(d, a, cc, o, kk, m) * d.e2_e1u[o] * d.e3u_n(o, kk, m) * umsk<double>(cc, kk);
-  }
-  __device__ __forceinline__ double abe2(int ii, int jj, int kk) const {
-    const long o = P.ij(ii, jj);
-    const ColInfo cc = d.ci[o];
-    return ahv(d, a, cc, o, kk, m) * d.e1_e2v[o] * d.e3v_n(o, kk, m) * vmsk<double>(cc, kk);
-  }
-  // zcoef3 / zcoef4 of the w-point (ii,jj,kk): interior column, 2 <= kk <= jpkm1
-  __device__ __forceinline__ void coef34(int ii, int jj, int kk, double& c3, double& c4) const {
-    const long o = P.ij(ii, jj);
-    const ColInfo cc = d.ci[o], cw = d.ci[o - 1], cs = d.ci[o - P.jpi];
-    const IsoW<double> w = iso_w(d, a, o, kk, m, cc, cw, cs);
-    const long qq = m3 + o + (long)(kk - 1) * P.n2;
-    c3 = -w.zahu_w * d.e2t[o] * w.zmsku * a.wslpi[qq];
-    c4 = -w.zahv_w * d.e1t[o] * w.zmskv * a.wslpj[qq];
-  }
-  // the vertical laplacian coefficients of the w-point on tb and on tbb
-  __device__ __forceinline__ void vlap(int ii, int jj, int kk, double& ctb, double& ctbb) const {
-    const long o = P.ij(ii, jj);
-    const long qq = m3 + o + (long)(kk - 1) * P.n2;
-    const double f = d.e1e2t[o] / d.e3w_n(o, kk, m) * wmsk<double>(d.ci[o], kk);
-    const double ahw = a.ah_wslp2[qq], akz = a.akz[qq];
-    ctbb = 0.0;
-    if (a.lap) ctb = f * (ahw - akz);
-    else if (a.kpass == 1) ctb = ahw * f;
-    else { ctb = ahw * f; ctbb = akz * f; }
-  }
-};
+// The vertical laplacian coefficients of the w-point (ij,k) on tb and on tbb, as the
+// forward kernel forms them (traldf_iso.F90:337-357).
+__device__ __forceinline__ void iso_adj_vlap(const Dom<double>& d, const LdfArgs<double>& a, long ij, int k, int m,
+                                             double& ctb, double& ctbb) {
+  const long qq = (long)m * d.n3 + ij + (long)(k - 1) * d.n2;
+  const double f = msel(over_e3w(d, d.e1e2t[ij], ij, k, m), wmsk<double>(d.ci[ij], k));
+  const double ahw = a.ah_wslp2[qq], akz = a.akz[qq];
+  ctbb = 0.0;
+  if (a.lap) ctb = f * (ahw - akz);
+  else if (a.kpass == 1) ctb = ahw * f;
+  else { ctb = ahw * f; ctbb = akz * f; }
+}
 
-// Stage 1: adjoints of the masked gradients zdit(i,j,k), zdjt(i,j,k) (u and v faces)
+// Stage 1: the products of the face and w-point coefficients (traldf_iso.F90:255-276
+// horizontal, :297-332 vertical) with the differences of G their fluxes see. su, sv:
+// cof1 (G - G(i+1)), cof2 (G - G(j+1)) at the u and v faces; t3, t4: zcoef3, zcoef4
+// times the adjoint G(k) - G(k-1) of the vertical flux at the interior w-points.
+__global__ void __launch_bounds__(128) k_iso_adj_prod(Dom<double> d, LdfArgs<double> a, LdfAdj b) {
+  const PtIdx c = pt_index(d);
+  if (!c.valid) return;
+  const Pt3 P = pt3(d);
+  const int i = c.i, j = c.j, k = c.k, m = c.m, jpi = d.jpi;
+  const long n3 = d.n3, q = c.q, qm = (long)m * n3 + q, ij = c.ij;
+  const bool face = P.uface(i, j, k), wpt = P.icol(i, j) && k >= 2 && k <= d.jpk - 1;
+  const ColInfo ci = d.ci[ij];
+  double cof1 = 0.0, cof2 = 0.0, c3 = 0.0, c4 = 0.0;
+  if (face) {
+    const ColInfo ce = d.ci[ij + 1], cn = d.ci[ij + jpi];
+    const double w0 = wmsk<double>(ci, k), w1 = wmsk<double>(ci, k + 1);
+    const double zu = rcount4(wmsk<double>(ce, k), w1, wmsk<double>(ce, k + 1), w0);
+    const double zv = rcount4(wmsk<double>(cn, k), w1, wmsk<double>(cn, k + 1), w0);
+    cof1 = msel(-ahu(d, a, ci, ij, k, m) * d.e2u[ij] * a.uslp[qm] * zu, umsk<double>(ci, k));
+    cof2 = msel(-ahv(d, a, ci, ij, k, m) * d.e1v[ij] * a.vslp[qm] * zv, vmsk<double>(ci, k));
+  }
+  if (wpt) {
+    const IsoW<double> w = iso_w(d, a, ij, k, m, ci, d.ci[ij - 1], d.ci[ij - jpi]);
+    c3 = -w.zahu_w * d.e2t[ij] * w.zmsku * a.wslpi[qm];
+    c4 = -w.zahv_w * d.e1t[ij] * w.zmskv * a.wslpj[qm];
+  }
+  for (int n = 0; n < a.kjpt; ++n) {
+    const long o = ((long)m * a.kjpt + n) * n3 + q;
+    const RO<double> G = b.G;
+    const double g = G[o];
+    b.su[o] = face ? cof1 * (g - G[o + 1]) : 0.0;
+    b.sv[o] = face ? cof2 * (g - G[o + jpi]) : 0.0;
+    double t3 = 0.0, t4 = 0.0;
+    if (wpt) {
+      const double t = g - G[o - d.n2];
+      if (nonzero(t)) {
+        t3 = c3 * t;
+        t4 = c4 * t;
+      }
+    }
+    b.t3[o] = t3;
+    b.t4[o] = t4;
+  }
+}
+
+// Stage 2: adjoints of the masked gradients zdit(i,j,k), zdjt(i,j,k) (u and v faces)
 // and of the vertical difference D(k) = (tb(k-1) - tb(k)) wmask(k) of column (i,j),
-// k = 2..jpk (zdkt(k) = D(k), zdk1t(k) = D(k+1), zdkt(1) = D(2); :246-254).
+// k = 2..jpk (zdkt(k) = D(k), zdk1t(k) = D(k+1), zdkt(1) = D(2); :246-254). zdit(i,j,k)
+// enters ztfw at (i,j) and (i+1,j), levels k and k+1, zdjt at (i,j) and (i,j+1); D(k)
+// is zdkt of level k and zdk1t of level k-1 for the u faces of columns i-1 and i and
+// the v faces of j-1 and j; at k = 2 also zdkt of level 1.
 __global__ void __launch_bounds__(128) k_iso_adj_grad(Dom<double> d, LdfArgs<double> a, LdfAdj b) {
   const PtIdx c = pt_index(d);
   if (!c.valid) return;
   const Pt3 P = pt3(d);
-  const int i = c.i, j = c.j, k = c.k, jpk = d.jpk;
-  const long n3 = d.n3;
-  const IsoAdjCoef C{d, a, P, c.m, (long)c.m * n3};
+  const int i = c.i, j = c.j, k = c.k, m = c.m, jpi = d.jpi, jpk = d.jpk;
+  const long n2 = d.n2, n3 = d.n3, ij = c.ij;
+  const ColInfo ci = d.ci[ij];
+  const bool face = P.uface(i, j, k), wpt = P.icol(i, j) && k >= 2 && k <= jpk - 1;
+  double abe1 = 0.0, abe2 = 0.0, ctb = 0.0, ctbb = 0.0;
+  if (face) {
+    abe1 = msel(ahu(d, a, ci, ij, k, m) * d.e2_e1u[ij] * d.e3u_n(ij, k, m), umsk<double>(ci, k));
+    abe2 = msel(ahv(d, a, ci, ij, k, m) * d.e1_e2v[ij] * d.e3v_n(ij, k, m), vmsk<double>(ci, k));
+  }
+  if (wpt) iso_adj_vlap(d, a, ij, k, m, ctb, ctbb);
+  // the faces of columns i-1 and j-1 lie outside the flux loops where these are 0
+  const bool hw = i > 1, hs = j > 1;
   for (int n = 0; n < a.kjpt; ++n) {
-    const long mo = ((long)c.m * a.kjpt + n) * n3;
-    const RO<double> G = b.G + mo;
-    auto gg = [&](int ii, int jj, int kk) -> double {
-      return (ii >= 1 && ii <= P.jpi && jj >= 1 && jj <= P.jpj && kk >= 1 && kk <= jpk) ? G[P.q(ii, jj, kk)] : 0.0;
-    };
-    // adjoint of the vertical flux ztfw at w-point (ii,jj,kk): G(kk) - G(kk-1)
-    auto tfw = [&](int ii, int jj, int kk) -> double {
-      if (!P.icol(ii, jj) || kk < 2 || kk > jpk - 1) return 0.0;
-      return gg(ii, jj, kk) - gg(ii, jj, kk - 1);
-    };
-    auto w34 = [&](int ii, int jj, int kk, double& s3, double& s4) {
-      const double t = tfw(ii, jj, kk);
-      if (t == 0.0) return;
-      double c3, c4;
-      C.coef34(ii, jj, kk, c3, c4);
-      s3 += c3 * t;
-      s4 += c4 * t;
-    };
+    const long o = ((long)m * a.kjpt + n) * n3 + c.q;
+    const RO<double> G = b.G, su = b.su, sv = b.sv, t3 = b.t3, t4 = b.t4;
     double di = 0.0, dj = 0.0, dk = 0.0;
-    if (P.uface(i, j, k)) {
-      double s3 = 0.0, s4 = 0.0, t3 = 0.0, t4 = 0.0;
-      // zdit(i,j,k) enters ztfw at (i,j,k+1), (i+1,j,k), (i+1,j,k+1), (i,j,k);
-      // zdjt(i,j,k) at (i,j,k+1), (i,j+1,k), (i,j+1,k+1), (i,j,k)
-      w34(i, j, k + 1, s3, s4);
-      w34(i, j, k, s3, s4);
-      double x;
-      w34(i + 1, j, k, t3, x);
-      w34(i + 1, j, k + 1, t3, x);
-      w34(i, j + 1, k, x, t4);
-      w34(i, j + 1, k + 1, x, t4);
-      const ColInfo cc = d.ci[P.ij(i, j)];
-      di = C.abe1(i, j, k) * (gg(i, j, k) - gg(i + 1, j, k)) + s3 + t3;
-      dj = C.abe2(i, j, k) * (gg(i, j, k) - gg(i, j + 1, k)) + s4 + t4;
-      if (a.zps && k == cc.mbku) di = 0.0;
-      if (a.zps && k == cc.mbkv) dj = 0.0;
+    if (face) {  // levels k, k+1 <= jpk
+      const double g = G[o];
+      di = abe1 * (g - G[o + 1]) + (t3[o + n2] + t3[o]) + (t3[o + 1] + t3[o + 1 + n2]);
+      dj = abe2 * (g - G[o + jpi]) + (t4[o + n2] + t4[o]) + (t4[o + jpi] + t4[o + jpi + n2]);
+      if (a.zps && k == ci.mbku) di = 0.0;
+      if (a.zps && k == ci.mbkv) dj = 0.0;
     }
     if (k >= 2) {
-      // D(k) is zdkt of level k and zdk1t of level k-1 for the u faces of columns
-      // i-1 and i (and the v faces of j-1 and j); at k = 2 also zdkt of level 1
-      auto su = [&](int ii, int jj, int kk) -> double {
-        return P.uface(ii, jj, kk) ? C.cof1(ii, jj, kk) * (gg(ii, jj, kk) - gg(ii + 1, jj, kk)) : 0.0;
-      };
-      auto sv = [&](int ii, int jj, int kk) -> double {
-        return P.uface(ii, jj, kk) ? C.cof2(ii, jj, kk) * (gg(ii, jj, kk) - gg(ii, jj + 1, kk)) : 0.0;
-      };
-      double s = su(i, j, k) + su(i - 1, j, k) + su(i, j, k - 1) + su(i - 1, j, k - 1);
-      s += sv(i, j, k) + sv(i, j - 1, k) + sv(i, j, k - 1) + sv(i, j - 1, k - 1);
-      if (k == 2) s += su(i, j, 1) + su(i - 1, j, 1) + sv(i, j, 1) + sv(i, j - 1, 1);
-      const double t = tfw(i, j, k);
-      if (t != 0.0) {
-        double ctb, ctbb;
-        C.vlap(i, j, k, ctb, ctbb);
-        s += ctb * t;
+      const double u0 = su[o], uw = hw ? su[o - 1] : 0.0, u1 = su[o - n2], uw1 = hw ? su[o - 1 - n2] : 0.0;
+      const double v0 = sv[o], vs = hs ? sv[o - jpi] : 0.0, v1 = sv[o - n2], vs1 = hs ? sv[o - jpi - n2] : 0.0;
+      double s = u0 + uw + u1 + uw1;
+      s += v0 + vs + v1 + vs1;
+      if (k == 2) s += u1 + uw1 + v1 + vs1;
+      if (wpt) {
+        const double t = G[o] - G[o - n2];
+        if (nonzero(t)) s += ctb * t;
       }
       dk = s;
     }
-    b.dit[mo + c.q] = di;
-    b.djt[mo + c.q] = dj;
-    b.dk[mo + c.q] = dk;
+    b.dit[o] = di;
+    b.djt[o] = dj;
+    b.dk[o] = dk;
   }
 }
 
-// Stage 2: tb_ad from the gradient adjoints (zdit = (tb(i+1)-tb(i)) umask, :218-227;
+// Stage 3: tb_ad from the gradient adjoints (zdit = (tb(i+1)-tb(i)) umask, :218-227;
 // D(k)), and tbb_ad from the second-pass vertical term (:343-356).
 __global__ void __launch_bounds__(128) k_iso_adj_tb(Dom<double> d, LdfArgs<double> a, LdfAdj b) {
   const PtIdx c = pt_index(d);
@@ -416,29 +529,28 @@ __global__ void __launch_bounds__(128) k_iso_adj_tb(Dom<double> d, LdfArgs<doubl
   const long q = c.q, n2 = d.n2, n3 = d.n3;
   const ColInfo ci = d.ci[c.ij];
   const bool tbb = !a.lap && a.kpass != 1;
-  const IsoAdjCoef C{d, a, P, c.m, (long)c.m * n3};
   for (int n = 0; n < a.kjpt; ++n) {
     const long mo = ((long)c.m * a.kjpt + n) * n3;
     const RO<double> di = b.dit + mo;
     const RO<double> dj = b.djt + mo;
     const RO<double> dk = b.dk + mo;
     double v = 0.0;
-    if (P.uface(i - 1, j, k)) v += umsk<double>(d.ci[c.ij - 1], k) * di[q - 1];
-    if (P.uface(i, j, k)) v -= umsk<double>(ci, k) * di[q];
-    if (P.uface(i, j - 1, k)) v += vmsk<double>(d.ci[c.ij - jpi], k) * dj[q - jpi];
-    if (P.uface(i, j, k)) v -= vmsk<double>(ci, k) * dj[q];
-    if (k + 1 <= jpk) v += wmsk<double>(ci, k + 1) * dk[q + n2];
-    if (k >= 2) v -= wmsk<double>(ci, k) * dk[q];
+    if (P.uface(i - 1, j, k)) v += msel(di[q - 1], umsk<double>(d.ci[c.ij - 1], k));
+    if (P.uface(i, j, k)) v -= msel(di[q], umsk<double>(ci, k));
+    if (P.uface(i, j - 1, k)) v += msel(dj[q - jpi], vmsk<double>(d.ci[c.ij - jpi], k));
+    if (P.uface(i, j, k)) v -= msel(dj[q], vmsk<double>(ci, k));
+    if (k + 1 <= jpk) v += msel(dk[q + n2], wmsk<double>(ci, k + 1));
+    if (k >= 2) v -= msel(dk[q], wmsk<double>(ci, k));
     b.tb_ad[mo + q] += v;
     if (tbb && P.icol(i, j)) {
       const RO<double> G = b.G + mo;
       double u = 0.0, ctb, ctbb;
       if (k + 1 >= 2 && k + 1 <= jpk - 1) {
-        C.vlap(i, j, k + 1, ctb, ctbb);
+        iso_adj_vlap(d, a, c.ij, k + 1, c.m, ctb, ctbb);
         u += ctbb * (G[q + n2] - G[q]);
       }
       if (k >= 2 && k <= jpk - 1) {
-        C.vlap(i, j, k, ctb, ctbb);
+        iso_adj_vlap(d, a, c.ij, k, c.m, ctb, ctbb);
         u -= ctbb * (G[q] - G[q - n2]);
       }
       b.tbb_ad[mo + q] += u;
@@ -450,7 +562,8 @@ __global__ void __launch_bounds__(128) k_iso_adj_tb(Dom<double> d, LdfArgs<doubl
 // Adjoint of tra_zdf_imp (trazdf.F90:143-264) on one interior column: the
 // back-substitution run forwards, then the elimination with its right-hand side
 // e3t_b tb + p2dt e3t_n ta run backwards. The matrix is built as k_zdf_imp builds
-// it in double precision.
+// it in double precision: one division a level, 1 / zwt, and every quotient corrected
+// from a reciprocal (divq); zwi(k+1) is zws(k).
 __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
   ColIdx<double> c = col_index(d);
   if (!c.valid || !c.interior) return;
@@ -458,7 +571,7 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
   const long n2 = d.n2, n3 = d.n3;
   const ColInfo ci = d.ci[c.ij];
   const long m3 = (long)c.m * n3;
-  double rat[KMAX], zws[KMAX], zwt[KMAX];
+  double rat[KMAX], zws[KMAX], zwt[KMAX], rz[KMAX];  // rz = 1 / zwt
   for (int n = 0; n < a.kjpt; ++n) {
     const bool build = (!a.is_trc && (n == 0 || (n == 1 && a.ddm))) || (a.is_trc && n == 0);
     if (build) {
@@ -470,15 +583,18 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
         if (a.add && k <= jpk - 1) v = v + a.add[q];
         return v;
       };
-      double wtk = wt(1);
+      double zwi = over_e3w(d, -a.p2dt * wt(1), c.ij, 1, c.m), tp = 0.0, rp = 0.0;
       for (int k = 1; k <= jpk - 1; ++k) {
-        const double wtk1 = wt(k + 1);
-        const double zwi = -a.p2dt * wtk / d.e3w_n(c.ij, k, c.m);
-        zws[k] = -a.p2dt * wtk1 / d.e3w_n(c.ij, k + 1, c.m);
-        if (k >= 2) rat[k] = zwi / zwt[k - 1];
-        const double zwd = d.e3t_a(c.ij, k, c.m) - zwi - zws[k];
-        zwt[k] = (k == 1) ? zwd : zwd - zwi * zws[k - 1] / zwt[k - 1];
-        wtk = wtk1;
+        const double zs = over_e3w(d, -a.p2dt * wt(k + 1), c.ij, k + 1, c.m);
+        double t = d.e3t_a(c.ij, k, c.m) - zwi - zs;
+        if (k >= 2) {
+          rat[k] = divq(zwi, tp, rp);
+          t = t - divq(zwi * zwi, tp, rp);  // zws(k-1) = zwi(k)
+        }
+        zws[k] = zs;
+        zwt[k] = tp = t;
+        rz[k] = rp = 1.0 / t;
+        zwi = zs;
       }
     }
     const long mo = ((long)c.m * a.kjpt + n) * n3;
@@ -488,13 +604,13 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
     double carry = 0.0;  // what level k receives from level k-1
     for (int k = 1; k <= jpk - 2; ++k) {
       const long q = c.ij + (long)(k - 1) * n2;
-      const double x = (lam[q] + carry) * tmsk<double>(ci, k) / zwt[k];
+      const double x = divq(msel(lam[q] + carry, tmsk<double>(ci, k)), zwt[k], rz[k]);
       carry = -zws[k] * x;
       lam[q] = x;
     }
     {
       const long q = c.ij + (long)(jpk - 2) * n2;
-      lam[q] = (lam[q] + carry) * tmsk<double>(ci, jpk - 1) / zwt[jpk - 1];
+      lam[q] = divq(msel(lam[q] + carry, tmsk<double>(ci, jpk - 1)), zwt[jpk - 1], rz[jpk - 1]);
     }
     // elimination (:238-250) run backwards
     double up = 0.0;  // what level k receives from level k+1

@@ -587,8 +587,8 @@ __device__ __forceinline__ IsoW<T> iso_w(const Dom<T>& d, const LdfArgs<T>& a, l
   const int jpi = d.jpi;
   const T wm = wmk<W, T>(ci, k);
   IsoW<T> w;
-  w.zmsku = wm * rcount(umk<W, T>(ci, k - 1) + umk<W, T>(ciw, k) + umk<W, T>(ciw, k - 1) + umk<W, T>(ci, k));
-  w.zmskv = wm * rcount(vmk<W, T>(ci, k - 1) + vmk<W, T>(cis, k) + vmk<W, T>(cis, k - 1) + vmk<W, T>(ci, k));
+  w.zmsku = msel(rcount4(umk<W, T>(ci, k - 1), umk<W, T>(ciw, k), umk<W, T>(ciw, k - 1), umk<W, T>(ci, k)), wm);
+  w.zmskv = msel(rcount4(vmk<W, T>(ci, k - 1), vmk<W, T>(cis, k), vmk<W, T>(cis, k - 1), vmk<W, T>(ci, k)), wm);
   w.zahu_w = (ahu<W>(d, a, ci, ij, k - 1, m) + ahu<W>(d, a, ciw, ij - 1, k, m) + ahu<W>(d, a, ciw, ij - 1, k - 1, m) +
               ahu<W>(d, a, ci, ij, k, m)) * w.zmsku;
   w.zahv_w = (ahv<W>(d, a, ci, ij, k - 1, m) + ahv<W>(d, a, cis, ij - jpi, k, m) + ahv<W>(d, a, cis, ij - jpi, k - 1, m) +
