@@ -57,7 +57,8 @@ cudaError_t launch_zdf_adj(const Dom<double>& d, const ZdfArgs<double>& a, const
 
 template <class T>
 cudaError_t launch_tra_nxt(const Dom<T>& d, T* tsb, T* tsn, T* tsa, T atfp, int euler, cudaStream_t s) {
-  k_tra_nxt<T><<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, tsb, tsn, tsa, atfp, euler);
+  const int kch = march_chunk(d);
+  k_tra_nxt<T><<<march_grid(d, kch), dim3(AX, MARCH_Y), 0, s>>>(d, tsb, tsn, tsa, atfp, euler, kch);
   ktick(NEMO_K_TRA_NXT, s);
   return cudaGetLastError();
 }

@@ -89,7 +89,6 @@ struct nemo_ctx {
   void* rab_w = nullptr;       // the model step's before expansion ratios rab_b (jpi,jpj,jpk,2)
   void* rab_n = nullptr;       // and the now ones rab_n, with the vertical physics
   void* zphy_w = nullptr;      // zdf_phy work: sh2, apdlr and the TKE system, 5 x n3 per member
-  void* zdyn_w = nullptr;      // dyn_zdf work: the implicit viscosity system, 2 x n3 per member
   double* fadj_w = nullptr;    // FCT adjoint with kn_fct_v = 4: 2 x n3 per member
   double* usr_s = nullptr;     // usrdef_sbc: the step's scalars (7), written before each step
   double usr_zsurf = 0.0;      // usrdef_sbc: GLOB_SUM(tmask(:,:,1))
@@ -1168,9 +1167,6 @@ int run_dyn_zdf_step(nemo_ctx* c, int kt) {
                                flux ? (const T*)F[NEMO_F_E3V_B] : nullptr, flux ? (const T*)F[NEMO_F_E3U_A] : nullptr,
                                flux ? (const T*)F[NEMO_F_E3V_A] : nullptr, c->stream);
   } else {
-    const size_t n = (size_t)c->n3 * c->nmem;
-    if (!c->zdyn_w && cudaMalloc(&c->zdyn_w, 2 * n * sizeof(T)) != cudaSuccess)
-      return fail(c, NEMO_ERR_NOMEM, "dyn_zdf work arrays");
     DynZdfArgs<T> a{};
     a.ub = (const T*)F[NEMO_F_UB]; a.vb = (const T*)F[NEMO_F_VB]; a.avm = (const T*)F[NEMO_F_AVM];
     a.rcdu = (const T*)F[NEMO_F_RCDU_BOT]; a.utau = (const T*)F[NEMO_F_UTAU]; a.vtau = (const T*)F[NEMO_F_VTAU];
@@ -1178,7 +1174,6 @@ int run_dyn_zdf_step(nemo_ctx* c, int kt) {
     a.vtau_b = F[NEMO_F_VTAU_B] ? (const T*)F[NEMO_F_VTAU_B] : a.vtau;
     a.ua_b = (const double*)F[NEMO_F_UA_B]; a.va_b = (const double*)F[NEMO_F_VA_B];
     a.ua = (T*)F[NEMO_F_UA]; a.va = (T*)F[NEMO_F_VA];
-    a.zwd = (T*)c->zdyn_w; a.zws = a.zwd + n;
     a.r2dt = (T)r2dt; a.zdt = (T)(r2dt * 0.5); a.rau0 = (T)nm.rau0;
     e = launch_dyn_zdf_imp<T>(dom_now<T>(c), a, c->stream);
   }
@@ -1957,7 +1952,7 @@ int nemo_gpu_destroy(nemo_ctx* c) {
   for (auto p : c->iso_w) cudaFree(p);
   for (auto p : c->adj_w) cudaFree(p);
   cudaFree(c->slp_w);
-  cudaFree(c->rab_w); cudaFree(c->rab_n); cudaFree(c->zphy_w); cudaFree(c->zdyn_w); cudaFree(c->usr_s); cudaFree(c->fadj_w);
+  cudaFree(c->rab_w); cudaFree(c->rab_n); cudaFree(c->zphy_w); cudaFree(c->usr_s); cudaFree(c->fadj_w);
   cudaFree(c->blp_w);
   for (auto p : c->spg_w) cudaFree(p);
   for (auto p : c->spg_cor) cudaFree(p);

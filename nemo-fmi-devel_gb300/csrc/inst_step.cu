@@ -23,11 +23,20 @@ int level_chunk(const Dom<T>& d, int block, int step) {
     if (planes * ((d.jpk + f * step - 1) / (f * step)) * block >= 152L * 64 * 32) return f * step;
   return step;
 }
+// the two components' columns: z = 2 member + component
+template <class T>
+dim3 s_cols2(const Dom<T>& d, int ty) { return dim3((d.jpi + SX - 1) / SX, (d.jpj + ty - 1) / ty, 2 * d.nmem); }
+// shared memory (dynamic, and a few KB static) beyond the 48 KB default needs the opt-in
+template <class K>
+cudaError_t smem_opt_in(K kern, int bytes) {
+  return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+}
 }  // namespace
 
 template <class T>
 cudaError_t launch_wzv(const Dom<T>& d, const T* un, const T* vn, T* wn, T z1_2dt, cudaStream_t s) {
-  k_wzv<T><<<s_col(d), dim3(SX, SY), 0, s>>>(d, un, vn, wn, z1_2dt);
+  const bool flat = d.e3t_n.s == 0 && d.e3u_n.s == 0 && d.e3v_n.s == 0 && d.e3t_a.s == 0 && d.e3t_b.s == 0;
+  (flat ? k_wzv<T, true> : k_wzv<T, false>)<<<s_col(d), dim3(SX, SY), 0, s>>>(d, un, vn, wn, z1_2dt);
   ktick(NEMO_K_WZV, s);
   return cudaGetLastError();
 }
@@ -40,7 +49,9 @@ cudaError_t launch_dyn_zdf_step(const Dom<T>& d, const T* ub, const T* vb, T* ua
 }
 template <class T>
 cudaError_t launch_dyn_nxt(const Dom<T>& d, const NxtArgs<T, double>& a, cudaStream_t s) {
-  k_dyn_nxt<T, double><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
+  const int smem = 32 * DN_Y * d.jpk * (int)sizeof(T);
+  if (cudaError_t e = smem_opt_in(k_dyn_nxt<T, double>, smem)) return e;
+  k_dyn_nxt<T, double><<<s_cols2<T>(d, DN_Y), dim3(SX, DN_Y), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_NXT, s);
   return cudaGetLastError();
 }
@@ -154,7 +165,11 @@ cudaError_t launch_zdf_mxl(const Dom<T>& d, const MxlArgs<T>& a, cudaStream_t s)
 
 template <class T>
 cudaError_t launch_dyn_zdf_imp(const Dom<T>& d, const DynZdfArgs<T>& a, cudaStream_t s) {
-  k_dyn_zdf_imp<T><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
+  const int smem = 3 * 32 * DZ_Y * d.jpk * (int)sizeof(T);
+  const bool flat = d.e3u_n.s == 0 && d.e3v_n.s == 0 && d.e3w_n.s == 0;
+  const auto kern = flat ? k_dyn_zdf_imp<T, true> : k_dyn_zdf_imp<T, false>;
+  if (cudaError_t e = smem_opt_in(kern, smem)) return e;
+  kern<<<s_cols2<T>(d, DZ_Y), dim3(SX, DZ_Y), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_ZDF_STEP, s);
   return cudaGetLastError();
 }
@@ -188,28 +203,38 @@ cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s
 template <class T>
 cudaError_t launch_dyn_ldf_lap(const Dom<T>& d, const T* ahmt, const T* ahmf, const T* pub, const T* pvb, T* pua, T* pva,
                                T zsign, cudaStream_t s) {
-  k_dyn_ldf_lap<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, ahmt, ahmf, pub, pvb, pua, pva, zsign);
+  const int kch = march_chunk(d);
+  const bool flat = d.e3f_n.s == 0 && d.e3t_b.s == 0 && d.e3u_n.s == 0 && d.e3v_n.s == 0;
+  const dim3 g = march_grid(d, kch, 30, 2);  // a warp writes 30 interior points
+  (flat ? k_dyn_ldf_lap<T, true> : k_dyn_ldf_lap<T, false>)<<<g, dim3(SX, MARCH_Y), 0, s>>>(
+      d, ahmt, ahmf, pub, pvb, pua, pva, zsign, kch);
   ktick(NEMO_K_DYN_LDF, s);
   return cudaGetLastError();
 }
 
 template <class T>
 cudaError_t launch_vor_ene(const Dom<T>& d, int kvor, const T* pun, const T* pvn, T* pua, T* pva, cudaStream_t s) {
-  k_vor_ene<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, kvor, pun, pvn, pua, pva);
+  const int kch = march_chunk(d);
+  (kvor == 1 ? k_vor_ene<T, 1> : kvor == 2 ? k_vor_ene<T, 2> : k_vor_ene<T, 4>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(
+      d, pun, pvn, pua, pva, kch);
   ktick(NEMO_K_DYN_VOR, s);
   return cudaGetLastError();
 }
 
 template <class T>
 cudaError_t launch_dyn_keg(const Dom<T>& d, const T* un, const T* vn, T* ua, T* va, cudaStream_t s) {
-  k_dyn_keg<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, un, vn, ua, va);
+  const int kch = march_chunk(d);
+  k_dyn_keg<T><<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, un, vn, ua, va, kch);
   ktick(NEMO_K_DYN_KEG, s);
   return cudaGetLastError();
 }
 
 template <class T>
 cudaError_t launch_dyn_zad(const Dom<T>& d, const T* un, const T* vn, const T* wn, T* ua, T* va, cudaStream_t s) {
-  k_dyn_zad<T><<<s_col(d), dim3(SX, SY), 0, s>>>(d, un, vn, wn, ua, va);
+  const int kch = march_chunk(d);
+  const bool flat = d.e3u_n.s == 0 && d.e3v_n.s == 0;
+  (flat ? k_dyn_zad<T, true> : k_dyn_zad<T, false>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, un, vn, wn, ua, va,
+                                                                                                 kch);
   ktick(NEMO_K_DYN_ZAD, s);
   return cudaGetLastError();
 }

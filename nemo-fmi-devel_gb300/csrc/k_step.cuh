@@ -11,32 +11,75 @@
 
 namespace nemo {
 
+// one column of a scale-factor field, or the 1-D profile (stride 1)
+template <class T>
+struct E3Col {
+  const T* p;
+  int st;
+  __device__ __forceinline__ E3Col(const E3<T>& e, long ij, int m) : p(e.p.p + m * e.sm + ij * (long)e.s), st((int)e.sk) {}
+  __device__ __forceinline__ T operator()(int k) const { return __ldg(p + (long)(k - 1) * st); }
+};
+// levels that the column kernels below load before they use the first of them
+template <class T>
+constexpr int BATCH = sizeof(T) == 4 ? 8 : 4;
+
 // div_hor (divhor.F90:76-106: the horizontal divergence of the interior, 0 on the
 // closed edges) and wzv (sshwzv.F90:172-189: w integrated up from w(jpk) = 0), one
-// column per thread. The loads of a level do not depend on the running sum, so the
-// unrolled k-loops keep several levels' loads in flight (the column kernels of this
-// file are otherwise bound by one memory round trip per level).
-template <class T>
-__global__ void k_wzv(Dom<T> d, RO<T> un, RO<T> vn, T* wn, T z1_2dt) {
-  ColIdx<T> c = col_index(d);
-  if (!c.valid) return;
-  const int jpi = d.jpi, jpk = d.jpk;
-  const long n2 = d.n2, m3 = (long)c.m * d.n3, ij = c.ij;
-  const ColInfo ci = d.ci[ij];
-  wn[m3 + ij + (long)(jpk - 1) * n2] = T(0);
-  T w = T(0);
-  #pragma unroll 4
-  for (int k = jpk - 1; k >= 1; --k) {
-    const long q = m3 + ij + (long)(k - 1) * n2;
-    const T e3n = d.e3t_n(ij, k, c.m);
-    T hdiv = T(0);
-    if (c.interior)
-      hdiv = (d.e2u[ij] * d.e3u_n(ij, k, c.m) * un[q] - d.e2u[ij - 1] * d.e3u_n(ij - 1, k, c.m) * un[q - 1] +
-              d.e1v[ij] * d.e3v_n(ij, k, c.m) * vn[q] - d.e1v[ij - jpi] * d.e3v_n(ij - jpi, k, c.m) * vn[q - jpi]) *
-             d.r1_e1e2t[ij] / e3n;
-    w = w - (e3n * hdiv + z1_2dt * (d.e3t_a(ij, k, c.m) - d.e3t_b(ij, k, c.m))) * tmsk<T>(ci, k);
-    wn[q] = w;
+// column per thread, the next level loaded ahead of the running sum, which alone links
+// the levels. FLAT: e3t, e3u, e3v are 1-D profiles, kept in shared memory with the
+// reciprocals of e3t. 77 us before at 752x502x31 in FP32 (seven scale-factor loads and an
+// IEEE division a level), 40 us now; 21 us by traffic.
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(128) k_wzv(Dom<T> d, const T* __restrict__ un, const T* __restrict__ vn,
+                                             T* __restrict__ wn, T z1_2dt) {
+  __shared__ E3Prof<T> pt;
+  __shared__ T pu[KMAX + 1], pv[KMAX + 1], pd[KMAX + 1];
+  const ColIdx<T> c = col_index(d);
+  const int jpi = d.jpi, jpk = d.jpk, m = c.m;
+  if constexpr (FLAT) {
+    pt.fill(d.e3t_n, m, jpk);
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= jpk) {
+      pu[k] = d.e3u_n(0, k, m);
+      pv[k] = d.e3v_n(0, k, m);
+      pd[k] = z1_2dt * (d.e3t_a(0, k, m) - d.e3t_b(0, k, m));
+    }
+    __syncthreads();
   }
+  if (!c.valid) return;
+  const long ij = c.ij, n2 = d.n2, c3 = (long)m * d.n3 + ij;
+  const ColInfo ci = d.ci[ij];
+  const int wst = c.interior ? 1 : 0, sst = wst * jpi;  // an edge column reads its own cells alone
+  const T e2u = d.e2u[ij], e2uw = d.e2u[ij - wst], e1v = d.e1v[ij], e1vs = d.e1v[ij - sst], r1 = d.r1_e1e2t[ij];
+  wn[c3 + (long)(jpk - 1) * n2] = T(0);
+  T w = T(0);
+  march<T, 4>(
+      1, jpk - 1,
+      [&](int x, T (&l)[4]) {
+        const long q = c3 + (long)(jpk - 1 - x) * n2;
+        l[0] = __ldg(un + q);
+        l[1] = __ldg(un + q - wst);
+        l[2] = __ldg(vn + q);
+        l[3] = __ldg(vn + q - sst);
+      },
+      [&](int x, T (&l)[4]) {
+        const int k = jpk - x;
+        T hdiv, e3n, de;
+        if constexpr (FLAT) {
+          e3n = pt.e[k];
+          de = pd[k];
+          hdiv = divr((e2u * pu[k] * l[0] - e2uw * pu[k] * l[1] + e1v * pv[k] * l[2] - e1vs * pv[k] * l[3]) * r1, e3n,
+                      pt.r[k]);
+        } else {
+          e3n = d.e3t_n(ij, k, m);
+          de = z1_2dt * (d.e3t_a(ij, k, m) - d.e3t_b(ij, k, m));
+          hdiv = (e2u * d.e3u_n(ij, k, m) * l[0] - e2uw * d.e3u_n(ij - wst, k, m) * l[1] +
+                  e1v * d.e3v_n(ij, k, m) * l[2] - e1vs * d.e3v_n(ij - sst, k, m) * l[3]) * r1 / e3n;
+        }
+        if (!c.interior) hdiv = T(0);
+        w = w - (e3n * hdiv + de) * tmsk<T>(ci, k);
+        wn[c3 + (long)(k - 1) * n2] = w;
+      });
 }
 
 // The time step of dyn_zdf (dynzdf.F90:112) with no vertical viscosity or drag.
@@ -56,175 +99,244 @@ __global__ void k_dyn_zdf_step(Dom<T> d, RO<T> ub, RO<T> vb, T* ua, T* va, T r2d
   }
 }
 
-// The implicit vertical viscosity of one U- (V-) column of dyn_zdf
-// (dynzdf.F90:127-141, :205-302) after its time step: the bottom stress of the
-// barotropic after velocity ab, then the system of avm (iso-level lateral mixing,
-// no adaptive-implicit advection) with the surface condition, the implicit drag on
-// the bottom diagonal and the wind stress in the surface right-hand side, assembled
-// and forward-eliminated in one downward sweep (its diagonals kept in zwd, zws) and
-// back-substituted upwards. The W-point scale factor across the U- (V-) point is the
-// MIN of the neighbouring e3w (the rest state of a linear free surface).
-template <bool U, class T>
-__device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs<T>& a, long ij, int m,
-                                               const ColInfo& ci, T* pa, const double* ab, const T* tau,
-                                               const T* tau_b) {
-  const long n2 = d.n2, m3 = (long)m * d.n3 + ij, p2 = (long)m * d.n2 + ij;
-  const long nb = U ? 1 : d.jpi;
-  const int jpk = d.jpk, kb = U ? ci.mbku : ci.mbkv;
-  auto mk = [&](int k) { return U ? umsk<T>(ci, k) : vmsk<T>(ci, k); };
-  auto e3 = [&](int k) { return U ? d.e3u_n(ij, k, m) : d.e3v_n(ij, k, m); };
-  auto e3xw = [&](int k) { return fmn(d.e3w_n(ij, k, m), d.e3w_n(ij + nb, k, m)); };
-  auto wxm = [&](int k) { return k == 1 ? mk(1) : mk(k) * mk(k - 1); };
-  const T rc = a.rcdu[p2 + nb] + a.rcdu[p2];
-  {
-    const long q = m3 + (long)(kb - 1) * n2;
-    pa[q] = pa[q] + a.r2dt * T(0.5) * rc * (T)ab[p2] / e3(kb);
-  }
-  T wd_p = T(1), ws_p = T(0), x_p = T(0);
-  for (int k = 1; k <= jpk - 1; ++k) {
-    const long q = m3 + (long)(k - 1) * n2;
-    const T ze3a = e3(k);
-    const T zzws = -a.zdt * (a.avm[q + n2 + nb] + a.avm[q + n2]) / (ze3a * e3xw(k + 1)) * wxm(k + 1);
-    T wd, x = pa[q];
-    if (k == 1) {
-      wd = T(1) - zzws;
-      if (k == kb) wd = wd - a.r2dt * T(0.5) * rc / e3(kb);
-      x = x + a.r2dt * T(0.5) * (tau_b[p2] + tau[p2]) / (ze3a * a.rau0) * mk(1);
-    } else {
-      const T zzwi = -a.zdt * (a.avm[q + nb] + a.avm[q]) / (ze3a * e3xw(k)) * wxm(k);
-      wd = T(1) - zzwi - zzws;
-      if (k == kb) wd = wd - a.r2dt * T(0.5) * rc / e3(kb);
-      wd = wd - zzwi * ws_p / wd_p;
-      x = x - zzwi / wd_p * x_p;
+// One U- (V-) column of dyn_zdf (dynzdf.F90:47-499) with the implicit vertical
+// viscosity: the time step and the removal of the barotropic after velocity ab (:112,
+// :122-126), then, on the interior, the bottom stress of ab and the system of avm
+// (:127-141, :205-302; iso-level lateral mixing, no adaptive-implicit advection) with
+// the surface condition, the implicit drag on the bottom diagonal and the wind stress
+// in the surface right-hand side, assembled and forward-eliminated in one downward
+// sweep and back-substituted upwards. The W-point scale factor across the U- (V-) point
+// is the MIN of the neighbouring e3w (the rest state of a linear free surface).
+template <class T>
+struct DynZdfProf {  // 1-D scale factors: e3, and the divisors e3(k) e3w(k+1), e3(k) e3w(k)
+  T e[KMAX + 1], ds[KMAX + 1], rs[KMAX + 1], di[KMAX + 1], ri[KMAX + 1];
+};
+template <bool U, bool FLAT, class T>
+__device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs<T>& a, const ColIdx<T>& c, int nt, T* sx,
+                                               T* sd, T* ss, const DynZdfProf<T>& pf) {
+  constexpr int B = 4;  // levels loaded together
+  const int jpk = d.jpk, K = jpk - 1, m = c.m, n2 = (int)d.n2;
+  const long ij = c.ij, m3 = (long)m * d.n3 + ij, p2 = (long)m * d.n2 + ij;
+  const int nb = U ? 1 : d.jpi;
+  const ColInfo ci = d.ci[ij];
+  const int kb = U ? ci.mbku : ci.mbkv, lo = U ? ci.ulo : ci.vlo, hi = U ? ci.uhi : ci.vhi;
+  T* __restrict__ pa = (U ? a.ua : a.va) + m3;
+  const T* __restrict__ pb = (U ? a.ub : a.vb) + m3;
+  const T ab = (T)(U ? a.ua_b : a.va_b)[p2], r2dt = a.r2dt;
+  auto mk = [&](int k) { return in_range(k, lo, hi) ? T(1) : T(0); };
+  auto stepped = [&](T b, T x, T mu) { return ((b + r2dt * x) * mu - ab) * mu; };
+  if (!c.interior) {
+    for (int k = 1; k <= K; ++k) {
+      const long o = (long)(k - 1) * n2;
+      pa[o] = stepped(pb[o], pa[o], mk(k));
     }
-    a.zwd[q] = wd;
-    a.zws[q] = zzws;
-    pa[q] = x;
-    wd_p = wd; ws_p = zzws; x_p = x;
+    return;
   }
+  const T* __restrict__ av = a.avm + m3 + n2;
+  auto e3 = [&](int k) { return FLAT ? pf.e[k] : (U ? d.e3u_n : d.e3v_n)(ij, k, m); };
+  auto e3xw = [&](int k) { return fmn(d.e3w_n(ij, k, m), d.e3w_n(ij + nb, k, m)); };
+  const T rc = a.rcdu[p2 + nb] + a.rcdu[p2];
+  T rd_p = T(1), wd_p = T(1), ws_p = T(0), x_p = T(0);  // rd = 1 / wd
+  T mk0 = mk(1), s0 = T(0), w0 = T(0), wx0 = T(0);  // of level k: mask; of w-level k: avm sum, e3, mask
+  auto load = [&](int kt, T (&l)[3 * B]) {
+    const long b = (long)(kt - 1) * n2;
+    const T *pbk = pb + b, *avk = av + b, *avn = avk + nb, *pak = pa + b;
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int o = min(y, K - kt) * n2;
+      l[y] = __ldg(pbk + o);
+      l[B + y] = pak[o];
+      l[2 * B + y] = __ldg(avn + o) + __ldg(avk + o);
+    }
+  };
+  auto sweep = [&](int kt, T (&l)[3 * B]) {
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int k = kt + y;
+      if (k > K) break;
+      const T ze3a = e3(k), mk1 = mk(k + 1), wx1 = mk1 * mk0, sv = l[2 * B + y];
+      T x = stepped(l[y], l[B + y], mk0), w1 = T(0), zzws, wd;
+      if constexpr (FLAT) {
+        zzws = divr(-a.zdt * sv, pf.ds[k], pf.rs[k]) * wx1;
+      } else {
+        w1 = e3xw(k + 1);
+        zzws = -a.zdt * sv / (ze3a * w1) * wx1;
+      }
+      if (k == kb) x = x + r2dt * T(0.5) * rc * ab / ze3a;
+      T zzwi = T(0);
+      if (k == 1) {
+        wd = T(1) - zzws;
+        x = x + r2dt * T(0.5) * ((U ? a.utau_b : a.vtau_b)[p2] + (U ? a.utau : a.vtau)[p2]) / (ze3a * a.rau0) * mk0;
+      } else {
+        zzwi = FLAT ? divr(-a.zdt * s0, pf.di[k], pf.ri[k]) * wx0 : -a.zdt * s0 / (ze3a * w0) * wx0;
+        wd = T(1) - zzwi - zzws;
+      }
+      if (k == kb) wd = wd - r2dt * T(0.5) * rc / ze3a;
+      if (k > 1) {
+        wd = wd - divr(zzwi * ws_p, wd_p, rd_p);
+        x = x - divr(zzwi, wd_p, rd_p) * x_p;
+      }
+      const int o = (k - 1) * nt;
+      sd[o] = wd;
+      ss[o] = zzws;
+      sx[o] = x;
+      wd_p = wd; rd_p = T(1) / wd; ws_p = zzws; x_p = x;
+      mk0 = mk1; s0 = sv; w0 = w1; wx0 = wx1;
+    }
+  };
+  T la[3 * B], lb[3 * B];
+  load(1, la);
+  for (int kt = 1; kt <= K; kt += 2 * B) {  // a batch is loaded while the one before it is swept
+    if (kt + B <= K) load(kt + B, lb);
+    sweep(kt, la);
+    if (kt + B > K) break;
+    if (kt + 2 * B <= K) load(kt + 2 * B, la);
+    sweep(kt + B, lb);
+  }
+  if (kb == jpk) pa[(long)(jpk - 1) * n2] = pa[(long)(jpk - 1) * n2] + r2dt * T(0.5) * rc * ab / e3(kb);
   T nxt = T(0);
-  for (int k = jpk - 1; k >= 1; --k) {
-    const long q = m3 + (long)(k - 1) * n2;
-    const T x = (k == jpk - 1) ? pa[q] / a.zwd[q] : (pa[q] - a.zws[q] * nxt) / a.zwd[q];
-    pa[q] = x;
-    nxt = x;
+#pragma unroll 4
+  for (int k = K; k >= 1; --k) {
+    const int o = (k - 1) * nt;
+    nxt = (k == K) ? sx[o] / sd[o] : (sx[o] - ss[o] * nxt) / sd[o];
+    pa[(long)(k - 1) * n2] = nxt;
   }
 }
 
-// dyn_zdf (dynzdf.F90:47-499) with the implicit vertical viscosity, one column per
-// thread: the time step and the removal of the barotropic after velocity on every
-// column (:112, :122-126), then the u and v systems of the interior columns.
-template <class T>
-__global__ void k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<T> a) {
+// dyn_zdf, one U- or V-column per thread (grid z = 2 member + component). The forward
+// values, diagonals and upper diagonals of the column stay in shared memory (3 jpk
+// values a thread), so that ua, va and avm are read once and the result is written
+// once, and four levels are loaded while the four before them are swept; the quotients
+// by scale factors (1-D with FLAT) and by the pivot are divr's. One thread for both
+// components, with the time step as a pass of its own and the diagonals in global
+// memory, took 340 us at 752x502x31 in FP32 (376 MB to move: 55 us).
+constexpr int DZ_Y = 2;
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(32 * DZ_Y) k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char col_smem[];
+  __shared__ DynZdfProf<T> pf;
+  constexpr int nt = 32 * DZ_Y;
+  ColIdx<T> c = col_index(d);
+  c.m = blockIdx.z >> 1;
+  const bool isv = blockIdx.z & 1;
+  if constexpr (FLAT) {
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= d.jpk) {
+      const T e = (isv ? d.e3v_n : d.e3u_n)(0, k, c.m);
+      pf.e[k] = e;
+      pf.ds[k] = e * d.e3w_n(0, min(k + 1, d.jpk), c.m);
+      pf.rs[k] = T(1) / pf.ds[k];
+      pf.di[k] = e * d.e3w_n(0, k, c.m);
+      pf.ri[k] = T(1) / pf.di[k];
+    }
+    __syncthreads();
+  }
+  if (!c.valid) return;
+  T* sx = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x;
+  T *sd = sx + d.jpk * nt, *ss = sd + d.jpk * nt;
+  if (isv) dyn_zdf_column<false, FLAT>(d, a, c, nt, sx, sd, ss, pf);
+  else dyn_zdf_column<true, FLAT>(d, a, c, nt, sx, sd, ss, pf);
+}
+
+// dyn_nxt (dynnxt.F90:114-358; linear free surface, ln_dynspg_ts with ln_bt_fw), one
+// U- or V-column per thread (grid z = 2 member + component): the barotropic part of the
+// after velocity replaced by the sub-steps' ua_b; lbc of ua, va (the closed edges 0);
+// the Euler swap or the Asselin filter and swap with the before velocity returned to
+// the time-split barotropic estimate; the now and before barotropic velocities. The
+// column waits for its sums in shared memory (the after velocity, then the filtered
+// before one), so that memory sees each field read once and written once: 564 MB at
+// 752x502x31 in FP32, 83 us; with the column read back from memory by each of four
+// passes it took 203 us.
+constexpr int DN_Y = 4;
+template <class T, class A>
+__global__ void __launch_bounds__(32 * DN_Y) k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a) {
+  extern __shared__ __align__(16) unsigned char col_smem[];
+  constexpr int nt = 32 * DN_Y, B = BATCH<T>;
+  T* s = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x;
   const ColIdx<T> c = col_index(d);
   if (!c.valid) return;
-  const long n2 = d.n2, m3 = (long)c.m * d.n3 + c.ij, p2 = (long)c.m * d.n2 + c.ij;
-  const ColInfo ci = d.ci[c.ij];
-  const T uab = (T)a.ua_b[p2], vab = (T)a.va_b[p2];
-  for (int k = 1; k <= d.jpk - 1; ++k) {
-    const long q = m3 + (long)(k - 1) * n2;
-    const T um = umsk<T>(ci, k), vm = vmsk<T>(ci, k);
-    a.ua[q] = ((a.ub[q] + a.r2dt * a.ua[q]) * um - uab) * um;
-    a.va[q] = ((a.vb[q] + a.r2dt * a.va[q]) * vm - vab) * vm;
-  }
-  if (!c.interior) return;
-  dyn_zdf_column<true>(d, a, c.ij, c.m, ci, a.ua, a.ua_b, a.utau, a.utau_b);
-  dyn_zdf_column<false>(d, a, c.ij, c.m, ci, a.va, a.va_b, a.vtau, a.vtau_b);
-}
-
-// dyn_nxt (dynnxt.F90:114-358; linear free surface, ln_dynspg_ts with ln_bt_fw),
-// one (i,j) column of u and of v per thread: the barotropic part of the after
-// velocity replaced by the sub-steps' ua_b; lbc of ua, va (the closed edges 0);
-// the Euler swap or the Asselin filter and swap with the before velocity returned
-// to the time-split barotropic estimate; the now and before barotropic velocities.
-template <class T, class A>
-__global__ void k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a) {
-  ColIdx<T> c = col_index(d);
-  if (!c.valid) return;
-  const int jpk = d.jpk;
-  const long n2 = d.n2, m3 = (long)c.m * d.n3, m2 = (long)c.m * n2, ij = c.ij;
+  const int jpk = d.jpk, m = blockIdx.z >> 1, n2 = (int)d.n2;
+  const bool isv = blockIdx.z & 1;
+  const long ij = c.ij, m3 = (long)m * d.n3 + ij, p2 = (long)m * d.n2 + ij;
   const ColInfo ci = d.ci[ij];
-  const T r1u = d.r1_hu_0[ij], r1v = d.r1_hv_0[ij];
-  const T uab = T(a.ua_b[m2 + ij]), vab = T(a.va_b[m2 + ij]);
-  // six distinct arrays: restrict lets the unrolled loops load ahead of the stores
-  T* __restrict__ ua = a.ua + m3;
-  T* __restrict__ va = a.va + m3;
-  T* __restrict__ un = a.un + m3;
-  T* __restrict__ vn = a.vn + m3;
-  T* __restrict__ ub = a.ub + m3;
-  T* __restrict__ vb = a.vb + m3;
-  auto Q = [&](int k) { return ij + (long)(k - 1) * n2; };
+  const int lo = isv ? ci.vlo : ci.ulo, hi = isv ? ci.vhi : ci.uhi;
+  const T r1 = isv ? d.r1_hv_0[ij] : d.r1_hu_0[ij];
+  const T ab = T((isv ? a.va_b : a.ua_b)[p2]);
+  // three distinct arrays: restrict lets a batch's loads go ahead of its stores
+  T* __restrict__ xa = (isv ? a.va : a.ua) + m3;
+  T* __restrict__ xn = (isv ? a.vn : a.un) + m3;
+  T* __restrict__ xb = (isv ? a.vb : a.ub) + m3;
+  const E3Col<T> e3(isv ? d.e3v_n : d.e3u_n, ij, m);
+  auto mk = [&](int k) { return in_range(k, lo, hi) ? T(1) : T(0); };
   // (:114-126)
-  T zue = T(0), zve = T(0);
-  #pragma unroll 4
-  for (int k = 1; k <= jpk - 1; ++k) {
-    const long q = Q(k);
-    zue = zue + d.e3u_n(ij, k, c.m) * ua[q] * umsk<T>(ci, k);
-    zve = zve + d.e3v_n(ij, k, c.m) * va[q] * vmsk<T>(ci, k);
-  }
-  #pragma unroll 4
-  for (int k = 1; k <= jpk - 1; ++k) {
-    const long q = Q(k);
-    ua[q] = (ua[q] - zue * r1u + uab) * umsk<T>(ci, k);
-    va[q] = (va[q] - zve * r1v + vab) * vmsk<T>(ci, k);
-  }
-  if (!c.interior)  // lbc_lnk of ua, va (:146): the closed edges, every level
-    for (int k = 1; k <= jpk; ++k) {
-      ua[Q(k)] = T(0);
-      va[Q(k)] = T(0);
+  T ze = T(0);
+  for (int kt = 1; kt <= jpk - 1; kt += B) {
+    const T* pk = xa + (long)(kt - 1) * n2;
+    T x[B], e[B];
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int z = min(y, jpk - 1 - kt);
+      x[y] = pk[z * n2];
+      e[y] = e3(kt + z);
     }
-  // the now and before barotropic velocities (:345-358) are summed where un and ub
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int k = kt + y;
+      if (k > jpk - 1) break;
+      ze = ze + e[y] * x[y] * mk(k);
+      s[(k - 1) * nt] = x[y];
+    }
+  }
+  // the now and before barotropic velocities (:345-358) are summed where xn and xb
   // take their final values, level by level in the same order
-  T sun = T(0), sub = T(0), svn = T(0), svb = T(0);
-  if (a.euler) {  // (:168-171)
-    #pragma unroll 4
-    for (int k = 1; k <= jpk - 1; ++k) {
-      const long q = Q(k);
-      const T eu = d.e3u_n(ij, k, c.m), ev = d.e3v_n(ij, k, c.m), um = umsk<T>(ci, k), vm = vmsk<T>(ci, k);
-      const T u = ua[q], v = va[q];
-      un[q] = u;
-      vn[q] = v;
-      sun = sun + eu * u * um;
-      sub = sub + eu * ub[q] * um;
-      svn = svn + ev * v * vm;
-      svb = svb + ev * vb[q] * vm;
+  T sn = T(0), sb = T(0), sf = T(0);
+  for (int kt = 1; kt <= jpk - 1; kt += B) {
+    const long b = (long)(kt - 1) * n2;
+    T* __restrict__ pa = xa + b;
+    T* __restrict__ pn = xn + b;
+    const T* pb = xb + b;
+    T vb[B], vn[B], ee[B];
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int z = min(y, jpk - 1 - kt), o = z * n2;
+      vb[y] = pb[o];
+      vn[y] = pn[o];
+      ee[y] = e3(kt + z);
     }
-  } else {  // (:197-211), then (:312-324)
-    T sb = T(0), tb = T(0);
-    #pragma unroll 4
-    for (int k = 1; k <= jpk - 1; ++k) {
-      const long q = Q(k);
-      const T eu = d.e3u_n(ij, k, c.m), ev = d.e3v_n(ij, k, c.m), um = umsk<T>(ci, k), vm = vmsk<T>(ci, k);
-      const T u = ua[q], v = va[q];
-      // FP32: the time laplacian from differences (see k_tra_nxt)
-      const T zuf = un[q] + a.atfp * (sizeof(T) == 4 ? (u - un[q]) - (un[q] - ub[q]) : ub[q] - T(2) * un[q] + u);
-      const T zvf = vn[q] + a.atfp * (sizeof(T) == 4 ? (v - vn[q]) - (vn[q] - vb[q]) : vb[q] - T(2) * vn[q] + v);
-      ub[q] = zuf;
-      vb[q] = zvf;
-      un[q] = u;
-      vn[q] = v;
-      sb = sb + eu * zuf * um;
-      tb = tb + ev * zvf * vm;
-      sun = sun + eu * u * um;
-      svn = svn + ev * v * vm;
-    }
-    const T unb = a.un_b[m2 + ij], vnb = a.vn_b[m2 + ij];
-    #pragma unroll 4
-    for (int k = 1; k <= jpk - 1; ++k) {
-      const long q = Q(k);
-      const T eu = d.e3u_n(ij, k, c.m), ev = d.e3v_n(ij, k, c.m), um = umsk<T>(ci, k), vm = vmsk<T>(ci, k);
-      const T ubk = ub[q] - (sb * r1u - unb) * um;
-      const T vbk = vb[q] - (tb * r1v - vnb) * vm;
-      ub[q] = ubk;
-      vb[q] = vbk;
-      sub = sub + eu * ubk * um;
-      svb = svb + ev * vbk * vm;
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int k = kt + y;
+      if (k > jpk - 1) break;
+      const T e = ee[y], mu = mk(k);
+      // lbc_lnk of ua, va (:146): the closed edges
+      const T u = c.interior ? (s[(k - 1) * nt] - ze * r1 + ab) * mu : T(0);
+      pa[y * n2] = u;
+      pn[y * n2] = u;
+      if (a.euler) {  // (:168-171)
+        sb = sb + e * vb[y] * mu;
+      } else {        // (:197-211); FP32: the time laplacian from differences (see k_tra_nxt)
+        const T zf = vn[y] + a.atfp * (sizeof(T) == 4 ? (u - vn[y]) - (vn[y] - vb[y]) : vb[y] - T(2) * vn[y] + u);
+        s[(k - 1) * nt] = zf;
+        sf = sf + e * zf * mu;
+      }
+      sn = sn + e * u * mu;
     }
   }
-  a.un_b[m2 + ij] = sun * r1u;
-  a.ub_b[m2 + ij] = sub * r1u;
-  a.vn_b[m2 + ij] = svn * r1v;
-  a.vb_b[m2 + ij] = svb * r1v;
+  if (!c.interior) xa[(long)(jpk - 1) * n2] = T(0);
+  if (!a.euler) {  // (:312-324)
+    const T nb = (isv ? a.vn_b : a.un_b)[p2];
+    const T* ps = s;
+    T* pb = xb;
+#pragma unroll 4
+    for (int k = 1; k <= jpk - 1; ++k, ps += nt, pb += n2) {
+      const T e = e3(k), mu = mk(k);
+      const T bk = *ps - (sf * r1 - nb) * mu;
+      *pb = bk;
+      sb = sb + e * bk * mu;
+    }
+  }
+  (isv ? a.vn_b : a.un_b)[p2] = sn * r1;
+  (isv ? a.vb_b : a.ub_b)[p2] = sb * r1;
 }
 
 // ssh_swp (sshwzv.F90:216-267), linear free surface, one point per thread.
@@ -899,27 +1011,57 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_consta
 }
 
 // hpg_zco (dynhpg.F90:258-323), one interior column per thread: the pressure
-// gradient integrated downwards from the surface in registers.
+// gradient integrated downwards from the surface in registers. The levels depend on one
+// another through the running sums alone, so a batch of them is loaded together (the
+// compiler cannot move the load of a trend over the store of the level above): 68 -> 41
+// us at 752x502x31 in FP32 (35 us by traffic).
 template <class T>
-__global__ void k_hpg_zco(Dom<T> d, const T* __restrict__ rhd, T* ua, T* va, T zcoef0) {
+__global__ void __launch_bounds__(128) k_hpg_zco(Dom<T> d, const T* __restrict__ rhd, T* __restrict__ ua,
+                                                 T* __restrict__ va, T zcoef0) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (i < 2 || i > d.jpi - 1 || j < 2 || j > d.jpj - 1) return;
   const int m = blockIdx.z;
   const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi;
   const long c3 = (long)m * d.n3 + ij;
   const T r1u = d.r1_e1u[ij], r1v = d.r1_e2v[ij];
-  T zcoef1 = zcoef0 * d.e3w_n(ij, 1, m);
-  T zhpi = zcoef1 * (rhd[c3 + 1] - rhd[c3]) * r1u;
-  T zhpj = zcoef1 * (rhd[c3 + d.jpi] - rhd[c3]) * r1v;
-  ua[c3] = ua[c3] + zhpi;
-  va[c3] = va[c3] + zhpj;
-  for (int k = 2; k <= d.jpk - 1; ++k) {
-    const long q = c3 + (long)(k - 1) * d.n2, qu = q - d.n2;
-    zcoef1 = zcoef0 * d.e3w_n(ij, k, m);
-    zhpi = zhpi + zcoef1 * ((rhd[q + 1] + rhd[qu + 1]) - (rhd[q] + rhd[qu])) * r1u;
-    zhpj = zhpj + zcoef1 * ((rhd[q + d.jpi] + rhd[qu + d.jpi]) - (rhd[q] + rhd[qu])) * r1v;
-    ua[q] = ua[q] + zhpi;
-    va[q] = va[q] + zhpj;
+  const int n2 = (int)d.n2;
+  const E3Col<T> e3w(d.e3w_n, ij, m);
+  T re = T(0), rn = T(0), r0 = T(0), zhpi = T(0), zhpj = T(0);
+  constexpr int U = BATCH<T>;
+  for (int kt = 1; kt <= d.jpk - 1; kt += U) {
+    const long b = c3 + (long)(kt - 1) * n2;
+    const T *pr = rhd + b, *prn = pr + d.jpi;
+    T* __restrict__ pu = ua + b;
+    T* __restrict__ pv = va + b;
+    T s0[U], se[U], sn[U], a0[U], a1[U], ew[U];
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+      const int z = min(x, d.jpk - 1 - kt), q = z * n2;
+      s0[x] = __ldg(pr + q);
+      se[x] = __ldg(pr + q + 1);
+      sn[x] = __ldg(prn + q);
+      a0[x] = pu[q];
+      a1[x] = pv[q];
+      ew[x] = e3w(kt + z);
+    }
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+      const int k = kt + x;
+      if (k > d.jpk - 1) break;
+      const T zcoef1 = zcoef0 * ew[x];
+      if (k == 1) {
+        zhpi = zcoef1 * (se[x] - s0[x]) * r1u;
+        zhpj = zcoef1 * (sn[x] - s0[x]) * r1v;
+      } else {
+        zhpi = zhpi + zcoef1 * ((se[x] + re) - (s0[x] + r0)) * r1u;
+        zhpj = zhpj + zcoef1 * ((sn[x] + rn) - (s0[x] + r0)) * r1v;
+      }
+      pu[x * n2] = a0[x] + zhpi;
+      pv[x * n2] = a1[x] + zhpj;
+      r0 = s0[x];
+      re = se[x];
+      rn = sn[x];
+    }
   }
 }
 
@@ -954,125 +1096,240 @@ __global__ void k_zdf_mxl(Dom<T> d, MxlArgs<T> a) {
   a.hmlpt[c2] = a.gdept[c3 + (long)(nmln - 2) * d.n2] * ssm;
 }
 
-// dyn_ldf_lap (dynldf_lap_blp.F90:37-104), linear free surface (e3*_b = e3*_n),
-// one (i,j,k) point per thread: -curl(curl) + grad(div) of the before velocity.
-// The relative vorticity zcur and divergence zdiv a point needs (three of each) are
-// formed where read, each with the reference's expression.
-template <class T>
-struct LdfDyn {
-  const Dom<T>& d;
-  const T *ahmt, *ahmf, *pub, *pvb;
-  long m3;
-  int k, m;
-  __device__ __forceinline__ long P(int i, int j) const { return (long)(i - 1) + (long)(j - 1) * d.jpi; }
-  __device__ __forceinline__ T cur(int a, int b) const {
-    const long p = P(a, b), q = m3 + p + (long)(k - 1) * d.n2;
-    return a_(ahmf, q) * d.e3f_n(p, k, m) * d.r1_e1e2f[p] *
-           (d.e2v[p + 1] * a_(pvb, q + 1) - d.e2v[p] * a_(pvb, q) - d.e1u[p + d.jpi] * a_(pub, q + d.jpi) +
-            d.e1u[p] * a_(pub, q));
+// ---------------------------------------------------------- momentum trends
+// dyn_ldf_lap, vor_ene, dyn_keg and dyn_zad: a thread owns one (i,j) and marches down a
+// chunk of levels. Each reads two or three 3-D fields at the point and its neighbours
+// and updates ua and va, so memory bounds them once the instructions are few enough and
+// a warp has its next level's loads in flight while it works on this one:
+// * the 2-D metrics of the stencil (26 in vor_ene) are loaded once a chunk instead of
+//   once a point;
+// * level k + 1 is loaded before level k is computed and stored (the compiler cannot
+//   move the load of a trend over the store of the level above);
+// * quotients by what a chunk shares (the e1, e2 of the column; with 1-D scale factors,
+//   FLAT, the e3 of the level, whose reciprocals the block forms once) are divr's.
+// One point a thread, they took 248, 150 and 73 us and, one column a thread, dyn_zad
+// 191 us at 752x502x31 in FP32; so they take 107, 65, 61 and 65 us (floors by traffic:
+// 56, 42, 42 and 49 us; the rest is instruction issue and the latency left).
+// dyn_ldf_lap (dynldf_lap_blp.F90:37-104), linear free surface (e3*_b = e3*_n):
+// -curl(curl) + grad(div) of the before velocity, each relative vorticity zcur and
+// divergence zdiv by the reference's expression. A warp covers 32 points of a row and
+// writes the inner 30: zcur of the western and zdiv of the eastern point come from the
+// neighbour lane, so that a point forms two of each instead of three.
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(32 * MARCH_Y) k_dyn_ldf_lap(Dom<T> d, const T* __restrict__ ahmt,
+                                                              const T* __restrict__ ahmf, const T* __restrict__ pub,
+                                                              const T* __restrict__ pvb, T* __restrict__ pua,
+                                                              T* __restrict__ pva, T zsign, int kch) {
+  __shared__ E3Prof<T> pt, pu, pv;
+  __shared__ T pf[KMAX + 1];
+  const MarchIdx c = march_index(d, kch, 30);
+  const int j = c.j, J = d.jpi;
+  if constexpr (FLAT) {
+    pt.fill(d.e3t_b, c.m, d.jpk);
+    pu.fill(d.e3u_n, c.m, d.jpk);
+    pv.fill(d.e3v_n, c.m, d.jpk);
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= d.jpk) pf[k] = d.e3f_n(0, k, c.m);
+    __syncthreads();
   }
-  __device__ __forceinline__ T div(int a, int b) const {
-    const long p = P(a, b), q = m3 + p + (long)(k - 1) * d.n2;
-    return a_(ahmt, q) * d.r1_e1e2t[p] / d.e3t_b(p, k, m) *
-           (d.e2u[p] * d.e3u_n(p, k, m) * a_(pub, q) - d.e2u[p - 1] * d.e3u_n(p - 1, k, m) * a_(pub, q - 1) +
-            d.e1v[p] * d.e3v_n(p, k, m) * a_(pvb, q) - d.e1v[p - d.jpi] * d.e3v_n(p - d.jpi, k, m) * a_(pvb, q - d.jpi));
-  }
-  __device__ __forceinline__ static T a_(const T* x, long q) { return __ldg(x + q); }
-};
-
-template <class T>
-__global__ void k_dyn_ldf_lap(Dom<T> d, const T* __restrict__ ahmt, const T* __restrict__ ahmf,
-                              const T* __restrict__ pub, const T* __restrict__ pvb, T* pua, T* pva, T zsign) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || c.k > d.jpk - 1 || c.i < 2 || c.i > d.jpi - 1 || c.j < 2 || c.j > d.jpj - 1) return;
-  const LdfDyn<T> L{d, ahmt, ahmf, pub, pvb, (long)c.m * d.n3, c.k, c.m};
-  const int i = c.i, j = c.j;
-  const long q = (long)c.m * d.n3 + c.q;
-  const T zc = L.cur(i, j), zd = L.div(i, j);
-  pua[q] = pua[q] + zsign * (-((zc - L.cur(i, j - 1)) * d.r1_e2u[c.ij] / d.e3u_n(c.ij, c.k, c.m)) +
-                             (L.div(i + 1, j) - zd) * d.r1_e1u[c.ij]);
-  pva[q] = pva[q] + zsign * ((zc - L.cur(i - 1, j)) * d.r1_e1v[c.ij] / d.e3v_n(c.ij, c.k, c.m) +
-                             (L.div(i, j + 1) - zd) * d.r1_e2v[c.ij]);
+  if (j < 2 || j > d.jpj - 1) return;  // whole warps
+  // lanes outside 2..jpi-1 feed their neighbours: zcur at i = 1, zdiv at i = jpi
+  const bool cu = c.i <= J - 1, dv = c.i >= 2 && c.i <= J;
+  const bool out = cu && dv && threadIdx.x >= 1 && threadIdx.x <= 30;
+  const long p = (long)(min(c.i, J) - 1) + (long)(j - 1) * J;
+  const int e = cu ? 1 : 0, w = dv ? 1 : 0;  // offsets that stay in the row
+  // metrics of the f-points p, p-J and of the t-points p, p+J
+  const T rf0 = d.r1_e1e2f[p], rfs = d.r1_e1e2f[p - J];
+  const T v0 = d.e2v[p], ve = d.e2v[p + e], vs = d.e2v[p - J], vse = d.e2v[p - J + e];
+  const T u0 = d.e1u[p], un = d.e1u[p + J], us = d.e1u[p - J];
+  const T rt0 = d.r1_e1e2t[p], rtn = d.r1_e1e2t[p + J];
+  const T x0 = d.e2u[p], xw = d.e2u[p - w], xn = d.e2u[p + J], xnw = d.e2u[p + J - w];
+  const T y0 = d.e1v[p], ys = d.e1v[p - J], yn = d.e1v[p + J];
+  const T r2u = d.r1_e2u[p], r1u = d.r1_e1u[p], r1v = d.r1_e1v[p], r2v = d.r1_e2v[p];
+  const long o = (long)c.m * d.n3 + p;
+  march<T, 16>(
+      c.k0, c.k1,
+      [&](int k, T (&l)[16]) {
+        const long q = o + (long)(k - 1) * d.n2;
+        const T *u = pub + q, *v = pvb + q, *hf = ahmf + q, *ht = ahmt + q;
+        l[0] = __ldg(u); l[1] = __ldg(u - w); l[2] = __ldg(u + J); l[3] = __ldg(u - J); l[4] = __ldg(u + J - w);
+        l[5] = __ldg(v); l[6] = __ldg(v + e); l[7] = __ldg(v - J); l[8] = __ldg(v - J + e); l[9] = __ldg(v + J);
+        l[10] = __ldg(hf); l[11] = __ldg(hf - J); l[12] = __ldg(ht); l[13] = __ldg(ht + J);
+        l[14] = pua[q]; l[15] = pva[q];
+      },
+      [&](int k, T (&l)[16]) {
+        T eu, ev, euw, eun, eunw, evs, evn, ef, efs;
+        if constexpr (FLAT) {
+          eu = euw = eun = eunw = pu.e[k];
+          ev = evs = evn = pv.e[k];
+          ef = efs = pf[k];
+        } else {
+          eu = d.e3u_n(p, k, c.m); euw = d.e3u_n(p - w, k, c.m);
+          eun = d.e3u_n(p + J, k, c.m); eunw = d.e3u_n(p + J - w, k, c.m);
+          ev = d.e3v_n(p, k, c.m); evs = d.e3v_n(p - J, k, c.m); evn = d.e3v_n(p + J, k, c.m);
+          ef = d.e3f_n(p, k, c.m); efs = d.e3f_n(p - J, k, c.m);
+        }
+        auto over_t = [&](T x, long r) { return FLAT ? divr(x, pt.e[k], pt.r[k]) : x / d.e3t_b(r, k, c.m); };
+        auto over_u = [&](T x) { return FLAT ? divr(x, eu, pu.r[k]) : x / eu; };
+        auto over_v = [&](T x) { return FLAT ? divr(x, ev, pv.r[k]) : x / ev; };
+        const T b0 = l[0], c0 = l[5];
+        const T cur0 = l[10] * ef * rf0 * (ve * l[6] - v0 * c0 - un * l[2] + u0 * b0);
+        const T curs = l[11] * efs * rfs * (vse * l[8] - vs * l[7] - u0 * b0 + us * l[3]);
+        const T h0 = y0 * ev * c0;
+        const T div0 = over_t(l[12] * rt0, p) * (x0 * eu * b0 - xw * euw * l[1] + h0 - ys * evs * l[7]);
+        const T divn = over_t(l[13] * rtn, p + J) * (xn * eun * l[2] - xnw * eunw * l[4] + yn * evn * l[9] - h0);
+        const T curw = __shfl_up_sync(0xffffffffu, cur0, 1), dive = __shfl_down_sync(0xffffffffu, div0, 1);
+        if (out) {
+          const long q = o + (long)(k - 1) * d.n2;
+          pua[q] = l[14] + zsign * (-over_u((cur0 - curs) * r2u) + (dive - div0) * r1u);
+          pva[q] = l[15] + zsign * (over_v((cur0 - curw) * r1v) + (divn - div0) * r2v);
+        }
+      });
 }
 
-// vor_ene (dynvor.F90:324-429), z-coordinate without ln_dynvor_msk, one (i,j,k)
-// point per thread; the vorticities zwz and transports zwx, zwy of the four
-// surrounding points are formed where read, each with the reference's expression.
-template <class T>
-__global__ void k_vor_ene(Dom<T> d, int kvor, const T* __restrict__ pun, const T* __restrict__ pvn, T* pua,
-                          T* pva) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || c.k > d.jpk - 1 || c.i < 2 || c.i > d.jpi - 1 || c.j < 2 || c.j > d.jpj - 1) return;
-  const long o = (long)c.m * d.n3 + (long)(c.k - 1) * d.n2;  // this level of this member
-  const long J = d.jpi;
-  auto zwz = [&](long p) -> T {
-    if (kvor == 1) return d.ff_f[p];
-    const T rv = (d.e2v[p + 1] * __ldg(pvn + o + p + 1) - d.e2v[p] * __ldg(pvn + o + p) -
-                  d.e1u[p + J] * __ldg(pun + o + p + J) + d.e1u[p] * __ldg(pun + o + p)) *
-                 d.r1_e1e2f[p];
-    if (kvor == 2) return rv;
-    return d.ff_f[p] + (d.e2v[p + 1] * __ldg(pvn + o + p + 1) - d.e2v[p] * __ldg(pvn + o + p) -
-                        d.e1u[p + J] * __ldg(pun + o + p + J) + d.e1u[p] * __ldg(pun + o + p)) *
-                           d.r1_e1e2f[p];
-  };
-  auto zwx = [&](long p) -> T { return d.e2u[p] * __ldg(pun + o + p); };
-  auto zwy = [&](long p) -> T { return d.e1v[p] * __ldg(pvn + o + p); };
-  const long p = c.ij, q = o + p;
-  const T zy1 = zwy(p - J) + zwy(p + 1 - J);
-  const T zy2 = zwy(p) + zwy(p + 1);
-  const T zx1 = zwx(p - 1) + zwx(p - 1 + J);
-  const T zx2 = zwx(p) + zwx(p + J);
-  const T zc = zwz(p);
-  pua[q] = pua[q] + T(0.25) * d.r1_e1u[p] * (zwz(p - J) * zy1 + zc * zy2);
-  pva[q] = pva[q] - T(0.25) * d.r1_e2v[p] * (zwz(p - 1) * zx1 + zc * zx2);
+// vor_ene (dynvor.F90:324-429), z-coordinate without ln_dynvor_msk; KV: the vorticity
+// (1 planetary, 2 relative, 4 total). The vorticities zwz and transports zwx, zwy of
+// the four surrounding points are formed where read, each with the reference's
+// expression.
+template <class T, int KV>
+__global__ void __launch_bounds__(32 * MARCH_Y) k_vor_ene(Dom<T> d, const T* __restrict__ pun, const T* __restrict__ pvn,
+                                                          T* __restrict__ pua, T* __restrict__ pva, int kch) {
+  const MarchIdx c = march_index(d, kch);
+  if (!c.inner) return;
+  const int J = d.jpi;
+  const long p = c.ij;
+  // metrics of the f-points p, s = p-J, w = p-1 (KV 1 reads ff_f alone)
+  T f0 = T(0), fs = T(0), fw = T(0), rf0 = T(0), rfs = T(0), rfw = T(0);
+  T v0 = T(0), ve = T(0), vs = T(0), vse = T(0), vw = T(0), u0 = T(0), un = T(0), us = T(0), uw = T(0), unw = T(0);
+  if constexpr (KV != 2) {
+    f0 = d.ff_f[p]; fs = d.ff_f[p - J]; fw = d.ff_f[p - 1];
+  }
+  if constexpr (KV != 1) {
+    rf0 = d.r1_e1e2f[p]; rfs = d.r1_e1e2f[p - J]; rfw = d.r1_e1e2f[p - 1];
+    v0 = d.e2v[p]; ve = d.e2v[p + 1]; vs = d.e2v[p - J]; vse = d.e2v[p - J + 1]; vw = d.e2v[p - 1];
+    u0 = d.e1u[p]; un = d.e1u[p + J]; us = d.e1u[p - J]; uw = d.e1u[p - 1]; unw = d.e1u[p - 1 + J];
+  }
+  const T x0 = d.e2u[p], xw = d.e2u[p - 1], xn = d.e2u[p + J], xnw = d.e2u[p - 1 + J];
+  const T y0 = d.e1v[p], ys = d.e1v[p - J], ye = d.e1v[p + 1], yse = d.e1v[p + 1 - J];
+  const T ru = T(0.25) * d.r1_e1u[p], rv = T(0.25) * d.r1_e2v[p];
+  auto zwz = [&](T ff, T rf, T rot) -> T { return KV == 1 ? ff : KV == 2 ? rot * rf : ff + rot * rf; };
+  const long o = (long)c.m * d.n3 + p;
+  march<T, 12>(
+      c.k0, c.k1,
+      [&](int k, T (&l)[12]) {
+        const long q = o + (long)(k - 1) * d.n2;
+        const T *u = pun + q, *v = pvn + q;
+        l[0] = __ldg(u); l[1] = __ldg(u - 1); l[2] = __ldg(u + J); l[3] = __ldg(u - 1 + J);
+        l[4] = KV == 1 ? T(0) : __ldg(u - J);
+        l[5] = __ldg(v); l[6] = __ldg(v + 1); l[7] = __ldg(v - J); l[8] = __ldg(v + 1 - J);
+        l[9] = KV == 1 ? T(0) : __ldg(v - 1);
+        l[10] = pua[q]; l[11] = pva[q];
+      },
+      [&](int k, T (&l)[12]) {
+        const T b0 = l[0], bw = l[1], bn = l[2], bnw = l[3], bs = l[4];
+        const T c0 = l[5], ce = l[6], cs = l[7], cse = l[8], cw = l[9];
+        const T zy1 = ys * cs + yse * cse;
+        const T zy2 = y0 * c0 + ye * ce;
+        const T zx1 = xw * bw + xnw * bnw;
+        const T zx2 = x0 * b0 + xn * bn;
+        const T zc = zwz(f0, rf0, ve * ce - v0 * c0 - un * bn + u0 * b0);
+        const T zs = zwz(fs, rfs, vse * cse - vs * cs - u0 * b0 + us * bs);
+        const T zw = zwz(fw, rfw, v0 * c0 - vw * cw - unw * bnw + uw * bw);
+        const long q = o + (long)(k - 1) * d.n2;
+        pua[q] = l[10] + ru * (zs * zy1 + zc * zy2);
+        pva[q] = l[11] - rv * (zw * zx1 + zc * zx2);
+      });
 }
 
-// dyn_keg (dynkeg.F90, nkeg_C2), one (i,j,k) interior point per thread: the kinetic
-// energy of the point and of its east / north neighbours formed where read.
+// dyn_keg (dynkeg.F90, nkeg_C2): the kinetic energy of the point and of its east /
+// north neighbours formed where read.
 template <class T>
-__global__ void k_dyn_keg(Dom<T> d, const T* __restrict__ un, const T* __restrict__ vn, T* ua, T* va) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || c.k > d.jpk - 1 || c.i < 2 || c.i > d.jpi - 1 || c.j < 2 || c.j > d.jpj - 1) return;
-  const long q = (long)c.m * d.n3 + c.q, J = d.jpi;
-  auto hke = [&](long r) -> T {
-    const T u0 = __ldg(un + r - 1), u1 = __ldg(un + r), v0 = __ldg(vn + r - J), v1 = __ldg(vn + r);
+__global__ void __launch_bounds__(32 * MARCH_Y) k_dyn_keg(Dom<T> d, const T* __restrict__ un, const T* __restrict__ vn,
+                                                          T* __restrict__ ua, T* __restrict__ va, int kch) {
+  const MarchIdx c = march_index(d, kch);
+  if (!c.inner) return;
+  const int J = d.jpi;
+  const T e1u = d.e1u[c.ij], e2v = d.e2v[c.ij], re1u = T(1) / e1u, re2v = T(1) / e2v;
+  auto hke = [](T u0, T u1, T v0, T v1) -> T {
     const T zu = u0 * u0 + u1 * u1;
     const T zv = v0 * v0 + v1 * v1;
     return T(0.25) * (zv + zu);
   };
-  const T h = hke(q);
-  ua[q] = ua[q] - (hke(q + 1) - h) / d.e1u[c.ij];
-  va[q] = va[q] - (hke(q + J) - h) / d.e2v[c.ij];
+  const long o = (long)c.m * d.n3 + c.ij;
+  march<T, 12>(
+      c.k0, c.k1,
+      [&](int k, T (&l)[12]) {
+        const long q = o + (long)(k - 1) * d.n2;
+        const T *u = un + q, *v = vn + q;
+        l[0] = __ldg(u); l[1] = __ldg(u - 1); l[2] = __ldg(u + 1); l[3] = __ldg(u + J); l[4] = __ldg(u - 1 + J);
+        l[5] = __ldg(v); l[6] = __ldg(v - J); l[7] = __ldg(v + 1); l[8] = __ldg(v + 1 - J); l[9] = __ldg(v + J);
+        l[10] = ua[q]; l[11] = va[q];
+      },
+      [&](int k, T (&l)[12]) {
+        const T b0 = l[0], bw = l[1], be = l[2], bn = l[3], bnw = l[4];
+        const T c0 = l[5], cs = l[6], ce = l[7], cse = l[8], cn = l[9];
+        const T h = hke(bw, b0, cs, c0);
+        const long q = o + (long)(k - 1) * d.n2;
+        ua[q] = l[10] - divr(hke(b0, be, cse, ce) - h, e1u, re1u);
+        va[q] = l[11] - divr(hke(bnw, bn, c0, cn) - h, e2v, re2v);
+      });
 }
 
-// dyn_zad (dynzad.F90), one interior column per thread: the w-level momentum fluxes
-// of the column carried down, each formed once.
-template <class T>
-__global__ void k_dyn_zad(Dom<T> d, const T* __restrict__ un, const T* __restrict__ vn, const T* __restrict__ wn,
-                          T* ua, T* va) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i < 2 || i > d.jpi - 1 || j < 2 || j > d.jpj - 1) return;
-  const int m = blockIdx.z;
-  const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi, J = d.jpi;
-  const long c3 = (long)m * d.n3 + ij;
-  const T e0 = d.e1e2t[ij], e1 = d.e1e2t[ij + 1], e2 = d.e1e2t[ij + J];
-  const T r1u = d.r1_e1e2u[ij], r1v = d.r1_e1e2v[ij];
-  T wu = T(0), wv = T(0);  // zwuw, zwvw at the top of level k
-  for (int k = 1; k <= d.jpk - 1; ++k) {
-    const long q = c3 + (long)(k - 1) * d.n2;
-    T wu1 = T(0), wv1 = T(0);  // at its bottom (w-level k+1), 0 at jpk
-    if (k + 1 <= d.jpk - 1) {
-      const long qb = q + d.n2;
-      const T z0 = T(0.25) * e0 * __ldg(wn + qb), zi = T(0.25) * e1 * __ldg(wn + qb + 1),
-              zj = T(0.25) * e2 * __ldg(wn + qb + J);
-      wu1 = (zi + z0) * (__ldg(un + q) - __ldg(un + qb));
-      wv1 = (zj + z0) * (__ldg(vn + q) - __ldg(vn + qb));
-    }
-    ua[q] = ua[q] - (wu + wu1) * r1u / d.e3u_n(ij, k, m);
-    va[q] = va[q] - (wv + wv1) * r1v / d.e3v_n(ij, k, m);
-    wu = wu1;
-    wv = wv1;
+// dyn_zad (dynzad.F90): the w-level momentum fluxes of the column carried down, each
+// formed once (the one at the top of a chunk by both its chunks).
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(32 * MARCH_Y) k_dyn_zad(Dom<T> d, const T* __restrict__ un, const T* __restrict__ vn,
+                                                          const T* __restrict__ wn, T* __restrict__ ua,
+                                                          T* __restrict__ va, int kch) {
+  __shared__ E3Prof<T> pu, pv;
+  const MarchIdx c = march_index(d, kch);
+  const int m = c.m, J = d.jpi, K = d.jpk - 1;
+  if constexpr (FLAT) {
+    pu.fill(d.e3u_n, m, d.jpk);
+    pv.fill(d.e3v_n, m, d.jpk);
+    __syncthreads();
   }
+  if (!c.inner) return;
+  const long ij = c.ij, n2 = d.n2, c3 = (long)m * d.n3 + ij;
+  const T e0 = T(0.25) * d.e1e2t[ij], e1 = T(0.25) * d.e1e2t[ij + 1], e2 = T(0.25) * d.e1e2t[ij + J];
+  const T r1u = d.r1_e1e2u[ij], r1v = d.r1_e1e2v[ij];
+  const long q0 = c3 + (long)(c.k0 - 1) * n2;
+  T wu = T(0), wv = T(0);  // zwuw, zwvw at the top of level k
+  T u0 = __ldg(un + q0), v0 = __ldg(vn + q0);
+  if (c.k0 > 1) {
+    const T z0 = e0 * __ldg(wn + q0), zi = e1 * __ldg(wn + q0 + 1), zj = e2 * __ldg(wn + q0 + J);
+    wu = (zi + z0) * (__ldg(un + q0 - n2) - u0);
+    wv = (zj + z0) * (__ldg(vn + q0 - n2) - v0);
+  }
+  march<T, 7>(
+      c.k0, c.k1,
+      [&](int k, T (&l)[7]) {  // wn, un, vn of the level below; ua, va
+        const long q = c3 + (long)(k - 1) * n2, qb = k < K ? q + n2 : q;
+        l[0] = __ldg(wn + qb); l[1] = __ldg(wn + qb + 1); l[2] = __ldg(wn + qb + J);
+        l[3] = __ldg(un + qb); l[4] = __ldg(vn + qb);
+        l[5] = ua[q]; l[6] = va[q];
+      },
+      [&](int k, T (&l)[7]) {
+        T wu1 = T(0), wv1 = T(0);  // at its bottom (w-level k+1), 0 at jpk
+        if (k < K) {
+          const T z0 = e0 * l[0], zi = e1 * l[1], zj = e2 * l[2];
+          wu1 = (zi + z0) * (u0 - l[3]);
+          wv1 = (zj + z0) * (v0 - l[4]);
+        }
+        u0 = l[3];
+        v0 = l[4];
+        const T tu = (wu + wu1) * r1u, tv = (wv + wv1) * r1v;
+        const long q = c3 + (long)(k - 1) * n2;
+        if constexpr (FLAT) {
+          ua[q] = l[5] - divr(tu, pu.e[k], pu.r[k]);
+          va[q] = l[6] - divr(tv, pv.e[k], pv.r[k]);
+        } else {
+          ua[q] = l[5] - tu / d.e3u_n(ij, k, m);
+          va[q] = l[6] - tv / d.e3v_n(ij, k, m);
+        }
+        wu = wu1;
+        wv = wv1;
+      });
 }
 
 // ---------------------------------------------------------------- usrdef_sbc (GYRE)

@@ -88,6 +88,67 @@ __device__ __forceinline__ KIdx k_index(const Dom<T>& d) {
   return c;
 }
 
+// Level-march kernels: grid x = i, y = j, z = member * nchunk + chunk; a thread walks the
+// levels of a chunk of 1..jpk-1 and loads level k + 1 before it computes and stores
+// level k (the compiler cannot move a load over a store that may alias it).
+constexpr int MARCH_Y = 4;
+struct MarchIdx {
+  int i, j, m, k0, k1;
+  long ij;
+  bool inner;
+};
+template <class T>
+__device__ __forceinline__ MarchIdx march_index(const Dom<T>& d, int kch, int width = 32) {
+  const int nch = (d.jpk - 1 + kch - 1) / kch;
+  MarchIdx c;
+  c.i = blockIdx.x * width + threadIdx.x + 1;
+  c.j = blockIdx.y * MARCH_Y + threadIdx.y + 1;
+  c.m = (int)(blockIdx.z / (unsigned)nch);
+  c.k0 = ((int)blockIdx.z - c.m * nch) * kch + 1;
+  c.k1 = min(c.k0 + kch - 1, d.jpk - 1);
+  c.ij = (long)(c.i - 1) + (long)(c.j - 1) * d.jpi;
+  c.inner = c.i >= 2 && c.i <= d.jpi - 1 && c.j >= 2 && c.j <= d.jpj - 1;
+  return c;
+}
+// Levels a thread walks: 32, 16, .. 1, the most that still gives every SM its resident
+// warps (64 of 32 points).
+template <class T>
+inline int march_chunk(const Dom<T>& d) {
+  int f = 32;
+  while (f > 1 && (long)d.n2 * d.nmem * ((d.jpk - 1 + f - 1) / f) < 152L * 64 * 32) f /= 2;
+  return f;
+}
+template <class T>
+inline dim3 march_grid(const Dom<T>& d, int kch, int width = 32, int edge = 0) {
+  return dim3((d.jpi - edge + width - 1) / width, (d.jpj + MARCH_Y - 1) / MARCH_Y, d.nmem * ((d.jpk - 1 + kch - 1) / kch));
+}
+// load(k, buffer) a level ahead of compute(k, buffer), for the levels k0..k1
+template <class T, int N, class L, class C>
+__device__ __forceinline__ void march(int k0, int k1, L load, C compute) {
+  T a[N], b[N];
+  load(k0, a);
+  for (int k = k0; k <= k1; k += 2) {
+    if (k + 1 <= k1) load(k + 1, b);
+    compute(k, a);
+    if (k + 1 > k1) break;
+    if (k + 2 <= k1) load(k + 2, a);
+    compute(k + 1, b);
+  }
+}
+// The 1-D profile of a scale factor and its reciprocals, for the levels of a block (one
+// thread a level; the caller synchronises).
+template <class T>
+struct E3Prof {
+  T e[KMAX + 1], r[KMAX + 1];
+  __device__ __forceinline__ void fill(const E3<T>& f, int m, int jpk) {
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= jpk) {
+      e[k] = f(0, k, m);
+      r[k] = T(1) / e[k];
+    }
+  }
+};
+
 // --------------------------------------------------------------------------------
 // traadv.F90:99-124: zun = e2u*e3u_n*un, zvn = e1v*e3v_n*vn, zwn = e1e2t*wn, 0 at jpk.
 template <class T>
@@ -226,6 +287,19 @@ __device__ __forceinline__ T divq(T x, T y, T ry) {
   }
 }
 
+// x / y given ry = 1 / y correctly rounded: divq's correction, in both precisions and
+// without a branch (three multiply-adds instead of the division's dozen instructions);
+// a quotient that is not finite is that of x ry. Exact for |x| > 2^-100 (2^-960).
+template <class T>
+__device__ __forceinline__ T divr(T x, T y, T ry) {
+  if constexpr (sizeof(T) == 8) {
+    const T q = __dmul_rn(x, ry);
+    return isfinite(q) ? __fma_rn(__fma_rn(-q, y, x), ry, q) : q;
+  } else {
+    const T q = __fmul_rn(x, ry);
+    return isfinite(q) ? __fmaf_rn(__fmaf_rn(-q, y, x), ry, q) : q;
+  }
+}
 // Upstream flux 0.5 * ((u + |u|) * tl + (u - |u|) * tr) (traadv_fct.F90:126-136):
 // exactly u * tl for u > 0 and u * tr for u < 0 (the doubled product scales exactly
 // and the other term is an exact 0), formed as one product of the selected value.

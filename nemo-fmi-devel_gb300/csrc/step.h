@@ -96,13 +96,12 @@ struct MxlArgs {
 
 // dyn_zdf with the implicit vertical viscosity: the ocean avm, the bottom drag
 // rcdu (2-D), the wind stress (utau_b may be utau), the barotropic after velocity of
-// dyn_spg_ts (FP64 in both precisions); work: the diagonal and upper diagonal of the
-// system, n3 per member each (u and v in turn)
+// dyn_spg_ts (FP64 in both precisions)
 template <class T>
 struct DynZdfArgs {
   const T *ub, *vb, *avm, *rcdu, *utau, *vtau, *utau_b, *vtau_b;
   const double *ua_b, *va_b;
-  T *ua, *va, *zwd, *zws;
+  T *ua, *va;
   T r2dt, zdt, rau0;
 };
 

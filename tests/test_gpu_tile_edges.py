@@ -5,7 +5,8 @@ import pytest
 
 import adj_cases
 from adj_cases import Case, GpuCase
-from harness import relerr
+from nemo_gpu import gyre
+from harness import Pair, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,53 @@ def test_tracer_adjoints(monkeypatch, jpi, jpj, jpk):
     c.o.tra_zdf_imp_adj(kt, c.kit, "TRA", c.p2dt, rtb, rta, 2)
     g.ctx.tra_zdf_imp_adj(kt, c.kit, "TRA", c.p2dt, tb_ad, ta_ad, 2)
     assert relerr(rtb, g.host(tb_ad, c.s4)[0]) <= tol and relerr(rta, g.host(ta_ad, c.s4)[0]) <= tol
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nn,jpk,flat", [(2, 9, True), (8, 18, True), (8, 18, False), (17, 26, True)])
+def test_level_march(prec, nn, jpk, flat):
+    """The momentum trends and the time stepping of velocities and tracers with 1 to 32
+    levels a thread (by the grid's size), with 1-D and with 3-D scale factors. Tolerances
+    of the routines' own parity tests."""
+    dom = gyre.domain(nn, jpk=jpk)
+    rng = np.random.default_rng(9)
+    if not flat:
+        f = 1.0 + 0.1 * rng.random((dom["jpi"], dom["jpj"], 1))
+        for n in "tuvwf":
+            dom[f"e3{n}_0"] = np.asfortranarray(dom[f"e3{n}_0"] * f)
+    p = Pair(dom=dom, nam=gyre.namelist(), prec=prec, seed=23)
+    st = p.states[0]
+    _, um, vm, wm = gyre.masks(dom)
+    st["ahmt"], st["ahmf"] = gyre.viscosity(dom)
+    st["avm"] = np.asfortranarray(2e-2 * (1.0 + rng.random(p.s3)) * wm)
+    st["avm"][:, :, [0, -1]] = 0.0
+    st["rhd"] = np.asfortranarray(1e-3 * rng.standard_normal(p.s3))
+    p.bind_spg()
+    for n in ("AHMT", "AHMF", "AVM", "RHD", "WN", "TSB", "TSN"):
+        p.bind(n)
+    p.bind("TSA", key="tsn")
+    p.set("UA_B", [np.asfortranarray(0.05 * rng.standard_normal(p.s2) * um[:, :, 0])])
+    p.set("VA_B", [np.asfortranarray(0.05 * rng.standard_normal(p.s2) * vm[:, :, 0])])
+    o, h, c = p.ora[0], p.host[0], p.ctx
+    for kvor in (1, 2, 4):
+        o.vor_ene(3, kvor, h["UN"], h["VN"], h["UA"], h["VA"])
+        c.vor_ene(3, kvor, p.dev["UN"], p.dev["VN"], p.dev["UA"], p.dev["VA"])
+    o.dyn_ldf_lap(3, h["UB"], h["VB"], h["UA"], h["VA"], 1)
+    c.dyn_ldf_lap(3, p.dev["UB"], p.dev["VB"], p.dev["UA"], p.dev["VA"], 1)
+    for f in ("dyn_keg", "dyn_zad", "dyn_hpg"):
+        getattr(o, f)(3)
+        getattr(c, f)(3)
+    c.synchronize()
+    t = 1e-12 if prec == "fp64" else 5e-5
+    p.compare("UA", p.s3, t)
+    p.compare("VA", p.s3, t)
+    for f in ("wzv", "dyn_zdf_step", "dyn_nxt", "tra_nxt"):
+        getattr(o, f)(3)
+        getattr(c, f)(3)
+    c.synchronize()
+    for n in ("WN", "UA", "VA", "UN", "VN", "UB", "VB"):
+        p.compare(n, p.s3, t)
+    for n in ("UN_B", "VN_B", "UB_B", "VB_B"):
+        p.compare(n, p.s2, t)
+    for n in ("TSB", "TSN"):
+        p.compare(n, p.s4, t)
