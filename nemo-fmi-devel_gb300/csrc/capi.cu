@@ -126,6 +126,7 @@ struct nemo_ctx {
   int bar_extra = 0;
   int p2_blocks = 0;
   int p2_cache = 0;  // the sub-step kernel keeps its constants in shared memory
+  int res_c = 0, res_rows = 0, res_v = 0, res_gen = 0;  // k_spg_p2_res: blocks a member (0: not used), rows, variant
   int p2_hot = 0;    // the sub-step kernel is k_spg_p2_ene (mixed, linear free surface, ENE/MIX)
   bool no_p2_hot = false;  // keep the general sub-step kernel (tests compare both)
   double* gs_part = nullptr;
@@ -987,6 +988,9 @@ int run_spg(nemo_ctx* c, int kt) {
   a.zmu = (T*)c->spg_x[6]; a.zmv = (T*)c->spg_x[7];
   a.cache = c->p2_cache;
   a.hot = c->p2_hot;
+  if (!c->bar_extra) {  // an injected arrival asks for a kernel with the grid barrier
+    a.res_c = c->res_c; a.res_rows = c->res_rows; a.res_v = c->res_v; a.res_gen = c->res_gen;
+  }
   a.ff = c->spg_ff;
   a.wgt1 = c->d_wgt1; a.wgt2 = c->d_wgt2; a.wgtf = c->d_wgtf; a.nwgt = (int)c->wgt1.size();
   a.ln_bt_fw = nm.ln_bt_fw; a.ln_apr_dyn = nm.ln_apr_dyn; a.nvor = nm.nvor_scheme; a.ll_init = ll_init;
@@ -1827,6 +1831,28 @@ void select_p2(nemo_ctx* c) {
   if (!c->p2_hot) {
     p2_grid(ene ? 1 : 0);
     if (c->p2_cache && (c->p2_blocks < 1 || need > (long)c->p2_blocks * P2_MAXT)) p2_grid(0);
+  }
+  // The mixed form's linear ENE/MIX sub-steps of a member that fits a cluster: the blocks
+  // a member with the least estimated time, rounds of resident clusters times a sub-step's
+  // (two barriers, as long as the arithmetic of some 700 points and 60 more for each block
+  // that joins them, and the block's points: 62x42 takes 107 us on 3 blocks, 72 on 6 and 82
+  // on 11), with the fewest points a thread.
+  c->res_c = 0;
+  c->res_gen = !c->p2_hot;
+  if (ene && !c->no_p2_hot && (c->p2_hot || !c->p2_cache)) {
+    double best = 0.0;
+    for (int v = 0; v < P2R_NV; ++v)
+      for (int cs = 1; cs <= P2R_MAXC; ++cs) {
+        const int rows = (c->jpj + cs - 1) / cs;
+        if ((c->jpj + rows - 1) / rows != cs) continue;  // a block without a row
+        const int n = spg_res_clusters<float>(v, c->res_gen, cs, rows, c->jpi);
+        if (n < 1) continue;
+        const double t = (double)((c->nmem + n - 1) / n) * (700.0 + 60.0 * cs + (double)rows * c->jpi);
+        if (c->res_c == 0 || t < best) {
+          best = t;
+          c->res_c = cs; c->res_rows = rows; c->res_v = v;
+        }
+      }
   }
 }
 

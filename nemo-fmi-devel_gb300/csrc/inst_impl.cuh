@@ -201,25 +201,33 @@ cudaError_t launch_iso_edges(const Dom<T>& d, const LdfArgs<T>& a, int copy_akz_
   return cudaGetLastError();
 }
 
+// FP32 with the GYRE's 31 levels: one thread a column (k_zdf_imp_async) from this many
+// columns on, where the march of all columns down the same planes is kinder to DRAM than
+// a block of columns at a time: 302x202 33 against 29 us, 362x242 35 against 38, 752x502
+// 118 against 150.
+constexpr long ZDF31_MIN = 65536;
 template <class T>
 cudaError_t launch_zdf(const Dom<T>& d, const ZdfArgs<T>& a, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
-    if (d.jpk == 31) {  // the GYRE levels: columns staged in shared memory
-      static bool attr = false;  // dynamic shared memory beyond 48 KB needs the opt-in
+    if (d.jpi < 3 || d.jpj < 3) return cudaSuccess;  // no interior column
+    if (d.jpk == 31 && d.n2 * d.nmem >= ZDF31_MIN) {  // the GYRE levels: columns staged in shared memory
       constexpr int smem_max = 4 * 31 * BX * BY * sizeof(float);
-      if (!attr) {
-        cudaFuncSetAttribute(k_zdf_imp_async<31>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-        attr = true;
-      }
+      static const cudaError_t attr31 =
+          cudaFuncSetAttribute(k_zdf_imp_async<31>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+      if (attr31 != cudaSuccess) return attr31;
       const int tz = kty(NEMO_K_ZDF_IMP);
-      const int smem = 4 * 31 * BX * tz * sizeof(float);
-      k_zdf_imp_async<31><<<col_grid(d, tz), dim3(BX, tz), smem, s>>>(d, a);
+      k_zdf_imp_async<31><<<col_grid(d, tz), dim3(BX, tz), 4 * 31 * BX * tz * sizeof(float), s>>>(d, a);
       ktick(NEMO_K_ZDF_IMP, s);
       return cudaGetLastError();
     }
+    static const cudaError_t attr =  // dynamic shared memory beyond 48 KB needs the opt-in
+        cudaFuncSetAttribute(k_zdf_imp32<ZW>, cudaFuncAttributeMaxDynamicSharedMemorySize, zdf32_smem(KMAX));
+    if (attr != cudaSuccess) return attr;
+    k_zdf_imp32<ZW><<<dim3((unsigned)((d.jpi + 31) / 32) * (d.jpj - 2), d.nmem), dim3(32, ZW), zdf32_smem(d.jpk), s>>>(d, a);
+  } else {
+    const int tz = kty(NEMO_K_ZDF_IMP);
+    k_zdf_imp<T><<<col_grid(d, tz), dim3(BX, tz), 0, s>>>(d, a);
   }
-  const int tz = kty(NEMO_K_ZDF_IMP);
-  k_zdf_imp<T><<<col_grid(d, tz), dim3(BX, tz), 0, s>>>(d, a);
   ktick(NEMO_K_ZDF_IMP, s);
   return cudaGetLastError();
 }
@@ -264,6 +272,68 @@ int spg_p2_ene_blocks_per_sm() {
   }
 }
 
+// the variants of k_spg_p2_res: threads, points a thread
+struct SpgRes {
+  void (*kern)(Dom<float>, SpgArgs<float>, int, int);
+  int nt, ppt;
+};
+static SpgRes spg_res(int v, bool gen) {
+  static const SpgRes t[2][P2R_NV] = {
+      {{k_spg_p2_res<512, 1, false>, 512, 1}, {k_spg_p2_res<512, 2, false>, 512, 2}, {k_spg_p2_res<512, 4, false>, 512, 4}},
+      {{k_spg_p2_res<512, 1, true>, 512, 1}, {k_spg_p2_res<512, 2, true>, 512, 2}, {k_spg_p2_res<512, 4, true>, 512, 4}}};
+  return t[gen ? 1 : 0][v];
+}
+// its launch: csize blocks a member, as clusters
+static cudaError_t spg_res_config(const SpgRes& v, bool gen, int csize, int rows, int jpi, int nmem,
+                                  cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+  cfg = {};
+  cfg.gridDim = dim3((unsigned)csize * nmem);
+  cfg.blockDim = dim3(v.nt);
+  cfg.dynamicSmemBytes = p2r_smem(v.nt * v.ppt, rows, jpi, gen);
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = csize;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (csize > 8) {  // more than the portable cluster size
+    const cudaError_t e = cudaFuncSetAttribute(v.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaFuncSetAttribute(v.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P2R_SMEM_MAX);
+}
+template <class T>
+cudaError_t launch_spg_res(const Dom<T>& d, const SpgArgs<T>& a, cudaStream_t s) {
+  if constexpr (sizeof(T) == 4) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    const SpgRes v = spg_res(a.res_v, a.res_gen);
+    const cudaError_t e = spg_res_config(v, a.res_gen, a.res_c, a.res_rows, d.jpi, d.nmem, cfg, attr);
+    cfg.stream = s;
+    return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, v.kern, d, a, a.res_c, a.res_rows);
+  } else {
+    return cudaErrorInvalidValue;
+  }
+}
+// clusters of k_spg_p2_res that the GPU holds at once (0: the shape does not fit)
+template <class T>
+int spg_res_clusters(int variant, int gen, int csize, int rows, int jpi) {
+  if constexpr (sizeof(T) == 4) {
+    const SpgRes v = spg_res(variant, gen);
+    if ((long)rows * jpi > v.nt * v.ppt || p2r_smem(v.nt * v.ppt, rows, jpi, gen) > P2R_SMEM_MAX) return 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    int n = 0;
+    if (spg_res_config(v, gen, csize, rows, jpi, 1, cfg, attr) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, v.kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  } else {
+    return 0;
+  }
+}
+
 template <class T>
 cudaError_t launch_spg(const Dom<T>& d, const SpgArgs<T>& a, const GridBar& bar, int p2_blocks, cudaStream_t s) {
   if (a.vvl) {  // Coriolis factors from the now depths (:241-343)
@@ -286,32 +356,36 @@ cudaError_t launch_spg(const Dom<T>& d, const SpgArgs<T>& a, const GridBar& bar,
   const int t1b = kty(NEMO_K_SPG_P1B);
   k_spg_p1b<T><<<col_grid(d, t1b), dim3(BX, t1b), 0, s>>>(d, a);
   ktick(NEMO_K_SPG_P1B, s);
-  {  // the barrier's arrival counter starts at 0 in every launch
-    cudaError_t ez = cudaMemsetAsync(bar.count, 0, sizeof(unsigned int), s);
-    if (ez != cudaSuccess) return ez;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p2_blocks);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = a.cache ? P2_CACHE_BYTES : 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   cudaError_t e;
-  if constexpr (sizeof(T) == 4) {
-    if (a.hot) {
-      cfg.dynamicSmemBytes = P2H_CACHE_BYTES;
-      e = cudaLaunchKernelEx(&cfg, k_spg_p2_ene<T>, d, a, bar);
+  if (a.res_c > 0) {
+    e = launch_spg_res(d, a, s);
+  } else {
+    {  // the barrier's arrival counter starts at 0 in every launch
+      cudaError_t ez = cudaMemsetAsync(bar.count, 0, sizeof(unsigned int), s);
+      if (ez != cudaSuccess) return ez;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p2_blocks);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = a.cache ? P2_CACHE_BYTES : 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if constexpr (sizeof(T) == 4) {
+      if (a.hot) {
+        cfg.dynamicSmemBytes = P2H_CACHE_BYTES;
+        e = cudaLaunchKernelEx(&cfg, k_spg_p2_ene<T>, d, a, bar);
+      } else {
+        e = a.vvl ? cudaLaunchKernelEx(&cfg, k_spg_p2<T, true>, d, a, bar)
+                  : cudaLaunchKernelEx(&cfg, k_spg_p2<T, false>, d, a, bar);
+      }
     } else {
       e = a.vvl ? cudaLaunchKernelEx(&cfg, k_spg_p2<T, true>, d, a, bar)
                 : cudaLaunchKernelEx(&cfg, k_spg_p2<T, false>, d, a, bar);
     }
-  } else {
-    e = a.vvl ? cudaLaunchKernelEx(&cfg, k_spg_p2<T, true>, d, a, bar)
-              : cudaLaunchKernelEx(&cfg, k_spg_p2<T, false>, d, a, bar);
   }
   if (e != cudaSuccess) return e;
   ktick(NEMO_K_SPG_P2, s);
@@ -350,6 +424,7 @@ cudaError_t launch_globsum(const T* x, const double* tmask_i, long n2, int nk, i
   template cudaError_t launch_clamp<T>(T*, long, cudaStream_t);                                              \
   template cudaError_t launch_spg<T>(const Dom<T>&, const SpgArgs<T>&, const GridBar&, int, cudaStream_t);   \
   template int spg_p2_blocks_per_sm<T>(int, int);                                                                 \
+  template int spg_res_clusters<T>(int, int, int, int, int);                                                      \
   template int spg_p2_ene_blocks_per_sm<T>();                                                                 \
   template cudaError_t launch_lbc<T>(T*, int, int, long, int, T, cudaStream_t);                              \
   template cudaError_t launch_globsum<T>(const T*, const double*, long, int, int, double*, int, double*, cudaStream_t);

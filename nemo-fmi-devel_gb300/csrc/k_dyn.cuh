@@ -42,6 +42,7 @@ struct SpgArgs {
   int ln_bt_fw, ln_apr_dyn, nvor, ll_init, icycle, ring0, phase3_filter;
   int cache;  // mixed form, ENE/MIX: the sub-step constants cached in shared memory
   int hot;    // mixed form, linear free surface, ENE/MIX: k_spg_p2_ene instead of k_spg_p2
+  int res_c, res_rows, res_v, res_gen;  // res_c > 0: k_spg_p2_res (variant res_v), res_c blocks of res_rows rows a member
   // Column depths (2-D): for a linear free surface the rest-state ht_0, hu_0, ...
   // shared by all members (member stride hs = 0); with a variable volume the bound
   // now / before depths of each member (hs = points per member). The Coriolis
@@ -1128,6 +1129,286 @@ __global__ void __launch_bounds__(256, 5) k_spg_p2_ene(Dom<T> d, SpgArgs<T> a, G
     a.ua_b[g] = uab;
     a.va_b[g] = vab;
     double uadv = (double)f1.z + (double)f1.w, vadv = (double)f2.x + (double)f2.y;
+    if (a.ln_bt_fw) {
+      const double zwx = uadv, zwy = vadv;
+      if (a.phase3_filter) {
+        uadv = 0.5 * (a.ub2_b[g] + zwx - a.rn_atfp * a.un_bf[g]);
+        vadv = 0.5 * (a.vb2_b[g] + zwy - a.rn_atfp * a.vn_bf[g]);
+        a.un_bf[g] = a.rn_atfp * a.un_bf[g] + (zwx - a.ub2_b[g]);
+        a.vn_bf[g] = a.rn_atfp * a.vn_bf[g] + (zwy - a.vb2_b[g]);
+      } else {
+        a.un_bf[g] = 0.0;
+        a.vn_bf[g] = 0.0;
+      }
+      a.ub2_b[g] = zwx;
+      a.vb2_b[g] = zwy;
+    }
+    a.un_adv[g] = uadv;
+    a.vn_adv[g] = vadv;
+    a.du[g] = (float)((uab - (double)a.ub_b[g]) * a.r1_2dt_b);
+    a.dv[g] = (float)((vab - (double)a.vb_b[g]) * a.r1_2dt_b);
+    a.cu[g] = (float)(uadv * (double)d.r1_hu_0[p]);
+    a.cv[g] = (float)(vadv * (double)d.r1_hv_0[p]);
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// The sub-steps of k_spg_p2_ene for a member that fits a thread-block cluster: block c
+// of a member's cluster owns the rows [c R, (c+1) R) and
+// keeps everything they need from the first to the last sub-step on the SM: the ssh and
+// velocity levels and the five compensated sums in registers, the constants, the
+// predictor fluxes and the AM4 ssh in shared memory. A block writes the row that its
+// neighbour needs into the neighbour's shared memory (fluxes after the predictor, the AM4
+// ssh after the new ssh), and two cluster barriers a sub-step take the place of the grid
+// barrier, its L2 round trips and the halo recomputation; members never wait for one
+// another, so an ensemble runs as independent clusters. No wait is open-ended: the blocks
+// of a cluster are resident together by definition and none leaves its loop early.
+// The grid-barrier kernels are bound by that barrier and by L2 latency at these sizes:
+// the sub-steps of GYRE nn_GYRE=1 (704 points) took 120 us and of 64 members of nn_GYRE=5
+// 1331 us, and take 52 and 733 us here, bound by instruction issue (250 a point).
+constexpr int P2R_MAXC = 16, P2R_NV = 3, P2R_SMEM_MAX = 227 * 1024;
+// shared memory of a block: five float4 of constants a point, five arrays of rows (six in
+// the GEN form), and what the last point of the last array reads as its eastern neighbour
+// (and does not use)
+inline int p2r_smem(int points, int rows, int jpi, bool gen) {
+  return (20 * points + (gen ? 6 : 5) * (rows + 1) * jpi + 4) * (int)sizeof(float);
+}
+__device__ __forceinline__ void st_cluster(float* p, unsigned rank, float v) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(r), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier(int csize) {
+  if (csize == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+// a x + b y + c z as the compiler contracts it in the grid-barrier kernels
+__device__ __forceinline__ float p2r_sum3(float a, float x, float b, float y, float c, float z) {
+  return __fmaf_rn(c, z, __fmaf_rn(a, x, __fmul_rn(b, y)));
+}
+// NT threads, PPT points a thread. Every slot is computed without a branch (a slot without
+// a point works on point 0 and stores nothing), so that a thread's points overlap. The
+// values are those of the kernel that such a grid had otherwise, to the bit: k_spg_p2_ene's,
+// with its combined constants, or (GEN) those of k_spg_p2 without its constant cache.
+template <int NT, int PPT, bool GEN>
+__global__ void __launch_bounds__(NT, 1) k_spg_p2_res(Dom<float> d, SpgArgs<float> a, int csize, int R) {
+  extern __shared__ float4 p2r[];
+  constexpr int CS = NT * PPT;  // stride of one float4 of constants
+  const int n2 = (int)d.n2, nmem2 = d.nmem * n2, W = d.jpi, jpj = d.jpj, tid = threadIdx.x;
+  const int c = (int)blockIdx.x % csize, m2 = ((int)blockIdx.x / csize) * n2;
+  const int j0 = c * R, nr = min(R, jpj - j0), FL = (R + 1) * W;  // rows j0 .. j0 + nr - 1 (0-based)
+  float4* const cst = p2r;
+  float* const zs = reinterpret_cast<float*>(cst + 5 * CS);  // own rows, then the first row of block c + 1
+  float* const fxb = zs + FL;      // two buffers of the u fluxes: own rows, then that of block c + 1
+  float* const fyb = fxb + 2 * FL; // two buffers of the v fluxes: the last row of block c - 1, own rows
+  float* const zq = fyb + 2 * FL;  // GEN: zwz, the row south of the own ones first
+  const float rdtbt = a.rdtbt;
+  float s0[PPT], s1[PPT], s2[PPT], un[PPT], ub[PPT], vn[PPT], vb[PPT];
+  FF fs[PPT], fu[PPT], fv[PPT], fau[PPT], fav[PPT];
+  int X[PPT];                                     // the point in the block's rows
+  bool own[PPT], inner[PPT], bot[PPT], top[PPT];  // bot / top: the row that block c - 1 / c + 1 reads
+  const int r0 = a.ring0;
+  // the row-0 (last-row) values of an array into its halo row of block c - 1 (c + 1)
+  auto push = [&](float* f, int row, int x, unsigned rank, float v) { st_cluster(f + row * W + x % W, rank, v); };
+  cluster_barrier(csize);  // every block of the cluster has started
+  {
+    float za1, za2, za3;
+    ab3(1, a.ll_init, za1, za2, za3);
+    const int sn = r0 & 3, sb = (r0 + 1) & 3, sbb = (r0 + 2) & 3;
+    const float w2 = a.wgtf[2 * a.nwgt];
+#pragma unroll
+    for (int s = 0; s < PPT; ++s) {
+      const int x = s * NT + tid, row = x / W, col = x - row * W;
+      own[s] = row < nr;
+      X[s] = own[s] ? x : 0;
+      inner[s] = own[s] && col >= 1 && col <= W - 2 && j0 + row >= 1 && j0 + row <= jpj - 2;
+      bot[s] = own[s] && row == 0 && c > 0;
+      top[s] = own[s] && row == nr - 1 && c < csize - 1;
+      s0[s] = s1[s] = s2[s] = un[s] = ub[s] = vn[s] = vb[s] = 0.f;
+      fs[s] = fu[s] = fv[s] = fau[s] = fav[s] = FF{0.f, 0.f};
+      float cv[20] = {};
+      if (own[s]) {
+        const int p = j0 * W + x, g = m2 + p;
+        if constexpr (GEN) {
+          cv[0] = d.r1_e1u[p]; cv[1] = d.r1_e2v[p];
+          cv[4] = d.r1_hu_0[p]; cv[5] = d.r1_hv_0[p];
+          cv[8] = d.e2u[p]; cv[9] = d.hu_0[p]; cv[10] = d.e1v[p]; cv[11] = d.hv_0[p];
+          cv[12] = d.ssumask[p]; cv[13] = d.ssvmask[p];
+          if (inner[s]) {
+            cv[2] = a.zCdU_u[g]; cv[3] = a.zCdU_v[g];
+            cv[6] = a.zu_frc[g]; cv[7] = a.zv_frc[g];
+            cv[16] = a.zssh_frc[g]; cv[17] = d.r1_e1e2t[p]; cv[18] = d.ssmask[p];
+          }
+          zq[W + x] = d.zwz[p];
+          if (row == 0) zq[x] = j0 > 0 ? d.zwz[p - W] : 0.f;
+        } else {
+          if (inner[s]) {
+            const float su = (1.0f - a.scal_load) * (-a.grav);
+            cv[0] = 0.25f * d.zwz[p - W] * d.r1_e1u[p];
+            cv[1] = 0.25f * d.zwz[p] * d.r1_e1u[p];
+            cv[2] = -0.25f * d.zwz[p - 1] * d.r1_e2v[p];
+            cv[3] = -0.25f * d.zwz[p] * d.r1_e2v[p];
+            cv[4] = a.zCdU_u[g] * d.r1_hu_0[p];
+            cv[5] = a.zCdU_v[g] * d.r1_hv_0[p];
+            cv[6] = su * d.r1_e1u[p];
+            cv[7] = su * d.r1_e2v[p];
+            cv[8] = a.zu_frc[g];
+            cv[9] = a.zv_frc[g];
+            cv[10] = d.ssumask[p];
+            cv[11] = d.ssvmask[p];
+            cv[16] = __fmul_rn(rdtbt, a.zssh_frc[g]);
+            cv[17] = __fmul_rn(rdtbt, d.r1_e1e2t[p]);
+            cv[18] = d.ssmask[p];
+          }
+          cv[12] = d.e2u[p] * d.hu_0[p];
+          cv[13] = d.e1v[p] * d.hv_0[p];
+        }
+        cv[14] = d.r1_e2u[p];
+        cv[15] = d.r1_e1v[p];
+        s0[s] = a.ring_ssh[sn * nmem2 + g];
+        s1[s] = a.ring_ssh[sb * nmem2 + g];
+        s2[s] = a.ring_ssh[sbb * nmem2 + g];
+        un[s] = a.ring_u[sn * nmem2 + g];
+        ub[s] = a.ring_u[sb * nmem2 + g];
+        vn[s] = a.ring_v[sn * nmem2 + g];
+        vb[s] = a.ring_v[sb * nmem2 + g];
+        const float ua_e = za1 * un[s] + za2 * ub[s] + za3 * a.ring_u[sbb * nmem2 + g];
+        const float va_e = za1 * vn[s] + za2 * vb[s] + za3 * a.ring_v[sbb * nmem2 + g];
+        const float zwx = d.e2u[p] * ua_e * d.hu_0[p];
+        const float zwy = d.e1v[p] * va_e * d.hv_0[p];
+        fxb[FL + x] = zwx;  // buffer 1 & 1
+        fyb[FL + W + x] = zwy;
+        if (bot[s]) push(fxb + FL, R, x, c - 1, zwx);
+        if (top[s]) push(fyb + FL, 0, x, c + 1, zwy);
+        fau[s].h = w2 * zwx * d.r1_e2u[p];
+        fav[s].h = w2 * zwy * d.r1_e1v[p];
+      }
+#pragma unroll
+      for (int q = 0; q < 5; ++q)
+        cst[q * CS + x] = make_float4(cv[4 * q], cv[4 * q + 1], cv[4 * q + 2], cv[4 * q + 3]);
+    }
+  }
+  cluster_barrier(csize);
+  float uo[PPT], vo[PPT];  // the oldest velocity levels, for the ring at the end
+  for (int jn = 1; jn <= a.icycle; ++jn) {
+    const float *fx = fxb + (jn & 1) * FL, *fy = fyb + (jn & 1) * FL;
+    const float w1h = a.wgtf[jn - 1], w1l = a.wgtf[a.nwgt + jn - 1];
+    float zb0, zb1, zb2, zb3;
+    am4(jn, a.ll_init, a.rn_bt_alpha, zb0, zb1, zb2, zb3);
+    // ---- ssha_e (:871-879) and zsshp2_e (:930-931), rounded as in k_spg_p2_ene
+    float za[PPT];
+#pragma unroll
+    for (int s = 0; s < PPT; ++s) {
+      const int x = X[s];
+      const float4 C = cst[4 * CS + s * NT + tid];
+      float e;
+      if constexpr (GEN) {
+        const float zhdiv = (fx[x] - fx[x - 1] + fy[W + x] - fy[x]) * C.y;
+        e = (s0[s] - rdtbt * (C.x + zhdiv)) * C.z;
+        e = inner[s] ? e : 0.f;
+        za[s] = zb0 * e + zb1 * s0[s] + zb2 * s1[s] + zb3 * s2[s];
+      } else {
+        const float dv = __fsub_rn(__fadd_rn(__fsub_rn(fx[x], fx[x - 1]), fy[W + x]), fy[x]);
+        e = __fmul_rn(__fsub_rn(s0[s], __fmaf_rn(C.y, dv, C.x)), C.z);
+        e = inner[s] ? e : 0.f;
+        za[s] = __fmaf_rn(zb3, s2[s], __fmaf_rn(zb2, s1[s], __fmaf_rn(zb1, s0[s], __fmul_rn(zb0, e))));
+      }
+      if (own[s]) zs[x] = za[s];
+      s2[s] = s1[s]; s1[s] = s0[s]; s0[s] = e;
+      ff_add_w(fs[s], w1h, w1l, e);
+    }
+#pragma unroll
+    for (int s = 0; s < PPT; ++s)
+      if (bot[s]) push(zs, R, X[s], c - 1, za[s]);
+    cluster_barrier(csize);
+    // ---- Coriolis, drag, pressure gradient, ua_e / va_e and their sums (:1000-1204), the
+    // predictor of sub-step jn+1 (:724-800) and its sums (:860-862)
+    float za1, za2, za3;
+    ab3(jn + 1, a.ll_init, za1, za2, za3);
+    const bool more = jn < a.icycle;
+    const float w2 = more ? a.wgtf[2 * a.nwgt + jn] : 0.f;
+    float *gx = fxb + ((jn + 1) & 1) * FL, *gy = fyb + ((jn + 1) & 1) * FL;
+    float zwx[PPT], zwy[PPT];
+#pragma unroll
+    for (int s = 0; s < PPT; ++s) {
+      const int x = X[s];
+      const float4* C = cst + s * NT + tid;
+      const float4 A = C[0], B = C[CS], F = C[2 * CS], P = C[3 * CS];
+      const float z0 = zs[x];
+      float ue, ve;
+      if constexpr (GEN) {
+        const float zy1 = (fy[x] + fy[x + 1]) * A.x, zy2 = (fy[W + x] + fy[W + x + 1]) * A.x;
+        const float zx1 = (fx[x - 1] + fx[x - 1 + W]) * A.y, zx2 = (fx[x] + fx[x + W]) * A.y;
+        const float zu_cor = 0.25f * (zq[x] * zy1 + zq[W + x] * zy2);
+        const float zv_cor = -0.25f * (zq[W + x - 1] * zx1 + zq[W + x] * zx2);
+        const float zu_trd = __fmaf_rn(__fmul_rn(A.z, un[s]), B.x, zu_cor);
+        const float zv_trd = __fmaf_rn(__fmul_rn(A.w, vn[s]), B.y, zv_cor);
+        const float zu_spg = -a.grav * (zs[x + 1] - z0) * A.x;
+        const float zv_spg = -a.grav * (zs[x + W] - z0) * A.y;
+        const float wxs = (1.0f - a.scal_load) * zu_spg;
+        const float wys = (1.0f - a.scal_load) * zv_spg;
+        ue = (un[s] + rdtbt * (wxs + zu_trd + B.z)) * P.x;
+        ve = (vn[s] + rdtbt * (wys + zv_trd + B.w)) * P.y;
+      } else {
+        const float zu_trd = A.x * (fy[x] + fy[x + 1]) + A.y * (fy[W + x] + fy[W + x + 1]) + B.x * un[s];
+        const float zv_trd = A.z * (fx[x - 1] + fx[x - 1 + W]) + A.w * (fx[x] + fx[x + W]) + B.y * vn[s];
+        const float wxs = B.z * (zs[x + 1] - z0);
+        const float wys = B.w * (zs[x + W] - z0);
+        ue = (un[s] + rdtbt * (wxs + zu_trd + F.x)) * F.z;
+        ve = (vn[s] + rdtbt * (wys + zv_trd + F.y)) * F.w;
+      }
+      const float ua_e = inner[s] ? ue : 0.f, va_e = inner[s] ? ve : 0.f;
+      ff_add_w(fu[s], w1h, w1l, ua_e);
+      ff_add_w(fv[s], w1h, w1l, va_e);
+      const float uex = p2r_sum3(za1, ua_e, za2, un[s], za3, ub[s]), vex = p2r_sum3(za1, va_e, za2, vn[s], za3, vb[s]);
+      zwx[s] = GEN ? F.x * uex * F.y : P.x * uex;
+      zwy[s] = GEN ? F.z * vex * F.w : P.y * vex;
+      if (more) {
+        if (own[s]) {
+          gx[x] = zwx[s];
+          gy[W + x] = zwy[s];
+        }
+        ff_add(fau[s], w2 * zwx[s] * P.z, 0.0f);
+        ff_add(fav[s], w2 * zwy[s] * P.w, 0.0f);
+      } else {
+        uo[s] = ub[s];
+        vo[s] = vb[s];
+      }
+      ub[s] = un[s]; un[s] = ua_e;
+      vb[s] = vn[s]; vn[s] = va_e;
+    }
+    if (more) {
+#pragma unroll
+      for (int s = 0; s < PPT; ++s) {
+        if (bot[s]) push(gx, R, X[s], c - 1, zwx[s]);
+        if (top[s]) push(gy, 0, X[s], c + 1, zwy[s]);
+      }
+    }
+    cluster_barrier(csize);
+  }
+  // ---- the levels into the ring (a next call without time averaging continues from
+  // them) and phase 3 per column, as in k_spg_p2_ene
+  const int r = (r0 + 3 * a.icycle) & 3, sn = r, sb = (r + 1) & 3, sbb = (r + 2) & 3;
+#pragma unroll
+  for (int s = 0; s < PPT; ++s) {
+    if (!own[s]) continue;
+    const int p = j0 * W + X[s], g = m2 + p;
+    a.ring_ssh[sn * nmem2 + g] = s0[s]; a.ring_ssh[sb * nmem2 + g] = s1[s]; a.ring_ssh[sbb * nmem2 + g] = s2[s];
+    a.ring_u[sn * nmem2 + g] = un[s]; a.ring_u[sb * nmem2 + g] = ub[s];
+    a.ring_v[sn * nmem2 + g] = vn[s]; a.ring_v[sb * nmem2 + g] = vb[s];
+    if (a.icycle >= 1) {
+      a.ring_u[sbb * nmem2 + g] = uo[s];
+      a.ring_v[sbb * nmem2 + g] = vo[s];
+    }
+    a.ssha[g] = (double)fs[s].h + (double)fs[s].l;
+    const double uab = (double)fu[s].h + (double)fu[s].l, vab = (double)fv[s].h + (double)fv[s].l;
+    a.ua_b[g] = uab;
+    a.va_b[g] = vab;
+    double uadv = (double)fau[s].h + (double)fau[s].l, vadv = (double)fav[s].h + (double)fav[s].l;
     if (a.ln_bt_fw) {
       const double zwx = uadv, zwy = vadv;
       if (a.phase3_filter) {

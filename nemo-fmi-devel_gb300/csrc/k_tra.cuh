@@ -1006,15 +1006,16 @@ struct ZdfArgs {
   int ddm, is_trc, clamp_sal;
 };
 
-// Any jpk <= KMAX, the reference's recurrences with the pivots in local memory; in
-// double precision the operations are those of trazdf.F90:218-264 in order, with
-// every quotient correctly rounded as the reference's division gives it, but formed
-// from a reciprocal (divq): one division per level (1 / zwt(k)) where the reference
-// divides six times (zwi, zws, the two pivot quotients of the 1st recurrence and the
-// 3rd recurrence of each of T and S); zwi(k+1) is zws(k), the same expression, formed
-// once; the divisions by e3w use the rest-state reciprocal profile where e3w is it.
+// tra_zdf_imp in FP64, one column a thread with the pivots in local memory: the operations
+// of trazdf.F90:218-264 in order, with every quotient correctly rounded as the reference's
+// division gives it, but formed from a reciprocal (divq): one division per level
+// (1 / zwt(k)) where the reference divides six times (zwi, zws, the two pivot quotients of
+// the 1st recurrence and the 3rd recurrence of each of T and S); zwi(k+1) is zws(k), the
+// same expression, formed once; the divisions by e3w use the rest-state reciprocal profile
+// where e3w is it.
 template <class T>
 __global__ void k_zdf_imp(Dom<T> d, ZdfArgs<T> a) {
+  static_assert(sizeof(T) == 8, "FP32: k_zdf_imp32");
   ColIdx<T> c = col_index(d);
   if (!c.valid || !c.interior) return;
   const int jpk = d.jpk;
@@ -1022,8 +1023,7 @@ __global__ void k_zdf_imp(Dom<T> d, ZdfArgs<T> a) {
   const ColInfo ci = d.ci[c.ij];
   const long m3 = (long)c.m * n3;
   // rat(k) = zwi(k) / zwt(k-1): the tracer-independent factor of the 2nd recurrence
-  T rat[KMAX], zws[KMAX], zwt[KMAX];
-  T aux[KMAX];  // FP32: the sub-diagonal zwi, for the increment form; FP64: 1 / zwt
+  T rat[KMAX], zws[KMAX], zwt[KMAX], aux[KMAX];  // aux = 1 / zwt
   for (int n = 0; n < a.kjpt; ++n) {
     const bool build = (!a.is_trc && (n == 0 || (n == 1 && a.ddm))) || (a.is_trc && n == 0);
     if (build) {
@@ -1036,78 +1036,30 @@ __global__ void k_zdf_imp(Dom<T> d, ZdfArgs<T> a) {
         if (a.add && k <= jpk - 1) v = v + a.add[q];
         return v;
       };
-      if constexpr (sizeof(T) == 8) {
-        // 1st recurrence as written in the reference (trazdf.F90:218-234)
-        const bool r3w = d.r1_e3w && d.e3w_n.s == 0;  // e3w is the rest-state profile
-        auto over_e3w = [&](T x, int k) {
-          const T e = d.e3w_n(c.ij, k, c.m);
-          return r3w ? divq(x, e, d.r1_e3w[k - 1]) : x / e;
-        };
-        T zwi = over_e3w(-a.p2dt * wt(1), 1);
-        for (int k = 1; k <= jpk - 1; ++k) {
-          zws[k] = over_e3w(-a.p2dt * wt(k + 1), k + 1);
-          const T zwd = d.e3t_a(c.ij, k, c.m) - zwi - zws[k];
-          if (k == 1) {
-            zwt[k] = zwd;
-          } else {
-            rat[k] = divq(zwi, zwt[k - 1], aux[k - 1]);
-            zwt[k] = zwd - divq(zwi * zws[k - 1], zwt[k - 1], aux[k - 1]);
-          }
-          aux[k] = T(1) / zwt[k];
-          zwi = zws[k];
-        }
-      } else {
-      T wtk = wt(1);
-      T g = T(0);
+      // 1st recurrence as written in the reference (trazdf.F90:218-234)
+      const bool r3w = d.r1_e3w && d.e3w_n.s == 0;  // e3w is the rest-state profile
+      auto over_e3w = [&](T x, int k) {
+        const T e = d.e3w_n(c.ij, k, c.m);
+        return r3w ? divq(x, e, d.r1_e3w[k - 1]) : x / e;
+      };
+      T zwi = over_e3w(-a.p2dt * wt(1), 1);
       for (int k = 1; k <= jpk - 1; ++k) {
-        const T wtk1 = wt(k + 1);
-        const T zwi = -a.p2dt * wtk / d.e3w_n(c.ij, k, c.m);
-        zws[k] = -a.p2dt * wtk1 / d.e3w_n(c.ij, k + 1, c.m);
-        const T e3a = d.e3t_a(c.ij, k, c.m);
-        if (k >= 2) rat[k] = zwi / zwt[k - 1];
-        aux[k] = zwi;
-        {
-          // FP32: the same pivots without cancellation. With g(k) = zwt(k) + zws(k),
-          // zwt(k) = zwd(k) - zwi(k) zws(k-1)/zwt(k-1) is g(k) - zws(k) where
-          // g(k) = e3t_a(k) - zwi(k) g(k-1)/zwt(k-1): a sum of non-negative terms
-          // (zwi, zws <= 0), whereas zwd - zwi zws/zwt cancels to O(e3t) from
-          // O(p2dt avt/e3w) when the vertical diffusivity is large.
-          g = (k == 1) ? e3a - zwi : e3a - zwi * (g / zwt[k - 1]);
-          zwt[k] = g - zws[k];
+        zws[k] = over_e3w(-a.p2dt * wt(k + 1), k + 1);
+        const T zwd = d.e3t_a(c.ij, k, c.m) - zwi - zws[k];
+        if (k == 1) {
+          zwt[k] = zwd;
+        } else {
+          rat[k] = divq(zwi, zwt[k - 1], aux[k - 1]);
+          zwt[k] = zwd - divq(zwi * zws[k - 1], zwt[k - 1], aux[k - 1]);
         }
-        wtk = wtk1;
-      }
+        aux[k] = T(1) / zwt[k];
+        zwi = zws[k];
       }
     }
     const long mo = ((long)c.m * a.kjpt + n) * n3;
     const RO<T> tb = a.ptb + mo;
     T* ta = a.pta + mo;
     const bool clamp = a.clamp_sal && !a.is_trc && n == 1;
-    if constexpr (sizeof(T) == 4) {
-      // FP32: the increment form of k_zdf_imp_async (d = x - tb, one rounding of the
-      // O(1) values in x = tb + d)
-      const int K1 = jpk - 1;
-      T prev = T(0);
-      for (int k = 1; k <= K1; ++k) {
-        const long q = c.ij + (long)(k - 1) * n2;
-        const T tbk = tb[q];
-        T r = a.p2dt * d.e3t_n(c.ij, k, c.m) * ta[q] + (d.e3t_b(c.ij, k, c.m) - d.e3t_a(c.ij, k, c.m)) * tbk;
-        if (k > 1) r = r - aux[k] * (tb[q - n2] - tbk);
-        if (k < K1) r = r - zws[k] * (tb[q + n2] - tbk);
-        else r = r + zws[k] * tbk;
-        prev = (k == 1) ? r : r - rat[k] * prev;
-        ta[q] = prev;
-      }
-      T dnx = T(0);
-      for (int k = K1; k >= 1; --k) {
-        const long q = c.ij + (long)(k - 1) * n2;
-        const T tbk = tb[q];
-        const T dk = (k == K1 ? ta[q] : ta[q] - zws[k] * dnx) / zwt[k];
-        const T x = (tbk + dk) * tmsk<T>(ci, k);
-        dnx = x - tbk;
-        ta[q] = (clamp && x < T(0)) ? T(0.1) : x;
-      }
-    } else {
     // 2nd recurrence (:238-250), the forward values kept in pta as in the reference
     T prev = T(0);
     for (int k = 1; k <= jpk - 1; ++k) {
@@ -1128,7 +1080,6 @@ __global__ void k_zdf_imp(Dom<T> d, ZdfArgs<T> a) {
       const long q = c.ij + (long)(k - 1) * n2;
       nxt = divq(ta[q] - zws[k] * nxt, zwt[k], aux[k]) * tmsk<T>(ci, k);
       ta[q] = (clamp && nxt < T(0)) ? T(0.1) : nxt;
-    }
     }
   }
 }
@@ -1231,6 +1182,168 @@ __global__ void __launch_bounds__(128, 3) k_zdf_imp_async(Dom<float> d, ZdfArgs<
       dnx = x - tbk;
       ta[(long)(k - 1) * n2] = (clamp && x < 0.0f) ? 0.1f : x;
     }
+  }
+}
+
+// tra_zdf_imp in FP32: a block owns 32 columns of a row and ZW warps share their levels.
+// Everything a level does by itself -- the loads, the off-diagonal zw(k) = zwi(k) (zws(k)
+// is zwi(k+1): both are -p2dt zwt(k+1) / e3w(k+1)), the right-hand side -- runs on all
+// warps; only the recurrences are serial, in shared memory: the pivots by one warp, each
+// tracer's elimination and back substitution by a warp of its own. A column is 6 to 8
+// planes deep in every field, so on a grid beyond L2 each access opens another DRAM row:
+// one level in flight a thread beats eight (189 against 274 us at 500x400x56), where one
+// thread a column with the pivots in local memory took 429 us (80 us by traffic).
+//
+// The pivots are formed without cancellation: with g(k) = zwt(k) + zws(k),
+// zwt(k) = zwd(k) - zwi(k) zws(k-1)/zwt(k-1) is g(k) - zws(k) where
+// g(k) = e3t_a(k) - zwi(k) g(k-1)/zwt(k-1): a sum of non-negative terms (zwi, zws <= 0),
+// whereas zwd - zwi zws/zwt cancels to O(e3t) from O(p2dt avt/e3w) when the vertical
+// diffusivity is large. The system is solved in increment form, for d = x - tb,
+// M d = rhs - M tb, whose right-hand side holds only the trend and differences of tb, so
+// the O(1) tracer values are rounded once, in x = tb + d (the reference's form rounds
+// the full values in both recurrences: ~10 ulps of salinity per step).
+constexpr int ZW = 6;
+inline int zdf32_smem(int jpk) { return 6 * (jpk + 1) * 32 * (int)sizeof(float); }
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_zdf_imp32(Dom<float> d, ZdfArgs<float> a) {
+  extern __shared__ float zsm[];
+  constexpr int NC = 32;
+  const int lane = threadIdx.x, w = threadIdx.y, jpk = d.jpk, K = jpk - 1, A = (jpk + 1) * NC;
+  float* zw = zsm + lane;  // [k * NC]: zwi(k), k = 1..jpk
+  float* rz = zw + A;      // e3t_a(k), then 1 / zwt(k), k = 1..K
+  float* sy = rz + A;      // two tracers: ta, then the right-hand side, then the forward values
+  float* sb = sy + 2 * A;  // two tracers: tb
+  const int nx = (d.jpi + NC - 1) / NC, j = (int)(blockIdx.x / nx) + 2, i0 = (int)(blockIdx.x % nx) * NC + lane + 1;
+  const int i = min(i0, d.jpi), m = blockIdx.y;
+  const bool ok = i0 >= 2 && i0 <= d.jpi - 1;
+  const long n2 = d.n2, n3 = d.n3, ij = (long)(i - 1) + (long)(j - 1) * d.jpi, c3 = (long)m * n3 + ij;
+  const float p2dt = a.p2dt;
+  bool built = false, built_avt = false;
+  for (int n0 = 0; n0 < a.kjpt;) {
+    // zwt = avt (T; S without double diffusion) or avs (S with it, passive tracers); two
+    // tracers of one matrix go together
+    auto from_avt = [&](int n) { return !a.is_trc && (n == 0 || !a.ddm); };
+    const bool use_avt = from_avt(n0);
+    const int nn = n0 + 1 < a.kjpt && from_avt(n0 + 1) == use_avt ? 2 : 1;
+    const bool build = !built || use_avt != built_avt;
+    const long mo = ((long)m * a.kjpt + n0) * n3 + ij;
+    const float *tb = a.ptb.p + mo, *coef = (use_avt ? a.avt : a.avs).p + c3, *add = a.add ? a.add.p + c3 : coef;
+    float* ta = a.pta + mo;
+    constexpr int U = 1;  // levels a thread loads together
+    for (int k0 = w + 1; k0 <= jpk; k0 += U * W) {
+      float v[U], x[U], t[2][U], b[2][U], ew[U], ea[U], en[U], eb[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = min(k0 + u * W, jpk);
+        const long o = (long)(k - 1) * n2;
+        for (int n = 0; n < 2; ++n) {
+          t[n][u] = n < nn ? ta[o + n * n3] : 0.0f;
+          b[n][u] = n < nn ? __ldg(tb + o + n * n3) : 0.0f;
+        }
+        v[u] = __ldg(coef + o);
+        x[u] = __ldg(add + o);
+        ew[u] = d.e3w_n(ij, k, m);
+        ea[u] = d.e3t_a(ij, k, m);
+        en[u] = d.e3t_n(ij, k, m);
+        eb[u] = d.e3t_b(ij, k, m);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + u * W;
+        if (k > jpk) break;
+        if (build) {
+          const float wt = k == 1 ? 0.0f : a.add && k <= K ? v[u] + x[u] : v[u];
+          zw[k * NC] = -p2dt * wt / ew[u];
+          rz[k * NC] = ea[u];
+        }
+        for (int n = 0; n < nn; ++n) {
+          sb[n * A + k * NC] = b[n][u];
+          sy[n * A + k * NC] = p2dt * en[u] * t[n][u] + (eb[u] - ea[u]) * b[n][u];
+        }
+      }
+    }
+    __syncthreads();
+    constexpr int C = 4;  // levels whose operands a serial warp reads together
+    if (w > 0) {          // right-hand sides
+      for (int k = w; k <= K; k += W - 1) {
+        const float zi = zw[k * NC], zs = zw[(k + 1) * NC];
+        for (int n = 0; n < nn; ++n) {
+          const float* b = sb + n * A + k * NC;
+          const float tbk = b[0];
+          float r = sy[n * A + k * NC];
+          if (k > 1) r = r - zi * (b[-NC] - tbk);  // zwi(k) (tb(k-1) - tb(k))
+          if (k < K) r = r - zs * (b[NC] - tbk);   // zws(k) (tb(k+1) - tb(k))
+          else r = r + zs * tbk;                   // last row: no x(k+1)
+          sy[n * A + k * NC] = r;
+        }
+      }
+    } else if (build) {  // pivots
+      float g = 0.0f, rprev = 0.0f, zk = zw[NC];
+      for (int k0 = 1; k0 <= K; k0 += C) {
+        float e[C], z[C];
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          const int k = min(k0 + u, K);
+          e[u] = rz[k * NC];
+          z[u] = zw[(k + 1) * NC];
+        }
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          if (k0 + u > K) break;
+          g = e[u] - (k0 + u == 1 ? zk : zk * (g * rprev));
+          rprev = 1.0f / (g - z[u]);
+          rz[(k0 + u) * NC] = rprev;
+          zk = z[u];
+        }
+      }
+    }
+    __syncthreads();
+    if (w < nn) {
+      float *y = sy + w * A, *b = sb + w * A, *to = ta + w * n3;
+      float prev = 0.0f, rp = 0.0f;
+      for (int k0 = 1; k0 <= K; k0 += C) {
+        float r[C], f[C];
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          const int k = min(k0 + u, K);
+          r[u] = y[k * NC];
+          f[u] = zw[k * NC] * rp;
+          rp = rz[k * NC];
+        }
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          if (k0 + u > K) break;
+          prev = k0 + u == 1 ? r[u] : r[u] - f[u] * prev;
+          y[(k0 + u) * NC] = prev;
+        }
+      }
+      const ColInfo ci = d.ci[ij];
+      const bool clamp = a.clamp_sal && !a.is_trc && n0 + w == 1;
+      float dnx = 0.0f;  // x(k+1) - tb(k+1) of the stored (masked) x(k+1)
+      for (int k0 = K; k0 >= 1; k0 -= C) {
+        float r[C], q[C], z[C], h[C];
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          const int k = max(k0 - u, 1);
+          r[u] = y[k * NC];
+          q[u] = rz[k * NC];
+          z[u] = k == K ? 0.0f : zw[(k + 1) * NC];
+          h[u] = b[k * NC];
+        }
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          const int k = k0 - u;
+          if (k < 1) break;
+          const float x = (h[u] + (r[u] - z[u] * dnx) * q[u]) * tmsk<float>(ci, k);
+          dnx = x - h[u];
+          if (ok) to[(long)(k - 1) * n2] = (clamp && x < 0.0f) ? 0.1f : x;
+        }
+      }
+    }
+    built = true;
+    built_avt = use_avt;
+    n0 += nn;
+    if (n0 < a.kjpt) __syncthreads();
   }
 }
 

@@ -89,3 +89,21 @@ def test_level_march(prec, nn, jpk, flat):
         p.compare(n, p.s2, t)
     for n in ("TSB", "TSN"):
         p.compare(n, p.s4, t)
+
+
+@pytest.mark.parametrize("nn,nmem,case", [(1, 3, dict()), (2, 1, dict(ln_bt_av=0)), (3, 2, dict(nvor_scheme=5)),
+                                          (4, 5, dict(ln_bt_fw=0)), (5, 1, dict(ln_bt_av=0)), (6, 1, dict()),
+                                          (9, 1, dict()), (3, 80, dict(sample=[0, 41, 79]))])
+def test_sub_steps_of_a_cluster(nn, nmem, case):
+    """The mixed form's linear ENE/MIX sub-steps with a member on one block (nn 1), on
+    clusters of several sizes and points a thread, past the largest (nn 9: the grid
+    barrier's kernel) and with more members than the combined constants serve (80); three calls, the second and third from the levels of the one before
+    without time averaging. Tolerance of the routine's mixed parity tests."""
+    from test_gpu_parity import _spg_compare, _spg_pair
+    p = _spg_pair("mixed", case, nn=nn, nmem=nmem)
+    for kt in (5, 6, 7):
+        for o in p.ora:
+            o.dyn_spg_ts(kt)
+        p.ctx.dyn_spg_ts(kt)
+        p.ctx.synchronize()
+    _spg_compare(p, "mixed")
