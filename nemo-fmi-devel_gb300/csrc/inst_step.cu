@@ -97,12 +97,15 @@ cudaError_t launch_ssh_swp_vvl(const Dom<T>& d, const VvlArgs<T>& a, T* sshb, T*
 
 template <class T>
 cudaError_t launch_ldf_slp(const Dom<T>& d, const SlpArgs<T>& a, cudaStream_t s) {
+  const int kch = march_chunk(d);
+  const dim3 g = march_grid(d, kch);
+  const bool flat = d.e3u_n.s == 0 && d.e3v_n.s == 0 && d.e3w_n.s == 0;
   if (a.gru_b) {  // partial steps: the bottom level's gradients from zps_hde
     k_slp_mxl<T, true><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
-    k_slp_pre<T, true><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
+    (flat ? k_slp_pre<T, true, true> : k_slp_pre<T, true, false>)<<<g, dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   } else {
     k_slp_mxl<T, false><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
-    k_slp_pre<T, false><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
+    (flat ? k_slp_pre<T, false, true> : k_slp_pre<T, false, false>)<<<g, dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   }
   k_slp_filter<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
   ktick(NEMO_K_LDF_SLP, s);
@@ -139,7 +142,7 @@ cudaError_t launch_tra_qsr(const Dom<T>& d, const QsrArgs<T>& a, cudaStream_t s)
 
 template <class T>
 cudaError_t launch_eos(const Dom<T>& d, const EosArgs<T>& a, cudaStream_t s) {
-  const int kch = level_chunk(d, EOS_BLOCK, EOS_U);
+  const int kch = level_chunk(d, EOS_BLOCK, EOS_LEV<T>);
   const dim3 g((unsigned)((d.n2 + EOS_BLOCK - 1) / EOS_BLOCK), (d.jpk - 1 + kch - 1) / kch, d.nmem);
   if (a.what == 3) k_bn2<T><<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
   else if (a.what == 0) (a.eos80 ? k_eos<T, 0, true> : k_eos<T, 0, false>)<<<g, EOS_BLOCK, 0, s>>>(d, a, kch);
@@ -193,9 +196,12 @@ cudaError_t launch_usr_put(double* dst, const double* v, cudaStream_t s) {
 
 template <class T>
 cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s) {
-  k_zdf_sh2<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
+  const int kch = march_chunk(d), smem = 4 * 32 * TKE_Y * d.jpk * (int)sizeof(T);
+  const auto tke = d.e3w_n.s == 0 && d.e3t_n.s == 0 ? k_zdf_tke<T, true> : k_zdf_tke<T, false>;
+  if (cudaError_t e = smem_opt_in(tke, smem)) return e;
+  (d.e3w_n.s == 0 ? k_zdf_sh2<T, true> : k_zdf_sh2<T, false>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   ktick(NEMO_K_ZDF_PHY, s);
-  k_zdf_tke<T><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
+  tke<<<dim3((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y - 1) / TKE_Y, d.nmem), dim3(SX, TKE_Y), smem, s>>>(d, a);
   ktick(NEMO_K_ZDF_PHY, s);
   return cudaGetLastError();
 }

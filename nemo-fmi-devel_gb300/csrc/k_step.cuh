@@ -445,56 +445,124 @@ __global__ void k_slp_mxl(Dom<T> d, SlpArgs<T> a) {
 }
 
 // The slopes before the filter: u, v (:197-233) and w (:281-315) at levels 2..jpkm1;
-// 0 on the closed edges (the lbc_lnk of :234 and :316).
-template <class T, bool ZPS>
-__global__ void k_slp_pre(Dom<T> d, SlpArgs<T> a) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || c.k < 2 || c.k > d.jpk - 1) return;
-  const long o = (long)c.m * d.n3 + c.q;
-  if (!c.interior) {
-    a.zu[o] = T(0); a.zv[o] = T(0); a.zwi[o] = T(0); a.zwj[o] = T(0);
+// 0 on the closed edges (the lbc_lnk of :234 and :316). Level march: the masks' level
+// ranges and the metrics of the column and its neighbours are loaded once a chunk, the
+// densities of the level above and N^2 of the level are carried, and with 1-D scale
+// factors (FLAT) the limits -7e3 / e3 come from a table. One point a thread, which looked
+// up some twenty masks through memory, it took 154 us at 481x323x31 in FP32.
+template <class T, bool ZPS, bool FLAT>
+__global__ void __launch_bounds__(32 * MARCH_Y) k_slp_pre(Dom<T> d, SlpArgs<T> a, int kch) {
+  __shared__ T pu[KMAX + 1], pv[KMAX + 1], pw[KMAX + 1];  // -7e3 / e3u, e3v, e3w
+  const MarchIdx c = march_index(d, kch);
+  const int m = c.m, J = d.jpi;
+  if constexpr (FLAT) {
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= d.jpk) {
+      pu[k] = T(-7.e+3) / d.e3u_n(0, k, m);
+      pv[k] = T(-7.e+3) / d.e3v_n(0, k, m);
+      pw[k] = T(-7.e+3) / d.e3w_n(0, k, m);
+    }
+    __syncthreads();
+  }
+  if (c.i > d.jpi || c.j > d.jpj) return;
+  const int k0 = max(c.k0, 2);
+  if (k0 > c.k1) return;
+  const long n2 = d.n2, ij = c.ij, o = (long)m * d.n3 + ij, p = (long)m * n2 + ij;
+  if (!c.inner) {
+    for (int k = k0; k <= c.k1; ++k) {
+      const long q = o + (long)(k - 1) * n2;
+      a.zu[q] = T(0); a.zv[q] = T(0); a.zwi[q] = T(0); a.zwj[q] = T(0);
+    }
     return;
   }
-  const SlpPt<T, ZPS> P{d, a, (long)c.m * d.n3, c.m};
-  const int i = c.i, j = c.j, k = c.k, jpi = d.jpi;
-  const long ij = c.ij, p = (long)c.m * d.n2 + ij;
-  // u- and v-points
-  {
-    const T zau = P.gru(i, j, k) * d.r1_e1u[ij];
-    const T zav = P.grv(i, j, k) * d.r1_e2v[ij];
-    const T dz0 = P.dzr(i, j, k);
-    T zbu = T(0.5) * (dz0 + P.dzr(i + 1, j, k));
-    T zbv = T(0.5) * (dz0 + P.dzr(i, j + 1, k));
-    zbu = fmn(fmn(zbu, -a.z1_slpmax * fabs(zau)), T(-7.e+3) / d.e3u_n(ij, k, c.m) * fabs(zau));
-    zbv = fmn(fmn(zbv, -a.z1_slpmax * fabs(zav)), T(-7.e+3) / d.e3v_n(ij, k, c.m) * fabs(zav));
-    const T o0 = P.oml(i, j, k);
-    const T zfi = fmx(o0, P.oml(i + 1, j, k));
-    const T zfj = fmx(o0, P.oml(i, j + 1, k));
-    const long m3 = P.m3;
-    const T g0 = a.gdept[m3 + c.q];
-    const T zdepu = T(0.5) * ((g0 + a.gdept[m3 + c.q + 1]) - T(2) * T(0) - d.e3u_n(ij, 1, c.m));
-    const T zdepv = T(0.5) * ((g0 + a.gdept[m3 + c.q + jpi]) - T(2) * T(0) - d.e3v_n(ij, 1, c.m));
-    a.zu[o] = ((T(1) - zfi) * zau / (zbu - a.zeps) + zfi * zdepu * a.hu[p]) * P.um(i, j, k);
-    a.zv[o] = ((T(1) - zfj) * zav / (zbv - a.zeps) + zfj * zdepv * a.hv[p]) * P.vm(i, j, k);
+  const ColInfo ci = d.ci[ij], ce = d.ci[ij + 1], cn = d.ci[ij + J], cw = d.ci[ij - 1], cs = d.ci[ij - J];
+  const T r1u = d.r1_e1u[ij], r1v = d.r1_e2v[ij], e1t = d.e1t[ij], e2t = d.e2t[ij];
+  const T hu = a.hu[p], hv = a.hv[p], wiml = a.wiml[p], wjml = a.wjml[p];
+  const int n0 = a.nmln[p], ne = a.nmln[p + 1], nn = a.nmln[p + J];
+  const T gw1 = a.gdepw[o], zml = fmx(a.hmlp[p] - gw1, T(10));
+  const T e3u1 = d.e3u_n(ij, 1, m), e3v1 = d.e3v_n(ij, 1, m);
+  // with partial steps the bottom level's gradients are zps_hde's (ldfslp.F90:144-151)
+  T gu0 = T(0), guw = T(0), gv0 = T(0), gvs = T(0);
+  if constexpr (ZPS) {
+    gu0 = a.gru_b[p]; guw = a.gru_b[p - 1]; gv0 = a.grv_b[p]; gvs = a.grv_b[p - J];
   }
-  // w-points
-  {
-    const long q = P.m3 + c.q;
-    const T zbw = a.zm1_2g * a.pn2[q] * (a.prd[q] + a.prd[q - d.n2] + T(2));
-    const T zci = fmx(P.um(i - 1, j, k) + P.um(i, j, k) + P.um(i - 1, j, k - 1) + P.um(i, j, k - 1), a.zeps) * d.e1t[ij];
-    const T zcj = fmx(P.vm(i, j - 1, k) + P.vm(i, j, k - 1) + P.vm(i, j - 1, k - 1) + P.vm(i, j, k), a.zeps) * d.e2t[ij];
-    const T wmk = P.wm(i, j, k);
-    const T zai = (P.gru(i - 1, j, k) + P.gru(i, j, k - 1) + P.gru(i - 1, j, k - 1) + P.gru(i, j, k)) / zci * wmk;
-    const T zaj = (P.grv(i, j - 1, k) + P.grv(i, j, k - 1) + P.grv(i, j - 1, k - 1) + P.grv(i, j, k)) / zcj * wmk;
-    const T e3w = d.e3w_n(ij, k, c.m);
-    const T zbi = fmn(fmn(zbw, T(-100) * fabs(zai)), T(-7.e+3) / e3w * fabs(zai));
-    const T zbj = fmn(fmn(zbw, T(-100) * fabs(zaj)), T(-7.e+3) / e3w * fabs(zaj));
-    const T zfk = fmx(P.oml(i, j, k), P.oml(i, j, k - 1));
-    const T gw1 = a.gdepw[P.m3 + ij];
-    const T zck = (a.gdepw[q] - gw1) / fmx(a.hmlp[p] - gw1, T(10));
-    a.zwi[o] = (zai / (zbi - a.zeps) * (T(1) - zfk) + zck * a.wiml[p] * zfk) * wmk;
-    a.zwj[o] = (zaj / (zbj - a.zeps) * (T(1) - zfk) + zck * a.wjml[p] * zfk) * wmk;
-  }
+  auto gru = [&](const ColInfo& x, int k, T lft, T rgt, T b) -> T {
+    if constexpr (ZPS) {
+      if (k == x.mbku) return b;
+    }
+    return umsk<T>(x, k) * (rgt - lft);
+  };
+  auto grv = [&](const ColInfo& x, int k, T lft, T rgt, T b) -> T {
+    if constexpr (ZPS) {
+      if (k == x.mbkv) return b;
+    }
+    return vmsk<T>(x, k) * (rgt - lft);
+  };
+  // carried: prd of the level above at the five points, the four gradients formed from
+  // them, N^2 of the level at p, p+1, p+J
+  const long qa = o + (long)(k0 - 2) * n2, qk = o + (long)(k0 - 1) * n2;
+  T r0 = __ldg(a.prd + qa);
+  T ui = gru(ci, k0 - 1, r0, __ldg(a.prd + qa + 1), gu0), uw = gru(cw, k0 - 1, __ldg(a.prd + qa - 1), r0, guw);
+  T vi = grv(ci, k0 - 1, r0, __ldg(a.prd + qa + J), gv0), vs = grv(cs, k0 - 1, __ldg(a.prd + qa - J), r0, gvs);
+  T b0 = __ldg(a.pn2 + qk), be = __ldg(a.pn2 + qk + 1), bn = __ldg(a.pn2 + qk + J);
+  march<T, 12>(
+      k0, c.k1,
+      [&](int k, T (&l)[12]) {
+        const long q = o + (long)(k - 1) * n2;
+        const T *r = a.prd + q, *b = a.pn2 + q + n2, *g = a.gdept + q;
+        l[0] = __ldg(r); l[1] = __ldg(r + 1); l[2] = __ldg(r - 1); l[3] = __ldg(r + J); l[4] = __ldg(r - J);
+        l[5] = __ldg(b); l[6] = __ldg(b + 1); l[7] = __ldg(b + J);
+        l[8] = __ldg(g); l[9] = __ldg(g + 1); l[10] = __ldg(g + J);
+        l[11] = __ldg(a.gdepw + q);
+      },
+      [&](int k, T (&l)[12]) {
+        const long q = o + (long)(k - 1) * n2;
+        auto lim_u = [&](T z) { return FLAT ? pu[k] * z : T(-7.e+3) / d.e3u_n(ij, k, m) * z; };
+        auto lim_v = [&](T z) { return FLAT ? pv[k] * z : T(-7.e+3) / d.e3v_n(ij, k, m) * z; };
+        auto lim_w = [&](T z) { return FLAT ? pw[k] * z : T(-7.e+3) / d.e3w_n(ij, k, m) * z; };
+        auto dzr = [&](T r, T n, T np, const ColInfo& x) -> T {
+          return a.zm1_g * (r + T(1)) * (n + np) * (T(1) - T(0.5) * tmsk<T>(x, k + 1));
+        };
+        auto oml = [&](int n, int kk) -> T { return kk <= n - 1 ? T(1) : T(0); };
+        const T u1 = gru(ci, k, l[0], l[1], gu0), uw1 = gru(cw, k, l[2], l[0], guw);
+        const T v1 = grv(ci, k, l[0], l[3], gv0), vs1 = grv(cs, k, l[4], l[0], gvs);
+        const T um0 = umsk<T>(ci, k), um0a = umsk<T>(ci, k - 1), umw = umsk<T>(cw, k), umwa = umsk<T>(cw, k - 1);
+        const T vm0 = vmsk<T>(ci, k), vm0a = vmsk<T>(ci, k - 1), vms = vmsk<T>(cs, k), vmsa = vmsk<T>(cs, k - 1);
+        // u- and v-points
+        {
+          const T zau = u1 * r1u, zav = v1 * r1v;
+          const T dz0 = dzr(l[0], b0, l[5], ci);
+          T zbu = T(0.5) * (dz0 + dzr(l[1], be, l[6], ce));
+          T zbv = T(0.5) * (dz0 + dzr(l[3], bn, l[7], cn));
+          zbu = fmn(fmn(zbu, -a.z1_slpmax * fabs(zau)), lim_u(fabs(zau)));
+          zbv = fmn(fmn(zbv, -a.z1_slpmax * fabs(zav)), lim_v(fabs(zav)));
+          const T o0 = oml(n0, k);
+          const T zfi = fmx(o0, oml(ne, k));
+          const T zfj = fmx(o0, oml(nn, k));
+          const T zdepu = T(0.5) * ((l[8] + l[9]) - T(2) * T(0) - e3u1);
+          const T zdepv = T(0.5) * ((l[8] + l[10]) - T(2) * T(0) - e3v1);
+          a.zu[q] = ((T(1) - zfi) * zau / (zbu - a.zeps) + zfi * zdepu * hu) * um0;
+          a.zv[q] = ((T(1) - zfj) * zav / (zbv - a.zeps) + zfj * zdepv * hv) * vm0;
+        }
+        // w-points
+        {
+          const T zbw = a.zm1_2g * b0 * (l[0] + r0 + T(2));
+          const T zci = fmx(umw + um0 + umwa + um0a, a.zeps) * e1t;
+          const T zcj = fmx(vms + vm0a + vmsa + vm0, a.zeps) * e2t;
+          const T wmk = wmsk<T>(ci, k);
+          const T zai = (uw1 + ui + uw + u1) / zci * wmk;
+          const T zaj = (vs1 + vi + vs + v1) / zcj * wmk;
+          const T zbi = fmn(fmn(zbw, T(-100) * fabs(zai)), lim_w(fabs(zai)));
+          const T zbj = fmn(fmn(zbw, T(-100) * fabs(zaj)), lim_w(fabs(zaj)));
+          const T zfk = fmx(oml(n0, k), oml(n0, k - 1));
+          const T zck = (l[11] - gw1) / zml;
+          a.zwi[q] = (zai / (zbi - a.zeps) * (T(1) - zfk) + zck * wiml * zfk) * wmk;
+          a.zwj[q] = (zaj / (zbj - a.zeps) * (T(1) - zfk) + zck * wjml * zfk) * wmk;
+        }
+        r0 = l[0];
+        ui = u1; uw = uw1; vi = v1; vs = vs1;
+        b0 = l[5]; be = l[6]; bn = l[7];
+      });
 }
 
 // 1-2-1 Shapiro filter of the nine neighbours at level k (:237-275, :319-353)
@@ -924,7 +992,9 @@ __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
 // 5 fields, eos_insitu 4) and by the FP64 pipe in FP64. As one point a thread, with
 // the coefficients loaded from global memory, the six calls of a step's density (two
 // rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32.
-constexpr int EOS_U = 4, EOS_BLOCK = 256;
+constexpr int EOS_BLOCK = 256;
+template <class T>
+constexpr int EOS_LEV = sizeof(T) == 4 ? 4 : 1;  // FP64: four levels in a row left a small grid's FP64 pipes idle
 template <class T, int WHAT, bool E80>
 __global__ void __launch_bounds__(EOS_BLOCK) k_eos(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
   const long p = (long)blockIdx.x * EOS_BLOCK + threadIdx.x;
@@ -934,6 +1004,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_eos(Dom<T> d, const __grid_consta
   const ColInfo ci = d.ci[p];
   const T* __restrict__ ts = a.pts + c4;
   const T* __restrict__ dep = (WHAT == 2 ? a.gdept : a.pdep) + c3;
+  constexpr int EOS_U = EOS_LEV<T>;
   for (int k = k0; k <= k1; k += EOS_U) {
     T t[EOS_U], s[EOS_U], h[EOS_U];
 #pragma unroll
@@ -984,6 +1055,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_consta
   const T* __restrict__ gw = a.gdepw + c3;
   long o = (long)(k0 - 2) * d.n2;
   T tu = __ldg(ts + o), su = __ldg(ts + n3 + o), au = __ldg(ab + o), bu = __ldg(ab + n3 + o), hu = __ldg(gt + o);
+  constexpr int EOS_U = EOS_LEV<T>;
   for (int k = k0; k <= k1; k += EOS_U) {
     T t[EOS_U], s[EOS_U], x[EOS_U], y[EOS_U], h[EOS_U], w[EOS_U];
 #pragma unroll
@@ -1412,40 +1484,59 @@ __global__ void k_usr_put(double* dst, double s0, double s1, double s2, double s
 __device__ __forceinline__ double lc_sin(double x) { return nemo_sin_0pi(x); }
 __device__ __forceinline__ float lc_sin(float x) { return sinf(x); }
 
-// 2 x the shear production at the uw-point (i+1/2, j, k) and the vw-point
-// (i, j+1/2, k) of column ij (zdfsh2.F90:57-66) with the closure's avm_k. With a
-// linear free surface e3uw_n = e3uw_b = the rest-state MIN of the neighbouring e3w.
-template <class T>
-__device__ __forceinline__ T zsh2_u(const Dom<T>& d, const ZphyArgs<T>& a, long m3, long ij, int k, int m) {
-  const ColInfo c = d.ci[ij];
-  const long q = m3 + ij + (long)(k - 1) * d.n2;
-  const T e = fmn(d.e3w_n(ij, k, m), d.e3w_n(ij + 1, k, m));
-  return (a.avm_k[q + 1] + a.avm_k[q]) * (a.un[q - d.n2] - a.un[q]) * (a.ub[q - d.n2] - a.ub[q]) / (e * e) *
-         (umsk<T>(c, k) * umsk<T>(c, k - 1));
-}
-template <class T>
-__device__ __forceinline__ T zsh2_v(const Dom<T>& d, const ZphyArgs<T>& a, long m3, long ij, int k, int m) {
-  const ColInfo c = d.ci[ij];
-  const long q = m3 + ij + (long)(k - 1) * d.n2;
-  const T e = fmn(d.e3w_n(ij, k, m), d.e3w_n(ij + d.jpi, k, m));
-  return (a.avm_k[q + d.jpi] + a.avm_k[q]) * (a.vn[q - d.n2] - a.vn[q]) * (a.vb[q - d.n2] - a.vb[q]) / (e * e) *
-         (vmsk<T>(c, k) * vmsk<T>(c, k - 1));
-}
-
-// zdf_sh2 (zdfsh2.F90:67-74): the shear production at the interior w-points of
-// levels 2..jpk-1, one point per thread; each of the four uw/vw terms it averages is
-// formed where read (two threads form each).
-template <class T>
-__global__ void k_zdf_sh2(Dom<T> d, ZphyArgs<T> a) {
-  const PtIdx c = pt_index(d);
-  if (!c.valid || !c.interior || c.k < 2 || c.k > d.jpk - 1) return;
-  const long m3 = (long)c.m * d.n3;
-  const int k = c.k;
-  const T u0 = zsh2_u(d, a, m3, c.ij - 1, k, c.m), u1 = zsh2_u(d, a, m3, c.ij, k, c.m);
-  const T v0 = zsh2_v(d, a, m3, c.ij - d.jpi, k, c.m), v1 = zsh2_v(d, a, m3, c.ij, k, c.m);
-  const ColInfo cw = d.ci[c.ij - 1], ch = d.ci[c.ij], cs = d.ci[c.ij - d.jpi];
-  a.sh2[m3 + c.q] = T(0.25) * ((u0 + u1) * (T(2) - umsk<T>(cw, k) * umsk<T>(ch, k)) +
-                               (v0 + v1) * (T(2) - vmsk<T>(cs, k) * vmsk<T>(ch, k)));
+// zdf_sh2 (zdfsh2.F90:57-74): the shear production at the interior w-points of levels
+// 2..jpk-1, from 2 x that of the four uw- and vw-points around (with the closure's avm_k;
+// with a linear free surface e3uw_n = e3uw_b = the rest-state MIN of the neighbouring
+// e3w). Level march: the velocities of the level above are carried, the quotients by the
+// squared e3 of the level are divr's with 1-D scale factors (FLAT). One point a thread
+// it took 67 us at 481x323x31 in FP32 (17 us by traffic).
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(32 * MARCH_Y) k_zdf_sh2(Dom<T> d, ZphyArgs<T> a, int kch) {
+  __shared__ T pe[KMAX + 1], pr[KMAX + 1];  // e3w^2 and its reciprocal
+  const MarchIdx c = march_index(d, kch);
+  const int m = c.m, J = d.jpi;
+  if constexpr (FLAT) {
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= d.jpk) {
+      const T e = d.e3w_n(0, k, m);
+      pe[k] = e * e;
+      pr[k] = T(1) / pe[k];
+    }
+    __syncthreads();
+  }
+  if (!c.inner) return;
+  const int k0 = max(c.k0, 2);
+  const long ij = c.ij, n2 = d.n2, o = (long)m * d.n3 + ij;
+  const ColInfo ci = d.ci[ij], cw = d.ci[ij - 1], cs = d.ci[ij - J];
+  const long qt = o + (long)(k0 - 2) * n2;  // the level above the first
+  T u0 = a.un[qt], uw = a.un[qt - 1], v0 = a.vn[qt], vs = a.vn[qt - J];
+  T x0 = a.ub[qt], xw = a.ub[qt - 1], y0 = a.vb[qt], ys = a.vb[qt - J];
+  if (k0 > c.k1) return;
+  march<T, 13>(
+      k0, c.k1,
+      [&](int k, T (&l)[13]) {
+        const long q = o + (long)(k - 1) * n2;
+        const T *un = a.un + q, *vn = a.vn + q, *ub = a.ub + q, *vb = a.vb + q, *av = a.avm_k + q;
+        l[0] = __ldg(un); l[1] = __ldg(un - 1); l[2] = __ldg(vn); l[3] = __ldg(vn - J);
+        l[4] = __ldg(ub); l[5] = __ldg(ub - 1); l[6] = __ldg(vb); l[7] = __ldg(vb - J);
+        l[8] = __ldg(av); l[9] = __ldg(av + 1); l[10] = __ldg(av - 1); l[11] = __ldg(av + J); l[12] = __ldg(av - J);
+      },
+      [&](int k, T (&l)[13]) {
+        auto over = [&](T x, long p, long nb) -> T {  // x / e^2, e = MIN(e3w(p), e3w(p + nb))
+          if constexpr (FLAT) return divr(x, pe[k], pr[k]);
+          const T e = fmn(d.e3w_n(p, k, m), d.e3w_n(p + nb, k, m));
+          return x / (e * e);
+        };
+        const T um0 = umsk<T>(ci, k), umw = umsk<T>(cw, k), vm0 = vmsk<T>(ci, k), vms = vmsk<T>(cs, k);
+        const T su1 = over((l[9] + l[8]) * (u0 - l[0]) * (x0 - l[4]), ij, 1) * (um0 * umsk<T>(ci, k - 1));
+        const T su0 = over((l[8] + l[10]) * (uw - l[1]) * (xw - l[5]), ij - 1, 1) * (umw * umsk<T>(cw, k - 1));
+        const T sv1 = over((l[11] + l[8]) * (v0 - l[2]) * (y0 - l[6]), ij, J) * (vm0 * vmsk<T>(ci, k - 1));
+        const T sv0 = over((l[8] + l[12]) * (vs - l[3]) * (ys - l[7]), ij - J, J) * (vms * vmsk<T>(cs, k - 1));
+        a.sh2[o + (long)(k - 1) * n2] =
+            T(0.25) * ((su0 + su1) * (T(2) - umw * um0) + (sv0 + sv1) * (T(2) - vms * vm0));
+        u0 = l[0]; uw = l[1]; v0 = l[2]; vs = l[3];
+        x0 = l[4]; xw = l[5]; y0 = l[6]; ys = l[7];
+      });
 }
 
 // The column part of zdf_phy, one water column per thread (its levels are coupled
@@ -1458,12 +1549,37 @@ __global__ void k_zdf_sh2(Dom<T> d, ZphyArgs<T> a) {
 //    Prandtl correction of avt_k, then zdf_phy's avt, avm (zdfphy.F90:269-270),
 //    zdf_evd (zdfevd.F90:76-109) and avs = avt (:284).
 // Edge columns get the closed lbc_lnk of the five coefficients (zdfphy.F90:301-303).
-// Each expression keeps the reference's association.
-template <class T>
-__global__ void k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
+// Each expression keeps the reference's association. The column's system, lengths and
+// Prandtl numbers stay in shared memory (four arrays of jpk a thread: the slots of the
+// diagonal, upper diagonal and forward values take the raw and limited lengths and en), so
+// that memory sees each field about once, and the next level is loaded ahead; with five
+// work arrays in memory the column made some 30 passes over it, 269 us at 481x323x31 in
+// FP32 (50 us by traffic).
+// With 1-D scale factors (FLAT) the quotients by e3t e3w, and always those by the pivot,
+// are divr's; where EVD acts is kept as a bit a level.
+constexpr int TKE_Y = 2;
+template <class T, bool FLAT>
+__global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char col_smem[];
+  __shared__ T pu[KMAX + 1], ru[KMAX + 1], pl[KMAX + 1], rl[KMAX + 1];  // e3t(k) e3w(k), e3t(k-1) e3w(k), reciprocals
+  constexpr int nt = 32 * TKE_Y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i > d.jpi || j > d.jpj) return;
   const int m = blockIdx.z, jpk = d.jpk;
+  if constexpr (FLAT) {
+    static_assert(nt >= KMAX, "one thread a level");
+    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    if (k <= jpk) {
+      const T e3w = d.e3w_n(0, k, m);
+      pu[k] = d.e3t_n(0, k, m) * e3w;
+      ru[k] = T(1) / pu[k];
+      pl[k] = d.e3t_n(0, k > 1 ? k - 1 : 1, m) * e3w;
+      rl[k] = T(1) / pl[k];
+    }
+    __syncthreads();
+  }
+  if (i > d.jpi || j > d.jpj) return;
+  T* const sd = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x - nt;  // [k * nt], k = 1..jpk
+  T *const su = sd + jpk * nt, *const sl = su + jpk * nt, *const sp = sl + jpk * nt;
   const long n2 = d.n2;
   const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi;
   const long c3 = (long)m * d.n3 + ij, c2 = (long)m * d.n2 + ij;
@@ -1498,78 +1614,87 @@ __global__ void k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
     if (zfr < T(0)) zfr = T(0);
   }
   // downward sweep: right-hand side, matrix, forward elimination
-  T dg_p = T(1), up_p = T(0), lw_p = T(0);
-  T avm_km1 = a.avm_k[c3];
-  for (int k = 2; k <= jpk - 1; ++k) {
-    const long q = c3 + (long)(k - 1) * n2;
-    const T wm = wmsk<T>(ci, k), tm = tmsk<T>(ci, k);
-    T en = a.en[q];
-    if (zfr != T(0)) {
-      const T dep = a.gdepw[q];
-      if (dep - zhlc < T(0) && wm != T(0)) {
-        const T zwlc = a.rn_lc * lc_sin(a.rpi * dep / zhlc);
-        en = en + a.rdt * zfr * (zwlc * zwlc * zwlc) / zhlc;
-      }
-    }
-    const T avm_k = a.avm_k[q], avm_kp1 = a.avm_k[q + n2];
-    const T sh2 = a.sh2[q], dissl = a.dissl[q], rn2 = a.rn2[q];
-    if (a.nn_pdl == 1) {
-      const T zri = fmx(a.rn2b[q], T(0)) * avm_k / (sh2 + a.rn_bshear);
-      a.apdlr[q] = fmx(T(0.1), a.ri_cri / fmx(a.ri_cri, zri));
-    }
-    const T zcof = a.zfact1 * tm;
-    const T e3w = d.e3w_n(ij, k, m);
-    const T up = zcof * fmx(avm_kp1 + avm_k, T(2.e-5)) / (d.e3t_n(ij, k, m) * e3w);
-    const T lw = zcof * fmx(avm_k + avm_km1, T(2.e-5)) / (d.e3t_n(ij, k - 1, m) * e3w);
-    T dg = T(1) - lw - up + a.zfact2 * dissl * wm;
-    const T rhs = en + a.rdt * (sh2 - a.avt_k[q] * rn2 + a.zfact3 * dissl * en) * wm;
-    T lf;
-    if (k == 2) {
-      lf = rhs - lw * en1;
-    } else {
-      dg = dg - lw * up_p / dg_p;
-      lf = rhs - lw / dg_p * lw_p;
-    }
-    a.zdiag[q] = dg; a.zd_up[q] = up; a.zd_lw[q] = lf;
-    dg_p = dg; up_p = up; lw_p = lf;
-    avm_km1 = avm_k;
-  }
-  // upward sweep: back substitution, the floor, and the buoyancy length (into zdiag)
+  T dg_p = T(1), rd_p = T(1), up_p = T(0), lw_p = T(0);  // rd = 1 / dg
+  T avm_km1 = a.avm_k[c3], avm_k = a.avm_k[c3 + n2];
+  unsigned long long evd_at = 0;  // levels (bit k - 1) where EVD acts
+  march<T, 7>(
+      2, jpk - 1,
+      [&](int k, T (&l)[7]) {
+        const long q = c3 + (long)(k - 1) * n2;
+        l[0] = a.en[q]; l[1] = a.avm_k[q + n2]; l[2] = __ldg(a.sh2 + q); l[3] = a.dissl[q];
+        l[4] = __ldg(a.rn2 + q); l[5] = __ldg(a.rn2b + q); l[6] = a.avt_k[q];
+      },
+      [&](int k, T (&l)[7]) {
+        const T wm = wmsk<T>(ci, k), tm = tmsk<T>(ci, k);
+        T en = l[0];
+        if (zfr != T(0)) {
+          const T dep = a.gdepw[c3 + (long)(k - 1) * n2];
+          if (dep - zhlc < T(0) && wm != T(0)) {
+            const T zwlc = a.rn_lc * lc_sin(a.rpi * dep / zhlc);
+            en = en + a.rdt * zfr * (zwlc * zwlc * zwlc) / zhlc;
+          }
+        }
+        const T avm_kp1 = l[1], sh2 = l[2], dissl = l[3];
+        if (a.nn_pdl == 1) {
+          const T zri = fmx(l[5], T(0)) * avm_k / (sh2 + a.rn_bshear);
+          sp[k * nt] = fmx(T(0.1), a.ri_cri / fmx(a.ri_cri, zri));
+        }
+        const T zcof = a.zfact1 * tm;
+        if (a.ln_zdfevd && fmn(l[4], l[5]) <= T(-1.e-12)) evd_at |= 1ULL << (k - 1);
+        T up = zcof * fmx(avm_kp1 + avm_k, T(2.e-5)), lw = zcof * fmx(avm_k + avm_km1, T(2.e-5));
+        if constexpr (FLAT) {
+          up = divr(up, pu[k], ru[k]);
+          lw = divr(lw, pl[k], rl[k]);
+        } else {
+          const T e3w = d.e3w_n(ij, k, m);
+          up = up / (d.e3t_n(ij, k, m) * e3w);
+          lw = lw / (d.e3t_n(ij, k - 1, m) * e3w);
+        }
+        T dg = T(1) - lw - up + a.zfact2 * dissl * wm;
+        const T rhs = en + a.rdt * (sh2 - l[6] * l[4] + a.zfact3 * dissl * en) * wm;
+        T lf;
+        if (k == 2) {
+          lf = rhs - lw * en1;
+        } else {
+          dg = dg - divr(lw * up_p, dg_p, rd_p);
+          lf = rhs - divr(lw, dg_p, rd_p) * lw_p;
+        }
+        sd[k * nt] = dg; su[k * nt] = up; sl[k * nt] = lf;
+        dg_p = dg; rd_p = T(1) / dg; up_p = up; lw_p = lf;
+        avm_km1 = avm_k;
+        avm_k = avm_kp1;
+      });
+  // upward sweep: back substitution, the floor, and the buoyancy length (into sd; en: sl)
   T en_p = T(0);
-  for (int k = jpk - 1; k >= 2; --k) {
-    const long q = c3 + (long)(k - 1) * n2;
-    const T en = (k == jpk - 1) ? a.zd_lw[q] / a.zdiag[q] : (a.zd_lw[q] - a.zd_up[q] * en_p) / a.zdiag[q];
-    en_p = en;
-    const T e = fmx(en, a.rn_emin) * wmsk<T>(ci, k);
-    a.en[q] = e;
-    a.zdiag[q] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(a.rn2[q], a.rsmall)));
-  }
-  T* zmxlm = a.zdiag;
-  T* zmxld = a.zd_up;
+  march<T, 1>(
+      2, jpk - 1, [&](int x, T (&l)[1]) { l[0] = __ldg(a.rn2 + c3 + (long)(jpk - x) * n2); },
+      [&](int x, T (&l)[1]) {
+        const int k = jpk + 1 - x;
+        const T en = (k == jpk - 1) ? sl[k * nt] / sd[k * nt] : (sl[k * nt] - su[k * nt] * en_p) / sd[k * nt];
+        en_p = en;
+        const T e = fmx(en, a.rn_emin) * wmsk<T>(ci, k);
+        a.en[c3 + (long)(k - 1) * n2] = e;
+        sl[k * nt] = e;
+        sd[k * nt] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(l[0], a.rsmall)));
+      });
   const T mxl1 = a.ln_mxl0 ? fmx(a.rn_mxl0, a.zraug * taum * tm1) : a.rn_mxl0;
-  // downward limits of nn_mxl = 2 (zmxlm) and 3 (zmxld, from the unlimited zmxlm)
-  if (a.nn_mxl == 2) {
+  // downward limits of nn_mxl = 2 (in place) and 3 (su, from the unlimited lengths)
+  if (a.nn_mxl == 2 || a.nn_mxl == 3) {
+    T* const out = a.nn_mxl == 2 ? sd : su;
     T p = mxl1;
     for (int k = 2; k <= jpk - 1; ++k) {
-      const long q = c3 + (long)(k - 1) * n2;
-      p = fmn(p + d.e3t_n(ij, k - 1, m), zmxlm[q]);
-      zmxlm[q] = p;
-    }
-  } else if (a.nn_mxl == 3) {
-    T p = mxl1;
-    for (int k = 2; k <= jpk - 1; ++k) {
-      const long q = c3 + (long)(k - 1) * n2;
-      p = fmn(p + d.e3t_n(ij, k - 1, m), zmxlm[q]);
-      zmxld[q] = p;
+      p = fmn(p + d.e3t_n(ij, k - 1, m), sd[k * nt]);
+      out[k * nt] = p;
     }
   }
   // upward sweep: the limited lengths, the coefficients, the ocean Kz
   const T evd = a.rn_evd;
   T nxt = a.rmxl_min;  // zmxlm(jpk)
+#pragma unroll 2
   for (int k = jpk - 1; k >= 2; --k) {
     const long q = c3 + (long)(k - 1) * n2;
     const T wm = wmsk<T>(ci, k), tm = tmsk<T>(ci, k);
-    const T raw = zmxlm[q];
+    const T raw = sd[k * nt];
     T lm, ld;
     if (a.nn_mxl == 2) {
       lm = fmn(nxt + d.e3t_n(ij, k + 1, m), raw);
@@ -1578,7 +1703,7 @@ __global__ void k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
     } else if (a.nn_mxl == 3) {
       const T dn = fmn(nxt + d.e3t_n(ij, k + 1, m), raw);
       nxt = dn;
-      const T lu = zmxld[q];
+      const T lu = su[k * nt];
       lm = fmn(lu, dn);
       ld = sqrt(lu * dn);
     } else if (a.nn_mxl == 1) {
@@ -1590,16 +1715,16 @@ __global__ void k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
       lm = z * wm + fmn(raw, e3w) * (T(1) - wm);
       ld = z * wm + fmn(lm, e3w) * (T(1) - wm);
     }
-    const T zsqen = sqrt(a.en[q]);
+    const T zsqen = sqrt(sl[k * nt]);
     const T zav = a.rn_ediff * lm * zsqen;
     const T avmk = fmx(zav, a.rn_avm0) * wm;
     T avtk = fmx(zav, a.rn_avt0) * wm;
     a.dissl[q] = zsqen / ld;
-    if (a.nn_pdl == 1) avtk = fmx(a.apdlr[q] * avtk, a.rn_avt0) * tm;
+    if (a.nn_pdl == 1) avtk = fmx(sp[k * nt] * avtk, a.rn_avt0) * tm;
     a.avm_k[q] = avmk;
     a.avt_k[q] = avtk;
     T avt = avtk, avm = avmk;
-    if (a.ln_zdfevd && fmn(a.rn2[q], a.rn2b[q]) <= T(-1.e-12)) {
+    if (evd_at >> (k - 1) & 1) {
       avt = evd * wm;
       if (a.nn_evdm == 1) avm = evd * wm;
     }
