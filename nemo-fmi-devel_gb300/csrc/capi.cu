@@ -441,6 +441,7 @@ template <class T>
 int build_dom(nemo_ctx* c, DomStore<T>& st) {
   Dom<T>& d = st.d;
   d.jpi = c->jpi; d.jpj = c->jpj; d.jpk = c->jpk; d.nmem = c->nmem; d.n2 = c->n2; d.n3 = c->n3;
+  d.kch = tra_chunk(c->n2, c->nmem, c->jpk, sizeof(T) == 8);
   int s = 0;
 #define UP(name) if ((s = upload(c, st, c->name, &d.name))) return s
   UP(e1t); UP(e2t); UP(e1u); UP(e2u); UP(e1v); UP(e2v);

@@ -19,10 +19,10 @@ static dim3 col_grid(const Dom<T>& d, int ty = BY) {
   return dim3((d.jpi + BX - 1) / BX, (d.jpj + ty - 1) / ty, d.nmem);
 }
 
-// one thread per KCH-level chunk of a column: z = member * nchunk + chunk
+// one thread per kch-level chunk of a column: z = member * nchunk + chunk
 template <class T>
 static dim3 kc_grid(const Dom<T>& d, int ty = BY) {
-  return dim3((d.jpi + BX - 1) / BX, (d.jpj + ty - 1) / ty, d.nmem * ((d.jpk + KCH - 1) / KCH));
+  return dim3((d.jpi + BX - 1) / BX, (d.jpj + ty - 1) / ty, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
 }
 
 // one thread per (i,j,k) point: z = member * jpk + (k - 1)
@@ -73,7 +73,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
   if (hot_fct_ok(d, a) && !a.lim) {  // the limiter is recorded by k_fct_c only
     if constexpr (sizeof(T) == 4) {
       if (a.tma && a.err && a.kjpt == 2) {  // planes staged by TMA
-        if (a.fused) {  // the three stages in one kernel
+        if (a.fused && a.trp && !a.pta_in) {  // the three stages in one kernel
           PlaneMaps<FF_NIN> maps;
           const bool ok = field_tensor_map(d, a.pun.p, 1, FF_BW, FF_BH, &maps.m[0]) &&
                           field_tensor_map(d, a.pvn.p, 1, FF_BW, FF_BH, &maps.m[1]) &&
@@ -111,7 +111,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
                 cudaFuncSetAttribute(k_fct_b_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
             if (attr_a != cudaSuccess) return attr_a;
             if (attr_b != cudaSuccess) return attr_b;
-            const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + KCH - 1) / KCH));
+            const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
             k_fct_a_tma<T><<<grid, dim3(TM_X, TM_Y), FA_SMEM, s>>>(d, a, ma, a.err, a.polls);
             ktick(NEMO_K_FCT_A_TMA, s);
             k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);
@@ -125,11 +125,14 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
       }
     }
     const int ta = kty(NEMO_K_FCT_A), tb = kty(NEMO_K_FCT_B), tc = kty(NEMO_K_FCT_C);
-    k_fct_a_hot<T><<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
+    (a.trp ? k_fct_a_hot<T, true> : k_fct_a_hot<T, false>)<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_A, s);
     k_fct_b_hot<T><<<kc_grid(d, tb), dim3(BX, tb), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_B, s);
-    k_fct_c_hot<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
+    // FP64 without the iso-neutral trend: the general kernel, two tracers a pass, is the
+    // faster (259 against 346 us at 362x242x31); with it (more loads a level) the other is
+    if (sizeof(T) == 8 && !a.with_iso) k_fct_c<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
+    else k_fct_c_hot<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_C, s);
     return cudaGetLastError();
   }
@@ -171,7 +174,7 @@ cudaError_t launch_iso_flux(const Dom<T>& d, const LdfArgs<T>& a, cudaStream_t s
           field_tensor_map(d, a.vslp.p, 1, TM_X, TM_Y, &maps.vslp) &&
           field_tensor_map(d, a.wslpi.p, 1, TM_X, TM_Y, &maps.wslpi) &&
           field_tensor_map(d, a.wslpj.p, 1, TM_X, TM_Y, &maps.wslpj)) {
-        const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + KCH - 1) / KCH));
+        const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
         k_iso_flux_tma<T><<<grid, dim3(TM_X, TM_Y), 0, s>>>(d, a, maps, a.err, a.polls);
         ktick(NEMO_K_ISO_FLUX_TMA, s);
         return cudaGetLastError();
@@ -191,7 +194,7 @@ cudaError_t launch_iso_flux(const Dom<T>& d, const LdfArgs<T>& a, cudaStream_t s
 template <class T>
 cudaError_t launch_iso_edges(const Dom<T>& d, const LdfArgs<T>& a, int copy_akz_edges, int msc_edges, cudaStream_t s) {
   if (copy_akz_edges && !hot_iso_ok(d, a)) {  // the specialised flux kernel copies them itself
-    k_iso_akz_copy_edges<T><<<col_grid(d), dim3(BX, BY), 0, s>>>(d, a);
+    k_iso_akz_copy_edges<T><<<dim3((unsigned)((d.n2 + 255) / 256), 1, 2 * d.nmem), 256, 0, s>>>(d, a);
     ktick(NEMO_K_ISO_AKZ_EDGES, s);
   }
   if (msc_edges) {

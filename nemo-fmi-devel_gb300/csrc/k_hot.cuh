@@ -65,6 +65,15 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
   const T e2_e1u = d.e2_e1u[ij], e1_e2v = d.e1_e2v[ij], e2u = d.e2u[ij], e1v = d.e1v[ij];
   const T e2t = icol ? d.e2t[ij] : T(0), e1t = icol ? d.e1t[ij] : T(0);
   const T aht = a.aht_c;
+  // FP64: the products of a column's constants once, and the averaged diffusivity of a
+  // w-point by the number n of its wet neighbours (the sums of n equal terms, whichever
+  // they are), off the FP64 pipe; the operations and their order are those below
+  constexpr bool D = sizeof(T) == 8;
+  const T abe1c = aht * e2_e1u, abe2c = aht * e1_e2v, cof1c = -aht * e2u, cof2c = -aht * e1v;
+  const T ah3 = ((aht + aht) + aht) * Third<T>::v, ah4 = (((aht + aht) + aht) + aht) * T(0.25);
+  const T cw3 = -ah4 * e2t * T(0.25), cw4 = -ah4 * e1t * T(0.25);  // zcoef3, zcoef4 at n = 4 before the slope
+  auto by_count = [&](int n) -> T { return n == 4 ? ah4 : n == 3 ? ah3 : n > 0 ? aht : T(0); };
+  auto wet = [](T m) { return __double2hiint((double)m) != 0 ? 1 : 0; };
   const T* e3u = d.e3u_n.p.p;
   const T* e3v = d.e3v_n.p.p;
   const long m3 = (long)c.m * d.n3;
@@ -110,14 +119,22 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
       const T wke = k == 1 ? te_ : msel(te_, tem), wk1e = msel(tep, te_);
       const T wkn = k == 1 ? tn_ : msel(tn_, tnm), wk1n = msel(tnp, tn_);
       // horizontal fluxes' coefficients (:255-276)
-      T pah = msel(aht, u0);
-      const T zabe1 = pah * e2_e1u * __ldg(e3u + k - 1);
       const T zmsku_h = rcount4(wke, wk1, wk1e, wk);
-      const T zcof1 = -pah * e2u * __ldg(uslp + q) * zmsku_h;
-      pah = msel(aht, v0);
-      const T zabe2 = pah * e1_e2v * __ldg(e3v + k - 1);
       const T zmskv_h = rcount4(wkn, wk1, wk1n, wk);
-      const T zcof2 = -pah * e1v * __ldg(vslp + q) * zmskv_h;
+      T zabe1, zabe2, zcof1, zcof2;
+      if constexpr (D) {  // of a wet face; the flux of a dry one is selected to 0
+        zabe1 = abe1c * __ldg(e3u + k - 1);
+        zcof1 = cof1c * __ldg(uslp + q) * zmsku_h;
+        zabe2 = abe2c * __ldg(e3v + k - 1);
+        zcof2 = cof2c * __ldg(vslp + q) * zmskv_h;
+      } else {
+        T pah = msel(aht, u0);
+        zabe1 = pah * e2_e1u * __ldg(e3u + k - 1);
+        zcof1 = -pah * e2u * __ldg(uslp + q) * zmsku_h;
+        pah = msel(aht, v0);
+        zabe2 = pah * e1_e2v * __ldg(e3v + k - 1);
+        zcof2 = -pah * e1v * __ldg(vslp + q) * zmskv_h;
+      }
       // vertical flux coefficients and ah_wslp2 = akz (:146-164, :200-201, :291-321).
       // The term (ah_wslp2 - akz) * dk(tb) of :323-332 is an exact 0 here (akz =
       // ah_wslp2) and adding it changes no value, so it is left out.
@@ -126,14 +143,25 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
       if (vface) {
         const T zmsku = msel(rcount4(u0m, uw, uwm, u0), wk);
         const T zmskv = msel(rcount4(v0m, vs, vsm, v0), wk);
-        const T zahu_w = (msel(aht, u0m) + msel(aht, uw) + msel(aht, uwm) + msel(aht, u0)) * zmsku;
-        const T zahv_w = (msel(aht, v0m) + msel(aht, vs) + msel(aht, vsm) + msel(aht, v0)) * zmskv;
+        T zahu_w, zahv_w;
+        int nu = 0, nv = 0;
+        if constexpr (D) {
+          if (wet(wk)) {
+            nu = wet(u0m) + wet(uw) + wet(uwm) + wet(u0);
+            nv = wet(v0m) + wet(vs) + wet(vsm) + wet(v0);
+          }
+          zahu_w = by_count(nu);
+          zahv_w = by_count(nv);
+        } else {
+          zahu_w = (msel(aht, u0m) + msel(aht, uw) + msel(aht, uwm) + msel(aht, u0)) * zmsku;
+          zahv_w = (msel(aht, v0m) + msel(aht, vs) + msel(aht, vsm) + msel(aht, v0)) * zmskv;
+        }
         const T wi = __ldg(wslpi + q), wj = __ldg(wslpj + q);
         const T ahw = zahu_w * wi * wi + zahv_w * wj * wj;
         ahw_out[q] = ahw;
         akz_out[q] = ahw;
-        zcoef3 = -zahu_w * e2t * zmsku * wi;
-        zcoef4 = -zahv_w * e1t * zmskv * wj;
+        zcoef3 = D && nu == 4 ? cw3 * wi : -zahu_w * e2t * zmsku * wi;
+        zcoef4 = D && nv == 4 ? cw4 * wj : -zahv_w * e1t * zmskv * wj;
       }
 #pragma unroll
       for (int nn = 0; nn < NT; ++nn) {
@@ -198,13 +226,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
 template <class T>
 inline bool hot_fct_ok(const Dom<T>& d, const FctArgs<T>& a) {
   auto flat = [](const E3<T>& e) { return e.s == 0 && e.sm == 0; };
-  return a.trp && a.kn_fct_h == 2 && a.kn_fct_v == 2 && !a.pta_in && flat(d.e3t_n) && flat(d.e3t_b) &&
+  return a.kn_fct_h == 2 && a.kn_fct_v == 2 && (long)a.kjpt * d.n3 < (1L << 31) && flat(d.e3t_n) && flat(d.e3t_b) &&
          flat(d.e3t_a) && flat(d.e3u_n) && flat(d.e3v_n);
 }
 
 // FCT stage a (traadv_fct.F90:119-280) of one column chunk; see k_fct_a. Tracer nn
-// of the member is at offset nn * n3 from tracer 0.
-template <class T>
+// of the member is at offset nn * n3 from tracer 0. TRP: pun, pvn, pwn are velocities, to
+// be scaled to transports.
+template <class T, bool TRP>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
@@ -215,11 +244,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T
   T* ay = a.ay + mb;
   T* az = a.az + mb;
   T* ta = a.pta + mb;
-  if (!c.interior) {  // edge columns: every level 0
+  const T* tai = a.pta_in ? a.pta_in + mb : nullptr;
+  if (!c.interior) {  // edge columns: every level 0 (ta: its input)
     for (int k = c.k0; k <= c.k1; ++k)
       for (int n = 0; n < a.kjpt; ++n) {
         const int q = (k - 1) * n2 + n * n3;
-        zwi[q] = T(0); ax[q] = T(0); ay[q] = T(0); az[q] = T(0); ta[q] = T(0);
+        zwi[q] = T(0); ax[q] = T(0); ay[q] = T(0); az[q] = T(0);
+        if (!tai) ta[q] = T(0);
+        else if (tai != ta) ta[q] = tai[q];
       }
     return;
   }
@@ -253,18 +285,21 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T
       if (k == jpk) {  // level jpk: no work, edge values
         for (int nn = 0; nn < nt; ++nn) {
           const int qq = q + no + nn * n3;
-          zwi[qq] = T(0); ax[qq] = T(0); ay[qq] = T(0); az[qq] = T(0); ta[qq] = T(0);
+          zwi[qq] = T(0); ax[qq] = T(0); ay[qq] = T(0); az[qq] = T(0);
+          if (!tai) ta[qq] = T(0);
+          else if (tai != ta) ta[qq] = tai[qq];
         }
         break;
       }
       const bool first = k == k0;
       const T e3uk = __ldg(e3u + k - 1), e3vk = __ldg(e3v + k - 1);
-      const T ue = e2u0 * e3uk * __ldg(un + q);
-      const T uw = e2uw * e3uk * __ldg(un + q - 1);
-      const T vn_ = e1v0 * e3vk * __ldg(vn + q);
-      const T vs = e1vs * e3vk * __ldg(vn + q - jpi);
-      if (first) wt = e1e2t * __ldg(wn + q);
-      const T wb = (k + 1 <= jpk - 1) ? e1e2t * __ldg(wn + q + n2) : T(0);
+      auto scaled = [](T f, T x) { return TRP ? f * x : x; };
+      const T ue = scaled(e2u0 * e3uk, __ldg(un + q));
+      const T uw = scaled(e2uw * e3uk, __ldg(un + q - 1));
+      const T vn_ = scaled(e1v0 * e3vk, __ldg(vn + q));
+      const T vs = scaled(e1vs * e3vk, __ldg(vn + q - jpi));
+      if (first) wt = scaled(e1e2t, __ldg(wn + q));
+      const T wb = (k + 1 <= jpk - 1) ? scaled(e1e2t, __ldg(wn + q + n2)) : T(0);
       const T e3n = __ldg(e3tn + k - 1), e3b = __ldg(e3tb + k - 1), e3a = __ldg(e3ta + k - 1);
       const T r1n = d.r1_e3t[k - 1];  // e3t_n, e3t_b and e3t_a are the one rest-state profile here
       const T tm = tk, wk = k == 1 ? tk : msel(tk, tkm), wk1 = msel(tkp, tk);
@@ -286,7 +321,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T
         const T zwz_t = (k == 1) ? (a.linssh ? wt * tb0 : T(0)) : zwzb[nn];
         const T zwz_b = (k + 1 <= jpk - 1) ? msel(ups(wb, __ldg(tb + q + n2), tb0), wk1) : T(0);
         const T ztra = -(zwx_e - zwx_w + zwy_n - zwy_s + zwz_t - zwz_b) * r1_e1e2t;
-        ta[o + q] = T(0) + msel(divq(ztra, e3n, r1n), tm);
+        ta[o + q] = (tai ? tai[o + q] : T(0)) + msel(divq(ztra, e3n, r1n), tm);
         zwi[o + q] = msel(divq(e3b * tb0 + p2dt * ztra, e3a, r1n), tm);
         // 2nd-order antidiffusive fluxes (:180-190, :255-263)
         const T tn0 = __ldg(tn + q), tne = __ldg(tn + q + 1), tnn = __ldg(tn + q + jpi);

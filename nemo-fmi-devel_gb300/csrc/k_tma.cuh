@@ -127,9 +127,9 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
   __shared__ alignas(8) unsigned long long bar[TM_NS];
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TM_X + tx;
   const int jpi = d.jpi, jpj = d.jpj, jpk = d.jpk, n2 = (int)d.n2;
-  const int nch = (jpk + KCH - 1) / KCH;
+  const int nch = (jpk + d.kch - 1) / d.kch;
   const int m = (int)blockIdx.z / nch, ch = (int)blockIdx.z - m * nch;
-  const int k0 = ch * KCH + 1, k1 = k0 + KCH - 1 < jpk ? k0 + KCH - 1 : jpk;
+  const int k0 = ch * d.kch + 1, k1 = k0 + d.kch - 1 < jpk ? k0 + d.kch - 1 : jpk;
   const int i0 = (int)blockIdx.x * TM_X, j0 = (int)blockIdx.y * TM_Y;  // tile origin (0-based)
   const int i = i0 + tx + 1, j = j0 + ty + 1;
   const bool valid = i <= jpi && j <= jpj;
@@ -657,11 +657,11 @@ template <class T>
 __device__ __forceinline__ TmaBlock tma_block(const Dom<T>& d) {
   TmaBlock b;
   b.tx = threadIdx.x; b.ty = threadIdx.y; b.tid = b.ty * TM_X + b.tx;
-  const int nch = (d.jpk + KCH - 1) / KCH;
+  const int nch = (d.jpk + d.kch - 1) / d.kch;
   b.m = (int)blockIdx.z / nch;
   const int ch = (int)blockIdx.z - b.m * nch;
-  b.k0 = ch * KCH + 1;
-  b.k1 = b.k0 + KCH - 1 < d.jpk ? b.k0 + KCH - 1 : d.jpk;
+  b.k0 = ch * d.kch + 1;
+  b.k1 = b.k0 + d.kch - 1 < d.jpk ? b.k0 + d.kch - 1 : d.jpk;
   b.i0 = (int)blockIdx.x * TM_X; b.j0 = (int)blockIdx.y * TM_Y;
   b.i = b.i0 + b.tx + 1; b.j = b.j0 + b.ty + 1;
   b.valid = b.i <= d.jpi && b.j <= d.jpj;
@@ -694,16 +694,21 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
   T* ay = a.ay + mb;
   T* az = a.az + mb;
   T* ta = a.pta + mb;
-  if (c.valid && !c.icol)  // edge columns: every level 0
+  const T* tai = a.pta_in ? a.pta_in + mb : nullptr;
+  if (c.valid && !c.icol)  // edge columns: every level 0 (ta: its input)
     for (int k = c.k0; k <= c.k1; ++k)
       for (int n = 0; n < a.kjpt; ++n) {
         const int q = (k - 1) * n2 + n * n3;
-        zwi[q] = T(0); ax[q] = T(0); ay[q] = T(0); az[q] = T(0); ta[q] = T(0);
+        zwi[q] = T(0); ax[q] = T(0); ay[q] = T(0); az[q] = T(0);
+        if (!tai) ta[q] = T(0);
+        else if (tai != ta) ta[q] = tai[q];
       }
   const ColInfo ci = c.icol ? d.ci[ij] : ColInfo{};
-  const T e2u0 = c.icol ? d.e2u[ij] : T(0), e2uw = c.icol ? d.e2u[ij - 1] : T(0);
-  const T e1v0 = c.icol ? d.e1v[ij] : T(0), e1vs = c.icol ? d.e1v[ij - jpi] : T(0);
-  const T e1e2t = c.icol ? d.e1e2t[ij] : T(0), r1_e1e2t = c.icol ? d.r1_e1e2t[ij] : T(0);
+  // velocities are scaled to transports; transports are taken as they are (x 1 is exact)
+  const bool trp = a.trp && c.icol;
+  const T e2u0 = trp ? d.e2u[ij] : T(1), e2uw = trp ? d.e2u[ij - 1] : T(1);
+  const T e1v0 = trp ? d.e1v[ij] : T(1), e1vs = trp ? d.e1v[ij - jpi] : T(1);
+  const T e1e2t = trp ? d.e1e2t[ij] : T(1), r1_e1e2t = c.icol ? d.r1_e1e2t[ij] : T(0);
   const T* e3u = d.e3u_n.p.p;
   const T* e3v = d.e3v_n.p.p;
   const T* e3tn = d.e3t_n.p.p;
@@ -735,16 +740,23 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
       if (c.icol)
         for (int nn = 0; nn < a.kjpt; ++nn) {
           const int qq = q + nn * n3;
-          zwi[qq] = T(0); ax[qq] = T(0); ay[qq] = T(0); az[qq] = T(0); ta[qq] = T(0);
+          zwi[qq] = T(0); ax[qq] = T(0); ay[qq] = T(0); az[qq] = T(0);
+          if (!tai) ta[qq] = T(0);
+          else if (tai != ta) ta[qq] = tai[qq];
         }
       break;
+    }
+    T tin[2] = {};  // the trend so far, in flight during the wait
+    if (tai && c.icol) {
+      tin[0] = tai[q];
+      if (a.kjpt > 1) tin[1] = tai[n3 + q];
     }
     ok = ring.wait((unsigned)p + 1, max_polls) && ok;
     if (c.icol) {
       auto L = [&](int f) { return ring.plane((unsigned)p, f); };
       auto L1 = [&](int f) { return ring.plane((unsigned)p + 1, f); };
       const bool first = k == k0;
-      const T e3uk = __ldg(e3u + k - 1), e3vk = __ldg(e3v + k - 1);
+      const T e3uk = trp ? __ldg(e3u + k - 1) : T(1), e3vk = trp ? __ldg(e3v + k - 1) : T(1);
       const T ue = e2u0 * e3uk * L(0)[o];
       const T uw = e2uw * e3uk * L(0)[o - 1];
       const T vn_ = e1v0 * e3vk * L(1)[o];
@@ -771,7 +783,7 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
         const T zwz_t = (k == 1) ? (a.linssh ? wt * tb0 : T(0)) : zwzb[nn];
         const T zwz_b = (k + 1 <= jpk - 1) ? ups(wb, L1(3 + nn)[o], tb0) * wk1 : T(0);
         const T ztra = -(zwx_e - zwx_w + zwy_n - zwy_s + zwz_t - zwz_b) * r1_e1e2t;
-        ta[on + q] = T(0) + ztra / e3n * tm;
+        ta[on + q] = tin[nn] + ztra / e3n * tm;
         zwi[on + q] = (e3b * tb0 + p2dt * ztra) / e3a * tm;
         // 2nd-order antidiffusive fluxes (:180-190, :255-263)
         const T tn0 = TN[o], tne = TN[o + 1], tnn = TN[o + TM_W];

@@ -64,9 +64,21 @@ __device__ __forceinline__ PtIdx pt_index(const Dom<T>& d) {
 }
 
 // k-march kernels: grid x = i, y = j, z = member * nchunk + chunk. A thread walks
-// the levels k0..k1 of one column (KCH levels per chunk), keeping in registers what
-// level k+1 shares with level k, so the vertical neighbours are loaded once.
+// the levels k0..k1 of one column (Dom::kch levels per chunk: KCH, fewer on a grid too
+// small to fill the chip), keeping in registers what level k+1 shares with level k, so
+// the vertical neighbours are loaded once.
 constexpr int KCH = 16;
+// Levels a chunk: the longest of 16, 8, 4, 2 with which the chunks of all columns still
+// give each SM eight warps. A chunk reloads its first level's neighbours, so a large grid
+// keeps 16 (8 costs 25 us of 1.35 ms a step at 752x502x31); at 32x22x31 a march of 16
+// levels is 16 memory round trips in a row on 3 % of the SMs (78 us for the four kernels).
+// In FP64 two warps already fill an SM's FP64 pipe, and what a chunk repeats costs more.
+inline int tra_chunk(long n2, int nmem, int jpk, bool fp64) {
+  const long want = 152L * 32 * (fp64 ? 2 : 8);
+  int c = KCH;
+  while (c > 2 && n2 * nmem * ((jpk + c - 1) / c) < want) c /= 2;
+  return c;
+}
 struct KIdx {
   int i, j, m, k0, k1;
   long ij;
@@ -74,14 +86,14 @@ struct KIdx {
 };
 template <class T>
 __device__ __forceinline__ KIdx k_index(const Dom<T>& d) {
-  const int nch = (d.jpk + KCH - 1) / KCH;
+  const int nch = (d.jpk + d.kch - 1) / d.kch;
   KIdx c;
   c.i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   c.j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   c.m = (int)(blockIdx.z / (unsigned)nch);
   const int ch = (int)blockIdx.z - c.m * nch;
-  c.k0 = ch * KCH + 1;
-  c.k1 = c.k0 + KCH - 1 < d.jpk ? c.k0 + KCH - 1 : d.jpk;
+  c.k0 = ch * d.kch + 1;
+  c.k1 = c.k0 + d.kch - 1 < d.jpk ? c.k0 + d.kch - 1 : d.jpk;
   c.valid = c.i <= d.jpi && c.j <= d.jpj;
   c.interior = c.i >= 2 && c.i <= d.jpi - 1 && c.j >= 2 && c.j <= d.jpj - 1;
   c.ij = (long)(c.i - 1) + (long)(c.j - 1) * d.jpi;
@@ -300,6 +312,21 @@ __device__ __forceinline__ T divr(T x, T y, T ry) {
     return isfinite(q) ? __fmaf_rn(__fmaf_rn(-q, y, x), ry, q) : q;
   }
 }
+// x / e3t_n(k): FP64 through the reciprocal profile where e3t_n is the rest-state profile
+template <class T>
+__device__ __forceinline__ T over_e3t_n(const Dom<T>& d, T x, T e3n, int k) {
+  if constexpr (sizeof(T) == 8) {
+    if (d.r1_e3t && d.e3t_n.s == 0) return divq(x, e3n, d.r1_e3t[k - 1]);
+  }
+  return x / e3n;
+}
+// z * x for z = 1 or -1, off the FP64 pipe
+template <class T>
+__device__ __forceinline__ T signed_by(T z, T x) {
+  if constexpr (sizeof(T) == 8) return z < T(0) ? -x : x;
+  else return z * x;
+}
+
 // Upstream flux 0.5 * ((u + |u|) * tl + (u - |u|) * tr) (traadv_fct.F90:126-136):
 // exactly u * tl for u > 0 and u * tr for u < 0 (the doubled product scales exactly
 // and the other term is an exact 0), formed as one product of the selected value.
@@ -854,8 +881,8 @@ __device__ __forceinline__ T iso_div(const Dom<T>& d, const LdfArgs<T>& a, const
   const RO<T> fu = a.zftu + mo;
   const RO<T> fv = a.zftv + mo;
   const RO<T> fw = a.ztfw + mo;
-  tav = tav + a.zsign * (fu[q] - fu[q - 1] + fv[q] - fv[q - d.jpi]) * r1 / e3tn;
-  tav = tav + a.zsign * (fw[q] - fw[q + d.n2]) * r1 / e3tn;
+  tav = tav + over_e3t_n(d, signed_by(a.zsign, fu[q] - fu[q - 1] + fv[q] - fv[q - d.jpi]) * r1, e3tn, c.k);
+  tav = tav + over_e3t_n(d, signed_by(a.zsign, fw[q] - fw[q + d.n2]) * r1, e3tn, c.k);
   return tav;
 }
 
@@ -928,7 +955,7 @@ __global__ void __launch_bounds__(128) k_fct_c(Dom<T> d, FctArgs<T> a) {
           L[n3 + q] = limit_mult(ay[q], b_d, bu[q + jpi], b_u, bd[q + jpi]);
           L[2 * n3 + qp] = limit_mult(az[qp], bdp, b_u, bup, b_d);
         }
-        T tav = ta[q] - (axl - axlw + ayl - ayls + azt[nn] - azl_b) * r1_e1e2t / e3n;
+        T tav = ta[q] - over_e3t_n(d, (axl - axlw + ayl - ayls + azt[nn] - azl_b) * r1_e1e2t, e3n, k);
         if (a.with_iso) {
           // iso-neutral divergence: horizontal (traldf_iso.F90:278-284), then
           // vertical (:359-366)
@@ -936,8 +963,8 @@ __global__ void __launch_bounds__(128) k_fct_c(Dom<T> d, FctArgs<T> a) {
           const RO<T> fv = a.iso.zftv + mo;
           const RO<T> fw = a.iso.ztfw + mo;
           const T fwb = fw[qp];
-          tav = tav + a.iso.zsign * (fu[q] - fu[q - 1] + fv[q] - fv[q - jpi]) * r1_e1e2t / e3n;
-          tav = tav + a.iso.zsign * (fwt[nn] - fwb) * r1_e1e2t / e3n;
+          tav = tav + over_e3t_n(d, signed_by(a.iso.zsign, fu[q] - fu[q - 1] + fv[q] - fv[q - jpi]) * r1_e1e2t, e3n, k);
+          tav = tav + over_e3t_n(d, signed_by(a.iso.zsign, fwt[nn] - fwb) * r1_e1e2t, e3n, k);
           fwt[nn] = fwb;
         }
         ta[q] = tav;
@@ -974,21 +1001,29 @@ __global__ void k_iso_msc_edges(Dom<T> d, LdfArgs<T> a) {
 
 // akz = ah_wslp2 on the whole array (traldf_iso.F90:200-201) for the points the
 // interior sweep does not write: levels 1 and jpk of interior columns, every level
-// of the edge columns.
+// of the edge columns. Blocks z = 2 member + 0: the two levels, one (i,j) a thread; + 1: the
+// edge columns, one point a thread (a thread that copied a whole edge column waited for
+// jpk memory round trips in a row: 27 us at 500x400x56).
 template <class T>
-__global__ void k_iso_akz_copy_edges(Dom<T> d, LdfArgs<T> a) {
-  ColIdx<T> c = col_index(d);
-  if (!c.valid) return;
-  const long base = (long)c.m * d.n3 + c.ij;
-  if (c.interior) {
-    const long qt = base + (long)(d.jpk - 1) * d.n2;
-    a.akz[base] = a.ah_wslp2[base];
-    a.akz[qt] = a.ah_wslp2[qt];
-    return;
-  }
-  for (int k = 1; k <= d.jpk; ++k) {
-    const long q = base + (long)(k - 1) * d.n2;
-    a.akz[q] = a.ah_wslp2[q];
+__global__ void __launch_bounds__(256) k_iso_akz_copy_edges(Dom<T> d, LdfArgs<T> a) {
+  const long t = (long)blockIdx.x * 256 + threadIdx.x, step = (long)gridDim.x * 256;
+  const long base = (long)(blockIdx.z >> 1) * d.n3;
+  if (blockIdx.z & 1) {
+    const int jpi = d.jpi, per = 2 * jpi + 2 * d.jpj;
+    for (long e = t; e < (long)per * d.jpk; e += step) {
+      const int k = (int)(e / per), x = (int)(e - (long)k * per);
+      const int i = x < 2 * jpi ? x % jpi : (x - 2 * jpi) & 1 ? jpi - 1 : 0;
+      const int j = x < 2 * jpi ? (x < jpi ? 0 : d.jpj - 1) : (x - 2 * jpi) >> 1;
+      const long q = base + (long)k * d.n2 + (long)j * jpi + i;
+      a.akz[q] = a.ah_wslp2[q];
+    }
+  } else {
+    const long bot = base + (long)(d.jpk - 1) * d.n2;
+    for (long p = t; p < d.n2; p += step) {
+      const T x = a.ah_wslp2[base + p], y = a.ah_wslp2[bot + p];
+      a.akz[base + p] = x;
+      a.akz[bot + p] = y;
+    }
   }
 }
 

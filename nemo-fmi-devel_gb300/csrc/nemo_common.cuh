@@ -61,6 +61,7 @@ struct E3 {
 template <class T>
 struct Dom {
   int jpi, jpj, jpk, nmem;
+  int kch;         // levels a thread of the tracer k-marches walks
   long n2, n3;  // points per member of a 2-D / 3-D field
   RO<T> e1t, e2t, e1u, e2u, e1v, e2v;
   RO<T> r1_e1u, r1_e2u, r1_e1v, r1_e2v;
