@@ -131,6 +131,8 @@ struct nemo_ctx {
   bool no_p2_hot = false;  // keep the general sub-step kernel (tests compare both)
   double* gs_part = nullptr;
   double* gs_out = nullptr;
+  double* gs_host = nullptr;      // the result again, in mapped host memory
+  unsigned* gs_ticket = nullptr;  // blocks done, a member
   int gs_nblk = 0;
   double r2dt = 0;
   std::map<int, cudaGraphExec_t> graphs;
@@ -1112,7 +1114,7 @@ int run_usrdef_sbc(nemo_ctx* c) {
   const Dom<T> d = dom<T>(c);
   CK(launch_usr_sbc_a<T>(d, a, c->stream), "usrdef_sbc launch");
   CK(launch_globsum<T>((const T*)F[NEMO_F_EMP], d.tmask_i.p, c->n2, 1, c->nmem, c->gs_part, c->gs_nblk,
-                       c->gs_out, c->stream),
+                       c->gs_ticket, c->gs_out, nullptr, c->stream),
      "usrdef_sbc glob_sum");
   CK(launch_usr_sbc_b<T>(d, a, c->stream), "usrdef_sbc launch");
   return NEMO_OK;
@@ -1960,6 +1962,10 @@ int nemo_gpu_create(const nemo_dom_desc* dm, const nemo_namelist* nam, int nmemb
   c->gs_nblk = c->nsm * 4;
   if (cudaMalloc(&c->gs_part, 2 * (size_t)c->gs_nblk * c->nmem * 8) != cudaSuccess) return bad(NEMO_ERR_NOMEM);
   if (cudaMalloc(&c->gs_out, (size_t)c->nmem * 8) != cudaSuccess) return bad(NEMO_ERR_NOMEM);
+  if (cudaMalloc(&c->gs_ticket, (size_t)c->nmem * sizeof(unsigned)) != cudaSuccess) return bad(NEMO_ERR_NOMEM);
+  cudaMemset(c->gs_ticket, 0, (size_t)c->nmem * sizeof(unsigned));
+  if (cudaHostAlloc((void**)&c->gs_host, (size_t)c->nmem * 8, cudaHostAllocMapped) != cudaSuccess)
+    return bad(NEMO_ERR_NOMEM);
   // work arrays of the hot path allocated here, so graph capture never allocates
   if (ensure_fct_work(c, 2, c->nam.nn_fct_v == 4)) return bad(NEMO_ERR_NOMEM);
   if ((c->nam.ln_traldf_iso || c->nam.ln_traldf_triad) && ensure_iso_work(c, 2)) return bad(NEMO_ERR_NOMEM);
@@ -1990,7 +1996,7 @@ int nemo_gpu_destroy(nemo_ctx* c) {
   cudaFree(c->bar_mem); cudaFree(c->err_flag);
   cudaFree(c->ctl_part); cudaFree(c->ctl_out); cudaFree(c->ctl_idx); cudaFree(c->ctl_flag);
   cudaFree(c->hsb_mem); cudaFree(c->hsb_part); cudaFree(c->hsb_state); cudaFree(c->hsb_out);
-  cudaFree(c->gs_part); cudaFree(c->gs_out);
+  cudaFree(c->gs_part); cudaFree(c->gs_out); cudaFree(c->gs_ticket); cudaFreeHost(c->gs_host);
   for (auto e : c->tev)
     if (e) cudaEventDestroy(e);
   for (auto e : c->kc.ev)
@@ -2986,12 +2992,12 @@ int nemo_gpu_glob_sum(nemo_ctx* c, const char* cdname, const void* ptab, int nk,
   if (join_copies(c)) return NEMO_ERR_CUDA;
   const double* tmi = c->prec == NEMO_PREC_FP64 ? c->dd.d.tmask_i.p : c->df.d.tmask_i.p;
   cudaError_t e = is_fp64 ? launch_globsum<double>((const double*)ptab, tmi, c->n2, nk, c->nmem, c->gs_part, c->gs_nblk,
-                                                   c->gs_out, c->stream)
+                                                   c->gs_ticket, c->gs_out, c->gs_host, c->stream)
                           : launch_globsum<float>((const float*)ptab, tmi, c->n2, nk, c->nmem, c->gs_part, c->gs_nblk,
-                                                  c->gs_out, c->stream);
+                                                  c->gs_ticket, c->gs_out, c->gs_host, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "glob_sum launch");
-  CK(cudaMemcpyAsync(out, c->gs_out, (size_t)c->nmem * 8, cudaMemcpyDeviceToHost, c->stream), "glob_sum result");
   CK(cudaStreamSynchronize(c->stream), "glob_sum");
+  memcpy(out, c->gs_host, (size_t)c->nmem * 8);
   return NEMO_OK;
 }
 

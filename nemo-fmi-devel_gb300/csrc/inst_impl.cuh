@@ -410,9 +410,10 @@ cudaError_t launch_lbc(T* p, int jpi, int jpj, long nslab, int is_f, T pval, cud
 
 template <class T>
 cudaError_t launch_globsum(const T* x, const double* tmask_i, long n2, int nk, int nmem, double* part, int nblk,
-                           double* out, cudaStream_t s) {
-  k_globsum_partial<T><<<dim3(nblk, nmem), 256, 0, s>>>(x, tmask_i, n2, nk, part);
-  k_globsum_final<<<nmem, 256, 0, s>>>(part, nblk, out);
+                           unsigned* ticket, double* out, double* out_host, cudaStream_t s) {
+  const long need = (n2 * nk + 256L * GS_PT - 1) / (256L * GS_PT);
+  k_globsum<T><<<dim3((unsigned)(need < nblk ? need : nblk), nmem), 256, 0, s>>>(x, tmask_i, n2, nk, part, ticket, out,
+                                                                                out_host);
   return cudaGetLastError();
 }
 
@@ -430,6 +431,7 @@ cudaError_t launch_globsum(const T* x, const double* tmask_i, long n2, int nk, i
   template int spg_res_clusters<T>(int, int, int, int, int);                                                      \
   template int spg_p2_ene_blocks_per_sm<T>();                                                                 \
   template cudaError_t launch_lbc<T>(T*, int, int, long, int, T, cudaStream_t);                              \
-  template cudaError_t launch_globsum<T>(const T*, const double*, long, int, int, double*, int, double*, cudaStream_t);
+  template cudaError_t launch_globsum<T>(const T*, const double*, long, int, int, double*, int, unsigned*, double*, \
+                                         double*, cudaStream_t);
 
 }  // namespace nemo

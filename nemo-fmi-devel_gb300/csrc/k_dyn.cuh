@@ -1565,4 +1565,123 @@ static __global__ void k_globsum_final(const double* __restrict__ part, int nblk
   if (threadIdx.x == 0) out[m] = sh[0][0];
 }
 
+// the pair (hi, lo) of every thread of a block, summed into thread 0's; sh: 2 x 256 doubles
+__device__ __forceinline__ void dd_block_sum(double& hi, double& lo, double (&sh)[2][256]) {
+  const int t = threadIdx.x;
+  sh[0][t] = hi;
+  sh[1][t] = lo;
+  __syncthreads();
+  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    if (t < s) {
+      dd_add(hi, lo, sh[0][t + s], sh[1][t + s]);
+      sh[0][t] = hi;
+      sh[1][t] = lo;
+    }
+    __syncthreads();
+  }
+}
+// a normal or zero float as double, on the integer pipe
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
+  const unsigned h = e ? ((b >> 3) & 0x0fffffffu) + 0x38000000u : 0u;
+  return __hiloint2double((int)((b & 0x80000000u) | h), (int)(b << 29));
+}
+
+// One block's share of the sum, GS_PT points a thread and pass; the last block of a member
+// to finish adds the blocks' pairs and writes the result. FP64 runs at 1/58 of the FP32
+// rate, so the double-double additions bound this kernel (11 operations a point, and eight
+// serial levels of them in the tree). FP32 fields mostly need none: where the exponents of
+// the points a block adds in one pass span at most 53 - 24 - 12 = 17 binary places, every
+// partial sum of the 2^12 values is exact in a double (24 bits each, 12 bits of carry), and
+// so plain additions give the exact sum of the pass; any other pass (and FP64) takes the
+// double-double path. 38 -> 9 us (one launch instead of two) at 2 x 93x61x62.
+constexpr int GS_PT = 16;
+template <class T>
+__global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const double* __restrict__ tmask_i, long n2,
+                                                 int nk, double* __restrict__ part, unsigned* __restrict__ ticket,
+                                                 double* __restrict__ out, volatile double* out_host) {
+  __shared__ double sh[2][256];
+  __shared__ int s_min[8], s_max[8];
+  __shared__ bool s_last;
+  const int m = blockIdx.y, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const long n = n2 * nk, step = (long)gridDim.x * 256 * GS_PT;
+  const T* xm = x + (long)m * n;
+  double hi = 0.0, lo = 0.0;  // thread 0 of the exact passes, every thread of the others
+  for (long e0 = (long)blockIdx.x * 256 * GS_PT; e0 < n; e0 += step) {
+    T v[GS_PT];
+    long p = (e0 + t) % n2;  // point of the 2-D mask
+#pragma unroll
+    for (int i = 0; i < GS_PT; ++i) {
+      const long e = e0 + i * 256 + t;
+      v[i] = e < n ? xm[e] * (tmask_i[p] != 0.0 ? T(1) : T(0)) : T(0);  // tmask_i is 0 or 1
+      p += 256;
+      while (p >= n2) p -= n2;
+    }
+    bool exact = false;
+    if constexpr (sizeof(T) == 4) {
+      int emin = 255, emax = 0;
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < GS_PT; ++i) {
+        const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
+        const int e = (int)(b >> 23);
+        bad |= e == 255 || (e == 0 && b != 0);  // not finite, or denormal
+        if (b != 0) {
+          emin = min(emin, e);
+          emax = max(emax, e);
+        }
+      }
+      emin = __reduce_min_sync(0xffffffffu, bad ? -256 : emin);
+      emax = __reduce_max_sync(0xffffffffu, emax);
+      if (lane == 0) {
+        s_min[w] = emin;
+        s_max[w] = emax;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        emin = min(emin, s_min[i]);
+        emax = max(emax, s_max[i]);
+      }
+      exact = emax - emin <= 17;
+      if (exact) {
+        double s = widen(v[0]);
+#pragma unroll
+        for (int i = 1; i < GS_PT; ++i) s += widen(v[i]);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sh[0][w] = s;
+        __syncthreads();
+        if (t == 0) {
+          s = sh[0][0];
+          for (int i = 1; i < 8; ++i) s += sh[0][i];
+          dd_add(hi, lo, s, 0.0);
+        }
+      }
+      __syncthreads();  // s_min, s_max and sh are written again
+    }
+    if (!exact)
+      for (int i = 0; i < GS_PT; ++i) dd_add(hi, lo, (double)v[i], 0.0);
+  }
+  // threads other than 0 hold something only after a pass that was not exact
+  if (__syncthreads_or(t != 0 && (hi != 0.0 || lo != 0.0))) dd_block_sum(hi, lo, sh);
+  if (t == 0) {
+    part[2 * ((long)m * gridDim.x + blockIdx.x)] = hi;
+    part[2 * ((long)m * gridDim.x + blockIdx.x) + 1] = lo;
+    __threadfence();
+    s_last = atomicAdd(&ticket[m], 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const volatile double* pv = part + 2 * (long)m * gridDim.x;
+  hi = lo = 0.0;
+  for (int b = t; b < (int)gridDim.x; b += 256) dd_add(hi, lo, pv[2 * b], pv[2 * b + 1]);
+  dd_block_sum(hi, lo, sh);
+  if (t == 0) {
+    ticket[m] = 0;  // for the next launch
+    out[m] = hi;
+    if (out_host) out_host[m] = hi;
+  }
+}
+
 }  // namespace nemo

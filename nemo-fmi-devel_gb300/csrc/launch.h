@@ -66,6 +66,6 @@ template <class T>
 cudaError_t launch_lbc(T* p, int jpi, int jpj, long nslab, int is_f, T pval, cudaStream_t s);
 template <class T>
 cudaError_t launch_globsum(const T* x, const double* tmask_i, long n2, int nk, int nmem, double* part, int nblk,
-                           double* out, cudaStream_t s);
+                           unsigned* ticket, double* out, double* out_host, cudaStream_t s);
 
 }  // namespace nemo
