@@ -68,6 +68,26 @@ static bool field_tensor_map(const Dom<T>& d, const T* base, int nf, unsigned bx
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// the tensor maps of stage b's planes (two tracers each); false: no TMA
+template <class T>
+static bool fct_b_maps(const Dom<T>& d, const FctArgs<T>& a, PlaneMaps<FB_NF>& mb) {
+  const T* fb[5] = {a.ptb.p, a.zwi, a.ax, a.ay, a.az};
+  for (int f = 0; f < 5; ++f) {
+    if (!field_tensor_map(d, fb[f], 2, TM_W, TM_H, &mb.m[2 * f])) return false;
+    mb.m[2 * f + 1] = mb.m[2 * f];
+  }
+  return true;
+}
+// the instance of the general stage a for a call's orders and transports
+template <class T, class I>
+static auto fct_a_of(const FctArgs<T>& a) {
+  const bool h = a.kn_fct_h == 4, v = a.kn_fct_v == 4;
+  if (a.trp)
+    return h ? (v ? k_fct_a<T, I, true, true, true> : k_fct_a<T, I, true, false, true>)
+             : (v ? k_fct_a<T, I, false, true, true> : k_fct_a<T, I, false, false, true>);
+  return h ? (v ? k_fct_a<T, I, true, true, false> : k_fct_a<T, I, true, false, false>)
+           : (v ? k_fct_a<T, I, false, true, false> : k_fct_a<T, I, false, false, false>);
+}
 template <class T>
 cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
   if (hot_fct_ok(d, a) && !a.lim) {  // the limiter is recorded by k_fct_c only
@@ -99,52 +119,74 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
                     field_tensor_map(d, a.ptn.p, 2, TM_W, TM_H, &ma.m[5]);
           ma.m[4] = ma.m[3];  // tb, tn: one map each, read at the two tracers' levels
           ma.m[6] = ma.m[5];
-          const T* fb[5] = {a.ptb.p, a.zwi, a.ax, a.ay, a.az};
-          for (int f = 0; f < 5 && ok; ++f) {
-            ok = field_tensor_map(d, fb[f], 2, TM_W, TM_H, &mb.m[2 * f]);
-            mb.m[2 * f + 1] = mb.m[2 * f];
-          }
+          ok = ok && fct_b_maps(d, a, mb);
           if (ok) {
             static const cudaError_t attr_a =
-                cudaFuncSetAttribute(k_fct_a_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
+                cudaFuncSetAttribute(k_fct_a_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
+            static const cudaError_t attr_a2 =
+                cudaFuncSetAttribute(k_fct_a_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
             static const cudaError_t attr_b =
                 cudaFuncSetAttribute(k_fct_b_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
             if (attr_a != cudaSuccess) return attr_a;
+            if (attr_a2 != cudaSuccess) return attr_a2;
             if (attr_b != cudaSuccess) return attr_b;
             const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
-            k_fct_a_tma<T><<<grid, dim3(TM_X, TM_Y), FA_SMEM, s>>>(d, a, ma, a.err, a.polls);
+            (a.trp && !a.pta_in ? k_fct_a_tma<T, true> : k_fct_a_tma<T, false>)<<<grid, dim3(TM_X, TM_Y), FA_SMEM, s>>>(
+                d, a, ma, a.err, a.polls);
             ktick(NEMO_K_FCT_A_TMA, s);
             k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);
             ktick(NEMO_K_FCT_B_TMA, s);
             const int tc = kty(NEMO_K_FCT_C);
-            k_fct_c_hot<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
+            k_fct_c_hot<T, false><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
             ktick(NEMO_K_FCT_C, s);
             return cudaGetLastError();
           }
         }
       }
     }
-    const int ta = kty(NEMO_K_FCT_A), tb = kty(NEMO_K_FCT_B), tc = kty(NEMO_K_FCT_C);
+    const int ta = kty(NEMO_K_FCT_A);
     (a.trp ? k_fct_a_hot<T, true> : k_fct_a_hot<T, false>)<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_A, s);
-    k_fct_b_hot<T><<<kc_grid(d, tb), dim3(BX, tb), 0, s>>>(d, a);
+  } else {
+    if (a.kn_fct_v == 4) {
+      const int smem = 32 * I4_Y * (d.jpk + 1) * (int)sizeof(T);
+      static const cudaError_t attr = cudaFuncSetAttribute(k_interp4<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           32 * I4_Y * (KMAX + 1) * (int)sizeof(T));
+      if (attr != cudaSuccess) return attr;
+      k_interp4<T><<<dim3((d.jpi + 31) / 32, (d.jpj + I4_Y - 1) / I4_Y, d.nmem * a.kjpt), dim3(32, I4_Y), smem, s>>>(
+          d, a.ptn, const_cast<T*>(a.ztw.p), a.kjpt);
+      ktick(NEMO_K_INTERP4, s);
+    }
+    const bool small = (long)a.kjpt * d.n3 < (1L << 31);
+    const auto kern = small ? fct_a_of<T, int>(a) : fct_a_of<T, long>(a);
+    kern<<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
+    ktick(NEMO_K_FCT_A, s);
+  }
+  bool b_done = false;
+  if constexpr (sizeof(T) == 4) {  // stage b takes any e3t_n (its planes staged by TMA: any orders of stage a)
+    PlaneMaps<FB_NF> mb;
+    if (a.tma && a.err && a.kjpt == 2 && !a.lim && d.n3 < (1L << 30) && fct_b_maps(d, a, mb)) {
+      static const cudaError_t attr =
+          cudaFuncSetAttribute(k_fct_b_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
+      if (attr != cudaSuccess) return attr;
+      const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
+      k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);
+      ktick(NEMO_K_FCT_B_TMA, s);
+      b_done = true;
+    }
+  }
+  if (!b_done) {
+    const int tb = kty(NEMO_K_FCT_B);
+    if (hot_fct_ok(d, a) && !a.lim) k_fct_b_hot<T><<<kc_grid(d, tb), dim3(BX, tb), 0, s>>>(d, a);
+    else k_fct_b<T><<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_B, s);
-    // FP64 without the iso-neutral trend: the general kernel, two tracers a pass, is the
-    // faster (259 against 346 us at 362x242x31); with it (more loads a level) the other is
-    if (sizeof(T) == 8 && !a.with_iso) k_fct_c<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
-    else k_fct_c_hot<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
-    ktick(NEMO_K_FCT_C, s);
-    return cudaGetLastError();
   }
-  if (a.kn_fct_v == 4) {
-    k_interp4<T><<<col_grid(d), dim3(BX, BY), 0, s>>>(d, a.ptn, const_cast<T*>(a.ztw.p), a.kjpt);
-    ktick(NEMO_K_INTERP4, s);
-  }
-  k_fct_a<T><<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
-  ktick(NEMO_K_FCT_A, s);
-  k_fct_b<T><<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
-  ktick(NEMO_K_FCT_B, s);
-  k_fct_c<T><<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
+  const int tc = kty(NEMO_K_FCT_C);
+  // FP64 without the iso-neutral trend: the general kernel, two tracers a pass, is the
+  // faster (259 against 346 us at 362x242x31); with it (more loads a level) the other is
+  if (!hot_fct_c_ok(d, a) || (sizeof(T) == 8 && !a.with_iso)) k_fct_c<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
+  else if (d.e3t_n.s == 0) k_fct_c_hot<T, false><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
+  else k_fct_c_hot<T, true><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
   ktick(NEMO_K_FCT_C, s);
   return cudaGetLastError();
 }
@@ -175,13 +217,14 @@ cudaError_t launch_iso_flux(const Dom<T>& d, const LdfArgs<T>& a, cudaStream_t s
           field_tensor_map(d, a.wslpi.p, 1, TM_X, TM_Y, &maps.wslpi) &&
           field_tensor_map(d, a.wslpj.p, 1, TM_X, TM_Y, &maps.wslpj)) {
         const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
-        k_iso_flux_tma<T><<<grid, dim3(TM_X, TM_Y), 0, s>>>(d, a, maps, a.err, a.polls);
+        (iso_3d(d, a) ? k_iso_flux_tma<T, true> : k_iso_flux_tma<T, false>)<<<grid, dim3(TM_X, TM_Y), 0, s>>>(
+            d, a, maps, a.err, a.polls);
         ktick(NEMO_K_ISO_FLUX_TMA, s);
         return cudaGetLastError();
       }
     }
     const int ti = kty(NEMO_K_ISO_FLUX);
-    k_iso_flux_hot<T><<<kc_grid(d, ti), dim3(BX, ti), 0, s>>>(d, a);
+    (iso_3d(d, a) ? k_iso_flux_hot<T, true> : k_iso_flux_hot<T, false>)<<<kc_grid(d, ti), dim3(BX, ti), 0, s>>>(d, a);
   } else {
     k_iso_flux<T><<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
   }

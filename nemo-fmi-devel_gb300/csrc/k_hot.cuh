@@ -1,7 +1,9 @@
-// k_hot.cuh -- the tracer kernels specialised for the configuration of the hot path:
-// horizontally uniform e3 (1-D profiles), constant eddy diffusivity (aht0 * mask),
-// no partial steps, standard iso-neutral operator (akz = ah_wslp2), laplacian,
-// first pass. Other configurations use the general kernels of k_tra.cuh.
+// k_hot.cuh -- the tracer kernels specialised for the configurations of the hot path:
+// constant eddy diffusivity (aht0 * mask), standard iso-neutral operator (akz = ah_wslp2),
+// laplacian, first pass; FCT 2/2 with horizontally uniform e3 (1-D profiles). Variable
+// volume and partial steps (3-D e3, bottom gradients) are a second instance of the
+// iso-neutral fluxes, and in FP32 the limiter and the final trend take any e3. Other
+// configurations use the general kernels of k_tra.cuh.
 //
 // Same arithmetic, in the same order, as the general kernels (and the reference);
 // what changes is the bookkeeping around it, which dominated the general kernels'
@@ -16,12 +18,16 @@
 
 namespace nemo {
 
-// true when the context's configuration is the one these kernels assume
+// true when the call is one that the specialised iso-neutral kernels take (32-bit offsets
+// within a field), and whether it needs their form for 3-D e3 or partial steps
 template <class T>
 inline bool hot_iso_ok(const Dom<T>& d, const LdfArgs<T>& a) {
+  return !a.pahu && !a.pahv && !a.msc && a.lap && a.kpass == 1 && d.n3 < (1L << 31);
+}
+template <class T>
+inline bool iso_3d(const Dom<T>& d, const LdfArgs<T>& a) {
   auto flat = [](const E3<T>& e) { return e.s == 0 && e.sm == 0; };
-  return !a.pahu && !a.pahv && !a.zps && !a.msc && a.lap && a.kpass == 1 && flat(d.e3u_n) && flat(d.e3v_n) &&
-         flat(d.e3w_n);
+  return a.zps || !flat(d.e3u_n) || !flat(d.e3v_n);
 }
 
 template <class T>
@@ -32,9 +38,12 @@ template <class T>
 __device__ __forceinline__ T v_in(const ColInfo& c, int k) { return (k >= c.vlo && k <= c.vhi) ? T(1) : T(0); }
 
 // Iso-neutral fluxes (traldf_iso.F90:146-357) of one column chunk; see k_iso_flux.
-// It also sets akz = ah_wslp2 on the points k_iso_akz_copy_edges covers in general.
-template <class T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Dom<T> d, LdfArgs<T> a) {
+// It also sets akz = ah_wslp2 on the points k_iso_akz_copy_edges covers in general. G3: 3-D
+// scale factors or partial steps, whose bottom gradients are loaded once a column. The
+// general kernel looks up some forty masks a level and spills at 64 registers: 490 us at
+// 500x400x56 in FP32, 276 in the TMA form of this one.
+template <class T, bool G3>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (G3 ? 5 : 6) : 3) k_iso_flux_hot(Dom<T> d, LdfArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpj = d.jpj, jpk = d.jpk;
@@ -74,8 +83,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
   const T cw3 = -ah4 * e2t * T(0.25), cw4 = -ah4 * e1t * T(0.25);  // zcoef3, zcoef4 at n = 4 before the slope
   auto by_count = [&](int n) -> T { return n == 4 ? ah4 : n == 3 ? ah3 : n > 0 ? aht : T(0); };
   auto wet = [](T m) { return __double2hiint((double)m) != 0 ? 1 : 0; };
-  const T* e3u = d.e3u_n.p.p;
-  const T* e3v = d.e3v_n.p.p;
+  const T* e3u = d.e3u_n.p.p + (G3 ? c.m * d.e3u_n.sm + (long)ij * d.e3u_n.s : 0);
+  const T* e3v = d.e3v_n.p.p + (G3 ? c.m * d.e3v_n.sm + (long)ij * d.e3v_n.s : 0);
+  const int su = G3 ? (int)d.e3u_n.sk : 1, sv = G3 ? (int)d.e3v_n.sk : 1;
   const long m3 = (long)c.m * d.n3;
   const T* uslp = a.uslp.p + m3 + ij;
   const T* vslp = a.vslp.p + m3 + ij;
@@ -96,6 +106,22 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
       fv[nn] = a.zftv + mo;
       fw[nn] = a.ztfw + mo;
     }
+    // partial steps: the bottom gradients of the four faces around, and their levels
+    T gu0[NT] = {}, guw[NT] = {}, gv0[NT] = {}, gvs[NT] = {};
+    if (G3 && a.zps)
+      for (int nn = 0; nn < nt; ++nn) {
+        const long go = ((long)c.m * a.kjpt + n0 + nn) * d.n2 + ij;
+        gu0[nn] = a.pgu[go]; gv0[nn] = a.pgv[go];
+        if (icol) { guw[nn] = a.pgu[go - 1]; gvs[nn] = a.pgv[go - jpi]; }
+      }
+    const int bu0 = G3 && a.zps ? ci.mbku : 0, buw = G3 && a.zps ? ciw.mbku : 0;
+    const int bv0 = G3 && a.zps ? ci.mbkv : 0, bvs = G3 && a.zps ? cis.mbkv : 0;
+    auto grad = [&](T x, T m, int kk, int kb, T g) -> T {  // masked gradient, or the bottom level's
+      if constexpr (G3) {
+        if (kk == kb) return g;
+      }
+      return msel(x, m);
+    };
     // carried masks: T at k-1, k, k+1 of (i,j), (i+1,j), (i,j+1); U at k-1, k of
     // (i,j), (i-1,j); V at k-1, k of (i,j), (i,j-1)
     T t0m = t_in<T>(ci, k0 - 1), t0 = t_in<T>(ci, k0), t0p = t_in<T>(ci, k0 + 1);
@@ -123,16 +149,16 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
       const T zmskv_h = rcount4(wkn, wk1, wk1n, wk);
       T zabe1, zabe2, zcof1, zcof2;
       if constexpr (D) {  // of a wet face; the flux of a dry one is selected to 0
-        zabe1 = abe1c * __ldg(e3u + k - 1);
+        zabe1 = abe1c * __ldg(e3u + (k - 1) * su);
         zcof1 = cof1c * __ldg(uslp + q) * zmsku_h;
-        zabe2 = abe2c * __ldg(e3v + k - 1);
+        zabe2 = abe2c * __ldg(e3v + (k - 1) * sv);
         zcof2 = cof2c * __ldg(vslp + q) * zmskv_h;
       } else {
         T pah = msel(aht, u0);
-        zabe1 = pah * e2_e1u * __ldg(e3u + k - 1);
+        zabe1 = pah * e2_e1u * __ldg(e3u + (k - 1) * su);
         zcof1 = -pah * e2u * __ldg(uslp + q) * zmsku_h;
         pah = msel(aht, v0);
-        zabe2 = pah * e1_e2v * __ldg(e3v + k - 1);
+        zabe2 = pah * e1_e2v * __ldg(e3v + (k - 1) * sv);
         zcof2 = -pah * e1v * __ldg(vslp + q) * zmskv_h;
       }
       // vertical flux coefficients and ah_wslp2 = akz (:146-164, :200-201, :291-321).
@@ -178,10 +204,10 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
             tup[nn] = a0;
             if (icol) {
               const T aw = __ldg(t + qm - 1), as = __ldg(t + qm - jpi);
-              di0[nn] = msel(ae - a0, u0m);
-              diw[nn] = msel(a0 - aw, uwm);
-              dj0[nn] = msel(an - a0, v0m);
-              djs[nn] = msel(a0 - as, vsm);
+              di0[nn] = grad(ae - a0, u0m, k - 1, bu0, gu0[nn]);
+              diw[nn] = grad(a0 - aw, uwm, k - 1, buw, guw[nn]);
+              dj0[nn] = grad(an - a0, v0m, k - 1, bv0, gv0[nn]);
+              djs[nn] = grad(a0 - as, vsm, k - 1, bvs, gvs[nn]);
             }
           }
         }
@@ -192,14 +218,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_iso_flux_hot(Do
         const T dk0_0 = k == 1 ? dk1_0 : k10[nn];
         const T dk0_e = k == 1 ? dk1_e : k1e[nn];
         const T dk0_n = k == 1 ? dk1_n : k1n[nn];
-        const T zdi = msel(te - tc, u0);
-        const T zdj = msel(tn - tc, v0);
+        const T zdi = grad(te - tc, u0, k, bu0, gu0[nn]);
+        const T zdj = grad(tn - tc, v0, k, bv0, gv0[nn]);
         fu[nn][q] = msel(zabe1 * zdi + zcof1 * (dk0_e + dk1_0 + dk1_e + dk0_0), u0);
         fv[nn][q] = msel(zabe2 * zdj + zcof2 * (dk0_n + dk1_0 + dk1_n + dk0_0), v0);
         if (icol) {
           const T tw = __ldg(t + q - 1), ts = __ldg(t + q - jpi);
-          const T zdiw = msel(tc - tw, uw);
-          const T zdjs = msel(tc - ts, vs);
+          const T zdiw = grad(tc - tw, uw, k, buw, guw[nn]);
+          const T zdjs = grad(tc - ts, vs, k, bvs, gvs[nn]);
           T z = T(0);
           if (vface) {
             const T sdi = di0[nn] + zdiw + diw[nn] + zdi;
@@ -228,6 +254,12 @@ inline bool hot_fct_ok(const Dom<T>& d, const FctArgs<T>& a) {
   auto flat = [](const E3<T>& e) { return e.s == 0 && e.sm == 0; };
   return a.kn_fct_h == 2 && a.kn_fct_v == 2 && (long)a.kjpt * d.n3 < (1L << 31) && flat(d.e3t_n) && flat(d.e3t_b) &&
          flat(d.e3t_a) && flat(d.e3u_n) && flat(d.e3v_n);
+}
+
+// stage c reads e3t_n alone: any scale factors in FP32 (FP64 needs their reciprocals)
+template <class T>
+inline bool hot_fct_c_ok(const Dom<T>& d, const FctArgs<T>& a) {
+  return !a.lim && (long)a.kjpt * d.n3 < (1L << 31) && (sizeof(T) == 4 || (d.e3t_n.s == 0 && d.r1_e3t));
 }
 
 // FCT stage a (traadv_fct.F90:119-280) of one column chunk; see k_fct_a. Tracer nn
@@ -435,14 +467,16 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_fct_b_hot(Dom<T
 // divergence (traldf_iso.F90:278-284, :359-366) of one column chunk; see k_fct_c.
 // One tracer per pass over the levels, and every value a level reads is loaded
 // before any of its arithmetic, so a level costs one memory round trip.
-template <class T>
+// G3: e3t_n is a 3-D field.
+template <class T, bool G3>
 __global__ void __launch_bounds__(128) k_fct_c_hot(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid || !c.interior) return;
   const int jpi = d.jpi, jpk = d.jpk, n2 = (int)d.n2, n3 = (int)d.n3, ij = (int)c.ij;
   const long mb = (long)c.m * a.kjpt * d.n3 + ij;
   const T r1_e1e2t = d.r1_e1e2t[ij];
-  const T* e3tn = d.e3t_n.p.p;
+  const T* e3tn = d.e3t_n.p.p + (G3 ? c.m * d.e3t_n.sm + (long)ij * d.e3t_n.s : 0);
+  const int se = G3 ? (int)d.e3t_n.sk : 1;
   const bool w_lim = c.i - 1 >= 2;  // the face i-1 is limited only for i-1 >= 2 (then lbc: 0)
   const bool s_lim = c.j - 1 >= 2;
   const int k1 = c.k1 < jpk - 1 ? c.k1 : jpk - 1;
@@ -468,7 +502,7 @@ __global__ void __launch_bounds__(128) k_fct_c_hot(Dom<T> d, FctArgs<T> a) {
     for (int k = c.k0; k <= k1; ++k, q += n2) {
       const int qp = q + n2;
       // every load of the level first
-      const T e3n = __ldg(e3tn + k - 1);
+      const T e3n = __ldg(e3tn + (k - 1) * se);
       const T bup = __ldg(bu + qp), bdp = __ldg(bd + qp), azp = __ldg(az + qp);
       const T ax0 = __ldg(ax + q), axw = __ldg(ax + q - 1), ay0 = __ldg(ay + q), ays = __ldg(ay + q - jpi);
       const T bue = __ldg(bu + q + 1), bde = __ldg(bd + q + 1), buw = __ldg(bu + q - 1), bdw = __ldg(bd + q - 1);
@@ -485,7 +519,7 @@ __global__ void __launch_bounds__(128) k_fct_c_hot(Dom<T> d, FctArgs<T> a) {
       const T ayl = limit(ay0, bd0, bun, bu0, bdn);
       const T ayls = s_lim ? limit(ays, bds, bu0, bus, bd0) : T(0);
       const T azl_b = limit(azp, bdp, bu0, bup, bd0);
-      const T r1n = d.r1_e3t[k - 1];
+      const T r1n = sizeof(T) == 8 ? d.r1_e3t[k - 1] : T(0);
       T tav = ta0 - divq((axl - axlw + ayl - ayls + azt - azl_b) * r1_e1e2t, e3n, r1n);
       if (iso) {
         tav = tav + divq(zsign * (fu0 - fuw + fv0 - fvs) * r1_e1e2t, e3n, r1n);

@@ -11,14 +11,6 @@
 
 namespace nemo {
 
-// one column of a scale-factor field, or the 1-D profile (stride 1)
-template <class T>
-struct E3Col {
-  const T* p;
-  int st;
-  __device__ __forceinline__ E3Col(const E3<T>& e, long ij, int m) : p(e.p.p + m * e.sm + ij * (long)e.s), st((int)e.sk) {}
-  __device__ __forceinline__ T operator()(int k) const { return __ldg(p + (long)(k - 1) * st); }
-};
 // levels that the column kernels below load before they use the first of them
 template <class T>
 constexpr int BATCH = sizeof(T) == 4 ? 8 : 4;

@@ -117,7 +117,7 @@ struct PlaneRing {
 // (jpi, jpj, jpk * nmem). Same arithmetic in the same order as
 // k_iso_flux_hot; the vertical term (ah_wslp2 - akz) * dk(tb) of :323-332 is exactly 0
 // here (akz = ah_wslp2) and is left out.
-template <class T>
+template <class T, bool G3>
 __global__ void __launch_bounds__(TM_X * TM_Y, 2)
     k_iso_flux_tma(Dom<T> d, LdfArgs<T> a, const __grid_constant__ IsoMaps maps, int* err, int max_polls) {
   static_assert(sizeof(T) == 4, "the TMA kernel is the FP32 form");
@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
     }
   }
   const T aht = a.aht_c;
-  const T* e3u = d.e3u_n.p.p;
-  const T* e3v = d.e3v_n.p.p;
+  const T* e3u = d.e3u_n.p.p + (G3 ? m * d.e3u_n.sm + (long)ij * d.e3u_n.s : 0);
+  const T* e3v = d.e3v_n.p.p + (G3 ? m * d.e3v_n.sm + (long)ij * d.e3v_n.s : 0);
+  const int su = G3 ? (int)d.e3u_n.sk : 1, sv = G3 ? (int)d.e3v_n.sk : 1;
   T* ahw_out = a.ah_wslp2 + m3 + ij;
   T* akz_out = a.akz + m3 + ij;
   const int o = (ty + 1) * TM_W + tx + 4;  // this column in a plane slot
@@ -206,6 +207,22 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
       fv[nn] = a.zftv + mo;
       fw[nn] = a.ztfw + mo;
     }
+    // partial steps: the bottom gradients of the four faces around, and their levels
+    T gu0[2] = {}, guw[2] = {}, gv0[2] = {}, gvs[2] = {};
+    if (G3 && a.zps && face)
+      for (int nn = 0; nn < nt; ++nn) {
+        const long go = ((long)m * a.kjpt + n0 + nn) * d.n2 + ij;
+        gu0[nn] = a.pgu[go]; gv0[nn] = a.pgv[go];
+        if (icol) { guw[nn] = a.pgu[go - 1]; gvs[nn] = a.pgv[go - jpi]; }
+      }
+    const int bu0 = G3 && a.zps ? ci.mbku : 0, buw = G3 && a.zps ? ciw.mbku : 0;
+    const int bv0 = G3 && a.zps ? ci.mbkv : 0, bvs = G3 && a.zps ? cis.mbkv : 0;
+    auto grad = [&](T x, T msk, int kk, int kb, T g) -> T {  // masked gradient, or the bottom level's
+      if constexpr (G3) {
+        if (kk == kb) return g;
+      }
+      return x * msk;
+    };
     // carried masks (as k_iso_flux_hot)
     T t0m = t_in<T>(ci, k0 - 1), t0 = t_in<T>(ci, k0), t0p = t_in<T>(ci, k0 + 1);
     T tem = t_in<T>(cie, k0 - 1), te_ = t_in<T>(cie, k0), tep = t_in<T>(cie, k0 + 1);
@@ -226,10 +243,10 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
         k1n[nn] = (an - __ldg(t + q0 + jpi)) * wkn;
         if (icol) {
           const T aw = __ldg(t + qm - 1), as = __ldg(t + qm - jpi);
-          di0[nn] = (ae - a0) * u0m;
-          diw[nn] = (a0 - aw) * uwm;
-          dj0[nn] = (an - a0) * v0m;
-          djs[nn] = (a0 - as) * vsm;
+          di0[nn] = grad(ae - a0, u0m, k0 - 1, bu0, gu0[nn]);
+          diw[nn] = grad(a0 - aw, uwm, k0 - 1, buw, guw[nn]);
+          dj0[nn] = grad(an - a0, v0m, k0 - 1, bv0, gv0[nn]);
+          djs[nn] = grad(a0 - as, vsm, k0 - 1, bvs, gvs[nn]);
         }
       }
     ok = mbar_wait(&bar[pb % TM_NS], (pb / TM_NS) & 1, max_polls);
@@ -240,6 +257,11 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
         if (icol)
           for (int nn = 0; nn < nt; ++nn) fw[nn][q] = T(0);
         break;
+      }
+      T eu = T(0), ev = T(0);  // in flight during the wait
+      if (face) {
+        eu = __ldg(e3u + (k - 1) * su);
+        ev = __ldg(e3v + (k - 1) * sv);
       }
       const unsigned g1 = pb + (unsigned)p + 1;
       ok = mbar_wait(&bar[g1 % TM_NS], (g1 / TM_NS) & 1, max_polls) && ok;
@@ -252,11 +274,11 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
         const T wkn = k == 1 ? tn_ : tnm * tn_, wk1n = tn_ * tnp;
         // horizontal fluxes' coefficients (:255-276)
         T pah = aht * u0;
-        const T zabe1 = pah * e2_e1u * __ldg(e3u + k - 1);
+        const T zabe1 = pah * e2_e1u * eu;
         const T zmsku_h = rcount(wke + wk1 + wk1e + wk);
         const T zcof1 = -pah * e2u * S0[os] * zmsku_h;
         pah = aht * v0;
-        const T zabe2 = pah * e1_e2v * __ldg(e3v + k - 1);
+        const T zabe2 = pah * e1_e2v * ev;
         const T zmskv_h = rcount(wkn + wk1 + wk1n + wk);
         const T zcof2 = -pah * e1v * S0[TM_TILE + os] * zmskv_h;
         // vertical flux coefficients and ah_wslp2 = akz (:146-164, :200-201, :291-321)
@@ -286,14 +308,14 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 2)
           const T dk0_0 = k == 1 ? dk1_0 : k10[nn];
           const T dk0_e = k == 1 ? dk1_e : k1e[nn];
           const T dk0_n = k == 1 ? dk1_n : k1n[nn];
-          const T zdi = (te - tc) * u0;
-          const T zdj = (tn - tc) * v0;
+          const T zdi = grad(te - tc, u0, k, bu0, gu0[nn]);
+          const T zdj = grad(tn - tc, v0, k, bv0, gv0[nn]);
           fu[nn][q] = (zabe1 * zdi + zcof1 * (dk0_e + dk1_0 + dk1_e + dk0_0)) * u0;
           fv[nn][q] = (zabe2 * zdj + zcof2 * (dk0_n + dk1_0 + dk1_n + dk0_0)) * v0;
           if (icol) {
             const T tw = B0[o - 1], ts = B0[o - TM_W];
-            const T zdiw = (tc - tw) * uw;
-            const T zdjs = (tc - ts) * vs;
+            const T zdiw = grad(tc - tw, uw, k, buw, guw[nn]);
+            const T zdjs = grad(tc - ts, vs, k, bvs, gvs[nn]);
             T z = T(0);
             if (vface) {
               const T sdi = di0[nn] + zdiw + diw[nn] + zdi;
@@ -670,7 +692,8 @@ __device__ __forceinline__ TmaBlock tma_block(const Dom<T>& d) {
   return b;
 }
 
-template <class T>
+// PLAIN: velocities, and a trend that starts here (the hot path's call).
+template <class T, bool PLAIN>
 __global__ void __launch_bounds__(TM_X * TM_Y, 3)
     k_fct_a_tma(Dom<T> d, FctArgs<T> a, const __grid_constant__ PlaneMaps<FA_NF> maps, int* err, int max_polls) {
   static_assert(sizeof(T) == 4, "the TMA kernel is the FP32 form");
@@ -694,7 +717,7 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
   T* ay = a.ay + mb;
   T* az = a.az + mb;
   T* ta = a.pta + mb;
-  const T* tai = a.pta_in ? a.pta_in + mb : nullptr;
+  const T* tai = !PLAIN && a.pta_in ? a.pta_in + mb : nullptr;
   if (c.valid && !c.icol)  // edge columns: every level 0 (ta: its input)
     for (int k = c.k0; k <= c.k1; ++k)
       for (int n = 0; n < a.kjpt; ++n) {
@@ -705,7 +728,7 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
       }
   const ColInfo ci = c.icol ? d.ci[ij] : ColInfo{};
   // velocities are scaled to transports; transports are taken as they are (x 1 is exact)
-  const bool trp = a.trp && c.icol;
+  const bool trp = (PLAIN || a.trp) && c.icol;
   const T e2u0 = trp ? d.e2u[ij] : T(1), e2uw = trp ? d.e2u[ij - 1] : T(1);
   const T e1v0 = trp ? d.e1v[ij] : T(1), e1vs = trp ? d.e1v[ij - jpi] : T(1);
   const T e1e2t = trp ? d.e1e2t[ij] : T(1), r1_e1e2t = c.icol ? d.r1_e1e2t[ij] : T(0);
@@ -756,7 +779,7 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
       auto L = [&](int f) { return ring.plane((unsigned)p, f); };
       auto L1 = [&](int f) { return ring.plane((unsigned)p + 1, f); };
       const bool first = k == k0;
-      const T e3uk = trp ? __ldg(e3u + k - 1) : T(1), e3vk = trp ? __ldg(e3v + k - 1) : T(1);
+      const T e3uk = PLAIN || trp ? __ldg(e3u + k - 1) : T(1), e3vk = PLAIN || trp ? __ldg(e3v + k - 1) : T(1);
       const T ue = e2u0 * e3uk * L(0)[o];
       const T uw = e2uw * e3uk * L(0)[o - 1];
       const T vn_ = e1v0 * e3vk * L(1)[o];
@@ -847,7 +870,8 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
   ColInfo ci{}, ciw{}, cie{}, cis{}, cin{};
   if (c.icol) { ci = d.ci[ij]; ciw = d.ci[ij - 1]; cie = d.ci[ij + 1]; cis = d.ci[ij - jpi]; cin = d.ci[ij + jpi]; }
   const T e1e2t = c.icol ? d.e1e2t[ij] : T(0);
-  const T* e3tn = d.e3t_n.p.p;
+  const T* e3tn = d.e3t_n.p.p + c.m * d.e3t_n.sm + (long)ij * d.e3t_n.s;
+  const int se = (int)d.e3t_n.sk;
   const T* tbg = a.ptb.p + mb;
   const T* zwig = a.zwi + mb;
   const T* azg = a.az + mb;
@@ -875,12 +899,13 @@ __global__ void __launch_bounds__(TM_X * TM_Y, 3)
         }
       break;
     }
+    const T e3k = c.icol ? __ldg(e3tn + (k - 1) * se) : T(0);  // in flight during the wait
     ok = ring.wait((unsigned)p + 1, max_polls) && ok;
     if (c.icol) {
       auto L = [&](int f) { return ring.plane((unsigned)p, f); };
       auto L1 = [&](int f) { return ring.plane((unsigned)p + 1, f); };
       const bool first = k == k0;
-      const T zbt = e1e2t * __ldg(e3tn + k - 1) / a.p2dt;
+      const T zbt = e1e2t * e3k / a.p2dt;
       const T tw = t_in<T>(ciw, k), te = t_in<T>(cie, k), ts = t_in<T>(cis, k), tn = t_in<T>(cin, k);
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn) {

@@ -161,6 +161,14 @@ struct E3Prof {
   }
 };
 
+// one column of a scale-factor field, or the 1-D profile (stride 1)
+template <class T>
+struct E3Col {
+  const T* p;
+  int st;
+  __device__ __forceinline__ E3Col(const E3<T>& e, long ij, int m) : p(e.p.p + m * e.sm + ij * (long)e.s), st((int)e.sk) {}
+  __device__ __forceinline__ T operator()(int k) const { return __ldg(p + (long)(k - 1) * st); }
+};
 // --------------------------------------------------------------------------------
 // traadv.F90:99-124: zun = e2u*e3u_n*un, zvn = e1v*e3v_n*vn, zwn = e1e2t*wn, 0 at jpk.
 template <class T>
@@ -226,22 +234,6 @@ struct FctArgs {
                              // ((member*kjpt + n)*3 + face)*n3, for the adjoint
 };
 
-// Upstream transports at the faces of column (i,j) (traadv_fct.F90:123-145).
-template <class T>
-__device__ __forceinline__ T trp_u(const Dom<T>& d, const FctArgs<T>& a, long ij, long q, int k, int m) {
-  T u = a.pun[q];
-  return a.trp ? d.e2u[ij] * d.e3u_n(ij, k, m) * u : u;
-}
-template <class T>
-__device__ __forceinline__ T trp_v(const Dom<T>& d, const FctArgs<T>& a, long ij, long q, int k, int m) {
-  T v = a.pvn[q];
-  return a.trp ? d.e1v[ij] * d.e3v_n(ij, k, m) * v : v;
-}
-template <class T>
-__device__ __forceinline__ T trp_w(const Dom<T>& d, const FctArgs<T>& a, long ij, long q) {
-  T w = a.pwn[q];
-  return a.trp ? d.e1e2t[ij] * w : w;
-}
 // ---- value-exact helpers of the FCT and iso-neutral kernels. FP64 runs at 1/64 of
 // the FP32 rate on this GPU, and compares, min/max and products by 0/1 masks all
 // occupy that pipe; these forms move them to the integer pipe or drop them while
@@ -346,119 +338,136 @@ __device__ __forceinline__ T ups(T u, T tl, T tr) {
 // (traadv_fct.F90:119-278) with the lbc_lnk of :280 folded in (edge values 0).
 // k-march: the upstream flux through the w-face between levels k and k+1 is
 // computed once (the bottom flux of k is the top flux of k+1), and tb, tn of
-// level k and the transport through that face are carried to level k+1.
-template <class T>
+// level k, the transport through that face and the T masks are carried to level k+1.
+// H4, V4: the orders (4) of the horizontal and vertical antidiffusive fluxes; TRP: pun,
+// pvn, pwn are velocities to be scaled; I: the index type within a member's tracers (int
+// where they fit, half the address arithmetic). With all of that decided at run time a
+// point took 690 instructions (T and S, FCT 4/4, FP32): 359 us at 500x400x56, 335 so (a
+// form with its planes staged by TMA 347: the seven other fields of a level bound it).
+template <class T, class I, bool H4, bool V4, bool TRP>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpk = d.jpk;
-  const long n2 = d.n2, n3 = d.n3, ij = c.ij;
-  if (!c.interior) {  // edge columns: every level 0 (pta: its input)
-    for (int k = c.k0; k <= c.k1; ++k) {
-      const long q = ij + (long)(k - 1) * n2;
-      for (int n = 0; n < a.kjpt; ++n) {
-        const long mo = ((long)c.m * a.kjpt + n) * n3;
-        a.zwi[mo + q] = T(0); a.ax[mo + q] = T(0); a.ay[mo + q] = T(0); a.az[mo + q] = T(0);
-        T* ta = a.pta + mo;
-        const T* tai = a.pta_in ? a.pta_in + mo : nullptr;
-        if (!tai) ta[q] = T(0);
-        else if (tai != ta) ta[q] = tai[q];
-      }
-    }
+  const I n2 = (I)d.n2, n3 = (I)d.n3;
+  const long ij = c.ij, mb = (long)c.m * a.kjpt * d.n3 + ij, mv = (long)c.m * d.n3 + ij;
+  T *zwi = a.zwi + mb, *ax = a.ax + mb, *ay = a.ay + mb, *az = a.az + mb, *ta = a.pta + mb;
+  const T* tai = a.pta_in ? a.pta_in + mb : nullptr;
+  auto edge = [&](I q) {  // no work: 0 (pta: its input)
+    zwi[q] = T(0); ax[q] = T(0); ay[q] = T(0); az[q] = T(0);
+    if (!tai) ta[q] = T(0);
+    else if (tai != ta) ta[q] = tai[q];
+  };
+  if (!c.interior) {
+    for (int k = c.k0; k <= c.k1; ++k)
+      for (int n = 0; n < a.kjpt; ++n) edge((I)(k - 1) * n2 + n * n3);
     return;
   }
-  const long mv = (long)c.m * n3;
-  const ColInfo ci = d.ci[ij], ciw = d.ci[ij - 1], cie = d.ci[ij + 1], cis = d.ci[ij - jpi], cin = d.ci[ij + jpi];
+  const ColInfo ci = d.ci[ij];
+  ColInfo ciw{}, cie{}, cis{}, cin{};
+  if constexpr (H4) {
+    ciw = d.ci[ij - 1]; cie = d.ci[ij + 1]; cis = d.ci[ij - jpi]; cin = d.ci[ij + jpi];
+  }
+  const bool e_in = c.i + 1 <= jpi - 1, n_in = c.j + 1 <= d.jpj - 1;
   const T r1_e1e2t = d.r1_e1e2t[ij];
   const T r1_6 = T(1) / T(6);
+  const T su0 = TRP ? d.e2u[ij] : T(1), suw = TRP ? d.e2u[ij - 1] : T(1);
+  const T sv0 = TRP ? d.e1v[ij] : T(1), svs = TRP ? d.e1v[ij - jpi] : T(1), sw = TRP ? d.e1e2t[ij] : T(1);
+  const E3Col<T> e3tn(d.e3t_n, ij, c.m), e3tb(d.e3t_b, ij, c.m), e3ta(d.e3t_a, ij, c.m);
+  const E3Col<T> e3u0(d.e3u_n, ij, c.m), e3uw(d.e3u_n, ij - 1, c.m), e3v0(d.e3v_n, ij, c.m), e3vs(d.e3v_n, ij - jpi, c.m);
+  const T *un = a.pun.p + mv, *vn = a.pvn.p + mv, *wn = a.pwn.p + mv;
+  const T *ptb = a.ptb.p + mb, *ptn = a.ptn.p + mb, *ztw = V4 ? a.ztw.p + mb : nullptr;
+  const T p2dt = a.p2dt;
   constexpr int NT = 2;  // tracers per pass over the levels
   for (int n0 = 0; n0 < a.kjpt; n0 += NT) {
     const int nt = a.kjpt - n0 < NT ? a.kjpt - n0 : NT;
     // carried from level k-1: tb(k-1), tn(k-1), the bottom upstream flux of k-1
     T tbp[NT] = {}, tnp[NT] = {}, zwzb[NT] = {};
     T wt = T(0);  // transport through the top face of level k
+    T tkm = c.k0 > 1 ? tmsk<T>(ci, c.k0 - 1) : T(1), tk = tmsk<T>(ci, c.k0);
     for (int k = c.k0; k <= c.k1; ++k) {
-      const long q = ij + (long)(k - 1) * n2;
-      if (k == jpk) {  // level jpk: no work, edge values
-        for (int nn = 0; nn < nt; ++nn) {
-          const long mo = ((long)c.m * a.kjpt + n0 + nn) * n3;
-          a.zwi[mo + q] = T(0); a.ax[mo + q] = T(0); a.ay[mo + q] = T(0); a.az[mo + q] = T(0);
-          T* ta = a.pta + mo;
-          const T* tai = a.pta_in ? a.pta_in + mo : nullptr;
-          if (!tai) ta[q] = T(0);
-          else if (tai != ta) ta[q] = tai[q];
-        }
+      const I q = (I)(k - 1) * n2;
+      if (k == jpk) {
+        for (int nn = 0; nn < nt; ++nn) edge(q + (n0 + nn) * n3);
         continue;
       }
       const bool first = k == c.k0;
-      const T ue = trp_u(d, a, ij, mv + q, k, c.m);
-      const T uw = trp_u(d, a, ij - 1, mv + q - 1, k, c.m);
-      const T vn_ = trp_v(d, a, ij, mv + q, k, c.m);
-      const T vs = trp_v(d, a, ij - jpi, mv + q - jpi, k, c.m);
-      if (first) wt = trp_w(d, a, ij, mv + q);
-      const T wb = (k + 1 <= jpk - 1) ? trp_w(d, a, ij, mv + q + n2) : T(0);
-      const T e3n = d.e3t_n(ij, k, c.m), e3b = d.e3t_b(ij, k, c.m), e3a = d.e3t_a(ij, k, c.m);
-      const T tm = tmsk<T>(ci, k), wk = wmsk<T>(ci, k), wk1 = wmsk<T>(ci, k + 1);
+      T ue = __ldg(un + q), uw = __ldg(un + q - 1), vn_ = __ldg(vn + q), vs = __ldg(vn + q - jpi);
+      if (first) wt = TRP ? sw * __ldg(wn + q) : __ldg(wn + q);
+      T wb = (k + 1 <= jpk - 1) ? __ldg(wn + q + n2) : T(0);
+      if constexpr (TRP) {
+        ue = su0 * e3u0(k) * ue;
+        uw = suw * e3uw(k) * uw;
+        vn_ = sv0 * e3v0(k) * vn_;
+        vs = svs * e3vs(k) * vs;
+        wb = sw * wb;
+      }
+      const T e3n = e3tn(k), e3b = e3tb(k), e3a = e3ta(k);
+      const T tkp = tmsk<T>(ci, k + 1);
+      const T tm = tk, wk = msel(tk, tkm), wk1 = msel(tkp, tk);
+      T um0 = T(0), umw = T(0), ume = T(0), vm0 = T(0), vms = T(0), vmn = T(0);
+      if constexpr (H4) {
+        um0 = umsk<T>(ci, k); umw = umsk<T>(ciw, k); ume = umsk<T>(cie, k);
+        vm0 = vmsk<T>(ci, k); vms = vmsk<T>(cis, k); vmn = vmsk<T>(cin, k);
+      }
 #pragma unroll
       for (int nn = 0; nn < NT; ++nn) {
         if (nn >= nt) break;
-        const long mo = ((long)c.m * a.kjpt + n0 + nn) * n3;
-        const RO<T> tb = a.ptb + mo;
-        const RO<T> tn = a.ptn + mo;
-        T* ta = a.pta + mo;
-        const T* tai = a.pta_in ? a.pta_in + mo : nullptr;
-        const T tb0 = tb[q];
+        const I o = q + (n0 + nn) * n3;
+        const T *tb = ptb + o, *tn = ptn + o;
+        const T tb0 = __ldg(tb);
         if (first && k > 1) {  // the carried values of level k-1
-          tbp[nn] = tb[q - n2];
-          tnp[nn] = tn[q - n2];
+          tbp[nn] = __ldg(tb - n2);
+          tnp[nn] = __ldg(tn - n2);
           zwzb[nn] = ups(wt, tb0, tbp[nn]) * wk;
         }
-        const T zwx_e = ups(ue, tb0, tb[q + 1]), zwx_w = ups(uw, tb[q - 1], tb0);
-        const T zwy_n = ups(vn_, tb0, tb[q + jpi]), zwy_s = ups(vs, tb[q - jpi], tb0);
+        const T tin = tai ? tai[o] : T(0);
+        const T zwx_e = ups(ue, tb0, __ldg(tb + 1)), zwx_w = ups(uw, __ldg(tb - 1), tb0);
+        const T zwy_n = ups(vn_, tb0, __ldg(tb + jpi)), zwy_s = ups(vs, __ldg(tb - jpi), tb0);
         // upstream vertical fluxes at the top (k) and bottom (k+1) faces (:137-156)
         const T zwz_t = (k == 1) ? (a.linssh ? wt * tb0 : T(0)) : zwzb[nn];
-        const T zwz_b = (k + 1 <= jpk - 1) ? ups(wb, tb[q + n2], tb0) * wk1 : T(0);
+        const T zwz_b = (k + 1 <= jpk - 1) ? ups(wb, __ldg(tb + n2), tb0) * wk1 : T(0);
         const T ztra = -(zwx_e - zwx_w + zwy_n - zwy_s + zwz_t - zwz_b) * r1_e1e2t;
-        const T tin = tai ? tai[q] : T(0);
-        ta[q] = tin + ztra / e3n * tm;
-        a.zwi[mo + q] = (e3b * tb0 + a.p2dt * ztra) / e3a * tm;
         // horizontal antidiffusive fluxes (:180-251)
-        const T tn0 = tn[q], tne = tn[q + 1], tnn = tn[q + jpi];
+        const T tn0 = __ldg(tn), tne = __ldg(tn + 1), tnn = __ldg(tn + jpi);
         T axv, ayv;
-        if (a.kn_fct_h == 2) {
+        if constexpr (!H4) {
           axv = T(0.5) * ue * (tn0 + tne) - zwx_e;
           ayv = T(0.5) * vn_ * (tn0 + tnn) - zwy_n;
         } else {
-          const T tnw = tn[q - 1], tns = tn[q - jpi];
-          const T ztu_w = (tn0 - tnw) * umsk<T>(ciw, k);
-          const T ztu_0 = (tne - tn0) * umsk<T>(ci, k);
+          const T ztu_w = (tn0 - __ldg(tn - 1)) * umw;
+          const T ztu_0 = (tne - tn0) * um0;
           const T zltu0 = (ztu_0 + ztu_w) * r1_6;
           T zltue = T(0);
-          if (c.i + 1 <= jpi - 1) zltue = ((tn[q + 2] - tne) * umsk<T>(cie, k) + ztu_0) * r1_6;
-          const T ztv_s = (tn0 - tns) * vmsk<T>(cis, k);
-          const T ztv_0 = (tnn - tn0) * vmsk<T>(ci, k);
+          if (e_in) zltue = ((__ldg(tn + 2) - tne) * ume + ztu_0) * r1_6;
+          const T ztv_s = (tn0 - __ldg(tn - jpi)) * vms;
+          const T ztv_0 = (tnn - tn0) * vm0;
           const T zltv0 = (ztv_0 + ztv_s) * r1_6;
           T zltvn = T(0);
-          if (c.j + 1 <= d.jpj - 1) zltvn = ((tn[q + 2 * jpi] - tnn) * vmsk<T>(cin, k) + ztv_0) * r1_6;
+          if (n_in) zltvn = ((__ldg(tn + 2 * jpi) - tnn) * vmn + ztv_0) * r1_6;
           const T zC2t_u = tn0 + tne;
           const T zC2t_v = tn0 + tnn;
           axv = T(0.5) * ue * (zC2t_u + zltu0 - zltue) - zwx_e;
           ayv = T(0.5) * vn_ * (zC2t_v + zltv0 - zltvn) - zwy_n;
         }
-        a.ax[mo + q] = axv;
-        a.ay[mo + q] = ayv;
         // vertical antidiffusive flux at the top face of level k (:253-278)
         T azv = T(0);
         if (k >= 2) {
-          if (a.kn_fct_v == 2) azv = (wt * T(0.5) * (tn0 + tnp[nn]) - zwz_t) * wk;
-          else azv = (wt * a.ztw[mo + q] - zwz_t) * wk;
+          if constexpr (!V4) azv = (wt * T(0.5) * (tn0 + tnp[nn]) - zwz_t) * wk;
+          else azv = (wt * __ldg(ztw + o) - zwz_t) * wk;
         }
-        a.az[mo + q] = azv;
+        ta[o] = tin + over_e3t_n(d, ztra, e3n, k) * tm;
+        zwi[o] = (e3b * tb0 + p2dt * ztra) / e3a * tm;
+        ax[o] = axv;
+        ay[o] = ayv;
+        az[o] = azv;
         tbp[nn] = tb0;
         tnp[nn] = tn0;
         zwzb[nn] = zwz_b;
       }
       wt = wb;
+      tkm = tk;
+      tk = tkp;
     }
   }
 }
@@ -573,43 +582,78 @@ __device__ __forceinline__ T limit(T f, T bdo0, T bup1, T bup0, T bdo1) {
 }
 
 // interp_4th_cpt (traadv_fct.F90:517-616): compact 4th-order tn at w-points for the
-// interior columns, levels 2..jpkm1, one tridiagonal solve per column.
+// interior columns, levels 2..jpkm1, one tridiagonal solve per column and tracer (grid z =
+// kjpt member + tracer). Rows: identity with the centred average at ikt = 2 (mikt + 1
+// without ice-shelf cavities) and ikb = mbkt, diagonal 4 with off-diagonals 1 between them
+// (wmask 1), identity with 0 elsewhere; so the pivots of a column's run of wet rows are
+// one sequence, 4, 4 - 1/4, ..., which the block forms once. The forward values stay in
+// shared memory, and four levels are loaded while the four before them are used. With
+// pivots and forward values in local memory and both tracers in a thread it took 156 us
+// at 500x400x56 in FP32, 66 so (27 us by traffic).
+constexpr int I4_Y = 4;
 template <class T>
-__global__ void k_interp4(Dom<T> d, RO<T> ptn, T* __restrict__ ztw, int kjpt) {
-  ColIdx<T> c = col_index(d);
-  if (!c.valid || !c.interior) return;
-  const int jpk = d.jpk;
-  const long n2 = d.n2, n3 = d.n3;
-  const ColInfo ci = d.ci[c.ij];
-  const int ikt = 2;  // mikt + 1 without ice-shelf cavities
-  const int ikb = d.mbkt[c.ij];
-  T zwt[KMAX], zws[KMAX], out[KMAX];
-  for (int n = 0; n < kjpt; ++n) {
-    const long mo = ((long)c.m * kjpt + n) * n3;
-    const RO<T> t = ptn + mo;
-    auto coef = [&](int k, T& zwd, T& zwi, T& zwsk, T& zwrm) {
-      const T tk = t[c.ij + (long)(k - 1) * n2], tkm = t[c.ij + (long)(k - 2) * n2];
-      if (k == ikt || k == ikb) {
-        zwd = T(1); zwi = T(0); zwsk = T(0);
-        zwrm = T(0.5) * (tkm + tk);
-      } else {
-        const T wm = wmsk<T>(ci, k);
-        zwd = T(3) * wm + T(1); zwi = wm; zwsk = wm;
-        zwrm = T(3) * wm * (tk + tkm);
-      }
-    };
-    T zwd, zwi, zwrm;
-    coef(2, zwd, zwi, zws[2], zwrm);
-    zwt[2] = zwd;
-    out[2] = zwrm;
-    for (int k = 3; k <= jpk - 1; ++k) {
-      coef(k, zwd, zwi, zws[k], zwrm);
-      zwt[k] = zwd - zwi * zws[k - 1] / zwt[k - 1];
-      out[k] = zwrm - zwi / zwt[k - 1] * out[k - 1];
+__global__ void __launch_bounds__(32 * I4_Y) k_interp4(Dom<T> d, RO<T> ptn, T* __restrict__ ztw, int kjpt) {
+  extern __shared__ __align__(16) unsigned char i4_smem[];
+  __shared__ T piv[KMAX + 1], rp[KMAX + 1];  // pivots of a run of wet rows, their reciprocals
+  constexpr int nt = 32 * I4_Y, B = 4;
+  T* const out = reinterpret_cast<T*>(i4_smem) + threadIdx.y * 32 + threadIdx.x;  // [k * nt]
+  const int jpk = d.jpk, K = jpk - 1, n2 = (int)d.n2;
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    T p = T(4);
+    for (int n = 0; n <= K; ++n) {
+      piv[n] = p;
+      rp[n] = T(1) / p;
+      p = T(4) - rp[n];
     }
-    out[jpk - 1] = out[jpk - 1] / zwt[jpk - 1];
-    for (int k = jpk - 2; k >= 2; --k) out[k] = (out[k] - zws[k] * out[k + 1]) / zwt[k];
-    for (int k = 2; k <= jpk - 1; ++k) ztw[mo + c.ij + (long)(k - 1) * n2] = out[k];
+  }
+  __syncthreads();
+  const int i = blockIdx.x * 32 + threadIdx.x + 1, j = blockIdx.y * I4_Y + threadIdx.y + 1;
+  if (i < 2 || i > d.jpi - 1 || j < 2 || j > d.jpj - 1) return;
+  const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi, mo = (long)blockIdx.z * d.n3 + ij;
+  const ColInfo ci = d.ci[ij];
+  const int ikb = d.mbkt[ij];
+  const int ks = max(3, ci.tlo + 1), ke = ikb < 3 ? 2 : min(min((int)ci.thi, ikb - 1), K);  // the run of wet rows
+  const T* __restrict__ t = ptn.p + mo;
+  auto load = [&](int k0, T (&l)[B]) {
+    const T* p = t + (long)(k0 - 1) * n2;
+#pragma unroll
+    for (int y = 0; y < B; ++y) l[y] = __ldg(p + min(y, K - k0) * n2);
+  };
+  T tm = __ldg(t), prev = T(0);
+  auto sweep = [&](int k0, T (&l)[B]) {
+#pragma unroll
+    for (int y = 0; y < B; ++y) {
+      const int k = k0 + y;
+      if (k > K) break;
+      const bool run = k >= ks && k <= ke;
+      const T sum = l[y] + tm;
+      T x = run ? T(3) * sum : (k == 2 || k == ikb) ? T(0.5) * sum : T(0);
+      if (run) x = x - (k == ks ? prev : rp[k - ks - 1] * prev);
+      out[k * nt] = x;
+      prev = x;
+      tm = l[y];
+    }
+  };
+  T la[B], lb[B];
+  load(2, la);
+  for (int k0 = 2; k0 <= K; k0 += 2 * B) {
+    if (k0 + B <= K) load(k0 + B, lb);
+    sweep(k0, la);
+    if (k0 + B > K) break;
+    if (k0 + 2 * B <= K) load(k0 + 2 * B, la);
+    sweep(k0 + B, lb);
+  }
+  T nxt = T(0);
+  T* __restrict__ w = ztw + mo;
+#pragma unroll 4
+  for (int k = K; k >= 2; --k) {
+    T x = out[k * nt];
+    if (k >= ks && k <= ke) {
+      if (k < K) x = x - nxt;
+      x = divq(x, piv[k - ks], rp[k - ks]);
+    }
+    nxt = x;
+    w[(long)(k - 1) * n2] = x;
   }
 }
 
