@@ -126,6 +126,7 @@ struct nemo_ctx {
   int bar_extra = 0;
   int p2_blocks = 0;
   int p2_cache = 0;  // the sub-step kernel keeps its constants in shared memory
+  int p2_five = 0;   // it is the instance for five blocks an SM
   int res_c = 0, res_rows = 0, res_v = 0, res_gen = 0;  // k_spg_p2_res: blocks a member (0: not used), rows, variant
   int p2_hot = 0;    // the sub-step kernel is k_spg_p2_ene (mixed, linear free surface, ENE/MIX)
   bool no_p2_hot = false;  // keep the general sub-step kernel (tests compare both)
@@ -990,7 +991,7 @@ int run_spg(nemo_ctx* c, int kt) {
   a.du = (T*)c->spg_x[2]; a.dv = (T*)c->spg_x[3]; a.cu = (T*)c->spg_x[4]; a.cv = (T*)c->spg_x[5];
   a.zmu = (T*)c->spg_x[6]; a.zmv = (T*)c->spg_x[7];
   a.cache = c->p2_cache;
-  a.hot = c->p2_hot;
+  a.hot = c->p2_hot; a.five = c->p2_five;
   if (!c->bar_extra) {  // an injected arrival asks for a kernel with the grid barrier
     a.res_c = c->res_c; a.res_rows = c->res_rows; a.res_v = c->res_v; a.res_gen = c->res_gen;
   }
@@ -1815,8 +1816,21 @@ void select_p2(nemo_ctx* c) {
   const int prec = c->prec;
   auto p2_grid = [&](int cache) {
     const int bps =
-        prec == NEMO_PREC_FP64 ? spg_p2_blocks_per_sm<double>(0, vvl) : spg_p2_blocks_per_sm<float>(cache, vvl);
-    const long maxb = (long)bps * c->nsm;
+        prec == NEMO_PREC_FP64 ? spg_p2_blocks_per_sm<double>(0, vvl, 0) : spg_p2_blocks_per_sm<float>(cache, vvl, 0);
+    long maxb = (long)bps * c->nsm;
+    // The block with the most tiles sets the pace: five blocks an SM (48 registers, a few
+    // more spills) where it then owns one tile instead of two or two instead of three
+    // (variable volume, 421x363: 644 tiles, 776 -> 670 us a call; 640x520: 1193 -> 1124).
+    // With more rounds the spills cost more than the shorter tail saves (4800 tiles, 7
+    // rounds instead of 8: 3861 -> 3897 us).
+    c->p2_five = 0;
+    if (prec != NEMO_PREC_FP64 && vvl && maxb > 0 && need <= 3 * maxb) {
+      const long max5 = (long)spg_p2_blocks_per_sm<float>(0, vvl, 1) * c->nsm;
+      if (max5 > maxb && (need + max5 - 1) / max5 < (need + maxb - 1) / maxb) {
+        c->p2_five = 1;
+        maxb = max5;
+      }
+    }
     c->p2_blocks = (int)(need < maxb ? need : maxb);
     c->p2_cache = cache;
   };

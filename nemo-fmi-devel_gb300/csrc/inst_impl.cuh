@@ -288,12 +288,20 @@ cudaError_t launch_clamp(T* x, long n, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// the general sub-step kernel; five: compiled for five blocks an SM (FP32, variable volume)
+template <class T>
+static auto spg_p2_kernel(int vvl, int five) -> void (*)(Dom<T>, SpgArgs<T>, GridBar) {
+  if constexpr (sizeof(T) == 4) {
+    if (five) return k_spg_p2<T, true, 5>;
+  }
+  return vvl ? k_spg_p2<T, true> : k_spg_p2<T, false>;
+}
 // co-resident blocks per SM of the sub-step kernel, with or without the constant
 // cache (dynamic shared memory beyond the 48 KB default needs the opt-in)
 template <class T>
-int spg_p2_blocks_per_sm(int cache, int vvl) {
+int spg_p2_blocks_per_sm(int cache, int vvl, int five) {
   const size_t dyn = cache ? P2_CACHE_BYTES : 0;
-  auto kern = vvl ? k_spg_p2<T, true> : k_spg_p2<T, false>;
+  auto kern = spg_p2_kernel<T>(vvl, five);
   if (cache && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
     return 0;
   int nb = 0;
@@ -425,12 +433,10 @@ cudaError_t launch_spg(const Dom<T>& d, const SpgArgs<T>& a, const GridBar& bar,
         cfg.dynamicSmemBytes = P2H_CACHE_BYTES;
         e = cudaLaunchKernelEx(&cfg, k_spg_p2_ene<T>, d, a, bar);
       } else {
-        e = a.vvl ? cudaLaunchKernelEx(&cfg, k_spg_p2<T, true>, d, a, bar)
-                  : cudaLaunchKernelEx(&cfg, k_spg_p2<T, false>, d, a, bar);
+        e = cudaLaunchKernelEx(&cfg, spg_p2_kernel<T>(a.vvl, a.five), d, a, bar);
       }
     } else {
-      e = a.vvl ? cudaLaunchKernelEx(&cfg, k_spg_p2<T, true>, d, a, bar)
-                : cudaLaunchKernelEx(&cfg, k_spg_p2<T, false>, d, a, bar);
+      e = cudaLaunchKernelEx(&cfg, spg_p2_kernel<T>(a.vvl, 0), d, a, bar);
     }
   }
   if (e != cudaSuccess) return e;
@@ -470,7 +476,7 @@ cudaError_t launch_globsum(const T* x, const double* tmask_i, long n2, int nk, i
   template cudaError_t launch_iso_flux<T>(const Dom<T>&, const LdfArgs<T>&, cudaStream_t);                   \
   template cudaError_t launch_clamp<T>(T*, long, cudaStream_t);                                              \
   template cudaError_t launch_spg<T>(const Dom<T>&, const SpgArgs<T>&, const GridBar&, int, cudaStream_t);   \
-  template int spg_p2_blocks_per_sm<T>(int, int);                                                                 \
+  template int spg_p2_blocks_per_sm<T>(int, int, int);                                                                 \
   template int spg_res_clusters<T>(int, int, int, int, int);                                                      \
   template int spg_p2_ene_blocks_per_sm<T>();                                                                 \
   template cudaError_t launch_lbc<T>(T*, int, int, long, int, T, cudaStream_t);                              \

@@ -107,7 +107,7 @@ cudaError_t launch_ldf_slp(const Dom<T>& d, const SlpArgs<T>& a, cudaStream_t s)
     k_slp_mxl<T, false><<<s_col(d), dim3(SX, SY), 0, s>>>(d, a);
     (flat ? k_slp_pre<T, false, true> : k_slp_pre<T, false, false>)<<<g, dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   }
-  k_slp_filter<T><<<s_pt(d), dim3(SX, SY), 0, s>>>(d, a);
+  k_slp_filter<T><<<march_grid(d, kch, 30, 2), dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);  // a warp writes 30 interior points
   ktick(NEMO_K_LDF_SLP, s);
   return cudaGetLastError();
 }

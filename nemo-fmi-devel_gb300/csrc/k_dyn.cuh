@@ -42,6 +42,7 @@ struct SpgArgs {
   int ln_bt_fw, ln_apr_dyn, nvor, ll_init, icycle, ring0, phase3_filter;
   int cache;  // mixed form, ENE/MIX: the sub-step constants cached in shared memory
   int hot;    // mixed form, linear free surface, ENE/MIX: k_spg_p2_ene instead of k_spg_p2
+  int five;   // k_spg_p2 compiled for five blocks an SM
   int res_c, res_rows, res_v, res_gen;  // res_c > 0: k_spg_p2_res (variant res_v), res_c blocks of res_rows rows a member
   // Column depths (2-D): for a linear free surface the rest-state ht_0, hu_0, ...
   // shared by all members (member stride hs = 0); with a variable volume the bound
@@ -434,8 +435,8 @@ __device__ __forceinline__ int p2_tiles(const Dom<T>& d) {
   return ((d.jpi + P2_TX - 1) / P2_TX) * ((d.jpj + P2_TY - 1) / P2_TY) * d.nmem;
 }
 
-template <class T, bool VVL>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_spg_p2(Dom<T> d, SpgArgs<T> a, GridBar bar) {
+template <class T, bool VVL, int BPS = (sizeof(T) == 4 ? 4 : 2)>
+__global__ void __launch_bounds__(256, BPS) k_spg_p2(Dom<T> d, SpgArgs<T> a, GridBar bar) {
   unsigned int bar_epoch = 0;  // barriers passed by this block
   // two buffers, alternating between a block's tiles: a warp may start the next
   // tile while others still read this one's (the block barrier between the two

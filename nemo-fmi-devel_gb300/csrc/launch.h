@@ -57,7 +57,7 @@ cudaError_t launch_clamp(T* x, long n, cudaStream_t s);
 template <class T>
 cudaError_t launch_spg(const Dom<T>& d, const SpgArgs<T>& a, const GridBar& bar, int p2_blocks, cudaStream_t s);
 template <class T>
-int spg_p2_blocks_per_sm(int cache, int vvl);
+int spg_p2_blocks_per_sm(int cache, int vvl, int five);
 template <class T>
 int spg_p2_ene_blocks_per_sm();
 template <class T>
