@@ -5,7 +5,7 @@ import pytest
 
 import adj_cases
 from adj_cases import Case, GpuCase
-from nemo_gpu import gyre
+from nemo_gpu import gyre, shelf
 from harness import Pair, relerr
 
 pytestmark = pytest.mark.gpu
@@ -107,3 +107,76 @@ def test_sub_steps_of_a_cluster(nn, nmem, case):
         p.ctx.dyn_spg_ts(kt)
         p.ctx.synchronize()
     _spg_compare(p, "mixed")
+
+
+def test_sub_steps_of_one_tile_a_block():
+    """The variable-volume sub-steps of a shelf whose tiles fit five blocks an SM and not
+    four. Tolerance of the routine's mixed parity tests."""
+    from test_gpu_parity import _spg_compare
+    dom, nam = shelf.domain(421, 363, jpk=8, seed=3), shelf.namelist()
+    p = Pair(prec="mixed", dom=dom, nam=nam, states=[shelf.state(dom, nam, seed=4)])
+    p.bind_spg()
+    p.bind("SSH_IB")
+    p.ora[0].dyn_spg_ts(5)
+    p.ctx.dyn_spg_ts(5)
+    p.ctx.synchronize()
+    _spg_compare(p, "mixed")
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("jpi,jpj,jpk", [(43, 37, 19), (64, 33, 33), (45, 17, 5)])
+def test_shelf_tracers(prec, jpi, jpj, jpk):
+    """The tracer routines of a step with variable volume and partial steps, with and
+    without tensor copies (jpi a multiple of 4 or not), at few levels and with
+    remainders of chunks. Tolerances of the hot path's parity tests."""
+    dom, nam = shelf.domain(jpi, jpj, jpk=jpk, seed=7), shelf.namelist()
+    p = Pair(prec=prec, dom=dom, nam=nam, states=[shelf.state(dom, nam, seed=8)])
+    p.bind_hotpath()
+    for n in ("GTSU", "GTSV", "SSH_IB"):
+        p.bind(n)
+    for kt in (5, 6):
+        p.ora[0].stp_hotpath(kt)
+        p.ctx.stp_hotpath(kt)
+        p.ctx.synchronize()
+    t = 1e-12 if prec == "fp64" else 5e-6
+    p.compare("TSA", p.s4, t)
+    p.compare("AH_WSLP2", p.s3, t)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_column_physics_of_a_larger_grid(monkeypatch, prec):
+    """zdf_phy and ldf_slp with more than one level a thread, by their own parity tests."""
+    import test_ldf_slp
+    import test_zdf_tke
+    real = gyre.domain
+    monkeypatch.setattr(gyre, "domain", lambda nn, **k: real(11, jpk=18))
+    test_ldf_slp.test_ldf_slp_gpu_matches_oracle(prec)
+    for nn_mxl in (0, 2, 3):
+        test_zdf_tke.test_gpu_zdf_phy(prec, nn_mxl, 1, 1)
+
+
+@pytest.mark.parametrize("nk", [1, 7, 62])
+@pytest.mark.parametrize("spread", [0, 3, 40])
+def test_glob_sum_of_floats(nk, spread):
+    """The FP32 sum against the exactly rounded one: values of one binary place, within the
+    exact passes' range, and far outside it; a pass of zeros; two members. The compensated
+    sum is off by at most n 2^-104 of the sum of magnitudes."""
+    import math
+    p = Pair(nn=2, prec="mixed", seed=3, nmem=2)
+    rng = np.random.default_rng(spread)
+    x = rng.standard_normal((2, nk, p.s2[1], p.s2[0])) * 2.0 ** rng.integers(-spread, spread + 1, (2, nk, 1, 1))
+    x = x.astype(np.float32)
+    if nk > 2:
+        x[:, 1] = 0
+    t = p.torch.from_numpy(x).cuda()
+    p.torch.cuda.synchronize()
+    mask = p.ora[0].array("tmask_i", 2).T
+    for m, got in enumerate(p.ctx.glob_sum(t, nk)):
+        v = (x[m].astype(np.float64) * mask).ravel()
+        assert abs(got - math.fsum(v)) <= 2.0**-52 * abs(math.fsum(v)) + 2.0**-85 * np.abs(v).sum()
+    bad = x.copy()
+    bad[1, 0, 5, 5] = np.inf
+    t.copy_(p.torch.from_numpy(bad))
+    p.torch.cuda.synchronize()
+    out = p.ctx.glob_sum(t, nk)
+    assert np.isfinite(out[0]) and not np.isfinite(out[1])
