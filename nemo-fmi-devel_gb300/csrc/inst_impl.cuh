@@ -145,7 +145,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
       }
     }
     const int ta = kty(NEMO_K_FCT_A);
-    (a.trp ? k_fct_a_hot<T, true> : k_fct_a_hot<T, false>)<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
+    (!a.trp ? k_fct_a_hot<T, false, true> : a.pta_in ? k_fct_a_hot<T, true, true> : k_fct_a_hot<T, true, false>)<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_A, s);
   } else {
     if (a.kn_fct_v == 4) {

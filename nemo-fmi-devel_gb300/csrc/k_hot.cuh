@@ -264,9 +264,9 @@ inline bool hot_fct_c_ok(const Dom<T>& d, const FctArgs<T>& a) {
 
 // FCT stage a (traadv_fct.F90:119-280) of one column chunk; see k_fct_a. Tracer nn
 // of the member is at offset nn * n3 from tracer 0. TRP: pun, pvn, pwn are velocities, to
-// be scaled to transports.
-template <class T, bool TRP>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
+// be scaled to transports; TIN: there may be a trend to add to (FP32 spills with it).
+template <class T, bool TRP, bool TIN>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpk = d.jpk, n2 = (int)d.n2, n3 = (int)d.n3, ij = (int)c.ij;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a_hot(Dom<T
   T* ay = a.ay + mb;
   T* az = a.az + mb;
   T* ta = a.pta + mb;
-  const T* tai = a.pta_in ? a.pta_in + mb : nullptr;
+  const T* tai = TIN && a.pta_in ? a.pta_in + mb : nullptr;
   if (!c.interior) {  // edge columns: every level 0 (ta: its input)
     for (int k = c.k0; k <= c.k1; ++k)
       for (int n = 0; n < a.kjpt; ++n) {
