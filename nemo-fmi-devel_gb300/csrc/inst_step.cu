@@ -168,11 +168,11 @@ cudaError_t launch_zdf_mxl(const Dom<T>& d, const MxlArgs<T>& a, cudaStream_t s)
 
 template <class T>
 cudaError_t launch_dyn_zdf_imp(const Dom<T>& d, const DynZdfArgs<T>& a, cudaStream_t s) {
-  const int smem = 3 * 32 * DZ_Y * d.jpk * (int)sizeof(T);
   const bool flat = d.e3u_n.s == 0 && d.e3v_n.s == 0 && d.e3w_n.s == 0;
+  const int smem = dyn_zdf_smem(32 * DZ_Y<T>, d.jpk, flat, (int)sizeof(T));
   const auto kern = flat ? k_dyn_zdf_imp<T, true> : k_dyn_zdf_imp<T, false>;
   if (cudaError_t e = smem_opt_in(kern, smem)) return e;
-  kern<<<s_cols2<T>(d, DZ_Y), dim3(SX, DZ_Y), smem, s>>>(d, a);
+  kern<<<s_cols2<T>(d, DZ_Y<T>), dim3(SX, DZ_Y<T>), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_ZDF_STEP, s);
   return cudaGetLastError();
 }
@@ -196,12 +196,12 @@ cudaError_t launch_usr_put(double* dst, const double* v, cudaStream_t s) {
 
 template <class T>
 cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s) {
-  const int kch = march_chunk(d), smem = 4 * 32 * TKE_Y * d.jpk * (int)sizeof(T);
+  const int kch = march_chunk(d), smem = (sizeof(T) == 4 ? 3 : 4) * 32 * TKE_Y<T> * d.jpk * (int)sizeof(T);
   const auto tke = d.e3w_n.s == 0 && d.e3t_n.s == 0 ? k_zdf_tke<T, true> : k_zdf_tke<T, false>;
   if (cudaError_t e = smem_opt_in(tke, smem)) return e;
   (d.e3w_n.s == 0 ? k_zdf_sh2<T, true> : k_zdf_sh2<T, false>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   ktick(NEMO_K_ZDF_PHY, s);
-  tke<<<dim3((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y - 1) / TKE_Y, d.nmem), dim3(SX, TKE_Y), smem, s>>>(d, a);
+  tke<<<dim3((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y<T> - 1) / TKE_Y<T>, d.nmem), dim3(SX, TKE_Y<T>), smem, s>>>(d, a);
   ktick(NEMO_K_ZDF_PHY, s);
   return cudaGetLastError();
 }

@@ -101,12 +101,16 @@ __global__ void k_dyn_zdf_step(Dom<T> d, RO<T> ub, RO<T> vb, T* ua, T* va, T r2d
 // is the MIN of the neighbouring e3w (the rest state of a linear free surface).
 template <class T>
 struct DynZdfProf {  // 1-D scale factors: e3, and the divisors e3(k) e3w(k+1), e3(k) e3w(k)
-  T e[KMAX + 1], ds[KMAX + 1], rs[KMAX + 1], di[KMAX + 1], ri[KMAX + 1];
+  T *e, *ds, *rs, *di, *ri;  // of jpk + 1 values each
+  __device__ __forceinline__ DynZdfProf(T* p, int n) : e(p), ds(p + n), rs(p + 2 * n), di(p + 3 * n), ri(p + 4 * n) {}
 };
+inline int dyn_zdf_smem(int nt, int jpk, bool flat, int b) {
+  return ((b == 4 ? 2 : 3) * nt * jpk + (flat ? 5 * (jpk + 1) : 0)) * b;
+}
 template <bool U, bool FLAT, class T>
 __device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs<T>& a, const ColIdx<T>& c, int nt, T* sx,
-                                               T* sd, T* ss, const DynZdfProf<T>& pf) {
-  constexpr int B = 4;  // levels loaded together
+                                               T* ss, T* sd, const DynZdfProf<T>& pf) {
+  constexpr int B = FLAT && sizeof(T) == 4 ? 5 : 4;  // levels loaded together
   const int jpk = d.jpk, K = jpk - 1, m = c.m, n2 = (int)d.n2;
   const long ij = c.ij, m3 = (long)m * d.n3 + ij, p2 = (long)m * d.n2 + ij;
   const int nb = U ? 1 : d.jpi;
@@ -128,7 +132,9 @@ __device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs
   auto e3 = [&](int k) { return FLAT ? pf.e[k] : (U ? d.e3u_n : d.e3v_n)(ij, k, m); };
   auto e3xw = [&](int k) { return fmn(d.e3w_n(ij, k, m), d.e3w_n(ij + nb, k, m)); };
   const T rc = a.rcdu[p2 + nb] + a.rcdu[p2];
-  T rd_p = T(1), wd_p = T(1), ws_p = T(0), x_p = T(0);  // rd = 1 / wd
+  // of the level above: the upper diagonal and the forward value (FP32: over the pivot),
+  // the pivot and its reciprocal
+  T ws_p = T(0), x_p = T(0), wd_p = T(1), rd_p = T(1);
   T mk0 = mk(1), s0 = T(0), w0 = T(0), wx0 = T(0);  // of level k: mask; of w-level k: avm sum, e3, mask
   auto load = [&](int kt, T (&l)[3 * B]) {
     const long b = (long)(kt - 1) * n2;
@@ -164,15 +170,25 @@ __device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs
         wd = T(1) - zzwi - zzws;
       }
       if (k == kb) wd = wd - r2dt * T(0.5) * rc / ze3a;
-      if (k > 1) {
-        wd = wd - divr(zzwi * ws_p, wd_p, rd_p);
-        x = x - divr(zzwi, wd_p, rd_p) * x_p;
-      }
       const int o = (k - 1) * nt;
-      sd[o] = wd;
-      ss[o] = zzws;
-      sx[o] = x;
-      wd_p = wd; rd_p = T(1) / wd; ws_p = zzws; x_p = x;
+      if constexpr (sizeof(T) == 4) {
+        if (k > 1) {
+          wd = wd - zzwi * ws_p;
+          x = x - zzwi * x_p;
+        }
+        rd_p = T(1) / wd;
+        ws_p = divr(zzws, wd, rd_p);
+        x_p = divr(x, wd, rd_p);
+      } else {
+        if (k > 1) {
+          wd = wd - divr(zzwi * ws_p, wd_p, rd_p);
+          x = x - divr(zzwi, wd_p, rd_p) * x_p;
+        }
+        sd[o] = wd;
+        wd_p = wd; rd_p = T(1) / wd; ws_p = zzws; x_p = x;
+      }
+      ss[o] = ws_p;
+      sx[o] = x_p;
       mk0 = mk1; s0 = sv; w0 = w1; wx0 = wx1;
     }
   };
@@ -190,24 +206,29 @@ __device__ __forceinline__ void dyn_zdf_column(const Dom<T>& d, const DynZdfArgs
 #pragma unroll 4
   for (int k = K; k >= 1; --k) {
     const int o = (k - 1) * nt;
-    nxt = (k == K) ? sx[o] / sd[o] : (sx[o] - ss[o] * nxt) / sd[o];
+    nxt = (k == K) ? sx[o] : sx[o] - ss[o] * nxt;
+    if constexpr (sizeof(T) == 8) nxt = nxt / sd[o];
     pa[(long)(k - 1) * n2] = nxt;
   }
 }
 
-// dyn_zdf, one U- or V-column per thread (grid z = 2 member + component). The forward
-// values, diagonals and upper diagonals of the column stay in shared memory (3 jpk
-// values a thread), so that ua, va and avm are read once and the result is written
-// once, and four levels are loaded while the four before them are swept; the quotients
-// by scale factors (1-D with FLAT) and by the pivot are divr's. One thread for both
-// components, with the time step as a pass of its own and the diagonals in global
-// memory, took 340 us at 752x502x31 in FP32 (376 MB to move: 55 us).
-constexpr int DZ_Y = 2;
+// dyn_zdf, one U- or V-column per thread (grid z = 2 member + component). What the back
+// substitution needs of the column stays in shared memory, so that ua, va and avm are read
+// once and the result is written once, and a batch of levels is loaded while the one
+// before it is swept; the quotients by scale factors (1-D with FLAT) and by the pivot are
+// divr's. One thread for both components, with the time step as a pass of its own and the
+// diagonals in global memory, took 340 us at 752x502x31 in FP32 (376 MB to move: 55 us).
+// Bound by the loads in flight, so by the shared memory of a column: in FP32 the upper
+// diagonal and the forward value are kept over the pivot (two values a level and no
+// division on the way up, 24 warps an SM: 136 us) and not beside it (three: 200 us); it
+// rounds less often (five times a level, not seven). FP64 keeps the reference's order.
+template <class T>
+constexpr int DZ_Y = sizeof(T) == 4 ? 4 : 2;
 template <class T, bool FLAT>
-__global__ void __launch_bounds__(32 * DZ_Y) k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<T> a) {
+__global__ void __launch_bounds__(32 * DZ_Y<T>, sizeof(T) == 8 ? 1 : FLAT ? 6 : 5) k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<T> a) {
   extern __shared__ __align__(16) unsigned char col_smem[];
-  __shared__ DynZdfProf<T> pf;
-  constexpr int nt = 32 * DZ_Y;
+  constexpr int nt = 32 * DZ_Y<T>;
+  const DynZdfProf<T> pf(reinterpret_cast<T*>(col_smem) + (sizeof(T) == 4 ? 2 : 3) * nt * d.jpk, d.jpk + 1);
   ColIdx<T> c = col_index(d);
   c.m = blockIdx.z >> 1;
   const bool isv = blockIdx.z & 1;
@@ -225,9 +246,9 @@ __global__ void __launch_bounds__(32 * DZ_Y) k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<
   }
   if (!c.valid) return;
   T* sx = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x;
-  T *sd = sx + d.jpk * nt, *ss = sd + d.jpk * nt;
-  if (isv) dyn_zdf_column<false, FLAT>(d, a, c, nt, sx, sd, ss, pf);
-  else dyn_zdf_column<true, FLAT>(d, a, c, nt, sx, sd, ss, pf);
+  T *ss = sx + d.jpk * nt, *sd = ss + d.jpk * nt;  // sd: FP64
+  if (isv) dyn_zdf_column<false, FLAT>(d, a, c, nt, sx, ss, sd, pf);
+  else dyn_zdf_column<true, FLAT>(d, a, c, nt, sx, ss, sd, pf);
 }
 
 // dyn_nxt (dynnxt.F90:114-358; linear free surface, ln_dynspg_ts with ln_bt_fw), one
@@ -235,15 +256,23 @@ __global__ void __launch_bounds__(32 * DZ_Y) k_dyn_zdf_imp(Dom<T> d, DynZdfArgs<
 // after velocity replaced by the sub-steps' ua_b; lbc of ua, va (the closed edges 0);
 // the Euler swap or the Asselin filter and swap with the before velocity returned to
 // the time-split barotropic estimate; the now and before barotropic velocities. The
-// column waits for its sums in shared memory (the after velocity, then the filtered
-// before one), so that memory sees each field read once and written once: 564 MB at
-// 752x502x31 in FP32, 83 us; with the column read back from memory by each of four
-// passes it took 203 us.
+// column waits for its sums in shared memory (the after velocity, copied there all levels
+// at once, then the filtered before one), and a batch of the now and before velocities is
+// loaded while the one before it is used: memory sees each field read once and written
+// once, 564 MB at 752x502x31 in FP32, 83 us. With the column read back from memory by each
+// of four passes it took 203 us; loaded four levels at a time, each batch waited for,
+// 142 us; so 112 us (batches of 4: 138; of 15: 123).
 constexpr int DN_Y = 4;
+// one value of global memory into the thread's own place in shared memory
+template <class T>
+__device__ __forceinline__ void cp_async_val(T* smem, const T* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sa), "l"(gmem), "n"((int)sizeof(T)) : "memory");
+}
 template <class T, class A>
 __global__ void __launch_bounds__(32 * DN_Y) k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a) {
   extern __shared__ __align__(16) unsigned char col_smem[];
-  constexpr int nt = 32 * DN_Y, B = 4;  // levels loaded together (8: 152 us)
+  constexpr int nt = 32 * DN_Y, B = BATCH<T>;  // levels loaded together
   T* s = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x;
   const ColIdx<T> c = col_index(d);
   if (!c.valid) return;
@@ -261,58 +290,54 @@ __global__ void __launch_bounds__(32 * DN_Y) k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a
   const E3Col<T> e3(isv ? d.e3v_n : d.e3u_n, ij, m);
   auto mk = [&](int k) { return in_range(k, lo, hi) ? T(1) : T(0); };
   // (:114-126)
-  T ze = T(0);
-  for (int kt = 1; kt <= jpk - 1; kt += B) {
-    const T* pk = xa + (long)(kt - 1) * n2;
-    T x[B], e[B];
-#pragma unroll
-    for (int y = 0; y < B; ++y) {
-      const int z = min(y, jpk - 1 - kt);
-      x[y] = pk[z * n2];
-      e[y] = e3(kt + z);
-    }
-#pragma unroll
-    for (int y = 0; y < B; ++y) {
-      const int k = kt + y;
-      if (k > jpk - 1) break;
-      ze = ze + e[y] * x[y] * mk(k);
-      s[(k - 1) * nt] = x[y];
-    }
-  }
-  // the now and before barotropic velocities (:345-358) are summed where xn and xb
-  // take their final values, level by level in the same order
-  T sn = T(0), sb = T(0), sf = T(0);
-  for (int kt = 1; kt <= jpk - 1; kt += B) {
-    const long b = (long)(kt - 1) * n2;
-    T* __restrict__ pa = xa + b;
-    T* __restrict__ pn = xn + b;
-    const T* pb = xb + b;
-    T vb[B], vn[B], ee[B];
+  for (int k = 1; k <= jpk - 1; ++k) cp_async_val(s + (k - 1) * nt, xa + (long)(k - 1) * n2);
+  auto load = [&](int kt, T (&l)[3 * B]) {
+    const T *pn = xn + (long)(kt - 1) * n2, *pb = xb + (long)(kt - 1) * n2;
 #pragma unroll
     for (int y = 0; y < B; ++y) {
       const int z = min(y, jpk - 1 - kt), o = z * n2;
-      vb[y] = pb[o];
-      vn[y] = pn[o];
-      ee[y] = e3(kt + z);
+      l[y] = pb[o];
+      l[B + y] = pn[o];
+      l[2 * B + y] = e3(kt + z);
     }
+  };
+  T la[3 * B], lb[3 * B];
+  load(1, la);
+  cp_async_wait_all();
+  T ze = T(0);
+#pragma unroll 4
+  for (int k = 1; k <= jpk - 1; ++k) ze = ze + e3(k) * s[(k - 1) * nt] * mk(k);
+  // the now and before barotropic velocities (:345-358) are summed where xn and xb
+  // take their final values, level by level in the same order
+  T sn = T(0), sb = T(0), sf = T(0);
+  auto level = [&](int kt, const T (&l)[3 * B]) {
+    T* pa = xa + (long)(kt - 1) * n2;
+    T* pn = xn + (long)(kt - 1) * n2;
 #pragma unroll
     for (int y = 0; y < B; ++y) {
       const int k = kt + y;
       if (k > jpk - 1) break;
-      const T e = ee[y], mu = mk(k);
+      const T e = l[2 * B + y], mu = mk(k), vb = l[y], vn = l[B + y];
       // lbc_lnk of ua, va (:146): the closed edges
       const T u = c.interior ? (s[(k - 1) * nt] - ze * r1 + ab) * mu : T(0);
       pa[y * n2] = u;
       pn[y * n2] = u;
       if (a.euler) {  // (:168-171)
-        sb = sb + e * vb[y] * mu;
+        sb = sb + e * vb * mu;
       } else {        // (:197-211); FP32: the time laplacian from differences (see k_tra_nxt)
-        const T zf = vn[y] + a.atfp * (sizeof(T) == 4 ? (u - vn[y]) - (vn[y] - vb[y]) : vb[y] - T(2) * vn[y] + u);
+        const T zf = vn + a.atfp * (sizeof(T) == 4 ? (u - vn) - (vn - vb) : vb - T(2) * vn + u);
         s[(k - 1) * nt] = zf;
         sf = sf + e * zf * mu;
       }
       sn = sn + e * u * mu;
     }
+  };
+  for (int kt = 1; kt <= jpk - 1; kt += 2 * B) {  // a batch is loaded while the one before it is used
+    if (kt + B <= jpk - 1) load(kt + B, lb);
+    level(kt, la);
+    if (kt + B > jpk - 1) break;
+    if (kt + 2 * B <= jpk - 1) load(kt + 2 * B, la);
+    level(kt + B, lb);
   }
   if (!c.interior) xa[(long)(jpk - 1) * n2] = T(0);
   if (!a.euler) {  // (:312-324)
@@ -1574,20 +1599,23 @@ __global__ void __launch_bounds__(32 * MARCH_Y) k_zdf_sh2(Dom<T> d, ZphyArgs<T> 
 //    Prandtl correction of avt_k, then zdf_phy's avt, avm (zdfphy.F90:269-270),
 //    zdf_evd (zdfevd.F90:76-109) and avs = avt (:284).
 // Edge columns get the closed lbc_lnk of the five coefficients (zdfphy.F90:301-303).
-// Each expression keeps the reference's association. The column's system, lengths and
-// Prandtl numbers stay in shared memory (four arrays of jpk a thread: the slots of the
-// diagonal, upper diagonal and forward values take the raw and limited lengths and en), so
-// that memory sees each field about once, and the next level is loaded ahead; with five
-// work arrays in memory the column made some 30 passes over it, 269 us at 481x323x31 in
-// FP32 (50 us by traffic).
+// Each expression keeps the reference's association (the solve's in FP64). The column's
+// system, lengths and Prandtl numbers stay in shared memory (the slots of the upper diagonal
+// and the forward value take the limited and raw lengths), so that memory sees each field
+// about once, and the next level is loaded ahead; with five work arrays in memory the column
+// made some 30 passes over it, 269 us at 481x323x31 in FP32 (50 us by traffic). Bound by
+// the loads in flight: three values a level (in FP32 the upper diagonal and the forward
+// value over the pivot; en is read back) let 16 warps an SM run, 117 us; four values (the
+// pivot, and en kept) 12 warps, 150 us. Blocks of 4 rows, not 2 (122) or 8 (156).
 // With 1-D scale factors (FLAT) the quotients by e3t e3w, and always those by the pivot,
 // are divr's; where EVD acts is kept as a bit a level.
-constexpr int TKE_Y = 2;
+template <class T>
+constexpr int TKE_Y = sizeof(T) == 4 ? 4 : 2;
 template <class T, bool FLAT>
-__global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
+__global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
   extern __shared__ __align__(16) unsigned char col_smem[];
   __shared__ T pu[KMAX + 1], ru[KMAX + 1], pl[KMAX + 1], rl[KMAX + 1];  // e3t(k) e3w(k), e3t(k-1) e3w(k), reciprocals
-  constexpr int nt = 32 * TKE_Y;
+  constexpr int nt = 32 * TKE_Y<T>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int m = blockIdx.z, jpk = d.jpk;
   if constexpr (FLAT) {
@@ -1603,8 +1631,8 @@ __global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a)
     __syncthreads();
   }
   if (i > d.jpi || j > d.jpj) return;
-  T* const sd = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x - nt;  // [k * nt], k = 1..jpk
-  T *const su = sd + jpk * nt, *const sl = su + jpk * nt, *const sp = sl + jpk * nt;
+  T* const su = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x - nt;  // [k * nt], k = 1..jpk
+  T *const sl = su + jpk * nt, *const sp = sl + jpk * nt, *const sd = sp + jpk * nt;  // sd: FP64
   const long n2 = d.n2;
   const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi;
   const long c3 = (long)m * d.n3 + ij, c2 = (long)m * d.n2 + ij;
@@ -1639,7 +1667,9 @@ __global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a)
     if (zfr < T(0)) zfr = T(0);
   }
   // downward sweep: right-hand side, matrix, forward elimination
-  T dg_p = T(1), rd_p = T(1), up_p = T(0), lw_p = T(0);  // rd = 1 / dg
+  // of the level above: the upper diagonal and the forward value (FP32: over the pivot),
+  // the pivot and its reciprocal
+  T up_p = T(0), lw_p = T(0), dg_p = T(1), rd_p = T(1);
   T avm_km1 = a.avm_k[c3], avm_k = a.avm_k[c3 + n2];
   unsigned long long evd_at = 0;  // levels (bit k - 1) where EVD acts
   march<T, 7>(
@@ -1680,46 +1710,56 @@ __global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a)
         T lf;
         if (k == 2) {
           lf = rhs - lw * en1;
+        } else if constexpr (sizeof(T) == 4) {
+          dg = dg - lw * up_p;
+          lf = rhs - lw * lw_p;
         } else {
           dg = dg - divr(lw * up_p, dg_p, rd_p);
           lf = rhs - divr(lw, dg_p, rd_p) * lw_p;
         }
-        sd[k * nt] = dg; su[k * nt] = up; sl[k * nt] = lf;
-        dg_p = dg; rd_p = T(1) / dg; up_p = up; lw_p = lf;
+        rd_p = T(1) / dg;
+        if constexpr (sizeof(T) == 4) {
+          up_p = divr(up, dg, rd_p);
+          lw_p = divr(lf, dg, rd_p);
+        } else {
+          sd[k * nt] = dg;
+          dg_p = dg; up_p = up; lw_p = lf;
+        }
+        su[k * nt] = up_p; sl[k * nt] = lw_p;
         avm_km1 = avm_k;
         avm_k = avm_kp1;
       });
-  // upward sweep: back substitution, the floor, and the buoyancy length (into sd; en: sl)
+  // upward sweep: back substitution, the floor, and the buoyancy length (into sl)
   T en_p = T(0);
   march<T, 1>(
       2, jpk - 1, [&](int x, T (&l)[1]) { l[0] = __ldg(a.rn2 + c3 + (long)(jpk - x) * n2); },
       [&](int x, T (&l)[1]) {
         const int k = jpk + 1 - x;
-        const T en = (k == jpk - 1) ? sl[k * nt] / sd[k * nt] : (sl[k * nt] - su[k * nt] * en_p) / sd[k * nt];
+        T en = (k == jpk - 1) ? sl[k * nt] : sl[k * nt] - su[k * nt] * en_p;
+        if constexpr (sizeof(T) == 8) en = en / sd[k * nt];
         en_p = en;
         const T e = fmx(en, a.rn_emin) * wmsk<T>(ci, k);
         a.en[c3 + (long)(k - 1) * n2] = e;
-        sl[k * nt] = e;
-        sd[k * nt] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(l[0], a.rsmall)));
+        sl[k * nt] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(l[0], a.rsmall)));
       });
   const T mxl1 = a.ln_mxl0 ? fmx(a.rn_mxl0, a.zraug * taum * tm1) : a.rn_mxl0;
   // downward limits of nn_mxl = 2 (in place) and 3 (su, from the unlimited lengths)
   if (a.nn_mxl == 2 || a.nn_mxl == 3) {
-    T* const out = a.nn_mxl == 2 ? sd : su;
+    T* const out = a.nn_mxl == 2 ? sl : su;
     T p = mxl1;
     for (int k = 2; k <= jpk - 1; ++k) {
-      p = fmn(p + d.e3t_n(ij, k - 1, m), sd[k * nt]);
+      p = fmn(p + d.e3t_n(ij, k - 1, m), sl[k * nt]);
       out[k * nt] = p;
     }
   }
   // upward sweep: the limited lengths, the coefficients, the ocean Kz
   const T evd = a.rn_evd;
   T nxt = a.rmxl_min;  // zmxlm(jpk)
-#pragma unroll 2
-  for (int k = jpk - 1; k >= 2; --k) {
+  auto limit = [&](int x, T (&l)[1]) {
+    const int k = jpk + 1 - x;
     const long q = c3 + (long)(k - 1) * n2;
     const T wm = wmsk<T>(ci, k), tm = tmsk<T>(ci, k);
-    const T raw = sd[k * nt];
+    const T raw = sl[k * nt];
     T lm, ld;
     if (a.nn_mxl == 2) {
       lm = fmn(nxt + d.e3t_n(ij, k + 1, m), raw);
@@ -1740,7 +1780,7 @@ __global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a)
       lm = z * wm + fmn(raw, e3w) * (T(1) - wm);
       ld = z * wm + fmn(lm, e3w) * (T(1) - wm);
     }
-    const T zsqen = sqrt(sl[k * nt]);
+    const T zsqen = sqrt(l[0]);
     const T zav = a.rn_ediff * lm * zsqen;
     const T avmk = fmx(zav, a.rn_avm0) * wm;
     T avtk = fmx(zav, a.rn_avt0) * wm;
@@ -1756,7 +1796,8 @@ __global__ void __launch_bounds__(32 * TKE_Y) k_zdf_tke(Dom<T> d, ZphyArgs<T> a)
     a.avt[q] = avt;
     a.avm[q] = avm;
     if (a.avs) a.avs[q] = avt;
-  }
+  };
+  march<T, 1>(2, jpk - 1, [&](int x, T (&l)[1]) { l[0] = a.en[c3 + (long)(jpk - x) * n2]; }, limit);
   // the surface level: coefficients from en(1) and the surface length; avt, avm
   // keep their values there unless zdf_evd acts
   {
