@@ -211,8 +211,9 @@ cudaError_t launch_dyn_ldf_lap(const Dom<T>& d, const T* ahmt, const T* ahmf, co
                                T zsign, cudaStream_t s) {
   const int kch = march_chunk(d);
   const bool flat = d.e3f_n.s == 0 && d.e3t_b.s == 0 && d.e3u_n.s == 0 && d.e3v_n.s == 0;
-  const dim3 g = march_grid(d, kch, 30, 2);  // a warp writes 30 interior points
-  (flat ? k_dyn_ldf_lap<T, true> : k_dyn_ldf_lap<T, false>)<<<g, dim3(SX, MARCH_Y), 0, s>>>(
+  dim3 g = march_grid(d, kch, 30, 2);  // a block writes 30 x (LDF_Y - 2) interior points
+  g.y = (max(d.jpj - 2, 1) + LDF_Y - 3) / (LDF_Y - 2);
+  (flat ? k_dyn_ldf_lap<T, true> : k_dyn_ldf_lap<T, false>)<<<g, dim3(SX, LDF_Y), 0, s>>>(
       d, ahmt, ahmf, pub, pvb, pua, pva, zsign, kch);
   ktick(NEMO_K_DYN_LDF, s);
   return cudaGetLastError();

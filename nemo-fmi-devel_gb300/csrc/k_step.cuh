@@ -1230,81 +1230,80 @@ __global__ void k_zdf_mxl(Dom<T> d, MxlArgs<T> a) {
 // * quotients by what a chunk shares (the e1, e2 of the column; with 1-D scale factors,
 //   FLAT, the e3 of the level, whose reciprocals the block forms once) are divr's.
 // One point a thread, they took 248, 150 and 73 us and, one column a thread, dyn_zad
-// 191 us at 752x502x31 in FP32; so they take 107, 65, 61 and 65 us (floors by traffic:
+// 191 us at 752x502x31 in FP32; so they take 93, 65, 60 and 65 us (floors by traffic:
 // 56, 42, 42 and 49 us; the rest is instruction issue and the latency left).
 // dyn_ldf_lap (dynldf_lap_blp.F90:37-104), linear free surface (e3*_b = e3*_n):
 // -curl(curl) + grad(div) of the before velocity, each relative vorticity zcur and
-// divergence zdiv by the reference's expression. A warp covers 32 points of a row and
-// writes the inner 30: zcur of the western and zdiv of the eastern point come from the
-// neighbour lane, so that a point forms two of each instead of three.
+// divergence zdiv by the reference's expression, formed once a tile: a block covers 32 x
+// LDF_Y points and writes the inner 30 x (LDF_Y - 2); zcur of the western and zdiv of the
+// eastern point come from the neighbour lane, zcur of the southern and zdiv of the northern
+// point from shared memory (two buffers, one barrier a level). A point that formed two of
+// each took 96 registers, 16 loads a level and 107 us at 752x502x31 in FP32, 93 so (blocks
+// of 10, 12, 16 rows: 94, 94, 97).
+constexpr int LDF_Y = 8;
 template <class T, bool FLAT>
-__global__ void __launch_bounds__(32 * MARCH_Y) k_dyn_ldf_lap(Dom<T> d, const T* __restrict__ ahmt,
-                                                              const T* __restrict__ ahmf, const T* __restrict__ pub,
-                                                              const T* __restrict__ pvb, T* __restrict__ pua,
-                                                              T* __restrict__ pva, T zsign, int kch) {
+__global__ void __launch_bounds__(32 * LDF_Y, FLAT && sizeof(T) == 4 ? 5 : 2) k_dyn_ldf_lap(Dom<T> d, const T* __restrict__ ahmt,
+                                                            const T* __restrict__ ahmf, const T* __restrict__ pub,
+                                                            const T* __restrict__ pvb, T* __restrict__ pua,
+                                                            T* __restrict__ pva, T zsign, int kch) {
   __shared__ E3Prof<T> pt, pu, pv;
-  __shared__ T pf[KMAX + 1];
+  __shared__ T pf[KMAX + 1], scur[2][LDF_Y][32], sdiv[2][LDF_Y][32];
   const MarchIdx c = march_index(d, kch, 30);
-  const int j = c.j, J = d.jpi;
+  const int J = d.jpi, x = threadIdx.x, y = threadIdx.y, j = blockIdx.y * (LDF_Y - 2) + y + 1;
   if constexpr (FLAT) {
     pt.fill(d.e3t_b, c.m, d.jpk);
     pu.fill(d.e3u_n, c.m, d.jpk);
     pv.fill(d.e3v_n, c.m, d.jpk);
-    const int k = threadIdx.y * 32 + threadIdx.x + 1;
+    const int k = y * 32 + x + 1;
     if (k <= d.jpk) pf[k] = d.e3f_n(0, k, c.m);
     __syncthreads();
   }
-  if (j < 2 || j > d.jpj - 1) return;  // whole warps
-  // lanes outside 2..jpi-1 feed their neighbours: zcur at i = 1, zdiv at i = jpi
-  const bool cu = c.i <= J - 1, dv = c.i >= 2 && c.i <= J;
-  const bool out = cu && dv && threadIdx.x >= 1 && threadIdx.x <= 30;
-  const long p = (long)(min(c.i, J) - 1) + (long)(j - 1) * J;
-  const int e = cu ? 1 : 0, w = dv ? 1 : 0;  // offsets that stay in the row
-  // metrics of the f-points p, p-J and of the t-points p, p+J
-  const T rf0 = d.r1_e1e2f[p], rfs = d.r1_e1e2f[p - J];
-  const T v0 = d.e2v[p], ve = d.e2v[p + e], vs = d.e2v[p - J], vse = d.e2v[p - J + e];
-  const T u0 = d.e1u[p], un = d.e1u[p + J], us = d.e1u[p - J];
-  const T rt0 = d.r1_e1e2t[p], rtn = d.r1_e1e2t[p + J];
-  const T x0 = d.e2u[p], xw = d.e2u[p - w], xn = d.e2u[p + J], xnw = d.e2u[p + J - w];
-  const T y0 = d.e1v[p], ys = d.e1v[p - J], yn = d.e1v[p + J];
+  const int i0 = min(c.i, J), j0 = min(j, d.jpj);
+  const bool out = c.i >= 2 && c.i <= J - 1 && x >= 1 && x <= 30 && j >= 2 && j <= d.jpj - 1 && y >= 1 && y <= LDF_Y - 2;
+  // offsets that stay in the domain (a value formed with one of 0 is not used)
+  const int e = i0 < J ? 1 : 0, w = i0 > 1 ? 1 : 0, n = j0 < d.jpj ? J : 0, s = j0 > 1 ? J : 0;
+  const long p = (long)(i0 - 1) + (long)(j0 - 1) * J;
+  const T rf0 = d.r1_e1e2f[p], rt0 = d.r1_e1e2t[p];
+  const T v0 = d.e2v[p], ve = d.e2v[p + e], u0 = d.e1u[p], un = d.e1u[p + n];
+  const T x0 = d.e2u[p], xw = d.e2u[p - w], y0 = d.e1v[p], ys = d.e1v[p - s];
   const T r2u = d.r1_e2u[p], r1u = d.r1_e1u[p], r1v = d.r1_e1v[p], r2v = d.r1_e2v[p];
   const long o = (long)c.m * d.n3 + p;
-  march<T, 16>(
+  march<T, 8>(
       c.k0, c.k1,
-      [&](int k, T (&l)[16]) {
+      [&](int k, T (&l)[8]) {
         const long q = o + (long)(k - 1) * d.n2;
-        const T *u = pub + q, *v = pvb + q, *hf = ahmf + q, *ht = ahmt + q;
-        l[0] = __ldg(u); l[1] = __ldg(u - w); l[2] = __ldg(u + J); l[3] = __ldg(u - J); l[4] = __ldg(u + J - w);
-        l[5] = __ldg(v); l[6] = __ldg(v + e); l[7] = __ldg(v - J); l[8] = __ldg(v - J + e); l[9] = __ldg(v + J);
-        l[10] = __ldg(hf); l[11] = __ldg(hf - J); l[12] = __ldg(ht); l[13] = __ldg(ht + J);
-        l[14] = pua[q]; l[15] = pva[q];
+        l[0] = __ldg(pub + q); l[1] = __ldg(pub + q + n); l[2] = __ldg(pvb + q); l[3] = __ldg(pvb + q - s);
+        l[4] = __ldg(ahmf + q); l[5] = __ldg(ahmt + q);
+        if (out) { l[6] = pua[q]; l[7] = pva[q]; }
       },
-      [&](int k, T (&l)[16]) {
-        T eu, ev, euw, eun, eunw, evs, evn, ef, efs;
+      [&](int k, T (&l)[8]) {
+        T eu, ev, euw, evs, ef;
         if constexpr (FLAT) {
-          eu = euw = eun = eunw = pu.e[k];
-          ev = evs = evn = pv.e[k];
-          ef = efs = pf[k];
+          eu = euw = pu.e[k];
+          ev = evs = pv.e[k];
+          ef = pf[k];
         } else {
           eu = d.e3u_n(p, k, c.m); euw = d.e3u_n(p - w, k, c.m);
-          eun = d.e3u_n(p + J, k, c.m); eunw = d.e3u_n(p + J - w, k, c.m);
-          ev = d.e3v_n(p, k, c.m); evs = d.e3v_n(p - J, k, c.m); evn = d.e3v_n(p + J, k, c.m);
-          ef = d.e3f_n(p, k, c.m); efs = d.e3f_n(p - J, k, c.m);
+          ev = d.e3v_n(p, k, c.m); evs = d.e3v_n(p - s, k, c.m);
+          ef = d.e3f_n(p, k, c.m);
         }
-        auto over_t = [&](T x, long r) { return FLAT ? divr(x, pt.e[k], pt.r[k]) : x / d.e3t_b(r, k, c.m); };
-        auto over_u = [&](T x) { return FLAT ? divr(x, eu, pu.r[k]) : x / eu; };
-        auto over_v = [&](T x) { return FLAT ? divr(x, ev, pv.r[k]) : x / ev; };
-        const T b0 = l[0], c0 = l[5];
-        const T cur0 = l[10] * ef * rf0 * (ve * l[6] - v0 * c0 - un * l[2] + u0 * b0);
-        const T curs = l[11] * efs * rfs * (vse * l[8] - vs * l[7] - u0 * b0 + us * l[3]);
-        const T h0 = y0 * ev * c0;
-        const T div0 = over_t(l[12] * rt0, p) * (x0 * eu * b0 - xw * euw * l[1] + h0 - ys * evs * l[7]);
-        const T divn = over_t(l[13] * rtn, p + J) * (xn * eun * l[2] - xnw * eunw * l[4] + yn * evn * l[9] - h0);
+        const T uw = __shfl_up_sync(0xffffffffu, l[0], 1), vr = __shfl_down_sync(0xffffffffu, l[2], 1);
+        const T cur0 = l[4] * ef * rf0 * (ve * vr - v0 * l[2] - un * l[1] + u0 * l[0]);
+        const T ht = l[5] * rt0;
+        const T div0 = (FLAT ? divr(ht, pt.e[k], pt.r[k]) : ht / d.e3t_b(p, k, c.m)) *
+                       (x0 * eu * l[0] - xw * euw * uw + y0 * ev * l[2] - ys * evs * l[3]);
+        T (&bc)[LDF_Y][32] = scur[k & 1], (&bd)[LDF_Y][32] = sdiv[k & 1];
+        bc[y][x] = cur0;
+        bd[y][x] = div0;
         const T curw = __shfl_up_sync(0xffffffffu, cur0, 1), dive = __shfl_down_sync(0xffffffffu, div0, 1);
+        __syncthreads();
         if (out) {
+          const T curs = bc[y - 1][x], divn = bd[y + 1][x];
+          auto over_u = [&](T a) { return FLAT ? divr(a, eu, pu.r[k]) : a / eu; };
+          auto over_v = [&](T a) { return FLAT ? divr(a, ev, pv.r[k]) : a / ev; };
           const long q = o + (long)(k - 1) * d.n2;
-          pua[q] = l[14] + zsign * (-over_u((cur0 - curs) * r2u) + (dive - div0) * r1u);
-          pva[q] = l[15] + zsign * (over_v((cur0 - curw) * r1v) + (divn - div0) * r2v);
+          pua[q] = l[6] + zsign * (-over_u((cur0 - curs) * r2u) + (dive - div0) * r1u);
+          pva[q] = l[7] + zsign * (over_v((cur0 - curw) * r1v) + (divn - div0) * r2v);
         }
       });
 }
