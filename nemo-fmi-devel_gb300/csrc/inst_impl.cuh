@@ -183,7 +183,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
   }
   const int tc = kty(NEMO_K_FCT_C);
   // FP64 without the iso-neutral trend: the general kernel, two tracers a pass, is the
-  // faster (259 against 346 us at 362x242x31); with it (more loads a level) the other is
+  // faster (210 against 346 us at 362x242x31); with it (more loads a level) the other is
   if (!hot_fct_c_ok(d, a) || (sizeof(T) == 8 && !a.with_iso)) k_fct_c<T><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
   else if (d.e3t_n.s == 0) k_fct_c_hot<T, false><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
   else k_fct_c_hot<T, true><<<kc_grid(d, tc), dim3(BX, tc), 0, s>>>(d, a);
@@ -217,9 +217,19 @@ cudaError_t launch_iso_flux(const Dom<T>& d, const LdfArgs<T>& a, cudaStream_t s
           field_tensor_map(d, a.wslpi.p, 1, TM_X, TM_Y, &maps.wslpi) &&
           field_tensor_map(d, a.wslpj.p, 1, TM_X, TM_Y, &maps.wslpj)) {
         const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
-        (iso_3d(d, a) ? k_iso_flux_tma<T, true> : k_iso_flux_tma<T, false>)<<<grid, dim3(TM_X, TM_Y), 0, s>>>(
+        (iso_3d(d, a) ? k_iso_flux_tma<T, true, true> : k_iso_flux_tma<T, false, true>)<<<grid, dim3(TM_X, TM_Y), 0, s>>>(
             d, a, maps, a.err, a.polls);
         ktick(NEMO_K_ISO_FLUX_TMA, s);
+        return cudaGetLastError();
+      }
+      // rows not 16 bytes apart: the planes copied by the threads. 281 against 342 us of
+      // k_iso_flux_hot at 749x502x31, 101 against 138 at 310x367, 18.3 against 19.0 at
+      // 121x152; on smaller grids (7.0 against 6.2 us at 62x42) a march is too short for it
+      if (a.tma && a.err && d.n2 * d.nmem >= 16384) {
+        const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
+        (iso_3d(d, a) ? k_iso_flux_tma<T, true, false> : k_iso_flux_tma<T, false, false>)<<<grid, dim3(TM_X, TM_Y), 0, s>>>(
+            d, a, maps, a.err, a.polls);
+        ktick(NEMO_K_ISO_FLUX, s);
         return cudaGetLastError();
       }
     }

@@ -180,3 +180,36 @@ def test_glob_sum_of_floats(nk, spread):
     p.torch.cuda.synchronize()
     out = p.ctx.glob_sum(t, nk)
     assert np.isfinite(out[0]) and not np.isfinite(out[1])
+
+
+@pytest.mark.parametrize("nn,jpk", [(6, 9), (8, 20), (8, 31)])
+def test_ragged_rows(nn, jpk):
+    """Rows that are no multiple of 16 bytes long: the tracer planes copied into shared
+    memory by the threads. The specialised kernels without shared memory do the same
+    operations in the same order, so the results are the same bits; both within the mixed
+    tolerance of the oracle. A wait that gives up at once is reported and leaves the
+    context usable."""
+    from nemo_gpu.api import NemoError
+    dom = gyre.domain(nn, jpk=jpk)
+    assert dom["jpi"] % 4
+    res = []
+    for tma in (1, 0):
+        p = Pair(dom=dom, nam=gyre.namelist(), prec="mixed", seed=31)
+        p.bind_hotpath()
+        p.ctx.set_tma(tma)
+        for kt in (5, 6):
+            p.ora[0].stp_hotpath(kt)
+            p.ctx.stp_hotpath(kt)
+            p.ctx.synchronize()
+        p.compare("TSA", p.s4, 5e-6)
+        res.append([np.asarray(p.ctx.to_host(p.dev[n], s)) for n, s in (("TSA", p.s4), ("AH_WSLP2", p.s3))])
+    for x, y in zip(*res):
+        assert np.array_equal(x, y)
+    p.ctx.set_tma(1)
+    p.ctx.set_tma_poll_limit(0)
+    p.ctx.stp_hotpath(7)
+    with pytest.raises(NemoError, match="tensor copy"):
+        p.ctx.synchronize()
+    p.ctx.set_tma_poll_limit(1 << 16)
+    p.ctx.stp_hotpath(8)
+    p.ctx.synchronize()
