@@ -1166,7 +1166,7 @@ __global__ void __launch_bounds__(256, 5) k_spg_p2_ene(Dom<T> d, SpgArgs<T> a, G
 // of a cluster are resident together by definition and none leaves its loop early.
 // The grid-barrier kernels are bound by that barrier and by L2 latency at these sizes:
 // the sub-steps of GYRE nn_GYRE=1 (704 points) took 120 us and of 64 members of nn_GYRE=5
-// 1331 us, and take 52 and 733 us here, bound by instruction issue (250 a point).
+// 1331 us, and take 58 and 750 us here, bound by instruction issue (250 a point).
 constexpr int P2R_MAXC = 16, P2R_NV = 3, P2R_SMEM_MAX = 227 * 1024;
 // shared memory of a block: five float4 of constants a point, five arrays of rows (six in
 // the GEN form), and what the last point of the last array reads as its eastern neighbour
@@ -1595,7 +1595,7 @@ __device__ __forceinline__ double widen(float x) {
 // the points a block adds in one pass span at most 53 - 24 - 12 = 17 binary places, every
 // partial sum of the 2^12 values is exact in a double (24 bits each, 12 bits of carry), and
 // so plain additions give the exact sum of the pass; any other pass (and FP64) takes the
-// double-double path. 38 -> 9 us (one launch instead of two) at 2 x 93x61x62.
+// double-double path. 38 -> 15 us (one launch instead of two) at 2 x 93x61x62.
 constexpr int GS_PT = 16;
 template <class T>
 __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const double* __restrict__ tmask_i, long n2,

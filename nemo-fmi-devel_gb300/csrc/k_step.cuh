@@ -466,7 +466,8 @@ __global__ void k_slp_mxl(Dom<T> d, SlpArgs<T> a) {
 // ranges and the metrics of the column and its neighbours are loaded once a chunk, the
 // densities of the level above and N^2 of the level are carried, and with 1-D scale
 // factors (FLAT) the limits -7e3 / e3 come from a table. One point a thread, which looked
-// up some twenty masks through memory, it took 154 us at 481x323x31 in FP32.
+// up some twenty masks through memory, it took 154 us at 481x323x31 in FP32, 74 so (101
+// registers; bounded to 80 or fewer it spills: 77 to 86 us).
 template <class T, bool ZPS, bool FLAT>
 __global__ void __launch_bounds__(32 * MARCH_Y) k_slp_pre(Dom<T> d, SlpArgs<T> a, int kch) {
   __shared__ T pu[KMAX + 1], pv[KMAX + 1], pw[KMAX + 1];  // -7e3 / e3u, e3v, e3w
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(32 * MARCH_Y) k_slp_pre(Dom<T> d, SlpArgs<T> a
 // Level march; a warp covers 32 points of a row and writes the inner 30, so that of the
 // nine neighbours of the 1-2-1 Shapiro filter (:237-275, :319-353) a point loads its own
 // column's three and gets the others from the neighbour lanes. One point a thread with 36
-// loads and 15 mask look-ups it took 58 us at 481x323x31 in FP32 (22 us by traffic).
+// loads and 15 mask look-ups it took 58 us at 481x323x31 in FP32, 39 so (22 us by traffic).
 template <class T>
 __global__ void __launch_bounds__(32 * MARCH_Y) k_slp_filter(Dom<T> d, SlpArgs<T> a, int kch) {
   const MarchIdx c = march_index(d, kch, 30);
@@ -1038,10 +1039,11 @@ __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
 // eos_insitu (WHAT 0), eos_insitu_pot (1) and rab_3d (2) on levels 1..jpk-1: a thread
 // owns one (i,j) of the flat 2-D plane (no stencil, so no ragged tiles) and a chunk of
 // levels, EOS_U of them loaded before the first polynomial. The polynomials' operands
-// come from the constant bank; the kernels are bound by memory in FP32 (rab_3d moves
-// 5 fields, eos_insitu 4) and by the FP64 pipe in FP64. As one point a thread, with
+// come from the constant bank; the kernels are bound by instruction issue in FP32 (66 to
+// 72 % of the slots: some 110 instructions a point of the polynomials; by traffic, 4 and 5
+// fields, 28 and 35 us of 48 and 55) and by the FP64 pipe in FP64. As one point a thread, with
 // the coefficients loaded from global memory, the six calls of a step's density (two
-// rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32.
+// rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32, 358 so.
 constexpr int EOS_BLOCK = 256;
 template <class T>
 constexpr int EOS_LEV = sizeof(T) == 4 ? 4 : 1;  // FP64: four levels in a row left a small grid's FP64 pipes idle
@@ -1538,7 +1540,7 @@ __device__ __forceinline__ float lc_sin(float x) { return sinf(x); }
 // with a linear free surface e3uw_n = e3uw_b = the rest-state MIN of the neighbouring
 // e3w). Level march: the velocities of the level above are carried, the quotients by the
 // squared e3 of the level are divr's with 1-D scale factors (FLAT). One point a thread
-// it took 67 us at 481x323x31 in FP32 (17 us by traffic).
+// it took 67 us at 481x323x31 in FP32, 34 so (17 us by traffic).
 template <class T, bool FLAT>
 __global__ void __launch_bounds__(32 * MARCH_Y) k_zdf_sh2(Dom<T> d, ZphyArgs<T> a, int kch) {
   __shared__ T pe[KMAX + 1], pr[KMAX + 1];  // e3w^2 and its reciprocal
