@@ -37,6 +37,14 @@ __device__ __forceinline__ T u_in(const ColInfo& c, int k) { return (k >= c.ulo 
 template <class T>
 __device__ __forceinline__ T v_in(const ColInfo& c, int k) { return (k >= c.vlo && k <= c.vhi) ? T(1) : T(0); }
 
+// x / y given ry = 1 / y correctly rounded: FP64 for finite x / y (its test for others
+// would run on the FP64 pipe)
+template <class T>
+__device__ __forceinline__ T div_by(T x, T y, T ry) {
+  if constexpr (sizeof(T) == 8) return divq(x, y, ry);
+  else return divr(x, y, ry);
+}
+
 // Iso-neutral fluxes (traldf_iso.F90:146-357) of one column chunk; see k_iso_flux.
 // It also sets akz = ah_wslp2 on the points k_iso_akz_copy_edges covers in general. G3: 3-D
 // scale factors or partial steps, whose bottom gradients are loaded once a column. The
@@ -265,8 +273,12 @@ inline bool hot_fct_c_ok(const Dom<T>& d, const FctArgs<T>& a) {
 // FCT stage a (traadv_fct.F90:119-280) of one column chunk; see k_fct_a. Tracer nn
 // of the member is at offset nn * n3 from tracer 0. TRP: pun, pvn, pwn are velocities, to
 // be scaled to transports; TIN: there may be a trend to add to (FP32 spills with it).
+// Bound by the loads in flight, so by the warps: 214 us at 749x502x31 in FP32 with 40 warps
+// an SM (48 registers, 40 bytes of spills, tn loaded with tb), 239 with 32, 290 with 24.
+// e3t is the one rest-state profile of the three time levels; its quotients as in the TMA
+// form, whose bits the two share.
 template <class T, bool TRP, bool TIN>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 10) : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpk = d.jpk, n2 = (int)d.n2, n3 = (int)d.n3, ij = (int)c.ij;
@@ -292,9 +304,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct
   const T e1e2t = d.e1e2t[ij], r1_e1e2t = d.r1_e1e2t[ij];
   const T* e3u = d.e3u_n.p.p;
   const T* e3v = d.e3v_n.p.p;
-  const T* e3tn = d.e3t_n.p.p;
-  const T* e3tb = d.e3t_b.p.p;
-  const T* e3ta = d.e3t_a.p.p;
+  const T* e3t = d.e3t_n.p.p;  // the rest-state profile of all three time levels
   const long mv = (long)c.m * d.n3 + ij;
   const T* un = a.pun.p + mv;
   const T* vn = a.pvn.p + mv;
@@ -332,8 +342,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct
       const T vs = scaled(e1vs * e3vk, __ldg(vn + q - jpi));
       if (first) wt = scaled(e1e2t, __ldg(wn + q));
       const T wb = (k + 1 <= jpk - 1) ? scaled(e1e2t, __ldg(wn + q + n2)) : T(0);
-      const T e3n = __ldg(e3tn + k - 1), e3b = __ldg(e3tb + k - 1), e3a = __ldg(e3ta + k - 1);
-      const T r1n = d.r1_e3t[k - 1];  // e3t_n, e3t_b and e3t_a are the one rest-state profile here
+      const T e3 = __ldg(e3t + k - 1), r1_e3 = d.r1_e3t[k - 1];
       const T tm = tk, wk = k == 1 ? tk : msel(tk, tkm), wk1 = msel(tkp, tk);
 #pragma unroll
       for (int nn = 0; nn < NT; ++nn) {
@@ -342,6 +351,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct
         const T* tb = tbp_ + o;
         const T* tn = tnp_ + o;
         const T tb0 = __ldg(tb + q);
+        const T tn0 = __ldg(tn + q), tne = __ldg(tn + q + 1), tnn = __ldg(tn + q + jpi);
         if (first && k > 1) {  // the carried values of level k-1
           tbc[nn] = __ldg(tb + q - n2);
           tnc[nn] = __ldg(tn + q - n2);
@@ -353,10 +363,9 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 8) : 3) k_fct
         const T zwz_t = (k == 1) ? (a.linssh ? wt * tb0 : T(0)) : zwzb[nn];
         const T zwz_b = (k + 1 <= jpk - 1) ? msel(ups(wb, __ldg(tb + q + n2), tb0), wk1) : T(0);
         const T ztra = -(zwx_e - zwx_w + zwy_n - zwy_s + zwz_t - zwz_b) * r1_e1e2t;
-        ta[o + q] = (tai ? tai[o + q] : T(0)) + msel(divq(ztra, e3n, r1n), tm);
-        zwi[o + q] = msel(divq(e3b * tb0 + p2dt * ztra, e3a, r1n), tm);
+        ta[o + q] = (tai ? tai[o + q] : T(0)) + msel(div_by(ztra, e3, r1_e3), tm);
+        zwi[o + q] = msel(div_by(e3 * tb0 + p2dt * ztra, e3, r1_e3), tm);
         // 2nd-order antidiffusive fluxes (:180-190, :255-263)
-        const T tn0 = __ldg(tn + q), tne = __ldg(tn + q + 1), tnn = __ldg(tn + q + jpi);
         ax[o + q] = T(0.5) * ue * (tn0 + tne) - zwx_e;
         ay[o + q] = T(0.5) * vn_ * (tn0 + tnn) - zwy_n;
         az[o + q] = k >= 2 ? msel(wt * T(0.5) * (tn0 + tnc[nn]) - zwz_t, wk) : T(0);
