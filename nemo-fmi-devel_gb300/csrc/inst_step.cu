@@ -26,10 +26,12 @@ int level_chunk(const Dom<T>& d, int block, int step) {
 // the two components' columns: z = 2 member + component
 template <class T>
 dim3 s_cols2(const Dom<T>& d, int ty) { return dim3((d.jpi + SX - 1) / SX, (d.jpj + ty - 1) / ty, 2 * d.nmem); }
-// shared memory (dynamic, and a few KB static) beyond the 48 KB default needs the opt-in
+// Shared memory beyond the 48 KB default needs the opt-in, which every context of the
+// device shares: always the most that any launch asks for (KMAX levels), so that no call
+// lowers what another thread's launch is about to use.
 template <class K>
-cudaError_t smem_opt_in(K kern, int bytes) {
-  return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+cudaError_t smem_opt_in(K kern, int most) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
 }
 }  // namespace
 
@@ -49,8 +51,8 @@ cudaError_t launch_dyn_zdf_step(const Dom<T>& d, const T* ub, const T* vb, T* ua
 }
 template <class T>
 cudaError_t launch_dyn_nxt(const Dom<T>& d, const NxtArgs<T, double>& a, cudaStream_t s) {
-  const int smem = 32 * DN_Y * d.jpk * (int)sizeof(T);
-  if (cudaError_t e = smem_opt_in(k_dyn_nxt<T, double>, smem)) return e;
+  const int level = 32 * DN_Y * (int)sizeof(T), smem = level * d.jpk;
+  if (cudaError_t e = smem_opt_in(k_dyn_nxt<T, double>, level * KMAX)) return e;
   k_dyn_nxt<T, double><<<s_cols2<T>(d, DN_Y), dim3(SX, DN_Y), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_NXT, s);
   return cudaGetLastError();
@@ -171,7 +173,7 @@ cudaError_t launch_dyn_zdf_imp(const Dom<T>& d, const DynZdfArgs<T>& a, cudaStre
   const bool flat = d.e3u_n.s == 0 && d.e3v_n.s == 0 && d.e3w_n.s == 0;
   const int smem = dyn_zdf_smem(32 * DZ_Y<T>, d.jpk, flat, (int)sizeof(T));
   const auto kern = flat ? k_dyn_zdf_imp<T, true> : k_dyn_zdf_imp<T, false>;
-  if (cudaError_t e = smem_opt_in(kern, smem)) return e;
+  if (cudaError_t e = smem_opt_in(kern, dyn_zdf_smem(32 * DZ_Y<T>, KMAX, flat, (int)sizeof(T)))) return e;
   kern<<<s_cols2<T>(d, DZ_Y<T>), dim3(SX, DZ_Y<T>), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_ZDF_STEP, s);
   return cudaGetLastError();
@@ -196,9 +198,9 @@ cudaError_t launch_usr_put(double* dst, const double* v, cudaStream_t s) {
 
 template <class T>
 cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s) {
-  const int kch = march_chunk(d), smem = (sizeof(T) == 4 ? 3 : 4) * 32 * TKE_Y<T> * d.jpk * (int)sizeof(T);
+  const int kch = march_chunk(d), level = (sizeof(T) == 4 ? 3 : 4) * 32 * TKE_Y<T> * (int)sizeof(T), smem = level * d.jpk;
   const auto tke = d.e3w_n.s == 0 && d.e3t_n.s == 0 ? k_zdf_tke<T, true> : k_zdf_tke<T, false>;
-  if (cudaError_t e = smem_opt_in(tke, smem)) return e;
+  if (cudaError_t e = smem_opt_in(tke, level * KMAX)) return e;
   (d.e3w_n.s == 0 ? k_zdf_sh2<T, true> : k_zdf_sh2<T, false>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   ktick(NEMO_K_ZDF_PHY, s);
   tke<<<dim3((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y<T> - 1) / TKE_Y<T>, d.nmem), dim3(SX, TKE_Y<T>), smem, s>>>(d, a);
