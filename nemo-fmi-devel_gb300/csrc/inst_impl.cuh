@@ -101,9 +101,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
                           field_tensor_map(d, a.ptb.p, a.kjpt, FF_BW, FF_BH, &maps.m[3]) &&
                           field_tensor_map(d, a.ptn.p, a.kjpt, FF_BW, FF_BH, &maps.m[4]);
           if (ok) {
-            static const cudaError_t attr =
-                cudaFuncSetAttribute(k_fct_fused_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FF_SMEM);
-            if (attr != cudaSuccess) return attr;
+            if (cudaError_t e = smem_opt_in(k_fct_fused_tma<T>, FF_SMEM)) return e;
             const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem);
             k_fct_fused_tma<T><<<grid, dim3(TM_X, TM_Y), FF_SMEM, s>>>(d, a, maps, a.err, a.polls);
             ktick(NEMO_K_FCT_FUSED, s);
@@ -121,18 +119,11 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
           ma.m[6] = ma.m[5];
           ok = ok && fct_b_maps(d, a, mb);
           if (ok) {
-            static const cudaError_t attr_a =
-                cudaFuncSetAttribute(k_fct_a_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
-            static const cudaError_t attr_a2 =
-                cudaFuncSetAttribute(k_fct_a_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
-            static const cudaError_t attr_b =
-                cudaFuncSetAttribute(k_fct_b_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
-            if (attr_a != cudaSuccess) return attr_a;
-            if (attr_a2 != cudaSuccess) return attr_a2;
-            if (attr_b != cudaSuccess) return attr_b;
+            const auto stage_a = a.trp && !a.pta_in ? k_fct_a_tma<T, true> : k_fct_a_tma<T, false>;
+            if (cudaError_t e = smem_opt_in(stage_a, FA_SMEM)) return e;
+            if (cudaError_t e = smem_opt_in(k_fct_b_tma<T>, FB_SMEM)) return e;
             const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
-            (a.trp && !a.pta_in ? k_fct_a_tma<T, true> : k_fct_a_tma<T, false>)<<<grid, dim3(TM_X, TM_Y), FA_SMEM, s>>>(
-                d, a, ma, a.err, a.polls);
+            stage_a<<<grid, dim3(TM_X, TM_Y), FA_SMEM, s>>>(d, a, ma, a.err, a.polls);
             ktick(NEMO_K_FCT_A_TMA, s);
             k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);
             ktick(NEMO_K_FCT_B_TMA, s);
@@ -149,10 +140,8 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
     ktick(NEMO_K_FCT_A, s);
   } else {
     if (a.kn_fct_v == 4) {
-      const int smem = 32 * I4_Y * (d.jpk + 1) * (int)sizeof(T);
-      static const cudaError_t attr = cudaFuncSetAttribute(k_interp4<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           32 * I4_Y * (KMAX + 1) * (int)sizeof(T));
-      if (attr != cudaSuccess) return attr;
+      const int level = 32 * I4_Y * (int)sizeof(T), smem = level * (d.jpk + 1);
+      if (cudaError_t e = smem_opt_in(k_interp4<T>, level * (KMAX + 1))) return e;
       k_interp4<T><<<dim3((d.jpi + 31) / 32, (d.jpj + I4_Y - 1) / I4_Y, d.nmem * a.kjpt), dim3(32, I4_Y), smem, s>>>(
           d, a.ptn, const_cast<T*>(a.ztw.p), a.kjpt);
       ktick(NEMO_K_INTERP4, s);
@@ -166,9 +155,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {  // stage b takes any e3t_n (its planes staged by TMA: any orders of stage a)
     PlaneMaps<FB_NF> mb;
     if (a.tma && a.err && a.kjpt == 2 && !a.lim && d.n3 < (1L << 30) && fct_b_maps(d, a, mb)) {
-      static const cudaError_t attr =
-          cudaFuncSetAttribute(k_fct_b_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM);
-      if (attr != cudaSuccess) return attr;
+      if (cudaError_t e = smem_opt_in(k_fct_b_tma<T>, FB_SMEM)) return e;
       const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
       k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);
       ktick(NEMO_K_FCT_B_TMA, s);
@@ -268,17 +255,13 @@ cudaError_t launch_zdf(const Dom<T>& d, const ZdfArgs<T>& a, cudaStream_t s) {
     if (d.jpi < 3 || d.jpj < 3) return cudaSuccess;  // no interior column
     if (d.jpk == 31 && d.n2 * d.nmem >= ZDF31_MIN) {  // the GYRE levels: columns staged in shared memory
       constexpr int smem_max = 4 * 31 * BX * BY * sizeof(float);
-      static const cudaError_t attr31 =
-          cudaFuncSetAttribute(k_zdf_imp_async<31>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-      if (attr31 != cudaSuccess) return attr31;
+      if (cudaError_t e = smem_opt_in(k_zdf_imp_async<31>, smem_max)) return e;
       const int tz = kty(NEMO_K_ZDF_IMP);
       k_zdf_imp_async<31><<<col_grid(d, tz), dim3(BX, tz), 4 * 31 * BX * tz * sizeof(float), s>>>(d, a);
       ktick(NEMO_K_ZDF_IMP, s);
       return cudaGetLastError();
     }
-    static const cudaError_t attr =  // dynamic shared memory beyond 48 KB needs the opt-in
-        cudaFuncSetAttribute(k_zdf_imp32<ZW>, cudaFuncAttributeMaxDynamicSharedMemorySize, zdf32_smem(KMAX));
-    if (attr != cudaSuccess) return attr;
+    if (cudaError_t e = smem_opt_in(k_zdf_imp32<ZW>, zdf32_smem(KMAX))) return e;
     k_zdf_imp32<ZW><<<dim3((unsigned)((d.jpi + 31) / 32) * (d.jpj - 2), d.nmem), dim3(32, ZW), zdf32_smem(d.jpk), s>>>(d, a);
   } else {
     const int tz = kty(NEMO_K_ZDF_IMP);

@@ -26,13 +26,6 @@ int level_chunk(const Dom<T>& d, int block, int step) {
 // the two components' columns: z = 2 member + component
 template <class T>
 dim3 s_cols2(const Dom<T>& d, int ty) { return dim3((d.jpi + SX - 1) / SX, (d.jpj + ty - 1) / ty, 2 * d.nmem); }
-// Shared memory beyond the 48 KB default needs the opt-in, which every context of the
-// device shares: always the most that any launch asks for (KMAX levels), so that no call
-// lowers what another thread's launch is about to use.
-template <class K>
-cudaError_t smem_opt_in(K kern, int most) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-}
 }  // namespace
 
 template <class T>

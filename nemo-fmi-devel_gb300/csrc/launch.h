@@ -37,6 +37,15 @@ inline void ktick(int id, cudaStream_t s) {
   }
 }
 
+// Shared memory beyond the 48 KB default needs the opt-in, which belongs to the kernel on
+// the current device and is shared by every context there: made at each launch (a process
+// may have contexts on several devices), and always for the most that any launch asks for,
+// so that no call lowers what another thread's launch is about to use.
+template <class K>
+cudaError_t smem_opt_in(K kern, int most) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 template <class T>
 cudaError_t launch_adv_trp(const Dom<T>& d, const T* un, const T* vn, const T* wn, T* zun, T* zvn, T* zwn,
                            cudaStream_t s);

@@ -1,0 +1,139 @@
+// A stand-in for the CUDA runtime on a machine without a GPU, preloaded in front of it: two
+// devices of 152 SMs, memory from the host's heap, no kernel runs. What the library asks for
+// is checked and written down: a launch whose dynamic shared memory is beyond 48 KB and
+// beyond what the kernel was opted in for on the current device is refused, as by the real
+// runtime, and every accepted launch is logged with its kernel, grid, block and shared memory.
+#include <cuda_runtime_api.h>
+#include <cudaTypedefs.h>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <string>
+#include <utility>
+
+namespace {
+int device = 0;
+std::map<const void*, std::string> name;                    // host stub -> kernel
+std::map<std::pair<int, const void*>, size_t> opted;        // (device, stub) -> opt-in
+std::string launches;
+struct Config {
+  dim3 grid, block;
+  size_t smem;
+  void* stream;
+} pushed;
+
+cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem) {
+  const auto it = opted.find({device, f});
+  const size_t most = it == opted.end() ? 48 * 1024 : it->second;
+  if (smem > 48 * 1024 && smem > most) return cudaErrorInvalidValue;
+  if (!g.x || !g.y || !g.z || g.y > 65535 || g.z > 65535 || !b.x || b.x * b.y * b.z > 1024)
+    return cudaErrorInvalidConfiguration;
+  launches += name[f] + " " + std::to_string(g.x) + " " + std::to_string(g.y) + " " + std::to_string(g.z) + " " +
+              std::to_string(b.x) + " " + std::to_string(b.y) + " " + std::to_string(smem) + "\n";
+  return cudaSuccess;
+}
+CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                CUtensorMapFloatOOBfill) {
+  return CUDA_SUCCESS;
+}
+void* handle() { return calloc(1, 8); }
+}  // namespace
+
+extern "C" {
+const char* fake_launches() { return launches.c_str(); }
+void fake_clear() { launches.clear(); }
+cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+
+void** __cudaRegisterFatBinary(void*) { return (void**)handle(); }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+void __cudaRegisterFunction(void**, const char* stub, char*, const char* kernel, int, void*, void*, void*, void*, int*) {
+  name[stub] = kernel;
+}
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, void* s) {
+  pushed = Config{g, b, smem, s};
+  return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) {
+  *g = pushed.grid; *b = pushed.block; *smem = pushed.smem;
+  *(void**)s = pushed.stream;
+  return cudaSuccess;
+}
+cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* stub) { *k = (cudaKernel_t)stub; return cudaSuccess; }
+static cudaError_t last = cudaSuccess;
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void**, size_t smem, cudaStream_t) {
+  const cudaError_t e = launch((const void*)k, g, b, smem);
+  if (e != cudaSuccess) last = e;
+  return e;
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+  return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes);
+}
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = last;
+  last = cudaSuccess;
+  return e;
+}
+const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorInvalidValue ? "invalid argument" : "error"; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
+  if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    if (v > 227 * 1024) return cudaErrorInvalidValue;
+    opted[{device, f}] = v;
+  }
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+  *v = a == cudaDevAttrMultiProcessorCount ? 152 : 0;
+  return cudaSuccess;
+}
+// blocks an SM by registers alone, as the kernels' launch bounds ask for; clusters by SMs
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int, size_t, unsigned) {
+  const std::string& k = name[f];
+  *n = k.find("k_spg_p2_ene") != std::string::npos || k.find("Li5E") != std::string::npos ? 5
+       : k.find("IdL") != std::string::npos ? 2 : 4;
+  return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* c) {
+  *n = 128 / (int)c->attrs[0].val.clusterDim.x;
+  return cudaSuccess;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* q) {
+  *f = (void*)encode;
+  *q = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
+
+cudaError_t cudaMalloc(void** p, size_t n) { *p = aligned_alloc(256, (n + 255) / 256 * 256); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaGetSymbolAddress(void** p, const void*) { *p = calloc(1, 1 << 20); return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)handle(); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)handle(); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)handle(); return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { free(e); return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+}

@@ -1,0 +1,32 @@
+"""What the library launches, checked without a GPU over a stand-in for the CUDA runtime."""
+import fakedev
+
+
+def test_shared_memory_on_a_second_device():
+    """A process with contexts on two devices: each kernel that needs more than 48 KB of
+    shared memory is opted in on both."""
+    out = fakedev.run(r"""
+seen = []
+for device in (0, 1):
+    fake.cudaSetDevice(device)
+    for prec, jpk, order, fused in (("mixed", 31, 2, 0), ("mixed", 31, 2, 1), ("mixed", 64, 4, 0), ("fp64", 64, 4, 0)):
+        dom = gyre.domain(1, jpk=jpk)
+        c = Ctx(dom, gyre.namelist(), prec, nmem=100 if fused else 1)  # enough columns for each form of tra_zdf
+        c.bind("AVT", "AH_WSLP2", "AKZ", "TSB", "TSN", "TSA", "UN", "VN", "WN", "USLP", "VSLP", "WSLPI", "WSLPJ")
+        c.bind("UA", "VA", "UB", "VB", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP", "RCDU_BOT",
+               "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")
+        c("set_fct_fused", fused)
+        t = [c.array(2 * c.n3) for _ in range(6)]
+        launches()
+        c("tra_adv_fct", 10, 1, b"TRA", 14400.0, *t, 2, order, order)
+        c("tra_zdf_imp", 10, 1, b"TRA", 14400.0, t[3], t[5], 2)
+        if order == 2:
+            c("stp_hotpath", 10)
+        seen += [[device, k[0]] for k in launches() if k[-1] > 48 * 1024]
+        c.close()
+print(json.dumps(seen))
+""")
+    first, second = ({k for d, k in out if d == dev} for dev in (0, 1))
+    assert first == second
+    for k in ("k_fct_b_tma", "k_fct_fused_tma", "k_interp4IdE", "k_zdf_imp_async", "k_zdf_imp32"):
+        assert any(k in name for name in second), k
