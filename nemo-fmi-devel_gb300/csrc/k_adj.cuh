@@ -37,18 +37,23 @@ struct Pt3 {
 template <class T>
 __device__ __forceinline__ Pt3 pt3(const Dom<T>& d) { return Pt3{d.jpi, d.jpj, d.jpk, d.n2}; }
 
-// x / e3t_n(k) and x / e3w_n(k): through the reciprocal profile (divq, the correctly
+// x / e3t_n(k) and x / e3w_n(k): through the reciprocal profile (divr, the correctly
 // rounded quotient) where the now scale factor is the rest-state profile
 __device__ __forceinline__ double over_e3t(const Dom<double>& d, double x, long ij, int k, int m) {
   const double e = d.e3t_n(ij, k, m);
-  return d.r1_e3t && d.e3t_n.s == 0 ? divq(x, e, d.r1_e3t[k - 1]) : x / e;
+  return d.r1_e3t && d.e3t_n.s == 0 ? divr(x, e, d.r1_e3t[k - 1]) : x / e;
 }
 __device__ __forceinline__ double over_e3w(const Dom<double>& d, double x, long ij, int k, int m) {
   const double e = d.e3w_n(ij, k, m);
-  return d.r1_e3w && d.e3w_n.s == 0 ? divq(x, e, d.r1_e3w[k - 1]) : x / e;
+  return d.r1_e3w && d.e3w_n.s == 0 ? divr(x, e, d.r1_e3w[k - 1]) : x / e;
 }
 // x != 0 on the integer pipe (NaN counts as nonzero)
 __device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+// x times a zero, on the integer pipe: NaN where x is not finite
+__device__ __forceinline__ double zero_of(double x) {
+  return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+}
 
 // ------------------------------------------------------------------ tra_adv_fct
 // Adjoint of tra_adv_fct (traadv_fct.F90:54-327) at one point; with kn_fct_h = 4 the
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
 // inside (30 x (FADJ_Y - 2) points are written). Bound by the FP64 pipe: a point of
 // k_fct_adj divides seven times a tracer and forms all six faces (1053 us at
 // 302x202x31, T and S), 420 so. Values as k_fct_adj's: an upstream flux's adjoint f reaches the
-// point upstream of its face as u f and the other as 0 (0.5 (u + |u|) is u or 0).
+// point upstream of its face as u f and the other as zero_of(u f) (0.5 (u + |u|) is u or 0).
 constexpr int FADJ_Y = 16, FADJ_K = 8;
 __global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj a) {
   constexpr int NT = 2;
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj 
           ry[nn] = v * (-ay + (msel(gn, tmsk<double>(cn, k)) - hc));
         }
         sp[nn][row][lane] = py[nn];
-        sr[nn][row][lane] = sgn_pos(v) ? 0.0 : ry[nn];  // for the northern point
+        sr[nn][row][lane] = sgn_pos(v) ? zero_of(ry[nn]) : ry[nn];  // for the northern point
       }
       __syncthreads();
       const double wt = own && k >= 2 ? wn[q] : 0.0;
@@ -247,7 +252,7 @@ __global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj 
 #pragma unroll
       for (int nn = 0; nn < NT; ++nn) {
         const double pw = __shfl_up_sync(0xffffffffu, px[nn], 1);
-        const double rw = __shfl_up_sync(0xffffffffu, sgn_pos(u) ? 0.0 : rx[nn], 1);
+        const double rw = __shfl_up_sync(0xffffffffu, sgn_pos(u) ? zero_of(rx[nn]) : rx[nn], 1);
         if (nn >= nt) continue;
         const int n = n0 + nn;
         const double gd = g(n, k + 1);
@@ -255,9 +260,10 @@ __global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj 
         zface(n, k + 1, gc[nn], gd, pb, rb);
         if (own) {
           const double tnv = px[nn] + pw + py[nn] + sp[nn][row - 1][lane] + pz[nn] + pb;
-          double tbv = (sgn_pos(u) ? rx[nn] : 0.0) + rw + (sgn_pos(v) ? ry[nn] : 0.0) + sr[nn][row - 1][lane];
-          tbv += sgn_pos(wt) ? rz[nn] : 0.0;
-          tbv += sgn_pos(wb) ? 0.0 : rb;
+          double tbv = (sgn_pos(u) ? rx[nn] : zero_of(rx[nn])) + rw + (sgn_pos(v) ? ry[nn] : zero_of(ry[nn])) +
+                       sr[nn][row - 1][lane];
+          tbv += sgn_pos(wt) ? rz[nn] : zero_of(rz[nn]);
+          tbv += sgn_pos(wb) ? zero_of(rb) : rb;
           if (k == 1 && a.linssh) tbv += wn[q] * -msel(gc[nn], tm);  // surface flux w tb (:146-156)
           const long o = ((long)m * a.kjpt + n) * n3 + q;
           a.tb_ad[o] += tbv;
@@ -563,7 +569,7 @@ __global__ void __launch_bounds__(128) k_iso_adj_tb(Dom<double> d, LdfArgs<doubl
 // back-substitution run forwards, then the elimination with its right-hand side
 // e3t_b tb + p2dt e3t_n ta run backwards. The matrix is built as k_zdf_imp builds
 // it in double precision: one division a level, 1 / zwt, and every quotient corrected
-// from a reciprocal (divq); zwi(k+1) is zws(k).
+// from a reciprocal (divr); zwi(k+1) is zws(k).
 __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
   ColIdx<double> c = col_index(d);
   if (!c.valid || !c.interior) return;
@@ -588,8 +594,8 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
         const double zs = over_e3w(d, -a.p2dt * wt(k + 1), c.ij, k + 1, c.m);
         double t = d.e3t_a(c.ij, k, c.m) - zwi - zs;
         if (k >= 2) {
-          rat[k] = divq(zwi, tp, rp);
-          t = t - divq(zwi * zwi, tp, rp);  // zws(k-1) = zwi(k)
+          rat[k] = divr(zwi, tp, rp);
+          t = t - divr(zwi * zwi, tp, rp);  // zws(k-1) = zwi(k)
         }
         zws[k] = zs;
         zwt[k] = tp = t;
@@ -604,13 +610,13 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
     double carry = 0.0;  // what level k receives from level k-1
     for (int k = 1; k <= jpk - 2; ++k) {
       const long q = c.ij + (long)(k - 1) * n2;
-      const double x = divq(msel(lam[q] + carry, tmsk<double>(ci, k)), zwt[k], rz[k]);
+      const double x = divr(msel(lam[q] + carry, tmsk<double>(ci, k)), zwt[k], rz[k]);
       carry = -zws[k] * x;
       lam[q] = x;
     }
     {
       const long q = c.ij + (long)(jpk - 2) * n2;
-      lam[q] = divq(msel(lam[q] + carry, tmsk<double>(ci, jpk - 1)), zwt[jpk - 1], rz[jpk - 1]);
+      lam[q] = divr(msel(lam[q] + carry, tmsk<double>(ci, jpk - 1)), zwt[jpk - 1], rz[jpk - 1]);
     }
     // elimination (:238-250) run backwards
     double up = 0.0;  // what level k receives from level k+1

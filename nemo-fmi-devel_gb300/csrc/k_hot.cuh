@@ -37,14 +37,6 @@ __device__ __forceinline__ T u_in(const ColInfo& c, int k) { return (k >= c.ulo 
 template <class T>
 __device__ __forceinline__ T v_in(const ColInfo& c, int k) { return (k >= c.vlo && k <= c.vhi) ? T(1) : T(0); }
 
-// x / y given ry = 1 / y correctly rounded: FP64 for finite x / y (its test for others
-// would run on the FP64 pipe)
-template <class T>
-__device__ __forceinline__ T div_by(T x, T y, T ry) {
-  if constexpr (sizeof(T) == 8) return divq(x, y, ry);
-  else return divr(x, y, ry);
-}
-
 // Iso-neutral fluxes (traldf_iso.F90:146-357) of one column chunk; see k_iso_flux.
 // It also sets akz = ah_wslp2 on the points k_iso_akz_copy_edges covers in general. G3: 3-D
 // scale factors or partial steps, whose bottom gradients are loaded once a column. The
@@ -363,8 +355,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 10) : 3) k_fc
         const T zwz_t = (k == 1) ? (a.linssh ? wt * tb0 : T(0)) : zwzb[nn];
         const T zwz_b = (k + 1 <= jpk - 1) ? msel(ups(wb, __ldg(tb + q + n2), tb0), wk1) : T(0);
         const T ztra = -(zwx_e - zwx_w + zwy_n - zwy_s + zwz_t - zwz_b) * r1_e1e2t;
-        ta[o + q] = (tai ? tai[o + q] : T(0)) + msel(div_by(ztra, e3, r1_e3), tm);
-        zwi[o + q] = msel(div_by(e3 * tb0 + p2dt * ztra, e3, r1_e3), tm);
+        ta[o + q] = (tai ? tai[o + q] : T(0)) + msel(divr(ztra, e3, r1_e3), tm);
+        zwi[o + q] = msel(divr(e3 * tb0 + p2dt * ztra, e3, r1_e3), tm);
         // 2nd-order antidiffusive fluxes (:180-190, :255-263)
         ax[o + q] = T(0.5) * ue * (tn0 + tne) - zwx_e;
         ay[o + q] = T(0.5) * vn_ * (tn0 + tnn) - zwy_n;

@@ -293,12 +293,14 @@ __device__ __forceinline__ T divq(T x, T y, T ry) {
 
 // x / y given ry = 1 / y correctly rounded: divq's correction, in both precisions and
 // without a branch (three multiply-adds instead of the division's dozen instructions);
-// a quotient that is not finite is that of x ry. Exact for |x| > 2^-100 (2^-960).
+// a quotient that is not finite is that of x ry (FP64 tests it on the integer pipe), where
+// divq's correction would turn an infinite one into NaN. Exact for |x| > 2^-100 (2^-960).
 template <class T>
 __device__ __forceinline__ T divr(T x, T y, T ry) {
   if constexpr (sizeof(T) == 8) {
     const T q = __dmul_rn(x, ry);
-    return isfinite(q) ? __fma_rn(__fma_rn(-q, y, x), ry, q) : q;
+    const bool finite = (__double2hiint(q) & 0x7ff00000) != 0x7ff00000;
+    return finite ? __fma_rn(__fma_rn(-q, y, x), ry, q) : q;
   } else {
     const T q = __fmul_rn(x, ry);
     return isfinite(q) ? __fmaf_rn(__fmaf_rn(-q, y, x), ry, q) : q;
@@ -308,7 +310,7 @@ __device__ __forceinline__ T divr(T x, T y, T ry) {
 template <class T>
 __device__ __forceinline__ T over_e3t_n(const Dom<T>& d, T x, T e3n, int k) {
   if constexpr (sizeof(T) == 8) {
-    if (d.r1_e3t && d.e3t_n.s == 0) return divq(x, e3n, d.r1_e3t[k - 1]);
+    if (d.r1_e3t && d.e3t_n.s == 0) return divr(x, e3n, d.r1_e3t[k - 1]);
   }
   return x / e3n;
 }
@@ -650,7 +652,7 @@ __global__ void __launch_bounds__(32 * I4_Y) k_interp4(Dom<T> d, RO<T> ptn, T* _
     T x = out[k * nt];
     if (k >= ks && k <= ke) {
       if (k < K) x = x - nxt;
-      x = divq(x, piv[k - ks], rp[k - ks]);
+      x = sizeof(T) == 8 ? divr(x, piv[k - ks], rp[k - ks]) : x / piv[k - ks];
     }
     nxt = x;
     w[(long)(k - 1) * n2] = x;

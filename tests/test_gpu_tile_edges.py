@@ -213,3 +213,57 @@ def test_ragged_rows(nn, jpk):
     p.ctx.set_tma_poll_limit(1 << 16)
     p.ctx.stp_hotpath(8)
     p.ctx.synchronize()
+
+
+def kinds(x):
+    """where x is +inf, -inf and NaN"""
+    return np.stack([np.isposinf(x), np.isneginf(x), np.isnan(x)])
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_fct_of_a_value_that_is_not_finite(value):
+    """tra_adv_fct with given transports in FP64 on a tracer with one infinite or undefined value:
+    what the specialised kernels leave infinite and undefined is what the general ones (a
+    bound tape asks for them) do."""
+    p = Pair(nn=2, prec="fp64", seed=5)
+    st, o, c = p.states[0], p.ora[0], p.ctx
+    tb = np.array(st["tsb"], order="F")
+    tb[20, 15, 6, 0] = value
+    zun, zvn, zwn = o.tra_adv_trp(*[np.array(st[n], order="F") for n in ("un", "vn", "wn")])
+    out = []
+    for general in (0, 1):
+        d = [p.to_dev([x]) for x in (zun, zvn, zwn, tb, st["tsn"], np.zeros(p.s4, order="F"))]
+        c.bind("FCT_TAPE", p.to_dev([np.zeros(6 * tb.size // 2)]) if general else None)
+        c.tra_adv_fct(5, 1, "TRA", 14400.0, *d, 2, 2, 2)
+        out.append(kinds(c.to_host(d[5], p.s4)))
+    assert out[1].any() and np.array_equal(*out)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_tracer_adjoints_of_a_value_that_is_not_finite(value):
+    """The tracer adjoints of a sensitivity with one infinite or undefined value are infinite
+    and undefined where the oracle's are."""
+    c = Case("gyre", seed=22)
+    g = GpuCase(c)
+    c.iso_coefficients()
+    g.iso_coefficients()
+    kt = c.kit + 2
+    lam = c.rand4(masked=False)
+    lam[15, 10, 6, 0] = value
+    zero = np.zeros(c.s4, order="F")
+    rb, ra, tb, ta = zero.copy(order="F"), lam.copy(order="F"), g.dev(zero), g.dev(lam)
+    c.o.tra_zdf_imp_adj(kt, c.kit, "TRA", c.p2dt, rb, ra, 2)
+    g.ctx.tra_zdf_imp_adj(kt, c.kit, "TRA", c.p2dt, tb, ta, 2)
+    pairs = [(rb, tb), (ra, ta)]
+    ri, ti = zero.copy(order="F"), g.dev(zero)
+    c.o.tra_ldf_iso_adj(kt, c.kit, "TRA", None, None, c.gtsu, c.gtsv, None, None, ri, None, lam, 2, 1)
+    g.ctx.tra_ldf_iso_adj(kt, c.kit, "TRA", None, None, g.gtsu, g.gtsv, None, None, ti, None, g.dev(lam), 2, 1)
+    pairs.append((ri, ti))
+    tape, _ = c.fct_record()
+    g.ctx.bind("FCT_TAPE", g.dev(tape))
+    fb, fn = g.dev(zero), g.dev(zero)
+    g.ctx.tra_adv_fct_adj(kt, c.kit, "TRA", c.p2dt, g.zun, g.zvn, g.zwn, fb, fn, g.dev(lam), 2, 2, 2)
+    pairs += zip(c.fct_adj(tape, lam), (fb, fn))
+    for ref, got in pairs:
+        ref = kinds(ref)
+        assert ref.any() and np.array_equal(ref, kinds(g.host(got, c.s4)[0]))
