@@ -836,6 +836,12 @@ int nemo_gpu_set_fct_fused(nemo_ctx *ctx, int on);
  * compare them). No counterpart in the reference. */
 int nemo_gpu_set_spg_specialised(nemo_ctx *ctx, int on);
 
+/* With the specialised sub-step kernels on, the one that keeps a member on a
+ * thread-block cluster: mode 0 never, 1 (default) where it is expected to be the
+ * faster, 2 wherever a member fits a cluster. Same results, to the bit. No counterpart
+ * in the reference. */
+int nemo_gpu_set_spg_cluster(nemo_ctx *ctx, int mode);
+
 /* ------------------------------------------------------------ test hook */
 
 /* Bound of the grid barriers of the persistent sub-step kernel: each wait gives up

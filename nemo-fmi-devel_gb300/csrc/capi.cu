@@ -130,6 +130,7 @@ struct nemo_ctx {
   int res_c = 0, res_rows = 0, res_v = 0, res_gen = 0;  // k_spg_p2_res: blocks a member (0: not used), rows, variant
   int p2_hot = 0;    // the sub-step kernel is k_spg_p2_ene (mixed, linear free surface, ENE/MIX)
   bool no_p2_hot = false;  // keep the general sub-step kernel (tests compare both)
+  int cluster = 1;         // k_spg_p2_res: 0 never, 1 by select_p2's rule, 2 wherever it fits
   double* gs_part = nullptr;
   double* gs_out = nullptr;
   double* gs_host = nullptr;      // the result again, in mapped host memory
@@ -1856,7 +1857,7 @@ void select_p2(nemo_ctx* c) {
   // on 11), with the fewest points a thread.
   c->res_c = 0;
   c->res_gen = !c->p2_hot;
-  if (ene && !c->no_p2_hot && (c->p2_hot || !c->p2_cache)) {
+  if (c->cluster && ene && !c->no_p2_hot && (c->p2_hot || !c->p2_cache)) {
     double best = 0.0;
     for (int v = 0; v < P2R_NV; ++v)
       for (int cs = 1; cs <= P2R_MAXC; ++cs) {
@@ -3217,6 +3218,15 @@ int nemo_gpu_set_spg_specialised(nemo_ctx* c, int on) {
   for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
   c->graphs.clear();
   return c->p2_blocks < 1 ? fail(c, NEMO_ERR_CUDA, "set_spg_specialised: no launch shape") : NEMO_OK;
+}
+
+int nemo_gpu_set_spg_cluster(nemo_ctx* c, int mode) {
+  if (!c || mode < 0 || mode > 2) return fail(c, NEMO_ERR_ARG, "set_spg_cluster: bad argument");
+  c->cluster = mode;
+  select_p2(c);
+  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
+  c->graphs.clear();
+  return NEMO_OK;
 }
 
 int nemo_gpu_set_tma_poll_limit(nemo_ctx* c, int max_polls) {

@@ -204,6 +204,7 @@ def load(path):
     _proto(lib, "nemo_gpu_dia_hsb", i, [vp, i])
     _proto(lib, "nemo_gpu_dia_hsb_result", i, [vp, vp])
     _proto(lib, "nemo_gpu_set_spg_specialised", i, [vp, i])
+    _proto(lib, "nemo_gpu_set_spg_cluster", i, [vp, i])
     _proto(lib, "nemo_gpu_set_fct_fused", i, [vp, i])
     _proto(lib, "nemo_gpu_get_timing", i, [vp, C.POINTER(d), C.POINTER(i)])
     _proto(lib, "nemo_gpu_get_kernel_timing", i, [vp, C.POINTER(d), C.POINTER(i), i])

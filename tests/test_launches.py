@@ -30,3 +30,28 @@ print(json.dumps(seen))
     assert first == second
     for k in ("k_fct_b_tma", "k_fct_fused_tma", "k_interp4IdE", "k_zdf_imp_async", "k_zdf_imp32"):
         assert any(k in name for name in second), k
+
+
+def test_sub_step_kernels():
+    """The sub-step kernel of a call by the cluster setting: 0 the grid-barrier kernel (with
+    the constants combined, or with many members in the general form without its cache), 2
+    the cluster kernel with one, two and four points a thread, or in its general form."""
+    out = fakedev.run(r"""
+seen = []
+for nn, nmem in ((1, 2), (4, 1), (5, 3), (7, 1), (3, 80)):
+    for mode in (0, 2):
+        c = Ctx(gyre.domain(nn, jpk=4), gyre.namelist(), "mixed", nmem)
+        c.bind("UA", "VA", "UB", "VB", "UN", "VN", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP",
+               "RCDU_BOT", "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")
+        c("set_spg_cluster", mode)
+        launches()
+        c("dyn_spg_ts", 10)
+        seen.append([k[0] for k in launches() if "spg_p2" in k[0]])
+        c.close()
+print(json.dumps(seen))
+""")
+    want = ["k_spg_p2_ene", "k_spg_p2_resILi512ELi1ELb0E", "k_spg_p2_ene", "k_spg_p2_resILi512ELi2ELb0E", "k_spg_p2_ene",
+            "k_spg_p2_resILi512ELi4ELb0E", "k_spg_p2_ene", "k_spg_p2_resILi512ELi4ELb0E", "k_spg_p2IfLb0ELi4E",
+            "ELb1EEEvNS_3DomIfEENS_7SpgArgsIfEEii"]
+    assert [len(x) for x in out] == [1] * len(want)
+    assert all(w in x[0] for w, x in zip(want, out)), out
