@@ -1855,6 +1855,13 @@ void select_p2(nemo_ctx* c) {
   // (two barriers, as long as the arithmetic of some 700 points and 60 more for each block
   // that joins them, and the block's points: 62x42 takes 107 us on 3 blocks, 72 on 6 and 82
   // on 11), with the fewest points a thread.
+  // Against the grid-barrier kernel: with one or two points a thread the cluster is the
+  // faster at any number of sub-steps (1.15 times and more of 8 to 89 at 700 to 15 000
+  // points, 1 to 64 members). With four points a thread a sub-step is only 0.55 us shorter
+  // for each block an SM of the grid-barrier kernel, and the start (constants, levels and
+  // sums of 2048 points a block) 5 to 20 us longer, so it takes enough sub-steps or blocks to
+  // gain: 212x142 alone 60 -> 76 us with 8 sub-steps, 194 -> 188 with 44; three members of
+  // 182x122 67 -> 71, and 410 -> 329 with 89.
   c->res_c = 0;
   c->res_gen = !c->p2_hot;
   if (c->cluster && ene && !c->no_p2_hot && (c->p2_hot || !c->p2_cache)) {
@@ -1871,6 +1878,10 @@ void select_p2(nemo_ctx* c) {
           c->res_c = cs; c->res_rows = rows; c->res_v = v;
         }
       }
+    const int per_sm = (c->p2_blocks + c->nsm - 1) / c->nsm;
+    if (c->cluster == 1 && c->res_c && c->res_v == P2R_NV - 1 && c->p2_hot && per_sm <= 3 &&
+        0.55 * per_sm * c->icycle < 5.0 + 0.0075 * c->res_rows * c->jpi)
+      c->res_c = 0;
   }
 }
 

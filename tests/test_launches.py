@@ -55,3 +55,22 @@ print(json.dumps(seen))
             "ELb1EEEvNS_3DomIfEENS_7SpgArgsIfEEii"]
     assert [len(x) for x in out] == [1] * len(want)
     assert all(w in x[0] for w, x in zip(want, out)), out
+
+
+def test_rule_of_the_cluster_kernel():
+    """With four points a thread the cluster kernel only takes calls whose sub-steps are
+    enough to pay its start; with fewer points a thread it takes all."""
+    out = fakedev.run(r"""
+seen = []
+for jpi, jpj, nmem, nb in ((212, 142, 1, 6), (212, 142, 1, 60), (182, 122, 3, 6), (182, 122, 3, 60), (152, 102, 12, 6), (62, 42, 1, 6)):
+    dom = gyre.domain((jpi - 2) // 30, jpk=4)
+    c = Ctx(dom, gyre.namelist(ln_bt_auto=0, nn_baro=nb), "mixed", nmem)
+    c.bind("UA", "VA", "UB", "VB", "UN", "VN", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP",
+           "RCDU_BOT", "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")
+    launches()
+    c("dyn_spg_ts", 10)
+    seen.append(["spg_p2_res" in k[0] for k in launches() if "spg_p2" in k[0]])
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [[False], [True], [False], [True], [True], [True]]
