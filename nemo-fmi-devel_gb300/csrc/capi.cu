@@ -1820,14 +1820,17 @@ void select_p2(nemo_ctx* c) {
         prec == NEMO_PREC_FP64 ? spg_p2_blocks_per_sm<double>(0, vvl, 0) : spg_p2_blocks_per_sm<float>(cache, vvl, 0);
     long maxb = (long)bps * c->nsm;
     // The block with the most tiles sets the pace: five blocks an SM (48 registers, a few
-    // more spills) where it then owns one tile instead of two or two instead of three
-    // (variable volume, 421x363: 644 tiles, 776 -> 670 us a call; 640x520: 1193 -> 1124).
-    // With more rounds the spills cost more than the shorter tail saves (4800 tiles, 7
-    // rounds instead of 8: 3861 -> 3897 us).
+    // more spills) where every block then owns one tile and not two (variable volume,
+    // 421x363, 644 tiles: the kernel 657 -> 560 us). The second round of four blocks an SM
+    // has its full price from some 13 tiles on (of 608 blocks), tiles of the last row with
+    // few points left out: 288x552, 13 more, 674 -> 536 us a call; 465x328, 7 more, 555 and
+    // 556; 672x228, one more, 470 -> 517. Two rounds for three are not worth it (669x465
+    // 837 -> 1028 us, 585x519 974 -> 1015, 800x448 1020 -> 1012).
     c->p2_five = 0;
-    if (prec != NEMO_PREC_FP64 && vvl && maxb > 0 && need <= 3 * maxb) {
+    if (prec != NEMO_PREC_FP64 && vvl && maxb > 0 && need > maxb) {
       const long max5 = (long)spg_p2_blocks_per_sm<float>(0, vvl, 1) * c->nsm;
-      if (max5 > maxb && (need + max5 - 1) / max5 < (need + maxb - 1) / maxb) {
+      const long more = need - maxb - ((c->jpj - 1) % 8 < 4 ? (c->jpi + 31) / 32 : 0);
+      if (need <= max5 && 50 * more >= maxb) {
         c->p2_five = 1;
         maxb = max5;
       }

@@ -74,3 +74,25 @@ for jpi, jpj, nmem, nb in ((212, 142, 1, 6), (212, 142, 1, 60), (182, 122, 3, 6)
 print(json.dumps(seen))
 """)
     assert out == [[False], [True], [False], [True], [True], [True]]
+
+
+def test_rule_of_five_blocks_an_sm():
+    """The variable-volume sub-steps take the instance for five blocks an SM where one round
+    of tiles then takes the place of two, and the second of four blocks an SM is not nearly
+    empty; elsewhere four."""
+    out = fakedev.run(r"""
+seen = []
+for jpi, jpj in ((421, 363), (288, 552), (449, 328), (672, 228), (321, 449), (577, 316), (669, 465), (366, 508)):
+    dom = shelf.domain(jpi, jpj, jpk=4, seed=3)
+    c = Ctx(dom, shelf.namelist(), "mixed")
+    c.bind("UA", "VA", "UB", "VB", "UN", "VN", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP",
+           "RCDU_BOT", "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF", "SSH_IB", "SSH_IBB",
+           "E3T_B", "E3T_N", "E3T_A", "E3U_N", "E3V_N", "E3W_N", "E3F_N", "HT_N", "HU_N", "HV_N", "R1_HU_N", "R1_HV_N",
+           "HU_B", "HV_B", "R1_HU_B", "R1_HV_B")
+    launches()
+    c("dyn_spg_ts", 10)
+    seen.append(["Li5E" in k[0] for k in launches() if "spg_p2" in k[0]])
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [[True], [True], [False], [False], [False], [True], [False], [False]]
