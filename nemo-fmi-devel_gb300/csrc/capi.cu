@@ -1481,7 +1481,7 @@ int run_zdf_phy(nemo_ctx* c) {
   a.rpi = (T)3.141592653589793;
   a.nn_pdl = nm.nn_pdl; a.nn_mxl = nm.nn_mxl; a.ln_mxl0 = nm.ln_mxl0; a.ln_lc = nm.ln_lc;
   a.ln_zdfevd = nm.ln_zdfevd; a.nn_evdm = nm.nn_evdm;
-  cudaError_t e = launch_zdf_phy<T>(dom_now<T>(c), a, c->stream);
+  cudaError_t e = launch_zdf_phy<T>(dom_now<T>(c), a, c->nsm, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "zdf_phy launch");
   return NEMO_OK;
 }

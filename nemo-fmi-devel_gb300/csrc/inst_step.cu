@@ -189,14 +189,47 @@ cudaError_t launch_usr_put(double* dst, const double* v, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// k_zdf_tke with SH values a level in shared memory, and the rounds of resident blocks that
+// the grid takes (0: it cannot run)
 template <class T>
-cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s) {
-  const int kch = march_chunk(d), level = (sizeof(T) == 4 ? 3 : 4) * 32 * TKE_Y<T> * (int)sizeof(T), smem = level * d.jpk;
-  const auto tke = d.e3w_n.s == 0 && d.e3t_n.s == 0 ? k_zdf_tke<T, true> : k_zdf_tke<T, false>;
-  if (cudaError_t e = smem_opt_in(tke, level * KMAX)) return e;
+struct TkeLaunch {
+  void (*kern)(Dom<T>, ZphyArgs<T>);
+  int smem, rounds;
+};
+template <class T, int SH>
+static TkeLaunch<T> tke_launch(const Dom<T>& d, dim3 g, int nsm) {
+  TkeLaunch<T> t{d.e3w_n.s == 0 && d.e3t_n.s == 0 ? k_zdf_tke<T, true, SH> : k_zdf_tke<T, false, SH>, 0, 0};
+  const int level = SH * 32 * TKE_Y<T> * (int)sizeof(T);
+  t.smem = level * d.jpk;
+  int n = 0;
+  if (smem_opt_in(t.kern, level * KMAX) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, t.kern, 32 * TKE_Y<T>, t.smem) != cudaSuccess || n < 1)
+    return t;
+  const long blocks = (long)g.x * g.y * g.z, wave = (long)n * nsm;
+  t.rounds = (int)((blocks + wave - 1) / wave);
+  return t;
+}
+template <class T>
+cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, int nsm, cudaStream_t s) {
+  const int kch = march_chunk(d);
+  const dim3 g((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y<T> - 1) / TKE_Y<T>, d.nmem);
+  TkeLaunch<T> t;
+  if constexpr (sizeof(T) == 4) {
+    t = tke_launch<T, 3>(d, g, nsm);
+  } else {
+    // FP64: a column's four values a level leave three blocks of two warps an SM at 31 levels
+    // and one at 62. Of the forms with four, two and no values in shared memory (the rest in
+    // work arrays) the one with the fewest rounds of blocks, then the most values: us a call
+    // of zdf_phy 121x83x31 208, 216, 219; 200x151x31 512, 381, 383; 302x202x31 807, 968, 666;
+    // 333x251x31 1039, 1051, 1303; 250x200x62 2499, 1237, 1163.
+    t = tke_launch<T, 4>(d, g, nsm);
+    for (const TkeLaunch<T>& x : {tke_launch<T, 2>(d, g, nsm), tke_launch<T, 0>(d, g, nsm)})
+      if (x.rounds && (!t.rounds || x.rounds < t.rounds)) t = x;
+  }
+  if (!t.rounds) return cudaErrorLaunchOutOfResources;
   (d.e3w_n.s == 0 ? k_zdf_sh2<T, true> : k_zdf_sh2<T, false>)<<<march_grid(d, kch), dim3(SX, MARCH_Y), 0, s>>>(d, a, kch);
   ktick(NEMO_K_ZDF_PHY, s);
-  tke<<<dim3((d.jpi + SX - 1) / SX, (d.jpj + TKE_Y<T> - 1) / TKE_Y<T>, d.nmem), dim3(SX, TKE_Y<T>), smem, s>>>(d, a);
+  t.kern<<<g, dim3(SX, TKE_Y<T>), t.smem, s>>>(d, a);
   ktick(NEMO_K_ZDF_PHY, s);
   return cudaGetLastError();
 }
@@ -293,7 +326,7 @@ cudaError_t launch_dia_hsb(const Dom<T>& d, const HsbArgs<T>& a, double* part, i
   template cudaError_t launch_dyn_zdf_imp<T>(const Dom<T>&, const DynZdfArgs<T>&, cudaStream_t);           \
   template cudaError_t launch_usr_sbc_a<T>(const Dom<T>&, const UsrSbcArgs<T>&, cudaStream_t);              \
   template cudaError_t launch_usr_sbc_b<T>(const Dom<T>&, const UsrSbcArgs<T>&, cudaStream_t);              \
-  template cudaError_t launch_zdf_phy<T>(const Dom<T>&, const ZphyArgs<T>&, cudaStream_t);                 \
+  template cudaError_t launch_zdf_phy<T>(const Dom<T>&, const ZphyArgs<T>&, int, cudaStream_t);                 \
   template cudaError_t launch_dyn_ldf_lap<T>(const Dom<T>&, const T*, const T*, const T*, const T*, T*, T*, T,   \
                                              cudaStream_t);                                             \
   template cudaError_t launch_vor_ene<T>(const Dom<T>&, int, const T*, const T*, T*, T*, cudaStream_t);       \

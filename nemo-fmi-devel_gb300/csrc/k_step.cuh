@@ -1608,11 +1608,13 @@ __global__ void __launch_bounds__(32 * MARCH_Y) k_zdf_sh2(Dom<T> d, ZphyArgs<T> 
 // the loads in flight: three values a level (in FP32 the upper diagonal and the forward
 // value over the pivot; en is read back) let 16 warps an SM run, 117 us; four values (the
 // pivot, and en kept) 12 warps, 150 us. Blocks of 4 rows, not 2 (122) or 8 (156).
+// SH: the values a level kept in shared memory, the others in work arrays (FP32 three; FP64,
+// with the pivot, four, two or none: launch_zdf_phy).
 // With 1-D scale factors (FLAT) the quotients by e3t e3w, and always those by the pivot,
 // are divr's; where EVD acts is kept as a bit a level.
 template <class T>
 constexpr int TKE_Y = sizeof(T) == 4 ? 4 : 2;
-template <class T, bool FLAT>
+template <class T, bool FLAT, int SH>
 __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T> a) {
   extern __shared__ __align__(16) unsigned char col_smem[];
   __shared__ T pu[KMAX + 1], ru[KMAX + 1], pl[KMAX + 1], rl[KMAX + 1];  // e3t(k) e3w(k), e3t(k-1) e3w(k), reciprocals
@@ -1632,11 +1634,28 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
     __syncthreads();
   }
   if (i > d.jpi || j > d.jpj) return;
-  T* const su = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x - nt;  // [k * nt], k = 1..jpk
-  T *const sl = su + jpk * nt, *const sp = sl + jpk * nt, *const sd = sp + jpk * nt;  // sd: FP64
   const long n2 = d.n2;
   const long ij = (long)(i - 1) + (long)(j - 1) * d.jpi;
   const long c3 = (long)m * d.n3 + ij, c2 = (long)m * d.n2 + ij;
+  // the column's values, k = 1..jpk: su, sl at [k * n1], sp and (FP64) sd at [k * n1d]
+  T *su = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x - nt, *sl = su + jpk * nt;
+  T *sp = sl + jpk * nt, *sd = sp + jpk * nt;
+  if constexpr (SH < 3) {
+    sp = a.apdlr + c3 - n2;
+    sd = a.zdiag + c3 - n2;
+  }
+  if constexpr (SH < 2) {
+    su = a.zd_up + c3 - n2;
+    sl = a.zd_lw + c3 - n2;
+  }
+  const auto n1 = [&] {
+    if constexpr (SH >= 2) return nt;
+    else return n2;
+  }();
+  const auto n1d = [&] {
+    if constexpr (SH >= 3) return nt;
+    else return n2;
+  }();
   if (i == 1 || i == d.jpi || j == 1 || j == d.jpj) {
     for (int k = 1; k <= jpk; ++k) {
       const long q = c3 + (long)(k - 1) * n2;
@@ -1693,7 +1712,7 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
         const T avm_kp1 = l[1], sh2 = l[2], dissl = l[3];
         if (a.nn_pdl == 1) {
           const T zri = fmx(l[5], T(0)) * avm_k / (sh2 + a.rn_bshear);
-          sp[k * nt] = fmx(T(0.1), a.ri_cri / fmx(a.ri_cri, zri));
+          sp[k * n1d] = fmx(T(0.1), a.ri_cri / fmx(a.ri_cri, zri));
         }
         const T zcof = a.zfact1 * tm;
         if (a.ln_zdfevd && fmn(l[4], l[5]) <= T(-1.e-12)) evd_at |= 1ULL << (k - 1);
@@ -1723,10 +1742,10 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
           up_p = divr(up, dg, rd_p);
           lw_p = divr(lf, dg, rd_p);
         } else {
-          sd[k * nt] = dg;
+          sd[k * n1d] = dg;
           dg_p = dg; up_p = up; lw_p = lf;
         }
-        su[k * nt] = up_p; sl[k * nt] = lw_p;
+        su[k * n1] = up_p; sl[k * n1] = lw_p;
         avm_km1 = avm_k;
         avm_k = avm_kp1;
       });
@@ -1736,12 +1755,12 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
       2, jpk - 1, [&](int x, T (&l)[1]) { l[0] = __ldg(a.rn2 + c3 + (long)(jpk - x) * n2); },
       [&](int x, T (&l)[1]) {
         const int k = jpk + 1 - x;
-        T en = (k == jpk - 1) ? sl[k * nt] : sl[k * nt] - su[k * nt] * en_p;
-        if constexpr (sizeof(T) == 8) en = en / sd[k * nt];
+        T en = (k == jpk - 1) ? sl[k * n1] : sl[k * n1] - su[k * n1] * en_p;
+        if constexpr (sizeof(T) == 8) en = en / sd[k * n1d];
         en_p = en;
         const T e = fmx(en, a.rn_emin) * wmsk<T>(ci, k);
         a.en[c3 + (long)(k - 1) * n2] = e;
-        sl[k * nt] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(l[0], a.rsmall)));
+        sl[k * n1] = fmx(a.rmxl_min, sqrt(T(2) * e / fmx(l[0], a.rsmall)));
       });
   const T mxl1 = a.ln_mxl0 ? fmx(a.rn_mxl0, a.zraug * taum * tm1) : a.rn_mxl0;
   // downward limits of nn_mxl = 2 (in place) and 3 (su, from the unlimited lengths)
@@ -1749,8 +1768,8 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
     T* const out = a.nn_mxl == 2 ? sl : su;
     T p = mxl1;
     for (int k = 2; k <= jpk - 1; ++k) {
-      p = fmn(p + d.e3t_n(ij, k - 1, m), sl[k * nt]);
-      out[k * nt] = p;
+      p = fmn(p + d.e3t_n(ij, k - 1, m), sl[k * n1]);
+      out[k * n1] = p;
     }
   }
   // upward sweep: the limited lengths, the coefficients, the ocean Kz
@@ -1760,7 +1779,7 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
     const int k = jpk + 1 - x;
     const long q = c3 + (long)(k - 1) * n2;
     const T wm = wmsk<T>(ci, k), tm = tmsk<T>(ci, k);
-    const T raw = sl[k * nt];
+    const T raw = sl[k * n1];
     T lm, ld;
     if (a.nn_mxl == 2) {
       lm = fmn(nxt + d.e3t_n(ij, k + 1, m), raw);
@@ -1769,7 +1788,7 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
     } else if (a.nn_mxl == 3) {
       const T dn = fmn(nxt + d.e3t_n(ij, k + 1, m), raw);
       nxt = dn;
-      const T lu = su[k * nt];
+      const T lu = su[k * n1];
       lm = fmn(lu, dn);
       ld = sqrt(lu * dn);
     } else if (a.nn_mxl == 1) {
@@ -1786,7 +1805,7 @@ __global__ void __launch_bounds__(32 * TKE_Y<T>) k_zdf_tke(Dom<T> d, ZphyArgs<T>
     const T avmk = fmx(zav, a.rn_avm0) * wm;
     T avtk = fmx(zav, a.rn_avt0) * wm;
     a.dissl[q] = zsqen / ld;
-    if (a.nn_pdl == 1) avtk = fmx(sp[k * nt] * avtk, a.rn_avt0) * tm;
+    if (a.nn_pdl == 1) avtk = fmx(sp[k * n1d] * avtk, a.rn_avt0) * tm;
     a.avm_k[q] = avmk;
     a.avt_k[q] = avtk;
     T avt = avtk, avm = avmk;

@@ -118,9 +118,9 @@ struct UsrSbcArgs {
 };
 
 // zdf_phy with the TKE closure and zdf_evd. Member strides n3 (3-D) and n2 (taum,
-// fr_i). Work arrays (n3 per member): sh2, apdlr (the inverse Prandtl number), and
-// the three diagonals of the TKE system, whose storage the mixing lengths zmxlm
-// (zdiag) and zmxld (zd_up) take over once the system is solved.
+// fr_i). Work arrays (n3 per member): sh2, and what the column kernel's form in use does
+// not keep in shared memory: apdlr (the inverse Prandtl number), the pivots zdiag, and the
+// upper diagonal zd_up and forward values zd_lw, whose storage the mixing lengths take over.
 template <class T>
 struct ZphyArgs {
   const T *ub, *vb, *un, *vn, *rn2, *rn2b, *taum, *gdepw, *fr_i;  // fr_i may be null
@@ -150,7 +150,7 @@ template <class T>
 cudaError_t launch_usr_sbc_b(const Dom<T>& d, const UsrSbcArgs<T>& a, cudaStream_t s);
 cudaError_t launch_usr_put(double* dst, const double* v, cudaStream_t s);
 template <class T>
-cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, cudaStream_t s);
+cudaError_t launch_zdf_phy(const Dom<T>& d, const ZphyArgs<T>& a, int nsm, cudaStream_t s);
 template <class T>
 cudaError_t launch_eos(const Dom<T>& d, const EosArgs<T>& a, cudaStream_t s);
 template <class T>

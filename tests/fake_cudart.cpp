@@ -5,6 +5,7 @@
 // runtime, and every accepted launch is logged with its kernel, grid, block and shared memory.
 #include <cuda_runtime_api.h>
 #include <cudaTypedefs.h>
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -89,11 +90,14 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrMultiProcessorCount ? 152 : 0;
   return cudaSuccess;
 }
-// blocks an SM by registers alone, as the kernels' launch bounds ask for; clusters by SMs
-cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int, size_t, unsigned) {
+// blocks an SM by the sub-step kernels' launch bounds, else by 128 registers a thread and the
+// shared memory; clusters by SMs
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int threads, size_t smem,
+                                                                   unsigned) {
   const std::string& k = name[f];
-  *n = k.find("k_spg_p2_ene") != std::string::npos || k.find("Li5E") != std::string::npos ? 5
-       : k.find("IdL") != std::string::npos ? 2 : 4;
+  const auto has = [&](const char* s) { return k.find(s) != std::string::npos; };
+  if (has("k_spg_p2")) *n = has("k_spg_p2_ene") || has("Li5E") ? 5 : has("IdL") ? 2 : 4;
+  else *n = std::min(512 / threads, (int)(228 * 1024 / (smem + 4096)));
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* c) {

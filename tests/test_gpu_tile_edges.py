@@ -267,3 +267,19 @@ def test_tracer_adjoints_of_a_value_that_is_not_finite(value):
     for ref, got in pairs:
         ref = kinds(ref)
         assert ref.any() and np.array_equal(ref, kinds(g.host(got, c.s4)[0]))
+
+
+@pytest.mark.parametrize("nn_mxl", [0, 2, 3])
+@pytest.mark.parametrize("nmem", [1, 4, 12])
+def test_tke_columns_of_many_levels(nmem, nn_mxl):
+    """zdf_phy in FP64 with 62 levels and so many columns that four, two and none of a level's
+    values stay in shared memory. Tolerance of its own parity test."""
+    from test_zdf_tke import OUT, TOL_TKE, tke_pair
+    p = tke_pair("fp64", nmem=nmem, jpk=62, nn_mxl=nn_mxl, sample=sorted({0, nmem - 1}))
+    for kt in (1, 2):
+        for o in p.ora:
+            o.zdf_phy(kt)
+        p.ctx.zdf_phy(kt)
+    p.ctx.synchronize()
+    for n in OUT:
+        p.compare(n, p.s3, TOL_TKE["fp64"])

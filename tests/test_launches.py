@@ -96,3 +96,20 @@ for jpi, jpj in ((421, 363), (288, 552), (449, 328), (672, 228), (321, 449), (57
 print(json.dumps(seen))
 """)
     assert out == [[True], [True], [False], [False], [False], [True], [False], [False]]
+
+
+def test_forms_of_the_tke_columns():
+    """FP64 zdf_phy: four, two or none of a level's values in shared memory, by which needs
+    the fewest rounds of blocks."""
+    out = fakedev.run(r"""
+seen = []
+for nmem in (1, 4, 12):
+    c = Ctx(gyre.domain(2, jpk=62), gyre.namelist(ln_zdftke=1, ln_zdfevd=1), "fp64", nmem)
+    c.bind("UB", "VB", "UN", "VN", "AVM_K", "AVT_K", "AVM", "AVT", "EN", "DISSL", "RN2", "RN2B", "TAUM", "GDEPW_N")
+    launches()
+    c("zdf_phy", 3)
+    seen.append([k[0] for k in launches() if "zdf_tke" in k[0]])
+    c.close()
+print(json.dumps(seen))
+""")
+    assert ["Li4E" in out[0][0], "Li2E" in out[1][0], "Li0E" in out[2][0]] == [True] * 3, out
