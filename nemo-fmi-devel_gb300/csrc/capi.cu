@@ -88,7 +88,7 @@ struct nemo_ctx {
   void* slp_w = nullptr;       // ldf_slp work: 4 3-D and 6 2-D arrays per member
   void* rab_w = nullptr;       // the model step's before expansion ratios rab_b (jpi,jpj,jpk,2)
   void* rab_n = nullptr;       // and the now ones rab_n, with the vertical physics
-  void* zphy_w = nullptr;      // zdf_phy work: sh2, apdlr and the TKE system, 5 x n3 per member
+  void* zphy_w = nullptr;      // zdf_phy work, n3 per member: sh2; FP64: apdlr and the TKE system too
   double* fadj_w = nullptr;    // FCT adjoint with kn_fct_v = 4: 2 x n3 per member
   double* usr_s = nullptr;     // usrdef_sbc: the step's scalars (7), written before each step
   double usr_zsurf = 0.0;      // usrdef_sbc: GLOB_SUM(tmask(:,:,1))
@@ -1452,7 +1452,8 @@ template <class T>
 int run_zdf_phy(nemo_ctx* c) {
   const nemo_namelist& nm = c->nam;
   const size_t n = (size_t)c->n3 * c->nmem;
-  if (!c->zphy_w && cudaMalloc(&c->zphy_w, 5 * n * sizeof(T)) != cudaSuccess)
+  constexpr bool D = sizeof(T) == 8;  // FP64: the columns' systems too, where shared memory does not keep them
+  if (!c->zphy_w && cudaMalloc(&c->zphy_w, (D ? 5 : 1) * n * sizeof(T)) != cudaSuccess)
     return fail(c, NEMO_ERR_NOMEM, "zdf_phy work arrays");
   void* const* F = c->f;
   ZphyArgs<T> a{};
@@ -1463,7 +1464,10 @@ int run_zdf_phy(nemo_ctx* c) {
   a.avm_k = (T*)F[NEMO_F_AVM_K]; a.avt_k = (T*)F[NEMO_F_AVT_K]; a.avm = (T*)F[NEMO_F_AVM];
   a.avt = (T*)F[NEMO_F_AVT]; a.avs = (T*)F[NEMO_F_AVS]; a.en = (T*)F[NEMO_F_EN]; a.dissl = (T*)F[NEMO_F_DISSL];
   T* w = (T*)c->zphy_w;
-  a.sh2 = w; a.apdlr = w + n; a.zdiag = w + 2 * n; a.zd_up = w + 3 * n; a.zd_lw = w + 4 * n;
+  a.sh2 = w;
+  if constexpr (D) {
+    a.apdlr = w + n; a.zdiag = w + 2 * n; a.zd_up = w + 3 * n; a.zd_lw = w + 4 * n;
+  }
   // the constants of zdf_tke_init (zdftke.F90:663-690), tke_tke and tke_avn
   const double rdt = nm.rn_rdt, zrhoa = 1.22, zcdrag = 1.5e-3;
   const double rmxl_min = 1.e-6 / (nm.rn_ediff * std::sqrt(nm.rn_emin));

@@ -118,8 +118,8 @@ struct UsrSbcArgs {
 };
 
 // zdf_phy with the TKE closure and zdf_evd. Member strides n3 (3-D) and n2 (taum,
-// fr_i). Work arrays (n3 per member): sh2, and what the column kernel's form in use does
-// not keep in shared memory: apdlr (the inverse Prandtl number), the pivots zdiag, and the
+// fr_i). Work arrays (n3 per member): sh2, and in FP64 what the column kernel's form in use
+// does not keep in shared memory: apdlr (the inverse Prandtl number), the pivots zdiag, and the
 // upper diagonal zd_up and forward values zd_lw, whose storage the mixing lengths take over.
 template <class T>
 struct ZphyArgs {

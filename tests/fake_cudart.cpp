@@ -17,6 +17,7 @@ int device = 0;
 std::map<const void*, std::string> name;                    // host stub -> kernel
 std::map<std::pair<int, const void*>, size_t> opted;        // (device, stub) -> opt-in
 std::string launches;
+std::map<void*, size_t> held;  // device memory
 struct Config {
   dim3 grid, block;
   size_t smem;
@@ -44,6 +45,11 @@ void* handle() { return calloc(1, 8); }
 extern "C" {
 const char* fake_launches() { return launches.c_str(); }
 void fake_clear() { launches.clear(); }
+size_t fake_held() {
+  size_t n = 0;
+  for (const auto& m : held) n += m.second;
+  return n;
+}
 cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
 
@@ -111,8 +117,16 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
   return cudaSuccess;
 }
 
-cudaError_t cudaMalloc(void** p, size_t n) { *p = aligned_alloc(256, (n + 255) / 256 * 256); return cudaSuccess; }
-cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  *p = aligned_alloc(256, (n + 255) / 256 * 256);
+  held[*p] = n;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+  held.erase(p);
+  free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(1, n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }

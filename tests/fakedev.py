@@ -39,6 +39,7 @@ if "FAKE_CUDART" in os.environ:
 
     fake = C.CDLL(os.environ["FAKE_CUDART"])
     fake.fake_launches.restype = C.c_char_p
+    fake.fake_held.restype = C.c_size_t
     lib = _ffi.load(_b.library_path())
 
     def launches():

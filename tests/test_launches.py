@@ -113,3 +113,21 @@ for nmem in (1, 4, 12):
 print(json.dumps(seen))
 """)
     assert ["Li4E" in out[0][0], "Li2E" in out[1][0], "Li0E" in out[2][0]] == [True] * 3, out
+
+
+def test_work_memory_of_the_vertical_physics():
+    """zdf_phy in the mixed form keeps one work array, the shear production; the FP64 form
+    the system of the columns beside it."""
+    out = fakedev.run(r"""
+seen = []
+for prec, b in (("mixed", 4), ("fp64", 8)):
+    c = Ctx(gyre.domain(2), gyre.namelist(ln_zdftke=1, ln_zdfevd=1), prec, 3)
+    c.bind("UB", "VB", "UN", "VN", "AVM_K", "AVT_K", "AVM", "AVT", "EN", "DISSL", "RN2", "RN2B", "TAUM", "GDEPW_N")
+    before = fake.fake_held()
+    c("zdf_phy", 3)
+    c("zdf_phy", 4)
+    seen.append((fake.fake_held() - before) / (b * c.n3 * 3))
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [1.0, 5.0]
