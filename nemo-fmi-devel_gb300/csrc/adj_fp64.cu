@@ -21,8 +21,15 @@ dim3 acol_grid(const Dom<T>& d) {
 
 cudaError_t launch_fct_adj(const Dom<double>& d, const FctAdj& a, cudaStream_t s) {
   if (a.kh == 2) {
-    const dim3 g((d.jpi + 29) / 30, (d.jpj + FADJ_Y - 3) / (FADJ_Y - 2), d.nmem * ((d.jpk - 1 + FADJ_K - 1) / FADJ_K));
-    k_fct_adj2<<<g, dim3(32, FADJ_Y), 0, s>>>(d, a);
+    const dim3 t((d.jpi + 29) / 30, (d.jpj + FADJ_Y - 3) / (FADJ_Y - 2), d.nmem);
+    // levels a chunk: the fewest of 1, 2, 4, 8 whose blocks still start at once (one an SM and
+    // some). A level is 10 us of FP64 latency, whatever the grid: 33x23x31 20 us with 1, 92 with
+    // 8; 92x62x31 69, 59, 54, 97 with 1, 2, 4, 8; 302x202x31 539, 460, 414, 426.
+    auto chunks = [&](int k) { return (d.jpk - 1 + k - 1) / k; };
+    int kch = 1;
+    while (kch < FADJ_K && (long)t.x * t.y * t.z * chunks(kch) > 200) kch *= 2;
+    const dim3 g(t.x, t.y, t.z * chunks(kch));
+    k_fct_adj2<<<g, dim3(32, FADJ_Y), 0, s>>>(d, a, kch);
   } else {
     k_fct_adj<<<apt_grid(d), dim3(AX, AY), 0, s>>>(d, a);
   }

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
   }
 }
 
-// tra_adv_fct's adjoint with kn_fct_h = 2: a block marches down a chunk of levels over
+// tra_adv_fct's adjoint with kn_fct_h = 2: a block marches down a chunk of kch levels over
 // a tile of 32 x FADJ_Y points, one column a thread; each weight g and each face adjoint
 // is formed once a tile, by the point that owns it, and passed to its neighbour by a
 // shuffle (i) or through shared memory (j). The outer ring of the tile only feeds its
@@ -170,14 +170,14 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
 // k_fct_adj divides seven times a tracer and forms all six faces (1053 us at
 // 302x202x31, T and S), 420 so. Values as k_fct_adj's: an upstream flux's adjoint f reaches the
 // point upstream of its face as u f and the other as zero_of(u f) (0.5 (u + |u|) is u or 0).
-constexpr int FADJ_Y = 16, FADJ_K = 8;
-__global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj a) {
+constexpr int FADJ_Y = 16, FADJ_K = 8;  // the tile's rows, the most levels a chunk
+__global__ void __launch_bounds__(32 * FADJ_Y) k_fct_adj2(Dom<double> d, FctAdj a, int kch) {
   constexpr int NT = 2;
   __shared__ double sg[NT][FADJ_Y][32], sp[NT][FADJ_Y][32], sr[NT][FADJ_Y][32];
   const int lane = threadIdx.x, row = threadIdx.y, jpi = d.jpi, jpk = d.jpk;
   const int i = blockIdx.x * 30 + lane, j = blockIdx.y * (FADJ_Y - 2) + row;  // 1-based, 0: outside
-  const int nch = (jpk - 1 + FADJ_K - 1) / FADJ_K, m = blockIdx.z / nch;
-  const int k0 = (int)(blockIdx.z - m * nch) * FADJ_K + 1, k1 = min(k0 + FADJ_K - 1, jpk - 1);
+  const int nch = (jpk - 1 + kch - 1) / kch, m = blockIdx.z / nch;
+  const int k0 = (int)(blockIdx.z - m * nch) * kch + 1, k1 = min(k0 + kch - 1, jpk - 1);
   const Pt3 P = pt3(d);
   const bool in = i >= 1 && i <= jpi && j >= 1 && j <= d.jpj;
   const bool own = in && lane >= 1 && lane <= 30 && row >= 1 && row <= FADJ_Y - 2;

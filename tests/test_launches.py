@@ -131,3 +131,21 @@ for prec, b in (("mixed", 4), ("fp64", 8)):
 print(json.dumps(seen))
 """)
     assert out == [1.0, 5.0]
+
+
+def test_chunks_of_the_fct_adjoint():
+    """The FCT adjoint's levels a chunk: one on a tiny grid, so that a call waits for one level,
+    eight on a large one."""
+    out = fakedev.run(r"""
+seen = []
+for nn in (1, 3, 8):
+    c = Ctx(gyre.domain(nn), gyre.namelist(), "fp64")
+    c.bind("FCT_TAPE")
+    t = [c.array(2 * c.n3) for _ in range(6)]
+    launches()
+    c("tra_adv_fct_adj", 10, 1, b"TRA", 14400.0, *t, 2, 2, 2)
+    seen += [[k[1], k[2], k[3]] for k in launches() if "k_fct_adj2" in k[0]]
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [[2, 2, 30], [4, 5, 8], [9, 12, 4]]
