@@ -1044,12 +1044,16 @@ __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
 // fields, 28 and 35 us of 48 and 55) and by the FP64 pipe in FP64. As one point a thread, with
 // the coefficients loaded from global memory, the six calls of a step's density (two
 // rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32, 358 so.
-constexpr int EOS_BLOCK = 256;
+// Blocks of 2 (FP64) and 4 warps: with 8, a small grid was a few blocks whose points shared an
+// SM's FP64 pipe (rab_3d 20x17x10 16, 62x42x31 43 us, 9 and 32 so), and a large one had a
+// longer last round (93x61x31x12 669, 648).
+template <class T>
+constexpr int EOS_BLOCK = sizeof(T) == 4 ? 128 : 64;
 template <class T>
 constexpr int EOS_LEV = sizeof(T) == 4 ? 4 : 1;  // FP64: four levels in a row left a small grid's FP64 pipes idle
 template <class T, int WHAT, bool E80>
-__global__ void __launch_bounds__(EOS_BLOCK) k_eos(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
-  const long p = (long)blockIdx.x * EOS_BLOCK + threadIdx.x;
+__global__ void __launch_bounds__(EOS_BLOCK<T>) k_eos(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
+  const long p = (long)blockIdx.x * EOS_BLOCK<T> + threadIdx.x;
   if (p >= d.n2) return;
   const int m = blockIdx.z, k0 = blockIdx.y * kch + 1, k1 = min(k0 + kch - 1, d.jpk - 1);
   const long c3 = (long)m * d.n3 + p, c4 = 2 * (long)m * d.n3 + p;
@@ -1092,10 +1096,10 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_eos(Dom<T> d, const __grid_consta
 
 // bn2 (eosbn2.F90:889-933) on levels 2..jpk-1: a thread marches down a chunk of one
 // flat (i,j)'s levels and carries T, S, the expansion coefficients and the depth of
-// the level above, so that each of the 7 fields is read once.
-template <class T>
-__global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
-  const long p = (long)blockIdx.x * EOS_BLOCK + threadIdx.x;
+// the level above, so that each of the 7 fields is read once; U of them are loaded together.
+template <class T, int U>
+__global__ void __launch_bounds__(EOS_BLOCK<T>) k_bn2(Dom<T> d, const __grid_constant__ EosArgs<T> a, int kch) {
+  const long p = (long)blockIdx.x * EOS_BLOCK<T> + threadIdx.x;
   if (p >= d.n2) return;
   const int m = blockIdx.z, k0 = blockIdx.y * kch + 2, k1 = min(k0 + kch - 1, d.jpk - 1);
   if (k0 > k1) return;
@@ -1107,11 +1111,10 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_consta
   const T* __restrict__ gw = a.gdepw + c3;
   long o = (long)(k0 - 2) * d.n2;
   T tu = __ldg(ts + o), su = __ldg(ts + n3 + o), au = __ldg(ab + o), bu = __ldg(ab + n3 + o), hu = __ldg(gt + o);
-  constexpr int EOS_U = EOS_LEV<T>;
-  for (int k = k0; k <= k1; k += EOS_U) {
-    T t[EOS_U], s[EOS_U], x[EOS_U], y[EOS_U], h[EOS_U], w[EOS_U];
+  for (int k = k0; k <= k1; k += U) {
+    T t[U], s[U], x[U], y[U], h[U], w[U];
 #pragma unroll
-    for (int u = 0; u < EOS_U; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int ku = k + u <= k1 ? k + u : k1;
       o = (long)(ku - 1) * d.n2;
       t[u] = __ldg(ts + o);
@@ -1122,7 +1125,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) k_bn2(Dom<T> d, const __grid_consta
       w[u] = __ldg(gw + o);
     }
 #pragma unroll
-    for (int u = 0; u < EOS_U; ++u) {
+    for (int u = 0; u < U; ++u) {
       if (k + u > k1) break;
       const T zrw = (w[u] - h[u]) / (hu - h[u]);
       const T zaw = x[u] * (T(1) - zrw) + au * zrw;

@@ -283,3 +283,14 @@ def test_tke_columns_of_many_levels(nmem, nn_mxl):
     p.ctx.synchronize()
     for n in OUT:
         p.compare(n, p.s3, TOL_TKE["fp64"])
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("eos", ["seos", "eos80"])
+def test_densities_of_a_larger_grid(monkeypatch, prec, eos):
+    """The equations of state and bn2 with chunks of several levels a thread and a remainder of
+    levels, by their own parity test."""
+    import test_eos_hpg
+    real = gyre.domain
+    monkeypatch.setattr(gyre, "domain", lambda nn, **k: real(5, jpk=16))
+    test_eos_hpg.test_gpu_eos_bn2_hpg(prec, eos)
