@@ -269,8 +269,9 @@ __device__ __forceinline__ void cp_async_val(T* smem, const T* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sa), "l"(gmem), "n"((int)sizeof(T)) : "memory");
 }
-template <class T, class A>
-__global__ void __launch_bounds__(32 * DN_Y) k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a) {
+// BPS: the blocks an SM it is compiled for.
+template <class T, class A, int BPS>
+__global__ void __launch_bounds__(32 * DN_Y, BPS) k_dyn_nxt(Dom<T> d, NxtArgs<T, A> a) {
   extern __shared__ __align__(16) unsigned char col_smem[];
   constexpr int nt = 32 * DN_Y, B = BATCH<T>;  // levels loaded together
   T* s = reinterpret_cast<T*>(col_smem) + threadIdx.y * 32 + threadIdx.x;
