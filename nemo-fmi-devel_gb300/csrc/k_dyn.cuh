@@ -1596,7 +1596,10 @@ __device__ __forceinline__ double widen(float x) {
 // partial sum of the 2^12 values is exact in a double (24 bits each, 12 bits of carry), and
 // so plain additions give the exact sum of the pass; any other pass (and FP64) takes the
 // double-double path. 38 -> 15 us (one launch instead of two) at 2 x 93x61x62.
-constexpr int GS_PT = 16;
+// FP64 takes four points a thread: with sixteen, 176 dependent additions, a small sum waited
+// longer than in two launches before (33x23x31 34 -> 38 us, 26 so; 302x202x62 119, 131, 112).
+template <class T>
+constexpr int GS_PT = sizeof(T) == 4 ? 16 : 4;
 template <class T>
 __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const double* __restrict__ tmask_i, long n2,
                                                  int nk, double* __restrict__ part, unsigned* __restrict__ ticket,
@@ -1604,17 +1607,19 @@ __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const 
   __shared__ double sh[2][256];
   __shared__ int s_min[8], s_max[8];
   __shared__ bool s_last;
+  constexpr int PT = GS_PT<T>;
   const int m = blockIdx.y, t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const long n = n2 * nk, step = (long)gridDim.x * 256 * GS_PT;
+  const long n = n2 * nk, step = (long)gridDim.x * 256 * PT;
   const T* xm = x + (long)m * n;
   double hi = 0.0, lo = 0.0;  // thread 0 of the exact passes, every thread of the others
-  for (long e0 = (long)blockIdx.x * 256 * GS_PT; e0 < n; e0 += step) {
-    T v[GS_PT];
+  for (long e0 = (long)blockIdx.x * 256 * PT; e0 < n; e0 += step) {
+    T v[PT];
     long p = (e0 + t) % n2;  // point of the 2-D mask
 #pragma unroll
-    for (int i = 0; i < GS_PT; ++i) {
+    for (int i = 0; i < PT; ++i) {
       const long e = e0 + i * 256 + t;
-      v[i] = e < n ? xm[e] * (tmask_i[p] != 0.0 ? T(1) : T(0)) : T(0);  // tmask_i is 0 or 1
+      if constexpr (sizeof(T) == 8) v[i] = e < n ? xm[e] * tmask_i[p] : 0.0;
+      else v[i] = e < n ? xm[e] * (tmask_i[p] != 0.0 ? 1.0f : 0.0f) : 0.0f;  // tmask_i is 0 or 1
       p += 256;
       while (p >= n2) p -= n2;
     }
@@ -1623,7 +1628,7 @@ __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const 
       int emin = 255, emax = 0;
       bool bad = false;
 #pragma unroll
-      for (int i = 0; i < GS_PT; ++i) {
+      for (int i = 0; i < PT; ++i) {
         const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
         const int e = (int)(b >> 23);
         bad |= e == 255 || (e == 0 && b != 0);  // not finite, or denormal
@@ -1648,7 +1653,7 @@ __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const 
       if (exact) {
         double s = widen(v[0]);
 #pragma unroll
-        for (int i = 1; i < GS_PT; ++i) s += widen(v[i]);
+        for (int i = 1; i < PT; ++i) s += widen(v[i]);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) sh[0][w] = s;
         __syncthreads();
@@ -1661,7 +1666,7 @@ __global__ void __launch_bounds__(256) k_globsum(const T* __restrict__ x, const 
       __syncthreads();  // s_min, s_max and sh are written again
     }
     if (!exact)
-      for (int i = 0; i < GS_PT; ++i) dd_add(hi, lo, (double)v[i], 0.0);
+      for (int i = 0; i < PT; ++i) dd_add(hi, lo, (double)v[i], 0.0);
   }
   // threads other than 0 hold something only after a pass that was not exact
   if (__syncthreads_or(t != 0 && (hi != 0.0 || lo != 0.0))) dd_block_sum(hi, lo, sh);

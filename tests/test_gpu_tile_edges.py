@@ -294,3 +294,19 @@ def test_densities_of_a_larger_grid(monkeypatch, prec, eos):
     real = gyre.domain
     monkeypatch.setattr(gyre, "domain", lambda nn, **k: real(5, jpk=16))
     test_eos_hpg.test_gpu_eos_bn2_hpg(prec, eos)
+
+
+@pytest.mark.parametrize("nmem,nk", [(1, 1), (1, 62), (5, 31), (12, 3)])
+def test_glob_sum_of_doubles(nmem, nk):
+    """The FP64 sum of one member and of an ensemble (whose members share the blocks) against
+    the exactly rounded one; the compensated sum is off by at most n 2^-104 of the sum of
+    magnitudes."""
+    import math
+    p = Pair(nn=2, prec="fp64", seed=3, nmem=nmem, sample=[0])
+    x = np.random.default_rng(nk).standard_normal((nmem, nk, p.s2[1], p.s2[0])) * 1e3
+    t = p.torch.from_numpy(x).cuda()
+    p.torch.cuda.synchronize()
+    mask = p.ora[0].array("tmask_i", 2).T
+    for m, got in enumerate(p.ctx.glob_sum(t, nk)):
+        v = (x[m] * mask).ravel()
+        assert abs(got - math.fsum(v)) <= 2.0**-52 * abs(math.fsum(v)) + 2.0**-85 * np.abs(v).sum()
