@@ -245,16 +245,24 @@ cudaError_t launch_iso_edges(const Dom<T>& d, const LdfArgs<T>& a, int copy_akz_
   return cudaGetLastError();
 }
 
-// FP32 with the GYRE's 31 levels: one thread a column (k_zdf_imp_async) from this many
-// columns on, where the march of all columns down the same planes is kinder to DRAM than
-// a block of columns at a time: 302x202 33 against 29 us, 362x242 35 against 38, 752x502
-// 118 against 150.
-constexpr long ZDF31_MIN = 65536;
+// FP32 with the GYRE's 31 levels: one thread a column (k_zdf_imp_async, columns of 32 x 4 in
+// shared memory, three blocks an SM) or a block a row of 32 columns (k_zdf_imp32)? The former
+// takes 20 to 23 us a round of blocks up to the second, and on a grid of more rounds its march
+// of all columns down the same planes is kinder to DRAM; the latter some 15 us and 13 more per
+// thousand blocks: 182x122 20 against 15, 212x142 20 and 21, 272x182 23 and 26, 302x202 35 and
+// 32, 400x260 40 and 47, 752x502 118 and 150, 60 members of 33x23 22 and 34.
+template <class T>
+static bool zdf31_by_column(const Dom<T>& d) {
+  const long tiles = (long)((d.jpi + 30) / 32) * ((d.jpj + 2) / 4) * d.nmem;  // with an interior column
+  const long rows = (long)((d.jpi + 31) / 32) * (d.jpj - 2) * d.nmem;         // blocks of k_zdf_imp32
+  const long rounds = (tiles + 3 * 152 - 1) / (3 * 152);
+  return rows >= (rounds == 1 ? 900 : rounds == 2 ? 2500 : 0);
+}
 template <class T>
 cudaError_t launch_zdf(const Dom<T>& d, const ZdfArgs<T>& a, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
     if (d.jpi < 3 || d.jpj < 3) return cudaSuccess;  // no interior column
-    if (d.jpk == 31 && d.n2 * d.nmem >= ZDF31_MIN) {  // the GYRE levels: columns staged in shared memory
+    if (d.jpk == 31 && zdf31_by_column(d)) {
       constexpr int smem_max = 4 * 31 * BX * BY * sizeof(float);
       if (cudaError_t e = smem_opt_in(k_zdf_imp_async<31>, smem_max)) return e;
       const int tz = kty(NEMO_K_ZDF_IMP);

@@ -63,3 +63,39 @@ def test_launch_shape_rejects_untunable_heights():
         p.ctx.set_launch_shape({"spg_p2": 2})
     with pytest.raises(NemoError):
         p.ctx.set_launch_shape({"fct_a": 3})
+
+
+def test_launch_shapes_of_a_larger_grid_give_the_same_bits():
+    """The same at a size whose vertical diffusion in the mixed form runs one thread a column
+    in blocks of the chosen height (31 levels, 242 x 162)."""
+    res = {}
+    for h in (4, 2, 1):
+        p = Pair(nn=8, prec="mixed", seed=29)
+        p.bind_hotpath()
+        p.ctx.set_launch_shape({k: h for k in TUNABLE})
+        for kt in (5, 6):
+            p.ctx.stp_hotpath(kt)
+        p.ctx.synchronize()
+        res[h] = {n: p.dev[n].detach().cpu().clone() for n in ("TSA", "UN", "VN", "SSHA", "AH_WSLP2")}
+    for h in (2, 1):
+        for n in res[4]:
+            assert torch.equal(res[4][n], res[h][n]), f"{n}: block height {h} differs from 4"
+
+
+@pytest.mark.parametrize("prec,nn,nmem", [("mixed", 2, 20), ("mixed", 3, 9), ("fp64", 2, 6)])
+def test_a_member_of_an_ensemble_is_the_member_alone(prec, nn, nmem):
+    """The kernels and chunks chosen by the columns of all members give the bits that the
+    member has by itself."""
+    names = ("TSA", "UN", "VN", "UA", "VA", "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "AH_WSLP2")
+    many = Pair(nn=nn, prec=prec, seed=7, nmem=nmem, sample=[0])
+    for m in (0, nmem - 1):
+        one = Pair(nn=nn, prec=prec, states=[many.states[m]], sample=[0])
+        res = []
+        for p, at in ((many, m), (one, 0)):
+            p.bind_hotpath()
+            for kt in (5, 6):
+                p.ctx.stp_hotpath(kt)
+            p.ctx.synchronize()
+            res.append([p.dev[n].detach().cpu().view(p.nmem, -1)[at] for n in names])
+        for n, a, b in zip(names, *res):
+            assert torch.equal(a, b), (n, m)

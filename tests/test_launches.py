@@ -149,3 +149,21 @@ for nn in (1, 3, 8):
 print(json.dumps(seen))
 """)
     assert out == [[2, 2, 30], [4, 5, 8], [9, 12, 4]]
+
+
+def test_rule_of_the_vertical_diffusion():
+    """tra_zdf_imp in the mixed form with 31 levels: a block a row of columns where those
+    blocks are few for the rounds that one thread a column would take."""
+    out = fakedev.run(r"""
+seen = []
+for nn, nmem in ((2, 1), (6, 1), (7, 1), (9, 1), (10, 1), (14, 1), (1, 60), (2, 20)):
+    c = Ctx(gyre.domain(nn), gyre.namelist(), "mixed", nmem)
+    c.bind("AVT", "AH_WSLP2", "AKZ")
+    t = [c.array(2 * c.n3) for _ in range(2)]
+    launches()
+    c("tra_zdf_imp", 10, 1, b"TRA", 14400.0, *t, 2)
+    seen += ["async" in k[0] for k in launches() if "zdf_imp" in k[0]]
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [False, False, True, True, False, True, True, True]
