@@ -123,11 +123,15 @@ __device__ __forceinline__ MarchIdx march_index(const Dom<T>& d, int kch, int wi
   return c;
 }
 // Levels a thread walks: 32, 16, .. 1, the most that still gives every SM its resident
-// warps (64 of 32 points).
+// warps (64 of 32 points); in FP32 up to 8 levels already at a quarter of them: a grid that
+// small is in L2, and one or two levels a thread cost more than the warps gain (tra_nxt
+// 152x102x31 8.4 us with 1 level, 6.6 with 4; 200x151x31 10.9 with 2, 9.9 with 4, 8.6 with 8;
+// FP64 vor_ene 92x62x31 23 us with 1 level, 27 with 2).
 template <class T>
 inline int march_chunk(const Dom<T>& d) {
+  const long full = 152L * 64 * 32;
   int f = 32;
-  while (f > 1 && (long)d.n2 * d.nmem * ((d.jpk - 1 + f - 1) / f) < 152L * 64 * 32) f /= 2;
+  while (f > 1 && (long)d.n2 * d.nmem * ((d.jpk - 1 + f - 1) / f) < (sizeof(T) == 4 && f <= 8 ? full / 4 : full)) f /= 2;
   return f;
 }
 template <class T>
