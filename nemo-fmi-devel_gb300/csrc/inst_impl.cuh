@@ -26,6 +26,15 @@ static dim3 kc_grid(const Dom<T>& d, int ty = BY) {
   return dim3((d.jpi + BX - 1) / BX, (d.jpj + ty - 1) / ty, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
 }
 
+// the rounds of blocks that such a grid takes with bps of them an SM (a last chunk of few
+// levels is left out: its blocks are short)
+template <class T>
+static long kc_rounds(const Dom<T>& d, int bps) {
+  const long tiles = (long)((d.jpi + BX - 1) / BX) * ((d.jpj + BY - 1) / BY) * d.nmem;
+  const long blocks = tiles * (d.jpk / d.kch + (d.jpk % d.kch > d.kch / 2 ? 1 : 0));
+  return (blocks + bps * 152 - 1) / (bps * 152);
+}
+
 // one thread per (i,j,k) point: z = member * jpk + (k - 1)
 template <class T>
 static dim3 pt_grid(const Dom<T>& d) {
@@ -79,10 +88,20 @@ static bool fct_b_maps(const Dom<T>& d, const FctArgs<T>& a, PlaneMaps<FB_NF>& m
   }
   return true;
 }
-// the instance of the general stage a for a call's orders and transports
+// The instance of the general stage a for a call's orders and transports. FP32: eight blocks
+// an SM spill, and 4th-order horizontal with 2nd-order vertical fluxes the most (100 bytes);
+// there the fewest of six, seven and eight blocks with the same rounds (us a call with 3-D e3:
+// 200x151x31 100, 103, 111; 302x202x31 187, 159, 169; 480x320x31 352, 347, 330).
 template <class T, class I>
-static auto fct_a_of(const FctArgs<T>& a) {
+static auto fct_a_of(const Dom<T>& d, const FctArgs<T>& a) {
   const bool h = a.kn_fct_h == 4, v = a.kn_fct_v == 4;
+  if constexpr (sizeof(T) == 4 && sizeof(I) == 4) {
+    if (h && !v) {
+      const long r = kc_rounds(d, 8);
+      if (kc_rounds(d, 6) == r) return a.trp ? k_fct_a<T, I, true, false, true, 6> : k_fct_a<T, I, true, false, false, 6>;
+      if (kc_rounds(d, 7) == r) return a.trp ? k_fct_a<T, I, true, false, true, 7> : k_fct_a<T, I, true, false, false, 7>;
+    }
+  }
   if (a.trp)
     return h ? (v ? k_fct_a<T, I, true, true, true> : k_fct_a<T, I, true, false, true>)
              : (v ? k_fct_a<T, I, false, true, true> : k_fct_a<T, I, false, false, true>);
@@ -137,7 +156,11 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
       }
     }
     const int ta = kty(NEMO_K_FCT_A);
-    (!a.trp ? k_fct_a_hot<T, false, true> : a.pta_in ? k_fct_a_hot<T, true, true> : k_fct_a_hot<T, true, false>)<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
+    auto kern = !a.trp ? k_fct_a_hot<T, false, true> : a.pta_in ? k_fct_a_hot<T, true, true> : k_fct_a_hot<T, true, false>;
+    if constexpr (sizeof(T) == 4) {
+      if (!a.trp && kc_rounds(d, 8) < kc_rounds(d, 6)) kern = k_fct_a_hot<T, false, true, 8>;
+    }
+    kern<<<kc_grid(d, ta), dim3(BX, ta), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_A, s);
   } else {
     if (a.kn_fct_v == 4) {
@@ -148,14 +171,18 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
       ktick(NEMO_K_INTERP4, s);
     }
     const bool small = (long)a.kjpt * d.n3 < (1L << 31);
-    const auto kern = small ? fct_a_of<T, int>(a) : fct_a_of<T, long>(a);
+    const auto kern = small ? fct_a_of<T, int>(d, a) : fct_a_of<T, long>(d, a);
     kern<<<kc_grid(d), dim3(BX, BY), 0, s>>>(d, a);
     ktick(NEMO_K_FCT_A, s);
   }
   bool b_done = false;
   if constexpr (sizeof(T) == 4) {  // stage b takes any e3t_n (its planes staged by TMA: any orders of stage a)
+    // ... unless the plain kernel's grid is one round of blocks and this one's more: tra_adv_fct
+    // 4/2 with 3-D e3 at 320x220x31 181 against 192 us; 352x260x31, two rounds of both, 245 and 229
     PlaneMaps<FB_NF> mb;
-    if (a.tma && a.err && a.kjpt == 2 && !a.lim && d.n3 < (1L << 30) && fct_b_maps(d, a, mb)) {
+    const long tiles = (long)((d.jpi + TM_X - 1) / TM_X) * ((d.jpj + TM_Y - 1) / TM_Y) * d.nmem * ((d.jpk + d.kch - 1) / d.kch);
+    const bool plain = kc_rounds(d, 8) == 1 && tiles > 3 * 152;
+    if (a.tma && a.err && a.kjpt == 2 && !a.lim && !plain && d.n3 < (1L << 30) && fct_b_maps(d, a, mb)) {
       if (cudaError_t e = smem_opt_in(k_fct_b_tma<T>, FB_SMEM)) return e;
       const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
       k_fct_b_tma<T><<<grid, dim3(TM_X, TM_Y), FB_SMEM, s>>>(d, a, mb, a.err, a.polls);

@@ -264,13 +264,15 @@ inline bool hot_fct_c_ok(const Dom<T>& d, const FctArgs<T>& a) {
 
 // FCT stage a (traadv_fct.F90:119-280) of one column chunk; see k_fct_a. Tracer nn
 // of the member is at offset nn * n3 from tracer 0. TRP: pun, pvn, pwn are velocities, to
-// be scaled to transports; TIN: there may be a trend to add to (FP32 spills with it).
+// be scaled to transports; TIN: there may be a trend to add to (FP32 spills with it, and is
+// compiled for six blocks an SM, or for eight where a grid then takes a round less: 302x202x31
+// 154 -> 134 us a call of tra_adv_fct).
 // Bound by the loads in flight, so by the warps: 214 us at 749x502x31 in FP32 with 40 warps
 // an SM (48 registers, 40 bytes of spills, tn loaded with tb), 239 with 32, 290 with 24.
 // e3t is the one rest-state profile of the three time levels; its quotients as in the TMA
 // form, whose bits the two share.
-template <class T, bool TRP, bool TIN>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (TIN ? 6 : 10) : 3) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
+template <class T, bool TRP, bool TIN, int BPS = (sizeof(T) == 4 ? (TIN ? 6 : 10) : 3)>
+__global__ void __launch_bounds__(128, BPS) k_fct_a_hot(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpk = d.jpk, n2 = (int)d.n2, n3 = (int)d.n3, ij = (int)c.ij;

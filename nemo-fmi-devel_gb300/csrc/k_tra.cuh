@@ -350,8 +350,8 @@ __device__ __forceinline__ T ups(T u, T tl, T tr) {
 // where they fit, half the address arithmetic). With all of that decided at run time a
 // point took 690 instructions (T and S, FCT 4/4, FP32): 359 us at 500x400x56, 335 so (a
 // form with its planes staged by TMA 347: the seven other fields of a level bound it).
-template <class T, class I, bool H4, bool V4, bool TRP>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 3) k_fct_a(Dom<T> d, FctArgs<T> a) {
+template <class T, class I, bool H4, bool V4, bool TRP, int BPS = (sizeof(T) == 4 ? 8 : 3)>
+__global__ void __launch_bounds__(128, BPS) k_fct_a(Dom<T> d, FctArgs<T> a) {
   const KIdx c = k_index(d);
   if (!c.valid) return;
   const int jpi = d.jpi, jpk = d.jpk;

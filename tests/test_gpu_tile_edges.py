@@ -310,3 +310,24 @@ def test_glob_sum_of_doubles(nmem, nk):
     for m, got in enumerate(p.ctx.glob_sum(t, nk)):
         v = (x[m] * mask).ravel()
         assert abs(got - math.fsum(v)) <= 2.0**-52 * abs(math.fsum(v)) + 2.0**-85 * np.abs(v).sum()
+
+
+@pytest.mark.parametrize("jpi,jpj,jpk,order", [(302, 202, 31, 2), (302, 202, 31, 4), (332, 222, 18, 4), (320, 220, 31, 4),
+                                               (62, 42, 9, 4)])
+def test_advection_of_given_transports(jpi, jpj, jpk, order):
+    """tra_adv_fct of given transports in the mixed form, 2nd and 4th order in the horizontal,
+    at sizes of each instance of its stages. Tolerance of the mixed tracer fields."""
+    dom = gyre.domain(int(-(-max((jpi - 2) / 30, (jpj - 2) / 20) // 1)), jpk=jpk)
+    dom = {k: (np.asfortranarray(v[:jpi, :jpj]) if isinstance(v, np.ndarray) and v.ndim > 1 else v) for k, v in dom.items()}
+    for n in ("k_top", "k_bot"):
+        dom[n][0], dom[n][-1], dom[n][:, 0], dom[n][:, -1] = 0, 0, 0, 0
+    dom.update(jpi=jpi, jpj=jpj)
+    p = Pair(dom=dom, nam=gyre.namelist(), prec="mixed", seed=6)
+    st, o, c = p.states[0], p.ora[0], p.ctx
+    tr = o.tra_adv_trp(*[np.array(st[n], order="F") for n in ("un", "vn", "wn")])
+    tb, tn, ta = (np.array(x, order="F") for x in (st["tsb"], st["tsn"], np.zeros(p.s4)))
+    d = [p.to_dev([x]) for x in list(tr) + [tb, tn, ta]]
+    o.tra_adv_fct(5, 1, "TRA", 14400.0, *tr, tb, tn, ta, 2, order, 2)
+    c.tra_adv_fct(5, 1, "TRA", 14400.0, *d, 2, order, 2)
+    e = relerr(14400.0 * ta + tb, 14400.0 * c.to_host(d[5], p.s4) + tb)
+    assert e <= 5e-6 and np.abs(ta).max() > 0

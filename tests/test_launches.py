@@ -11,7 +11,7 @@ for device in (0, 1):
     fake.cudaSetDevice(device)
     for prec, jpk, order, fused in (("mixed", 31, 2, 0), ("mixed", 31, 2, 1), ("mixed", 64, 4, 0), ("fp64", 64, 4, 0)):
         dom = gyre.domain(1, jpk=jpk)
-        c = Ctx(dom, gyre.namelist(), prec, nmem=100 if fused else 1)  # enough columns for each form of tra_zdf
+        c = Ctx(dom, gyre.namelist(), prec, nmem=140 if fused else 1)  # enough columns for each form of tra_zdf
         c.bind("AVT", "AH_WSLP2", "AKZ", "TSB", "TSN", "TSA", "UN", "VN", "WN", "USLP", "VSLP", "WSLPI", "WSLPJ")
         c.bind("UA", "VA", "UB", "VB", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP", "RCDU_BOT",
                "SSHA", "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")
@@ -167,3 +167,29 @@ for nn, nmem in ((2, 1), (6, 1), (7, 1), (9, 1), (10, 1), (14, 1), (1, 60), (2, 
 print(json.dumps(seen))
 """)
     assert out == [False, False, True, True, False, True, True, True]
+
+
+def test_instances_of_the_advection():
+    """tra_adv_fct in the mixed form with given transports: stage a for six, seven or eight
+    blocks an SM by the rounds that the grid takes, stage b with copied planes but where its
+    second round is the plain kernel's first."""
+    out = fakedev.run(r"""
+seen = []
+def domain(jpi, jpj):
+    dom = gyre.domain(-(-max((jpi - 2) // 30, (jpj - 2) // 20) // 1) + 1)
+    import numpy as np
+    dom = {k: (np.asfortranarray(v[:jpi, :jpj]) if isinstance(v, np.ndarray) and v.ndim > 1 else v) for k, v in dom.items()}
+    dom.update(jpi=jpi, jpj=jpj)
+    return dom
+for jpi, jpj, h in ((200, 151, 4), (302, 202, 4), (480, 320, 4), (320, 220, 4), (352, 260, 4), (250, 180, 2), (302, 202, 2)):
+    c = Ctx(domain(jpi, jpj), gyre.namelist(), "mixed")
+    t = [c.array(2 * c.n3) for _ in range(6)]
+    launches()
+    c("tra_adv_fct", 10, 1, b"TRA", 14400.0, *t, 2, h, 2)
+    seen.append([k[0][:40] for k in launches() if "fct_" in k[0]][:2])
+    c.close()
+print(json.dumps(seen))
+""")
+    a = ["Lb0ELi6E", "Lb0ELi7E", "Lb0ELi8E", "Lb0ELi8E", "Lb0ELi6E", "Lb0ELb1ELi6E", "Lb0ELb1ELi8E"]
+    b = ["tma", "fct_bI", "tma", "fct_bI", "tma", "fct_b_hot", "fct_b_hot"]
+    assert all(x in k[0] and y in k[1] for x, y, k in zip(a, b, out)), out
