@@ -3129,6 +3129,7 @@ int nemo_gpu_autotune(nemo_ctx* c, int kt, int nrep) {
   unsigned char pick[NEMO_K_COUNT] = {};
   for (double& b : best) b = 1e300;
   int st = NEMO_OK;
+  for (bool& b : c->shape.asked) b = false;
   for (int ty : {4, 2, 1}) {
     for (int id : kTunable) c->shape.ty[id] = (unsigned char)ty;
     for (int r = 0; r <= nrep && st == NEMO_OK; ++r) {
@@ -3140,8 +3141,8 @@ int nemo_gpu_autotune(nemo_ctx* c, int kt, int nrep) {
       else st = c->prec == NEMO_PREC_FP64 ? run_hotpath<double>(c, kt, false) : run_hotpath<float>(c, kt, false);
     }
     if (st) break;
-    for (int id : kTunable)
-      if (c->kcnt[id] > 0 && c->kms[id] / c->kcnt[id] < best[id]) {
+    for (int id : kTunable)  // of the kernels whose form in this configuration has a height
+      if (c->shape.asked[id] && c->kcnt[id] > 0 && c->kms[id] / c->kcnt[id] < best[id]) {
         best[id] = c->kms[id] / c->kcnt[id];
         pick[id] = (unsigned char)ty;
       }

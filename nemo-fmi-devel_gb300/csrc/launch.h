@@ -23,10 +23,12 @@ extern thread_local KernelClock* t_kclock;
 // calling thread while it runs the hot path; elsewhere the default 4 (32 x 4).
 struct LaunchShape {
   unsigned char ty[NEMO_K_COUNT] = {};
+  mutable bool asked[NEMO_K_COUNT] = {};  // a launch took its height from here
 };
 extern thread_local const LaunchShape* t_shape;
 inline int kty(int id) {
   const LaunchShape* s = t_shape;
+  if (s) s->asked[id] = true;
   return (s && s->ty[id]) ? s->ty[id] : 4;
 }
 inline void ktick(int id, cudaStream_t s) {

@@ -193,3 +193,26 @@ print(json.dumps(seen))
     a = ["Lb0ELi6E", "Lb0ELi7E", "Lb0ELi8E", "Lb0ELi8E", "Lb0ELi6E", "Lb0ELb1ELi6E", "Lb0ELb1ELi8E"]
     b = ["tma", "fct_bI", "tma", "fct_bI", "tma", "fct_b_hot", "fct_b_hot"]
     assert all(x in k[0] and y in k[1] for x, y, k in zip(a, b, out)), out
+
+
+def test_autotune_of_kernels_without_a_height():
+    """nemo_gpu_autotune with timings that get shorter from one candidate to the next: it picks
+    the last for the kernels that have a block height, and leaves those whose form in the
+    configuration has none (the vertical diffusion of a small grid, and with tensor copies the
+    tracer fluxes) as they are."""
+    out = fakedev.run(r"""
+seen = []
+for nn in (1, 9):
+    c = Ctx(gyre.domain(nn), gyre.namelist(), "mixed")
+    c.bind("AVT", "AH_WSLP2", "AKZ", "TSB", "TSN", "TSA", "UN", "VN", "WN", "USLP", "VSLP", "WSLPI", "WSLPJ", "UA", "VA",
+           "UB", "VB", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP", "RCDU_BOT", "SSHA", "UA_B",
+           "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")
+    c("autotune", 10, 1)
+    ty = (C.c_int * 64)()
+    c("get_launch_shape", ty, 64)
+    from nemo_gpu._ffi import K
+    seen.append([ty[K[n]] for n in ("ZDF_IMP", "ISO_FLUX", "FCT_C", "SPG_P3")])
+    c.close()
+print(json.dumps(seen))
+""")
+    assert out == [[4, 4, 1, 1], [1, 4, 1, 1]]
