@@ -32,7 +32,7 @@ template <class T>
 static long kc_rounds(const Dom<T>& d, int bps) {
   const long tiles = (long)((d.jpi + BX - 1) / BX) * ((d.jpj + BY - 1) / BY) * d.nmem;
   const long blocks = tiles * (d.jpk / d.kch + (d.jpk % d.kch > d.kch / 2 ? 1 : 0));
-  return (blocks + bps * 152 - 1) / (bps * 152);
+  return (blocks + bps * SMS - 1) / (bps * SMS);
 }
 
 // one thread per (i,j,k) point: z = member * jpk + (k - 1)
@@ -181,7 +181,7 @@ cudaError_t launch_fct(const Dom<T>& d, const FctArgs<T>& a, cudaStream_t s) {
     // 4/2 with 3-D e3 at 320x220x31 181 against 192 us; 352x260x31, two rounds of both, 245 and 229
     PlaneMaps<FB_NF> mb;
     const long tiles = (long)((d.jpi + TM_X - 1) / TM_X) * ((d.jpj + TM_Y - 1) / TM_Y) * d.nmem * ((d.jpk + d.kch - 1) / d.kch);
-    const bool plain = kc_rounds(d, 8) == 1 && tiles > 3 * 152;
+    const bool plain = kc_rounds(d, 8) == 1 && tiles > 3 * SMS;
     if (a.tma && a.err && a.kjpt == 2 && !a.lim && !plain && d.n3 < (1L << 30) && fct_b_maps(d, a, mb)) {
       if (cudaError_t e = smem_opt_in(k_fct_b_tma<T>, FB_SMEM)) return e;
       const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
@@ -282,7 +282,7 @@ template <class T>
 static bool zdf31_by_column(const Dom<T>& d) {
   const long tiles = (long)((d.jpi + 30) / 32) * ((d.jpj + 2) / 4) * d.nmem;  // with an interior column
   const long rows = (long)((d.jpi + 31) / 32) * (d.jpj - 2) * d.nmem;         // blocks of k_zdf_imp32
-  const long rounds = (tiles + 3 * 152 - 1) / (3 * 152);
+  const long rounds = (tiles + 3 * SMS - 1) / (3 * SMS);
   return rows >= (rounds == 1 ? 900 : rounds == 2 ? 2500 : 0);
 }
 template <class T>
@@ -310,7 +310,7 @@ cudaError_t launch_zdf(const Dom<T>& d, const ZdfArgs<T>& a, cudaStream_t s) {
 template <class T>
 cudaError_t launch_clamp(T* x, long n, cudaStream_t s) {
   long nb = (n + 255) / 256;
-  if (nb > 152L * 16) nb = 152L * 16;
+  if (nb > SMS * 16) nb = SMS * 16;
   if (nb < 1) nb = 1;
   k_clamp_neg<T><<<(unsigned)nb, 256, 0, s>>>(x, n);
   ktick(NEMO_K_CLAMP, s);

@@ -20,7 +20,7 @@ template <class T>
 int level_chunk(const Dom<T>& d, int block, int step) {
   const long planes = (d.n2 + block - 1) / block * d.nmem;
   for (int f = 4; f > 1; f /= 2)
-    if (planes * ((d.jpk + f * step - 1) / (f * step)) * block >= 152L * 64 * 32) return f * step;
+    if (planes * ((d.jpk + f * step - 1) / (f * step)) * block >= SMS * 64L * 32) return f * step;
   return step;
 }
 // the two components' columns: z = 2 member + component
@@ -49,7 +49,7 @@ cudaError_t launch_dyn_nxt(const Dom<T>& d, const NxtArgs<T, double>& a, cudaStr
   // FP64: 94 registers let five blocks an SM run, 72 (some spills) seven. More than one block an
   // SM takes the latter: 302x202x31 250 -> 183 us, 200x151x31 109 -> 105; 62x42x31 33 -> 39.
   constexpr int more = sizeof(T) == 8 ? 7 : 1;
-  const auto kern = (long)g.x * g.y * g.z > 152 ? k_dyn_nxt<T, double, more> : k_dyn_nxt<T, double, 1>;
+  const auto kern = (long)g.x * g.y * g.z > SMS ? k_dyn_nxt<T, double, more> : k_dyn_nxt<T, double, 1>;
   if (cudaError_t e = smem_opt_in(kern, level * KMAX)) return e;
   kern<<<g, dim3(SX, DN_Y), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_NXT, s);

@@ -56,10 +56,10 @@ __device__ __forceinline__ double zero_of(double x) {
 }
 
 // ------------------------------------------------------------------ tra_adv_fct
-// Adjoint of tra_adv_fct (traadv_fct.F90:54-327) at one point; with kn_fct_h = 4 the
-// 4th-order centred horizontal fluxes (:191-227), with kn_fct_v = 4 the compact
-// vertical interpolation's part is k_fct_adj_v4's (below). With g = lam r1_e1e2t / e3t_n and h = g tmask on the interior cells (0
-// elsewhere), the limited antidiffusive flux of face f has the adjoint
+// Adjoint of tra_adv_fct (traadv_fct.F90:54-327) with kn_fct_h = 4, the 4th-order centred
+// horizontal fluxes (:191-227), at one point (2: k_fct_adj2 below); with kn_fct_v = 4 the
+// compact vertical interpolation's part is k_fct_adj_v4's. With g = lam r1_e1e2t / e3t_n
+// and h = g tmask on the interior cells (0 elsewhere), the limited antidiffusive flux of face f has the adjoint
 // -(g(f) - g(f+1)); times the recorded multiplier (0 where the forward zeroed the
 // flux) it is the adjoint of the flux before limiting, the centred flux of tn minus
 // the upstream flux of tb (:182-190, :255-263). The upstream flux gets minus that,
@@ -120,31 +120,29 @@ __global__ void __launch_bounds__(128) k_fct_adj(Dom<double> d, FctAdj a) {
       if (zt) tnv += wn[q] * 0.5 * azt;
       if (zb) tnv += wn[q + n2] * 0.5 * azb;
     }
-    if (a.kh == 4) {
-      // zltu(m) = (ztu(m) + ztu(m-1)) / 6 enters the flux of u-face m with + and that
-      // of face m-1 with -; ztu(m) = (tn(m+1) - tn(m)) umask(m). S: the adjoint of a
-      // face's centred bracket; Z: of zltu (interior points only, lbc_lnk zeroes the
-      // edges). Likewise in j.
-      auto Su = [&](int fi) -> double {
-        if (!P.uface(fi, j, k)) return 0.0;
-        const long qf = P.q(fi, j, k);
-        return 0.5 * un[qf] * (tx[qf] * (g(fi + 1, j, k) - g(fi, j, k)));
-      };
-      auto Sv = [&](int fj) -> double {
-        if (!P.uface(i, fj, k)) return 0.0;
-        const long qf = P.q(i, fj, k);
-        return 0.5 * vn[qf] * (ty[qf] * (g(i, fj + 1, k) - g(i, fj, k)));
-      };
-      auto Zu = [&](int mi) -> double { return P.cell(mi, j, k) ? Su(mi) - Su(mi - 1) : 0.0; };
-      auto Zv = [&](int mj) -> double { return P.cell(i, mj, k) ? Sv(mj) - Sv(mj - 1) : 0.0; };
-      const double zu0 = Zu(i - 1), zu1 = Zu(i), zu2 = Zu(i + 1);
-      const double zv0 = Zv(j - 1), zv1 = Zv(j), zv2 = Zv(j + 1);
-      const double r1_6 = 1. / 6.;
-      if (i >= 2) tnv += r1_6 * (zu0 + zu1) * umsk<double>(d.ci[c.ij - 1], k);
-      tnv -= r1_6 * (zu1 + zu2) * umsk<double>(ci, k);
-      if (j >= 2) tnv += r1_6 * (zv0 + zv1) * vmsk<double>(d.ci[c.ij - jpi], k);
-      tnv -= r1_6 * (zv1 + zv2) * vmsk<double>(ci, k);
-    }
+    // zltu(m) = (ztu(m) + ztu(m-1)) / 6 enters the flux of u-face m with + and that
+    // of face m-1 with -; ztu(m) = (tn(m+1) - tn(m)) umask(m). S: the adjoint of a
+    // face's centred bracket; Z: of zltu (interior points only, lbc_lnk zeroes the
+    // edges). Likewise in j.
+    auto Su = [&](int fi) -> double {
+      if (!P.uface(fi, j, k)) return 0.0;
+      const long qf = P.q(fi, j, k);
+      return 0.5 * un[qf] * (tx[qf] * (g(fi + 1, j, k) - g(fi, j, k)));
+    };
+    auto Sv = [&](int fj) -> double {
+      if (!P.uface(i, fj, k)) return 0.0;
+      const long qf = P.q(i, fj, k);
+      return 0.5 * vn[qf] * (ty[qf] * (g(i, fj + 1, k) - g(i, fj, k)));
+    };
+    auto Zu = [&](int mi) -> double { return P.cell(mi, j, k) ? Su(mi) - Su(mi - 1) : 0.0; };
+    auto Zv = [&](int mj) -> double { return P.cell(i, mj, k) ? Sv(mj) - Sv(mj - 1) : 0.0; };
+    const double zu0 = Zu(i - 1), zu1 = Zu(i), zu2 = Zu(i + 1);
+    const double zv0 = Zv(j - 1), zv1 = Zv(j), zv2 = Zv(j + 1);
+    const double r1_6 = 1. / 6.;
+    if (i >= 2) tnv += r1_6 * (zu0 + zu1) * umsk<double>(d.ci[c.ij - 1], k);
+    tnv -= r1_6 * (zu1 + zu2) * umsk<double>(ci, k);
+    if (j >= 2) tnv += r1_6 * (zv0 + zv1) * vmsk<double>(d.ci[c.ij - jpi], k);
+    tnv -= r1_6 * (zv1 + zv2) * vmsk<double>(ci, k);
     // upstream fluxes: minus the antidiffusive adjoint plus their own trend's
     const double fxe = -axe + (he - hc), fxw = -axw + (hc - hw);
     const double fyn = -ayn + (hn - hc), fys = -ays + (hc - hs);

@@ -404,7 +404,7 @@ constexpr size_t P2_CACHE_BYTES = (size_t)P2_NC * P2_MAXT * 256 * sizeof(float);
 // sum is a float pair hi + lo, updated with an exact product (the FMA residual) and
 // a two-sum on the FP32 pipe -- error ~2^-46 of the sum, far below the FP32 storage
 // of the summed values -- and converted to the FP64 fields once, at the end of the
-// kernel. (FP64 arithmetic runs at 1/64 of the FP32 rate on this GPU, and five FP64
+// kernel. (FP64 arithmetic runs at 1/58 of the FP32 rate on this GPU, and five FP64
 // sums per point per sub-step would occupy its FP64 pipe.) The intrinsics keep the
 // compiler from contracting the compensated steps.
 struct FF {

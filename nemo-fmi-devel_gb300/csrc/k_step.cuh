@@ -374,10 +374,10 @@ __global__ void k_ssh_swp(Dom<T> d, T* sshb, T* sshn, const A* __restrict__ ssha
 // ldf_slp (ldfslp.F90:83-374) with ldf_slp_mxl (:620-729), z-coordinate with or
 // without partial steps, without cavities, in three kernels: the slopes just below the mixed
 // layer (one column per thread), the slopes before the Shapiro filter at u-, v- and
-// w-points (one point per thread), the filter with the coastal decrease and lbc.
-// The density gradients zgru, zgrv and zdzr of the reference's work arrays are
+// w-points (a chunk of levels per thread), the filter with the coastal decrease and lbc
+// (the same). The density gradients zgru, zgrv and zdzr of the reference's work arrays are
 // formed where they are read, from the same operands in the same order.
-template <class T, bool ZPS = false>
+template <class T, bool ZPS>
 struct SlpPt {
   const Dom<T>& d;
   const SlpArgs<T>& a;
@@ -389,7 +389,6 @@ struct SlpPt {
   __device__ __forceinline__ T um(int i, int j, int k) const { return umsk<T>(d.ci[Q(i, j, 1)], k); }
   __device__ __forceinline__ T vm(int i, int j, int k) const { return vmsk<T>(d.ci[Q(i, j, 1)], k); }
   __device__ __forceinline__ T tm(int i, int j, int k) const { return tmsk<T>(d.ci[Q(i, j, 1)], k); }
-  __device__ __forceinline__ T wm(int i, int j, int k) const { return wmsk<T>(d.ci[Q(i, j, 1)], k); }
   __device__ __forceinline__ T prd(int i, int j, int k) const { return a.prd[m3 + Q(i, j, k)]; }
   // with partial steps (ZPS) the bottom level's gradients are zps_hde's
   // (ldfslp.F90:144-151); the z-coordinate form compiles without the test
@@ -409,9 +408,6 @@ struct SlpPt {
     if (k == 1) return T(0);
     const long q = m3 + Q(i, j, k);
     return a.zm1_g * (a.prd[q] + T(1)) * (a.pn2[q] + a.pn2[q + d.n2]) * (T(1) - T(0.5) * tm(i, j, k + 1));
-  }
-  __device__ __forceinline__ T oml(int i, int j, int k) const {
-    return k <= a.nmln[(long)m * d.n2 + Q(i, j, 1)] - 1 ? T(1) : T(0);
   }
 };
 

@@ -74,7 +74,7 @@ constexpr int KCH = 16;
 // levels is 16 memory round trips in a row on 3 % of the SMs (78 us for the four kernels).
 // In FP64 two warps already fill an SM's FP64 pipe, and what a chunk repeats costs more.
 inline int tra_chunk(long n2, int nmem, int jpk, bool fp64) {
-  const long want = 152L * 32 * (fp64 ? 2 : 8);
+  const long want = SMS * 32L * (fp64 ? 2 : 8);
   int c = KCH;
   while (c > 2 && n2 * nmem * ((jpk + c - 1) / c) < want) c /= 2;
   return c;
@@ -129,7 +129,7 @@ __device__ __forceinline__ MarchIdx march_index(const Dom<T>& d, int kch, int wi
 // FP64 vor_ene 92x62x31 23 us with 1 level, 27 with 2).
 template <class T>
 inline int march_chunk(const Dom<T>& d) {
-  const long full = 152L * 64 * 32;
+  const long full = SMS * 64L * 32;
   int f = 32;
   while (f > 1 && (long)d.n2 * d.nmem * ((d.jpk - 1 + f - 1) / f) < (sizeof(T) == 4 && f <= 8 ? full / 4 : full)) f /= 2;
   return f;
@@ -238,7 +238,7 @@ struct FctArgs {
                              // ((member*kjpt + n)*3 + face)*n3, for the adjoint
 };
 
-// ---- value-exact helpers of the FCT and iso-neutral kernels. FP64 runs at 1/64 of
+// ---- value-exact helpers of the FCT and iso-neutral kernels. FP64 runs at 1/58 of
 // the FP32 rate on this GPU, and compares, min/max and products by 0/1 masks all
 // occupy that pipe; these forms move them to the integer pipe or drop them while
 // giving the reference's values (at most the sign of a zero differs, which no later
@@ -1314,37 +1314,23 @@ __global__ void __launch_bounds__(32 * W) k_zdf_imp32(Dom<float> d, ZdfArgs<floa
     const long mo = ((long)m * a.kjpt + n0) * n3 + ij;
     const float *tb = a.ptb.p + mo, *coef = (use_avt ? a.avt : a.avs).p + c3, *add = a.add ? a.add.p + c3 : coef;
     float* ta = a.pta + mo;
-    constexpr int U = 1;  // levels a thread loads together
-    for (int k0 = w + 1; k0 <= jpk; k0 += U * W) {
-      float v[U], x[U], t[2][U], b[2][U], ew[U], ea[U], en[U], eb[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = min(k0 + u * W, jpk);
-        const long o = (long)(k - 1) * n2;
-        for (int n = 0; n < 2; ++n) {
-          t[n][u] = n < nn ? ta[o + n * n3] : 0.0f;
-          b[n][u] = n < nn ? __ldg(tb + o + n * n3) : 0.0f;
-        }
-        v[u] = __ldg(coef + o);
-        x[u] = __ldg(add + o);
-        ew[u] = d.e3w_n(ij, k, m);
-        ea[u] = d.e3t_a(ij, k, m);
-        en[u] = d.e3t_n(ij, k, m);
-        eb[u] = d.e3t_b(ij, k, m);
+    for (int k = w + 1; k <= jpk; k += W) {  // one level in flight a thread
+      const long o = (long)(k - 1) * n2;
+      float t[2], b[2];
+      for (int n = 0; n < 2; ++n) {
+        t[n] = n < nn ? ta[o + n * n3] : 0.0f;
+        b[n] = n < nn ? __ldg(tb + o + n * n3) : 0.0f;
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = k0 + u * W;
-        if (k > jpk) break;
-        if (build) {
-          const float wt = k == 1 ? 0.0f : a.add && k <= K ? v[u] + x[u] : v[u];
-          zw[k * NC] = -p2dt * wt / ew[u];
-          rz[k * NC] = ea[u];
-        }
-        for (int n = 0; n < nn; ++n) {
-          sb[n * A + k * NC] = b[n][u];
-          sy[n * A + k * NC] = p2dt * en[u] * t[n][u] + (eb[u] - ea[u]) * b[n][u];
-        }
+      const float v = __ldg(coef + o), x = __ldg(add + o);
+      const float ew = d.e3w_n(ij, k, m), ea = d.e3t_a(ij, k, m), en = d.e3t_n(ij, k, m), eb = d.e3t_b(ij, k, m);
+      if (build) {
+        const float wt = k == 1 ? 0.0f : a.add && k <= K ? v + x : v;
+        zw[k * NC] = -p2dt * wt / ew;
+        rz[k * NC] = ea;
+      }
+      for (int n = 0; n < nn; ++n) {
+        sb[n * A + k * NC] = b[n];
+        sy[n * A + k * NC] = p2dt * en * t[n] + (eb - ea) * b[n];
       }
     }
     __syncthreads();

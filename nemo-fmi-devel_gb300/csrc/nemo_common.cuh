@@ -16,6 +16,8 @@
 
 namespace nemo {
 
+constexpr int SMS = 152;  // SMs of a GB300: what the rules of grids and chunks count on
+
 struct __align__(8) ColInfo {
   uint8_t tlo, thi, ulo, uhi, vlo, vhi, mbku, mbkv;
 };
