@@ -48,8 +48,8 @@ cudaError_t launch_dyn_nxt(const Dom<T>& d, const NxtArgs<T, double>& a, cudaStr
   const dim3 g = s_cols2<T>(d, DN_Y);
   // FP64: 94 registers let five blocks an SM run, 72 (some spills) seven. More than one block an
   // SM takes the latter: 302x202x31 250 -> 183 us, 200x151x31 109 -> 105; 62x42x31 33 -> 39.
-  constexpr int more = sizeof(T) == 8 ? 7 : 1;
-  const auto kern = (long)g.x * g.y * g.z > SMS ? k_dyn_nxt<T, double, more> : k_dyn_nxt<T, double, 1>;
+  constexpr int more = sizeof(T) == 8 ? 7 : 5;
+  const auto kern = (long)g.x * g.y * g.z > SMS ? k_dyn_nxt<T, double, more> : k_dyn_nxt<T, double, 5>;
   if (cudaError_t e = smem_opt_in(kern, level * KMAX)) return e;
   kern<<<g, dim3(SX, DN_Y), smem, s>>>(d, a);
   ktick(NEMO_K_DYN_NXT, s);
