@@ -42,8 +42,6 @@ struct SpgArgs {
   int ln_bt_fw, ln_apr_dyn, nvor, ll_init, icycle, ring0, phase3_filter;
   int cache;  // mixed form, ENE/MIX: the sub-step constants cached in shared memory
   int hot;    // mixed form, linear free surface, ENE/MIX: k_spg_p2_ene instead of k_spg_p2
-  int five;   // k_spg_p2 compiled for five blocks an SM
-  int res_c, res_rows, res_v, res_gen;  // res_c > 0: k_spg_p2_res (variant res_v), res_c blocks of res_rows rows a member
   // Column depths (2-D): for a linear free surface the rest-state ht_0, hu_0, ...
   // shared by all members (member stride hs = 0); with a variable volume the bound
   // now / before depths of each member (hs = points per member). The Coriolis
@@ -58,6 +56,8 @@ struct SpgArgs {
   int een_e3f, sco;
   T rdtbt, grav, r1_rau0, scal_load, rn_bt_alpha;
   double rn_atfp, r1_2dt_b;
+  int five;   // k_spg_p2 compiled for five blocks an SM
+  int res_c, res_rows, res_v, res_gen;  // res_c > 0: k_spg_p2_res (variant res_v), res_c blocks of res_rows rows a member
 };
 
 template <class T>

@@ -63,7 +63,6 @@ struct E3 {
 template <class T>
 struct Dom {
   int jpi, jpj, jpk, nmem;
-  int kch;         // levels a thread of the tracer k-marches walks
   long n2, n3;  // points per member of a 2-D / 3-D field
   RO<T> e1t, e2t, e1u, e2u, e1v, e2v;
   RO<T> r1_e1u, r1_e2u, r1_e1v, r1_e2v;
@@ -80,6 +79,7 @@ struct Dom {
   // 1 / e3t_0 and 1 / e3w_0 per level (correctly rounded) where the rest-state scale
   // factor is a 1-D profile, else NULL: the divisors of the hot-path tracer kernels
   RO<T> r1_e3t, r1_e3w;
+  int kch;  // levels a thread of the tracer k-marches walks
 };
 
 __device__ __forceinline__ bool in_range(int k, int lo, int hi) { return k >= lo && k <= hi; }
