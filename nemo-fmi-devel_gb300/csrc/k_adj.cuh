@@ -37,15 +37,16 @@ struct Pt3 {
 template <class T>
 __device__ __forceinline__ Pt3 pt3(const Dom<T>& d) { return Pt3{d.jpi, d.jpj, d.jpk, d.n2}; }
 
-// x / e3t_n(k) and x / e3w_n(k): through the reciprocal profile (divr, the correctly
-// rounded quotient) where the now scale factor is the rest-state profile
+// x / e3t_n(k) and x / e3w_n(k): through the reciprocal profile (the correctly rounded
+// quotient; divr for the first, whose x holds sensitivities that may be infinite) where the
+// now scale factor is the rest-state profile
 __device__ __forceinline__ double over_e3t(const Dom<double>& d, double x, long ij, int k, int m) {
   const double e = d.e3t_n(ij, k, m);
   return d.r1_e3t && d.e3t_n.s == 0 ? divr(x, e, d.r1_e3t[k - 1]) : x / e;
 }
 __device__ __forceinline__ double over_e3w(const Dom<double>& d, double x, long ij, int k, int m) {
   const double e = d.e3w_n(ij, k, m);
-  return d.r1_e3w && d.e3w_n.s == 0 ? divr(x, e, d.r1_e3w[k - 1]) : x / e;
+  return d.r1_e3w && d.e3w_n.s == 0 ? divq(x, e, d.r1_e3w[k - 1]) : x / e;
 }
 // x != 0 on the integer pipe (NaN counts as nonzero)
 __device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(128) k_iso_adj_tb(Dom<double> d, LdfArgs<doubl
 // back-substitution run forwards, then the elimination with its right-hand side
 // e3t_b tb + p2dt e3t_n ta run backwards. The matrix is built as k_zdf_imp builds
 // it in double precision: one division a level, 1 / zwt, and every quotient corrected
-// from a reciprocal (divr); zwi(k+1) is zws(k).
+// from a reciprocal (divq; divr for the sensitivities); zwi(k+1) is zws(k).
 __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
   ColIdx<double> c = col_index(d);
   if (!c.valid || !c.interior) return;
@@ -592,8 +593,8 @@ __global__ void k_zdf_adj(Dom<double> d, ZdfArgs<double> a, ZdfAdj b) {
         const double zs = over_e3w(d, -a.p2dt * wt(k + 1), c.ij, k + 1, c.m);
         double t = d.e3t_a(c.ij, k, c.m) - zwi - zs;
         if (k >= 2) {
-          rat[k] = divr(zwi, tp, rp);
-          t = t - divr(zwi * zwi, tp, rp);  // zws(k-1) = zwi(k)
+          rat[k] = divq(zwi, tp, rp);
+          t = t - divq(zwi * zwi, tp, rp);  // zws(k-1) = zwi(k)
         }
         zws[k] = zs;
         zwt[k] = tp = t;

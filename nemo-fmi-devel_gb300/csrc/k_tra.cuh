@@ -303,8 +303,10 @@ template <class T>
 __device__ __forceinline__ T divr(T x, T y, T ry) {
   if constexpr (sizeof(T) == 8) {
     const T q = __dmul_rn(x, ry);
-    const bool finite = (__double2hiint(q) & 0x7ff00000) != 0x7ff00000;
-    return finite ? __fma_rn(__fma_rn(-q, y, x), ry, q) : q;
+    const T r = __fma_rn(__fma_rn(-q, y, x), ry, q);
+    const int h = __double2hiint(q);
+    const bool finite = (h & 0x7ff00000) != 0x7ff00000;
+    return __hiloint2double(finite ? __double2hiint(r) : h, finite ? __double2loint(r) : __double2loint(q));
   } else {
     const T q = __fmul_rn(x, ry);
     return isfinite(q) ? __fmaf_rn(__fmaf_rn(-q, y, x), ry, q) : q;
