@@ -820,8 +820,9 @@ int nemo_gpu_get_kernel_timing(nemo_ctx *ctx, double *ms, int *launches, int n);
 int nemo_gpu_set_fusion(nemo_ctx *ctx, int on);
 
 /* on = 1 (default): in a mixed-precision context, the iso-neutral flux kernel of that
- * configuration stages the tracer planes in shared memory with tensor copies (TMA)
- * when jpi is a multiple of 4; on = 0 forces the kernel without TMA. Same results. */
+ * configuration stages the tracer planes in shared memory, with tensor copies (TMA)
+ * when jpi is a multiple of 4, else from 16384 columns on with copies by its threads;
+ * on = 0 forces the kernels that read global memory. Same results. */
 int nemo_gpu_set_tma(nemo_ctx *ctx, int on);
 
 /* on = 1: with TMA on (nemo_gpu_set_tma), the three FCT stages of that configuration

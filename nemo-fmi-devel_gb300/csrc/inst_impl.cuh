@@ -239,7 +239,10 @@ cudaError_t launch_iso_flux(const Dom<T>& d, const LdfArgs<T>& a, cudaStream_t s
       }
       // rows not 16 bytes apart: the planes copied by the threads. 281 against 342 us of
       // k_iso_flux_hot at 749x502x31, 101 against 138 at 310x367, 18.3 against 19.0 at
-      // 121x152; on smaller grids (7.0 against 6.2 us at 62x42) a march is too short for it
+      // 121x152; on smaller grids (7.0 against 6.2 us at 62x42) a march is too short for it.
+      // At 230 to 270 points a row, with the data in L2, the other is the faster by itself
+      // (242x162x31 50 against 62 us), but its blocks leave no room for the sub-steps that a
+      // step runs beside it: 418 us a step against 348
       if (a.tma && a.err && d.n2 * d.nmem >= 16384) {
         const dim3 grid((d.jpi + TM_X - 1) / TM_X, (d.jpj + TM_Y - 1) / TM_Y, d.nmem * ((d.jpk + d.kch - 1) / d.kch));
         (iso_3d(d, a) ? k_iso_flux_tma<T, true, false> : k_iso_flux_tma<T, false, false>)<<<grid, dim3(TM_X, TM_Y), 0, s>>>(

@@ -1040,7 +1040,7 @@ __device__ __forceinline__ T eos_rd_2d(const EosArgs<T>& a, T t, T sal, T dep) {
 // 72 % of the slots: some 110 instructions a point of the polynomials; by traffic, 4 and 5
 // fields, 28 and 35 us of 48 and 55) and by the FP64 pipe in FP64. As one point a thread, with
 // the coefficients loaded from global memory, the six calls of a step's density (two
-// rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32, 358 so.
+// rab_3d, two bn2, eos_insitu, eos_insitu_pot) took 679 us at 752x502x31 in FP32, 343 so.
 // Blocks of 2 (FP64) and 4 warps: with 8, a small grid was a few blocks whose points shared an
 // SM's FP64 pipe (rab_3d 20x17x10 16, 62x42x31 43 us, 9 and 32 so), and a large one had a
 // longer last round (93x61x31x12 669, 648).
