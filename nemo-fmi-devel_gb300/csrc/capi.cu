@@ -700,10 +700,18 @@ Dom<T> dom_now(nemo_ctx* c) {
   return d;
 }
 
+// The captured steps hold the addresses of the fields and work arrays, the launch shapes and
+// the switches: whatever changes one of these drops them, and the next step is captured again.
+void drop_graphs(nemo_ctx* c) {
+  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
+  c->graphs.clear();
+}
+
 int ensure_fct_work(nemo_ctx* c, int kjpt, int need_ztw) {
   const size_t es = c->prec == NEMO_PREC_FP64 ? 8 : 4;
   const size_t bytes = (size_t)kjpt * c->n3 * c->nmem * es;
   if (kjpt > c->fct_kjpt) {
+    drop_graphs(c);
     for (auto& p : c->fct_w) { cudaFree(p); p = nullptr; }
     cudaFree(c->fct_ztw); c->fct_ztw = nullptr;
     for (auto& p : c->fct_w) {
@@ -723,6 +731,7 @@ int ensure_fct_work(nemo_ctx* c, int kjpt, int need_ztw) {
 int ensure_iso_work(nemo_ctx* c, int kjpt) {
   if (kjpt <= c->iso_kjpt) return NEMO_OK;
   const size_t bytes = (size_t)kjpt * c->n3 * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
+  drop_graphs(c);
   for (auto& p : c->iso_w) {
     cudaFree(p);
     p = nullptr;
@@ -731,6 +740,12 @@ int ensure_iso_work(nemo_ctx* c, int kjpt) {
     if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "iso-neutral flux arrays (%zu bytes)", bytes);
   c->iso_kjpt = kjpt;
   return NEMO_OK;
+}
+
+// The step's own work arrays (two tracers), held before a capture: none can be allocated in one.
+int ensure_step_work(nemo_ctx* c) {
+  if (int s = ensure_fct_work(c, 2, c->nam.nn_fct_v == 4)) return s;
+  return c->nam.ln_traldf_iso || c->nam.ln_traldf_triad ? ensure_iso_work(c, 2) : NEMO_OK;
 }
 
 int check_cdtype(nemo_ctx* c, const char* cdtype, int* is_trc) {
@@ -1999,9 +2014,7 @@ int nemo_gpu_create(const nemo_dom_desc* dm, const nemo_namelist* nam, int nmemb
   cudaMemset(c->gs_ticket, 0, (size_t)c->nmem * sizeof(unsigned));
   if (cudaHostAlloc((void**)&c->gs_host, (size_t)c->nmem * 8, cudaHostAllocMapped) != cudaSuccess)
     return bad(NEMO_ERR_NOMEM);
-  // work arrays of the hot path allocated here, so graph capture never allocates
-  if (ensure_fct_work(c, 2, c->nam.nn_fct_v == 4)) return bad(NEMO_ERR_NOMEM);
-  if ((c->nam.ln_traldf_iso || c->nam.ln_traldf_triad) && ensure_iso_work(c, 2)) return bad(NEMO_ERR_NOMEM);
+  if (ensure_step_work(c)) return bad(NEMO_ERR_NOMEM);
   if (cudaDeviceSynchronize() != cudaSuccess) return bad(NEMO_ERR_CUDA);
   *out = c;
   return NEMO_OK;
@@ -2092,8 +2105,7 @@ int nemo_gpu_synchronize(nemo_ctx* c) {
 int nemo_gpu_bind(nemo_ctx* c, int id, void* p) {
   if (!c || id < 0 || id >= NEMO_F_COUNT) return fail(c, NEMO_ERR_ARG, "bad field id %d", id);
   c->f[id] = p;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
@@ -2677,8 +2689,7 @@ int nemo_gpu_dia_hsb_init(nemo_ctx* c) {
                       : launch_hsb_init<float>(dom<float>(c), hsb_args<float>(c), 4 * c->nsm, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "dia_hsb_init launch");
   c->hsb_on = true;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);  // the model step now runs dia_hsb
-  c->graphs.clear();
+  drop_graphs(c);  // the model step now runs dia_hsb
   return NEMO_OK;
 }
 
@@ -3057,6 +3068,7 @@ static int stp_common(nemo_ctx* c, int kt, bool model) {
       CK(cudaGraphLaunch(it->second, c->stream), "graph launch");
       return NEMO_OK;
     }
+    if (int s = ensure_step_work(c)) return s;
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       int s = c->prec == NEMO_PREC_FP64 ? run_hotpath<double>(c, kt, false, model)
@@ -3152,8 +3164,7 @@ int nemo_gpu_autotune(nemo_ctx* c, int kt, int nrep) {
   cudaStreamSynchronize(c->stream);
   cleanup();
   nemo_gpu_set_timing(c, was_timing);
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);  // recaptured with the chosen shapes
-  c->graphs.clear();
+  drop_graphs(c);  // recaptured with the chosen shapes
   return st;
 }
 
@@ -3165,8 +3176,7 @@ int nemo_gpu_set_launch_shape(nemo_ctx* c, const int* ty, int n) {
     if (!(ty[i] == 0 || ty[i] == 4 || (tunable[i] && (ty[i] == 1 || ty[i] == 2))))
       return fail(c, NEMO_ERR_ARG, "set_launch_shape: kernel %d cannot take block height %d", i, ty[i]);
   for (int i = 0; i < n; ++i) c->shape.ty[i] = (unsigned char)(ty[i] == 4 ? 0 : ty[i]);
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);  // recaptured with the new shapes
-  c->graphs.clear();
+  drop_graphs(c);  // recaptured with the new shapes
   return NEMO_OK;
 }
 
@@ -3209,24 +3219,21 @@ int nemo_gpu_get_timing(nemo_ctx* c, double* ms, int* ncalls) {
 int nemo_gpu_set_fusion(nemo_ctx* c, int on) {
   if (!c) return NEMO_ERR_ARG;
   c->no_fusion = !on;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
 int nemo_gpu_set_fct_fused(nemo_ctx* c, int on) {
   if (!c) return NEMO_ERR_ARG;
   c->fct_fused = on != 0;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
 int nemo_gpu_set_tma(nemo_ctx* c, int on) {
   if (!c) return NEMO_ERR_ARG;
   c->no_tma = !on;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
@@ -3234,8 +3241,7 @@ int nemo_gpu_set_spg_specialised(nemo_ctx* c, int on) {
   if (!c) return NEMO_ERR_ARG;
   c->no_p2_hot = !on;
   select_p2(c);
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return c->p2_blocks < 1 ? fail(c, NEMO_ERR_CUDA, "set_spg_specialised: no launch shape") : NEMO_OK;
 }
 
@@ -3243,16 +3249,14 @@ int nemo_gpu_set_spg_cluster(nemo_ctx* c, int mode) {
   if (!c || mode < 0 || mode > 2) return fail(c, NEMO_ERR_ARG, "set_spg_cluster: bad argument");
   c->cluster = mode;
   select_p2(c);
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
 int nemo_gpu_set_tma_poll_limit(nemo_ctx* c, int max_polls) {
   if (!c || max_polls < 0) return fail(c, NEMO_ERR_ARG, "set_tma_poll_limit: bad argument");
   c->tma_polls = max_polls;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 
@@ -3260,8 +3264,7 @@ int nemo_gpu_set_barrier_limit(nemo_ctx* c, long long max_spins, int extra_arriv
   if (!c || max_spins < 1 || extra_arrivals < 0) return fail(c, NEMO_ERR_ARG, "set_barrier_limit: bad argument");
   c->bar_spins = max_spins;
   c->bar_extra = extra_arrivals;
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.second);
-  c->graphs.clear();
+  drop_graphs(c);
   return NEMO_OK;
 }
 

@@ -18,6 +18,7 @@ std::map<const void*, std::string> name;                    // host stub -> kern
 std::map<std::pair<int, const void*>, size_t> opted;        // (device, stub) -> opt-in
 std::string launches;
 std::map<void*, size_t> held;  // device memory
+bool capturing = false;
 struct Config {
   dim3 grid, block;
   size_t smem;
@@ -40,6 +41,7 @@ CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuui
   return CUDA_SUCCESS;
 }
 void* handle() { return calloc(1, 8); }
+cudaError_t last = cudaSuccess;
 }  // namespace
 
 extern "C" {
@@ -70,7 +72,6 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) 
   return cudaSuccess;
 }
 cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* stub) { *k = (cudaKernel_t)stub; return cudaSuccess; }
-static cudaError_t last = cudaSuccess;
 cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void**, size_t smem, cudaStream_t) {
   const cudaError_t e = launch((const void*)k, g, b, smem);
   if (e != cudaSuccess) last = e;
@@ -118,6 +119,7 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
 }
 
 cudaError_t cudaMalloc(void** p, size_t n) {
+  if (capturing) return last = cudaErrorStreamCaptureUnsupported;
   *p = aligned_alloc(256, (n + 255) / 256 * 256);
   held[*p] = n;
   return cudaSuccess;
@@ -142,12 +144,26 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStr
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*) { return cudaErrorNotSupported; }
-cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
-cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
+// a captured launch is logged like any other, its graph's launch as "graph"
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+  capturing = true;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+  capturing = false;
+  *g = (cudaGraph_t)handle();
+  return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) { free(g); return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t g) { free(g); return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) {
+  *x = (cudaGraphExec_t)handle();
+  return cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
+  launches += "graph 0 0 0 0 0 0\n";
+  return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)handle(); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)handle(); return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { free(e); return cudaSuccess; }

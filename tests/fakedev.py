@@ -42,6 +42,10 @@ if "FAKE_CUDART" in os.environ:
     fake.fake_held.restype = C.c_size_t
     lib = _ffi.load(_b.library_path())
 
+    HOTPATH = ("AVT", "AH_WSLP2", "AKZ", "TSB", "TSN", "TSA", "UN", "VN", "WN", "USLP", "VSLP", "WSLPI", "WSLPJ", "UA", "VA",
+               "UB", "VB", "SSHN", "SSHB", "UN_B", "VN_B", "UB_B", "VB_B", "UTAU", "VTAU", "EMP", "RCDU_BOT", "SSHA",
+               "UA_B", "VA_B", "UN_ADV", "VN_ADV", "UB2_B", "VB2_B", "UN_BF", "VN_BF")  # fields of stp_hotpath
+
     def launches():
         """[(kernel, grid x y z, block x y, shared memory)] since the last call"""
         out = [line.split() for line in fake.fake_launches().decode().splitlines()]
