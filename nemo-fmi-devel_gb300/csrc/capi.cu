@@ -742,10 +742,23 @@ int ensure_iso_work(nemo_ctx* c, int kjpt) {
   return NEMO_OK;
 }
 
+int ensure_blp_work(nemo_ctx* c, int kjpt) {
+  if (kjpt <= c->blp_kjpt) return NEMO_OK;
+  const size_t bytes = (size_t)kjpt * (c->n3 + 2 * c->n2) * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
+  drop_graphs(c);
+  cudaFree(c->blp_w);
+  c->blp_w = nullptr;
+  if (cudaMalloc(&c->blp_w, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "tra_ldf_blp work array");
+  c->blp_kjpt = kjpt;
+  return NEMO_OK;
+}
+
 // The step's own work arrays (two tracers), held before a capture: none can be allocated in one.
 int ensure_step_work(nemo_ctx* c) {
   if (int s = ensure_fct_work(c, 2, c->nam.nn_fct_v == 4)) return s;
-  return c->nam.ln_traldf_iso || c->nam.ln_traldf_triad ? ensure_iso_work(c, 2) : NEMO_OK;
+  if (c->nam.ln_traldf_iso || c->nam.ln_traldf_triad)
+    if (int s = ensure_iso_work(c, 2)) return s;
+  return c->nam.ln_traldf_blp ? ensure_blp_work(c, 2) : NEMO_OK;
 }
 
 int check_cdtype(nemo_ctx* c, const char* cdtype, int* is_trc) {
@@ -892,12 +905,7 @@ template <class T>
 int run_ldf_blp(nemo_ctx* c, int kt, int kit000, const void* pahu, const void* pahv, const void* pgu,
                 const void* pgv, const void* ptb, void* pta, int kjpt, int kldf) {
   const size_t n3b = (size_t)kjpt * c->n3 * c->nmem * sizeof(T), n2b = (size_t)kjpt * c->n2 * c->nmem * sizeof(T);
-  if (kjpt > c->blp_kjpt) {
-    cudaFree(c->blp_w);
-    c->blp_w = nullptr;
-    if (cudaMalloc(&c->blp_w, n3b + 2 * n2b) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "tra_ldf_blp work array");
-    c->blp_kjpt = kjpt;
-  }
+  if (int s = ensure_blp_work(c, kjpt)) return s;
   T* zlap = (T*)c->blp_w;
   T* zglu = (T*)((char*)c->blp_w + n3b);
   T* zglv = (T*)((char*)c->blp_w + n3b + n2b);

@@ -223,8 +223,9 @@ def test_graph_after_work_arrays_grow():
     at; the next step is captured again, with what its own vertical scheme needs."""
     out = fakedev.run(r"""
 seen = []
-for routine, scheme in (("tra_adv_fct", 2), ("tra_adv_fct", 4), ("tra_ldf_iso", 2)):
-    c = Ctx(gyre.domain(1, jpk=6), gyre.namelist(nn_fct_v=scheme), "fp64")
+for routine, over in (("tra_adv_fct", {}), ("tra_adv_fct", dict(nn_fct_v=4)), ("tra_ldf_iso", {}),
+                      ("tra_ldf_blp", dict(ln_traldf_lap=0, ln_traldf_blp=1, ln_traldf_iso=0, rn_aht_0=1.e11))):
+    c = Ctx(gyre.domain(1, jpk=6), gyre.namelist(**over), "fp64")
     c.bind(*HOTPATH)
     t = [c.array(3 * c.n3) for _ in range(6)]
     for kt in (10, 11):
@@ -234,14 +235,16 @@ for routine, scheme in (("tra_adv_fct", 2), ("tra_adv_fct", 4), ("tra_ldf_iso", 
     for n in (2, 3):
         if routine == "tra_adv_fct":
             c(routine, 12, 1, b"TRC", 14400.0, *t, n, 2, 2)
-        else:
+        elif routine == "tra_ldf_iso":
             c(routine, 12, 1, b"TRC", None, None, None, None, None, None, t[0], t[0], t[1], n, 1)
+        else:
+            c(routine, 12, 1, b"TRC", None, None, None, None, None, None, t[0], t[1], n, 20)
         launches()
         c("stp_hotpath", 13)
         seen.append([k[0] for k in launches()])
     c.close()
 print(json.dumps(seen))
 """)
-    for first, second, same, more in (out[:4], out[4:8], out[8:]):
+    for first, second, same, more in (out[:4], out[4:8], out[8:12], out[12:]):
         assert len(first) > 5 and first[-1] == "graph" and second == ["graph"] and same == ["graph"]
         assert more == first
