@@ -753,6 +753,22 @@ int ensure_blp_work(nemo_ctx* c, int kjpt) {
   return NEMO_OK;
 }
 
+// work arrays that keep their size, made at their first use
+int held(nemo_ctx* c, void** p, size_t bytes, const char* what) {
+  if (*p || cudaMalloc(p, bytes) == cudaSuccess) return NEMO_OK;
+  return fail(c, NEMO_ERR_NOMEM, "%s (%zu bytes)", what, bytes);
+}
+int ensure_rab(nemo_ctx* c, void** p) {
+  return held(c, p, 2 * (size_t)c->n3 * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4), "expansion ratios");
+}
+int ensure_zphy_work(nemo_ctx* c) {  // FP64: the columns' systems too, where shared memory does not keep them
+  return held(c, &c->zphy_w, (size_t)c->n3 * c->nmem * (c->prec == NEMO_PREC_FP64 ? 5 * 8 : 4), "zdf_phy work arrays");
+}
+int ensure_slp_work(nemo_ctx* c) {
+  return held(c, &c->slp_w, (4 * (size_t)c->n3 + 6 * (size_t)c->n2) * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4),
+              "ldf_slp work arrays");
+}
+
 // The step's own work arrays (two tracers), held before a capture: none can be allocated in one.
 int ensure_step_work(nemo_ctx* c) {
   if (int s = ensure_fct_work(c, 2, c->nam.nn_fct_v == 4)) return s;
@@ -1060,8 +1076,7 @@ template <class T>
 int run_ldf_slp(nemo_ctx* c, const void* prd, const void* pn2) {
   const nemo_namelist& nm = c->nam;
   const size_t n3 = (size_t)c->n3 * c->nmem, n2 = (size_t)c->n2 * c->nmem;
-  if (!c->slp_w && cudaMalloc(&c->slp_w, (4 * n3 + 6 * n2) * sizeof(T)) != cudaSuccess)
-    return fail(c, NEMO_ERR_NOMEM, "ldf_slp work arrays");
+  if (int s = ensure_slp_work(c)) return s;
   T* w = (T*)c->slp_w;
   SlpArgs<T> a{};
   a.prd = (const T*)prd; a.pn2 = (const T*)pn2;
@@ -1439,8 +1454,7 @@ int run_slopes(nemo_ctx* c, bool rn2b_done) {
   void* const* F = c->f;
   int s = NEMO_OK;
   if (!rn2b_done) {
-    if (!c->rab_w && cudaMalloc(&c->rab_w, 2 * (size_t)c->n3 * c->nmem * sizeof(T)) != cudaSuccess)
-      return fail(c, NEMO_ERR_NOMEM, "rab_b work array");
+    if ((s = ensure_rab(c, &c->rab_w))) return s;
     s = run_eos<T>(c, 2, F[NEMO_F_TSB], nullptr, nullptr, nullptr, c->rab_w, nullptr, nullptr);
     if (!s) s = run_eos<T>(c, 3, F[NEMO_F_TSB], nullptr, nullptr, nullptr, nullptr, c->rab_w, F[NEMO_F_RN2B]);
   }
@@ -1476,8 +1490,7 @@ int run_zdf_phy(nemo_ctx* c) {
   const nemo_namelist& nm = c->nam;
   const size_t n = (size_t)c->n3 * c->nmem;
   constexpr bool D = sizeof(T) == 8;  // FP64: the columns' systems too, where shared memory does not keep them
-  if (!c->zphy_w && cudaMalloc(&c->zphy_w, (D ? 5 : 1) * n * sizeof(T)) != cudaSuccess)
-    return fail(c, NEMO_ERR_NOMEM, "zdf_phy work arrays");
+  if (int s = ensure_zphy_work(c)) return s;
   void* const* F = c->f;
   ZphyArgs<T> a{};
   a.ub = (const T*)F[NEMO_F_UB]; a.vb = (const T*)F[NEMO_F_VB];
@@ -1557,10 +1570,9 @@ bool zphy_on(const nemo_ctx* c) {
 template <class T>
 int run_vphys(nemo_ctx* c) {
   void* const* F = c->f;
-  const size_t b2 = 2 * (size_t)c->n3 * c->nmem * sizeof(T);
-  if (!c->rab_w && cudaMalloc(&c->rab_w, b2) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "rab_b work array");
-  if (!c->rab_n && cudaMalloc(&c->rab_n, b2) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "rab_n work array");
-  int s = run_eos<T>(c, 2, F[NEMO_F_TSB], nullptr, nullptr, nullptr, c->rab_w, nullptr, nullptr);
+  int s = ensure_rab(c, &c->rab_w);
+  if (!s) s = ensure_rab(c, &c->rab_n);
+  if (!s) s = run_eos<T>(c, 2, F[NEMO_F_TSB], nullptr, nullptr, nullptr, c->rab_w, nullptr, nullptr);
   if (!s) s = run_eos<T>(c, 2, F[NEMO_F_TSN], nullptr, nullptr, nullptr, c->rab_n, nullptr, nullptr);
   if (!s) s = run_eos<T>(c, 3, F[NEMO_F_TSB], nullptr, nullptr, nullptr, nullptr, c->rab_w, F[NEMO_F_RN2B]);
   if (!s) s = run_eos<T>(c, 3, F[NEMO_F_TSN], nullptr, nullptr, nullptr, nullptr, c->rab_n, F[NEMO_F_RN2]);
@@ -3053,6 +3065,16 @@ int nemo_gpu_glob_sum(nemo_ctx* c, const char* cdname, const void* ptab, int nk,
   return NEMO_OK;
 }
 
+// ensure_step_work for what the model step adds
+static int ensure_model_work(nemo_ctx* c) {
+  const bool vphys = zphy_on(c), slopes = slopes_on(c);
+  int s = vphys || slopes ? ensure_rab(c, &c->rab_w) : NEMO_OK;
+  if (!s && vphys) s = ensure_rab(c, &c->rab_n);
+  if (!s && vphys) s = ensure_zphy_work(c);
+  if (!s && slopes) s = ensure_slp_work(c);
+  return s;
+}
+
 static int stp_common(nemo_ctx* c, int kt, bool model) {
   if (!c) return NEMO_ERR_ARG;
   NvtxRange nvtx_range(model ? "stp" : "stp_hotpath");
@@ -3077,6 +3099,8 @@ static int stp_common(nemo_ctx* c, int kt, bool model) {
       return NEMO_OK;
     }
     if (int s = ensure_step_work(c)) return s;
+    if (model)
+      if (int s = ensure_model_work(c)) return s;
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       int s = c->prec == NEMO_PREC_FP64 ? run_hotpath<double>(c, kt, false, model)

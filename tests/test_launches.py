@@ -1,5 +1,6 @@
 """What the library launches, checked without a GPU over a stand-in for the CUDA runtime."""
 import fakedev
+import pytest
 
 
 def test_shared_memory_on_a_second_device():
@@ -248,3 +249,22 @@ print(json.dumps(seen))
     for first, second, same, more in (out[:4], out[4:8], out[8:12], out[12:]):
         assert len(first) > 5 and first[-1] == "graph" and second == ["graph"] and same == ["graph"]
         assert more == first
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("fields", ["FULL_3D + gyre.FULL_2D", "FULL_3D[1:] + gyre.FULL_2D"])
+def test_model_step_captured_first(prec, fields):
+    """The first step asked of a context is a captured one: the closure's and the slopes' work
+    arrays are made before the capture."""
+    out = fakedev.run(f"""
+dom, base = gyre.domain(1), gyre.namelist()
+c = Ctx(dom, gyre.full_physics(dom, base, gyre.state(dom, base, seed=5))[0], "{prec}")
+c.bind(*HOTPATH, "NMLN", *(n.upper() for n in gyre.{fields}))
+c("stp_model", 10)
+first = [k[0] for k in launches()]
+c("stp_model", 11)
+print(json.dumps([first, [k[0] for k in launches()]]))
+""")
+    # the forcing's scalars are put ahead of the graph
+    assert out[0][-1] == "graph" and len(out[1]) == 2 and "usr_put" in out[1][0] and out[1][1] == "graph"
+    assert ("FULL_3D[" in fields) == (not any("zdf_sh2" in k for k in out[0]))
