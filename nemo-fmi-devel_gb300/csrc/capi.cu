@@ -92,7 +92,7 @@ struct nemo_ctx {
   double* fadj_w = nullptr;    // FCT adjoint with kn_fct_v = 4: 2 x n3 per member
   double* usr_s = nullptr;     // usrdef_sbc: the step's scalars (7), written before each step
   double usr_zsurf = 0.0;      // usrdef_sbc: GLOB_SUM(tmask(:,:,1))
-  void* blp_w = nullptr;       // tra_ldf_blp: the first laplacian (jpi,jpj,jpk,kjpt) per member
+  void* blp_w[1] = {};         // tra_ldf_blp: the first laplacian (jpi,jpj,jpk,kjpt) per member
   int blp_kjpt = 0;
   int iso_kjpt = 0;
   int fct_kjpt = 0;
@@ -190,6 +190,7 @@ thread_local const LaunchShape* t_shape = nullptr;
 namespace {
 
 int fail(nemo_ctx* c, int code, const char* fmt, ...) {
+  if (code == NEMO_ERR_NOMEM) cudaGetLastError();  // or the next launch's check would report it
   if (c) {
     char buf[512];
     va_list ap;
@@ -707,50 +708,48 @@ void drop_graphs(nemo_ctx* c) {
   c->graphs.clear();
 }
 
+// Work arrays of `kjpt` tracers in place of those of `have`, `bytes` each. Without the memory
+// none is held, and the next call makes them again.
+template <size_t N>
+int renew(nemo_ctx* c, void* (&w)[N], int& have, int kjpt, size_t bytes, const char* what) {
+  drop_graphs(c);
+  have = 0;
+  bool ok = true;
+  for (auto& p : w) { cudaFree(p); p = nullptr; }
+  for (auto& p : w) ok = ok && cudaMalloc(&p, bytes) == cudaSuccess;
+  if (!ok) {
+    for (auto& p : w) { cudaFree(p); p = nullptr; }
+    return fail(c, NEMO_ERR_NOMEM, "%s (%zu bytes)", what, bytes);
+  }
+  have = kjpt;
+  return NEMO_OK;
+}
+
 int ensure_fct_work(nemo_ctx* c, int kjpt, int need_ztw) {
-  const size_t es = c->prec == NEMO_PREC_FP64 ? 8 : 4;
-  const size_t bytes = (size_t)kjpt * c->n3 * c->nmem * es;
+  const size_t es = c->prec == NEMO_PREC_FP64 ? 8 : 4, n = c->n3 * c->nmem * es;
   if (kjpt > c->fct_kjpt) {
-    drop_graphs(c);
-    for (auto& p : c->fct_w) { cudaFree(p); p = nullptr; }
     cudaFree(c->fct_ztw); c->fct_ztw = nullptr;
-    for (auto& p : c->fct_w) {
-      if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "FCT work arrays (%zu bytes)", bytes);
-      cudaMemset(p, 0, bytes);
-    }
-    c->fct_kjpt = kjpt;
+    if (int s = renew(c, c->fct_w, c->fct_kjpt, kjpt, kjpt * n, "FCT work arrays")) return s;
+    for (void* p : c->fct_w) cudaMemset(p, 0, kjpt * n);
   }
   if (need_ztw && !c->fct_ztw) {
-    if (cudaMalloc(&c->fct_ztw, (size_t)c->fct_kjpt * c->n3 * c->nmem * es) != cudaSuccess)
+    if (cudaMalloc(&c->fct_ztw, c->fct_kjpt * n) != cudaSuccess)
       return fail(c, NEMO_ERR_NOMEM, "FCT compact-interpolation array");
-    cudaMemset(c->fct_ztw, 0, (size_t)c->fct_kjpt * c->n3 * c->nmem * es);
+    cudaMemset(c->fct_ztw, 0, c->fct_kjpt * n);
   }
   return NEMO_OK;
 }
 
 int ensure_iso_work(nemo_ctx* c, int kjpt) {
   if (kjpt <= c->iso_kjpt) return NEMO_OK;
-  const size_t bytes = (size_t)kjpt * c->n3 * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
-  drop_graphs(c);
-  for (auto& p : c->iso_w) {
-    cudaFree(p);
-    p = nullptr;
-  }
-  for (auto& p : c->iso_w)
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "iso-neutral flux arrays (%zu bytes)", bytes);
-  c->iso_kjpt = kjpt;
-  return NEMO_OK;
+  const size_t n = c->n3 * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
+  return renew(c, c->iso_w, c->iso_kjpt, kjpt, kjpt * n, "iso-neutral flux arrays");
 }
 
 int ensure_blp_work(nemo_ctx* c, int kjpt) {
   if (kjpt <= c->blp_kjpt) return NEMO_OK;
-  const size_t bytes = (size_t)kjpt * (c->n3 + 2 * c->n2) * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
-  drop_graphs(c);
-  cudaFree(c->blp_w);
-  c->blp_w = nullptr;
-  if (cudaMalloc(&c->blp_w, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "tra_ldf_blp work array");
-  c->blp_kjpt = kjpt;
-  return NEMO_OK;
+  const size_t n = (c->n3 + 2 * c->n2) * c->nmem * (c->prec == NEMO_PREC_FP64 ? 8 : 4);
+  return renew(c, c->blp_w, c->blp_kjpt, kjpt, kjpt * n, "tra_ldf_blp work array");
 }
 
 // work arrays that keep their size, made at their first use
@@ -922,9 +921,9 @@ int run_ldf_blp(nemo_ctx* c, int kt, int kit000, const void* pahu, const void* p
                 const void* pgv, const void* ptb, void* pta, int kjpt, int kldf) {
   const size_t n3b = (size_t)kjpt * c->n3 * c->nmem * sizeof(T), n2b = (size_t)kjpt * c->n2 * c->nmem * sizeof(T);
   if (int s = ensure_blp_work(c, kjpt)) return s;
-  T* zlap = (T*)c->blp_w;
-  T* zglu = (T*)((char*)c->blp_w + n3b);
-  T* zglv = (T*)((char*)c->blp_w + n3b + n2b);
+  T* zlap = (T*)c->blp_w[0];
+  T* zglu = (T*)((char*)c->blp_w[0] + n3b);
+  T* zglv = (T*)((char*)c->blp_w[0] + n3b + n2b);
   CK(cudaMemsetAsync(zlap, 0, n3b, c->stream), "zlap = 0");
   int s = kldf == 20 ? run_ldf_lap<T>(c, pahu, pahv, pgu, pgv, ptb, zlap, kjpt, 1)
           : kldf == 21 ? run_ldf_iso<T>(c, kt, kit000, pahu, pahv, pgu, pgv, ptb, ptb, zlap, kjpt, 1)
@@ -2052,7 +2051,7 @@ int nemo_gpu_destroy(nemo_ctx* c) {
   for (auto p : c->adj_w) cudaFree(p);
   cudaFree(c->slp_w);
   cudaFree(c->rab_w); cudaFree(c->rab_n); cudaFree(c->zphy_w); cudaFree(c->usr_s); cudaFree(c->fadj_w);
-  cudaFree(c->blp_w);
+  cudaFree(c->blp_w[0]);
   for (auto p : c->spg_w) cudaFree(p);
   for (auto p : c->spg_cor) cudaFree(p);
   for (auto p : c->ring) cudaFree(p);
@@ -2680,8 +2679,10 @@ int nemo_gpu_dia_hsb_init(nemo_ctx* c) {
     if (cudaMalloc(&c->hsb_mem, words * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&c->hsb_part, (size_t)c->hsb_nblk * nm * HSB_NS * 2 * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&c->hsb_state, nm * 8 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&c->hsb_out, nm * NEMO_HSB_N * sizeof(double)) != cudaSuccess)
+        cudaMalloc(&c->hsb_out, nm * NEMO_HSB_N * sizeof(double)) != cudaSuccess) {
+      for (double** p : {&c->hsb_mem, &c->hsb_part, &c->hsb_state, &c->hsb_out}) { cudaFree(*p); *p = nullptr; }
       return fail(c, NEMO_ERR_NOMEM, "dia_hsb work arrays");
+    }
     CK(cudaMemset(c->hsb_mem, 0, words * sizeof(double)), "dia_hsb = 0");
   }
   // surf = e1e2t * tmask_i (diahsb.F90:411), tmask_h (dommsk.F90:213-217, closed
@@ -2781,15 +2782,7 @@ static int adj_check(nemo_ctx* c, const char* cdtype, int* is_trc, const char* w
 
 static int ensure_adj_work(nemo_ctx* c, int kjpt) {
   if (kjpt <= c->adj_kjpt) return NEMO_OK;
-  const size_t bytes = (size_t)kjpt * c->n3 * c->nmem * sizeof(double);
-  for (auto& p : c->adj_w) {
-    cudaFree(p);
-    p = nullptr;
-  }
-  for (auto& p : c->adj_w)
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(c, NEMO_ERR_NOMEM, "adjoint work arrays (%zu bytes)", bytes);
-  c->adj_kjpt = kjpt;
-  return NEMO_OK;
+  return renew(c, c->adj_w, c->adj_kjpt, kjpt, kjpt * (c->n3 * c->nmem * sizeof(double)), "adjoint work arrays");
 }
 
 int nemo_gpu_tra_adv_fct_adj(nemo_ctx* c, int kt, int kit000, const char* cdtype, double p2dt, const void* pun,

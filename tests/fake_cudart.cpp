@@ -19,6 +19,7 @@ std::map<std::pair<int, const void*>, size_t> opted;        // (device, stub) ->
 std::string launches;
 std::map<void*, size_t> held;  // device memory
 bool capturing = false;
+long mallocs_left = -1;        // the device's memory is full after so many more (-1: never)
 struct Config {
   dim3 grid, block;
   size_t smem;
@@ -46,6 +47,7 @@ cudaError_t last = cudaSuccess;
 
 extern "C" {
 const char* fake_launches() { return launches.c_str(); }
+void fake_mallocs_left(long n) { mallocs_left = n; }
 void fake_clear() { launches.clear(); }
 size_t fake_held() {
   size_t n = 0;
@@ -120,6 +122,8 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
 
 cudaError_t cudaMalloc(void** p, size_t n) {
   if (capturing) return last = cudaErrorStreamCaptureUnsupported;
+  if (mallocs_left == 0) return last = cudaErrorMemoryAllocation;
+  if (mallocs_left > 0) --mallocs_left;
   *p = aligned_alloc(256, (n + 255) / 256 * 256);
   held[*p] = n;
   return cudaSuccess;

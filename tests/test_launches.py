@@ -268,3 +268,38 @@ print(json.dumps([first, [k[0] for k in launches()]]))
     # the forcing's scalars are put ahead of the graph
     assert out[0][-1] == "graph" and len(out[1]) == 2 and "usr_put" in out[1][0] and out[1][1] == "graph"
     assert ("FULL_3D[" in fields) == (not any("zdf_sh2" in k for k in out[0]))
+
+
+@pytest.mark.parametrize("routine,arrays", [("tra_adv_fct", 6), ("tra_ldf_iso", 3), ("tra_ldf_blp", 1),
+                                            ("tra_ldf_iso_adj", 4), ("dia_hsb_init", 4)])
+def test_device_memory_runs_out(routine, arrays):
+    """A call that has not the memory for its work arrays is refused and keeps none of them; a
+    smaller call after it has all of its own, and so has the same call once there is memory."""
+    out = fakedev.run(rf"""
+c = Ctx(gyre.domain(1, jpk=6), gyre.namelist(), "fp64")
+c.bind(*HOTPATH)
+t = [c.array(3 * c.n3) for _ in range(6)]
+call = dict(
+    tra_adv_fct=lambda n: c("tra_adv_fct", 12, 1, b"TRC", 14400.0, *t, n, 2, 2),
+    tra_ldf_iso=lambda n: c("tra_ldf_iso", 12, 1, b"TRC", *[None] * 6, t[0], t[0], t[1], n, 1),
+    tra_ldf_blp=lambda n: c("tra_ldf_blp", 12, 1, b"TRC", *[None] * 6, t[0], t[1], n, 20),
+    tra_ldf_iso_adj=lambda n: c("tra_ldf_iso_adj", 12, 1, b"TRC", *[None] * 6, t[0], t[0], t[1], n, 1),
+    dia_hsb_init=lambda n: n > 2 and c("dia_hsb_init"))["{routine}"]
+call(2)
+held, refused = [fake.fake_held()], []
+for room in range({arrays}):
+    fake.fake_mallocs_left(C.c_long(room))
+    try:
+        call(3)
+    except AssertionError as e:
+        refused.append(str(e))
+    fake.fake_mallocs_left(C.c_long(-1))
+    call(2)
+    held.append(fake.fake_held())
+call(3)
+held.append(fake.fake_held())
+print(json.dumps([refused, held]))
+""")
+    refused, held = out
+    assert len(refused) == arrays and all("array" in e for e in refused), refused
+    assert held[1:-1] == held[:1] * arrays and held[-1] > held[0]
